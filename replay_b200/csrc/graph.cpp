@@ -564,6 +564,7 @@ int32_t plan_window_ranges(const Graph &g, int64_t ws, int64_t we, float scale, 
     out.qe = we;
   }
   out.range_off = 0;
+  out.hit_off = 0;
   out.n_ranges = 0;
   out.n_candidates = 0;
   for (int c = 0; c < kClasses; ++c) {

@@ -274,9 +274,11 @@ struct rp_sim {
   std::vector<int32_t> step_win;  // window index per step
   std::vector<WinDesc> wins;
   std::vector<CandRange> ranges;
+  std::vector<WindowGroup> groups;
+  std::vector<int32_t> win_group;  // group of each window
   WindowWorkspace wsp;
-  // per-step mode: window w + 1 is built on a side stream into the other
-  // workspace while window w's steps run
+  // per-step mode: group g + 1 is built on a side stream into the other
+  // workspace while group g's steps run
   WindowWorkspace wsp2;
   bool overlap = false;
   cudaStream_t side = nullptr;
@@ -377,15 +379,17 @@ struct rp_sim {
     return RP_OK;
   }
 
-  WindowWorkspace &ws_of(int w) { return overlap && (w & 1) ? wsp2 : wsp; }
-  const WindowWorkspace &ws_of(int w) const { return overlap && (w & 1) ? wsp2 : wsp; }
+  WindowWorkspace &ws_of(int grp) { return overlap && (grp & 1) ? wsp2 : wsp; }
+  const WindowWorkspace &ws_of(int grp) const { return overlap && (grp & 1) ? wsp2 : wsp; }
   const int32_t *rp_of(int t) const {
-    if (prebuilt) return arena_rp.as<int32_t>() + arena_rp_off[step_win[t]];
-    return ws_of(step_win[t]).row_ptr.as<int32_t>();
+    const int w = step_win[t], grp = win_group[w];
+    if (prebuilt) return arena_rp.as<int32_t>() + arena_rp_off[w];
+    return ws_of(grp).row_ptr.as<int32_t>() + (int64_t)(w - groups[grp].first) * (N + 1);
   }
   const int2 *ent_of(int t) const {
-    if (prebuilt) return arena_ent.as<int2>() + arena_ent_off[step_win[t]];
-    return ws_of(step_win[t]).entries.as<int2>();
+    const int w = step_win[t];
+    if (prebuilt) return arena_ent.as<int2>() + arena_ent_off[w];
+    return ws_of(win_group[w]).entries.as<int2>() + 2 * wins[w].hit_off;
   }
 
   // Optional event marks around kernel groups (rp_sim_profile).
@@ -463,35 +467,28 @@ struct rp_sim {
     mark(kMarkOther);
     RP_TRY(emit_states(0, p.start_time));
     const int per_row = n_nets * M;
-    const int n_win = (int)wins.size();
-    auto build = [&](int w, cudaStream_t bs) {
-      enqueue_window_build(*g, ws_of(w), w, wins[w], cap, weight_kind,
-                           weight_kind == kWeightF32, bs);
-      // k_hits, k_scan_tiles, k_scan_apply, k_fill (+ k_trunc, + the two row sorts)
-      k += 4 + (wins[w].may_truncate ? 1 : 0) + (weight_kind == kWeightF32 ? 2 : 0);
+    auto build = [&](int grp, cudaStream_t bs) {
+      k += enqueue_window_build(*g, ws_of(grp), groups[grp], cap, weight_kind,
+                                weight_kind == kWeightF32, bs);
     };
+    const int n_groups = T > 0 ? win_group[step_win[T - 1]] + 1 : 0;  // groups these steps use
     bool side_used = false;
-    if (!prebuilt && overlap && T > 0) {
-      build(step_win[0], st);
+    if (!prebuilt && T > 0) {
+      build(0, st);
       mark(kMarkBuild);
     }
     for (int32_t t = 0; t < T; ++t) {
-      const int w = step_win[t];
-      if (!prebuilt && (t == 0 || w != step_win[t - 1])) {
-        if (!overlap) {
-          build(w, st);
-          mark(kMarkBuild);
-        } else {
-          if (t > 0) RP_TRY_CUDA(cudaStreamWaitEvent(st, ev_built[w & 1], 0));
-          if (w + 1 < n_win) {
-            // window w-1's steps, the last users of the other workspace, are
-            // all enqueued before this point
-            RP_TRY_CUDA(cudaEventRecord(ev_free, st));
-            RP_TRY_CUDA(cudaStreamWaitEvent(side, ev_free, 0));
-            build(w + 1, side);
-            RP_TRY_CUDA(cudaEventRecord(ev_built[(w + 1) & 1], side));
-            side_used = true;
-          }
+      const int grp = win_group[step_win[t]];
+      if (!prebuilt && (t == 0 || grp != win_group[step_win[t - 1]])) {
+        if (t > 0) RP_TRY_CUDA(cudaStreamWaitEvent(st, ev_built[grp & 1], 0));
+        if (grp + 1 < n_groups) {
+          // group grp-1's steps, the last users of the other workspace, are
+          // all enqueued before this point
+          RP_TRY_CUDA(cudaEventRecord(ev_free, st));
+          RP_TRY_CUDA(cudaStreamWaitEvent(side, ev_free, 0));
+          build(grp + 1, side);
+          RP_TRY_CUDA(cudaEventRecord(ev_built[(grp + 1) & 1], side));
+          side_used = true;
         }
       }
       if (path == RP_PATH_PLAIN) {
@@ -599,7 +596,7 @@ rp_status prebuild(rp_sim &s) {
   RP_TRY(tmp_ent.alloc(sizeof(int2) * (size_t)s.wsp.cap_entries));
   cudaStream_t st = s.stream;
   for (int w = 0; w < nw; ++w) {
-    enqueue_window_build(*s.g, s.wsp, w, s.wins[w], s.cap, s.weight_kind, true, st);
+    enqueue_window_build(*s.g, s.wsp, s.groups[w], s.cap, s.weight_kind, true, st);
     enqueue_window_compact(s.wsp, tmp_rp.as<int32_t>(), tmp_ent.as<int2>(), st);
     int32_t total = 0;
     RP_TRY_CUDA(cudaMemcpyAsync(&total, tmp_rp.as<int32_t>() + N, sizeof(int32_t),
@@ -620,12 +617,24 @@ rp_status prebuild(rp_sim &s) {
   // two spare pairs for the step kernel's 16-byte bulk staging
   RP_TRY(s.arena_ent.alloc(sizeof(int2) * (size_t)(ent + 2)));
   for (int w = 0; w < nw; ++w) {
-    enqueue_window_build(*s.g, s.wsp, w, s.wins[w], s.cap, s.weight_kind, true, st);
+    enqueue_window_build(*s.g, s.wsp, s.groups[w], s.cap, s.weight_kind, true, st);
     enqueue_window_compact(s.wsp, s.arena_rp.as<int32_t>() + s.arena_rp_off[w],
                            s.arena_ent.as<int2>() + s.arena_ent_off[w], st);
   }
   RP_TRY_CUDA(cudaStreamSynchronize(st));
   return RP_OK;
+}
+
+// A workspace for any of the simulation's window groups.
+rp_status sim_window_workspace(rp_sim &s, WindowWorkspace &w) {
+  int32_t slots = 1;
+  int64_t hits = 0;
+  for (const WindowGroup &g : s.groups) {
+    slots = std::max(slots, g.count);
+    hits = std::max(hits, g.candidates);
+  }
+  const bool sorted = s.weight_kind == kWeightF32 || s.p.csr_mode == RP_CSR_PREBUILT;
+  return window_workspace_alloc(w, s.N, slots, hits, sorted, s.wins, s.ranges);
 }
 
 rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
@@ -708,8 +717,19 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
               (long long)max_cand);
     return RP_ERR_RANGE;
   }
-  RP_TRY(window_workspace_alloc(s.wsp, s.N, max_cand, (int64_t)s.wins.size(), s.wins,
-                                s.ranges));
+  const bool prebuilt = p.csr_mode == RP_CSR_PREBUILT;
+  plan_window_groups(s.wins, s.N, prebuilt, s.groups);
+  s.win_group.resize(s.wins.size());
+  for (size_t k = 0; k < s.groups.size(); ++k)
+    for (int32_t w = 0; w < s.groups[k].count; ++w) s.win_group[s.groups[k].first + w] = (int32_t)k;
+  RP_TRY(sim_window_workspace(s, s.wsp));
+  if (!prebuilt && s.groups.size() > 1) {  // groups alternate between two workspaces
+    RP_TRY(sim_window_workspace(s, s.wsp2));
+    RP_TRY_CUDA(cudaStreamCreateWithFlags(&s.side, cudaStreamNonBlocking));
+    for (cudaEvent_t *e : {&s.ev_built[0], &s.ev_built[1], &s.ev_free, &s.ev_join})
+      RP_TRY_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    s.overlap = true;
+  }
 
   // ---- constants ----
   s.c.key0 = (uint32_t)p.seed;
@@ -1140,12 +1160,14 @@ RP_API rp_status rp_window_csr(rp_graph *h, int64_t ws, int64_t we, float scale,
   std::vector<CandRange> ranges;
   plan_window(g, ws, we, scale, cap, ranges, wins[0]);
   WindowWorkspace w;
-  RP_TRY(window_workspace_alloc(w, g.n_nodes, wins[0].n_candidates, 1, wins, ranges));
+  std::vector<WindowGroup> one;
+  plan_window_groups(wins, g.n_nodes, true, one);
+  RP_TRY(window_workspace_alloc(w, g.n_nodes, 1, wins[0].n_candidates, true, wins, ranges));
   DevBuf out_rp, out_ent;
   RP_TRY(out_rp.alloc(sizeof(int32_t) * ((size_t)g.n_nodes + 1)));
   RP_TRY(out_ent.alloc(sizeof(int2) * (size_t)w.cap_entries));
   cudaStream_t st = nullptr;
-  enqueue_window_build(g, w, 0, wins[0], cap, weight_kind, true, st);
+  enqueue_window_build(g, w, one[0], cap, weight_kind, true, st);
   unsigned long long hits_raw = 0;
   RP_TRY_CUDA(cudaMemcpyAsync(&hits_raw, w.counters.as<unsigned long long>() + 3,
                               sizeof(hits_raw), cudaMemcpyDeviceToHost, st));
@@ -1255,16 +1277,6 @@ RP_API rp_status rp_sim_create_batch(const rp_graph *h, const rp_params *p,
   if (s->prebuilt) {
     RP_TRY(prebuild(*s));
     s->prebuild_ms = ms_since(t0);
-  } else if (s->wins.size() > 1) {
-    int64_t max_cand = 0;
-    for (const WinDesc &d : s->wins) max_cand = std::max(max_cand, d.n_candidates);
-    RP_TRY(window_workspace_alloc(s->wsp2, s->N, max_cand, (int64_t)s->wins.size(), s->wins,
-                                  s->ranges));
-    RP_TRY_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
-    for (cudaEvent_t *e : {&s->ev_built[0], &s->ev_built[1], &s->ev_free, &s->ev_join})
-      RP_TRY_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    s->overlap = true;
-    s->setup_ms += ms_since(t0);
   }
   for (int32_t t = 0; t < s->T; ++t) {
     // nnz multiplied per step (for the roofline); per-step mode counts the

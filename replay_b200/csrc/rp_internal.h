@@ -174,6 +174,16 @@ struct WinDesc {
   int32_t range_off;     // first CandRange of this window
   int32_t n_ranges;
   int32_t may_truncate;  // candidates exceed the hit cap
+  int64_t hit_off;       // first hit of this window in its group's list
+};
+
+// Consecutive windows built by one chain of launches.  In the workspace the
+// window in slot k holds its hits from hit_off, its pairs and ranks from
+// 2 * hit_off, and its per-node arrays from k * n (row pointers: k * (n + 1)).
+struct WindowGroup {
+  int32_t first = 0, count = 0;
+  int32_t truncate = 0;  // some window's candidates exceed the hit cap
+  int64_t candidates = 0, max_candidates = 0;
 };
 
 struct Graph {
@@ -233,24 +243,30 @@ struct WindowWorkspace {
   int32_t n_nodes = 0;
   int64_t cap_hits = 0, cap_entries = 0;
   int32_t n_tiles = 0;
+  // a group of windows, slot after slot (WindowGroup); G slots
   DevBuf hits;      // Hit[cap_hits]
   DevBuf entries;   // int2 {col, weight}[cap_entries]
-  DevBuf erank;     // int32[cap_entries]
+  DevBuf erank;     // int32[cap_entries], sorted rows only (as the next two)
   DevBuf tmp_e;     // int2[cap_entries]  radix ping-pong for hub rows
   DevBuf tmp_r;     // int32[cap_entries]
-  DevBuf row_ptr;   // int32[n+1]
-  DevBuf deg;       // int32[n] degree, then fill cursor
-  DevBuf tiles;     // int32[n_tiles]
-  DevBuf counters;  // u64[4]: recorded hits, long rows, spare, predicate hits
-  DevBuf long_rows; // int32[n]
+  DevBuf row_ptr;   // int32[G][n+1]
+  DevBuf deg;       // int32[G][n] degree, then fill cursor
+  DevBuf tiles;     // int32[G][n_tiles]
+  DevBuf counters;  // u64[G][4]: spare, long rows, spare, predicate hits
+  DevBuf long_rows; // int32[G][n]
   DevBuf win;       // WinDesc[n_windows]
   DevBuf ranges;    // CandRange[...]
 };
 
-rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes,
-                                 int64_t cap_hits, int64_t n_windows,
+// Room for any group of at most `slots` windows and `cap_hits` candidates.
+rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t slots,
+                                 int64_t cap_hits, bool sort_rows,
                                  const std::vector<WinDesc> &wins,
                                  const std::vector<CandRange> &ranges);
+// Splits the windows into groups (`single`: one window each) and places each
+// window's hits in its group's list.
+void plan_window_groups(std::vector<WinDesc> &wins, int32_t n_nodes, bool single,
+                        std::vector<WindowGroup> &groups);
 
 // ---- mean-field replay (meanfield.cu) ----
 struct MfRates {
@@ -279,13 +295,13 @@ int32_t window_scan_tiles(int32_t n_nodes);
 
 enum WeightKind { kWeightF32 = 0, kWeightI32 = 1 };
 
-// Enqueues the CSR build of window `wi` into ws.row_ptr / ws.entries.
-// sort_rows: order each row by (col, rank) and merge duplicates in place
-// (merged-away entries keep their column with weight 0).
-void enqueue_window_build(const Graph &g, WindowWorkspace &ws, int wi,
-                          const WinDesc &desc, int64_t cap, int weight_kind,
-                          bool sort_rows, cudaStream_t st);
-// Compacts the sorted, merged CSR in ws into (row_ptr_out, entries_out):
+// Enqueues the CSR build of a group of windows into ws.row_ptr / ws.entries;
+// returns the kernels launched.  sort_rows: order each row by (col, rank) and
+// merge duplicates in place (merged-away entries keep their column with
+// weight 0).
+int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup &grp, int64_t cap,
+                         int weight_kind, bool sort_rows, cudaStream_t st);
+// Compacts the sorted, merged CSR in ws (slot 0) into (row_ptr_out, entries_out):
 // drops merged-away entries.  tmp_rows: int32[n+1] scratch.
 void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out,
                             int2 *entries_out, cudaStream_t st);

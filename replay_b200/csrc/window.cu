@@ -6,13 +6,14 @@
 // (tool/gpu_cpu_temporal_sim.cu:238-350: overlap weights, symmetric
 // emission, qsort by (row, col), FP32 duplicate merge, counting sort).
 //
-// Kernels, in launch order for one window:
+// Kernels, in launch order for one group of consecutive windows (grid y):
 //   k_hits      candidates of the duration-class index -> hit list (+degrees)
 //   k_trunc     only when the reference's hit cap can bind: keep the cap
 //               smallest ranks (radix select), then count degrees
 //   k_scan_*    degrees -> row_ptr (exclusive scan), cursors reset
 //   k_fill      hits -> row segments {col, weight} + rank
 //   k_rowsort_* rows ordered by (col, rank), duplicates merged in rank order
+#include <algorithm>
 #include <cstdio>
 
 #include "rp_device.cuh"
@@ -70,16 +71,28 @@ __device__ __forceinline__ int block_sum(int v, int *warp_tot) {
 }
 
 // ---------------------------------------------------------------------------
+// Every kernel below builds a group of consecutive windows: blockIdx.y is the
+// window's slot in the group, and the per-window arrays of the workspace lie
+// slot after slot (WindowGroup in rp_internal.h).
+//
+// k_hits writes candidate t's hit at slot t of the window's list (u = -2
+// where the candidate does not overlap the window): the class ranges hold few
+// candidates that miss, and a dense list would take one atomic per warp on
+// one address (180,000 candidates of a replica-sweep window: 5,600 of them).
 __global__ void __launch_bounds__(256)
-    k_hits(const WinDesc *__restrict__ wins, int wi,
-           const CandRange *__restrict__ ranges, const int64_t *__restrict__ cs,
-           const int64_t *__restrict__ ce, const int32_t *__restrict__ cu,
-           const int32_t *__restrict__ cv, const int32_t *__restrict__ crank,
-           Hit *__restrict__ hits, unsigned long long *__restrict__ counters,
-           int32_t *__restrict__ deg, int weight_f32) {
+    k_hits(const WinDesc *__restrict__ wins, const CandRange *__restrict__ ranges,
+           const int64_t *__restrict__ cs, const int64_t *__restrict__ ce,
+           const int32_t *__restrict__ cu, const int32_t *__restrict__ cv,
+           const int32_t *__restrict__ crank, Hit *__restrict__ hits_all,
+           unsigned long long *__restrict__ counters, int32_t *__restrict__ deg_all, int32_t n,
+           int weight_f32) {
   __shared__ CandRange sr[kClasses];
   __shared__ WinDesc sw;
-  if (threadIdx.x == 0) sw = wins[wi];
+  __shared__ int s_pred;
+  if (threadIdx.x == 0) {
+    sw = wins[blockIdx.y];
+    s_pred = 0;
+  }
   __syncthreads();
   if ((int)threadIdx.x < sw.n_ranges) sr[threadIdx.x] = ranges[sw.range_off + threadIdx.x];
   __syncthreads();
@@ -87,69 +100,66 @@ __global__ void __launch_bounds__(256)
   const int64_t total = sw.n_candidates;
   const int count_deg = !sw.may_truncate;
   const int query_neg = sw.ws < 0;
-  const unsigned lane = threadIdx.x & 31;
-  const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) - lane;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = warp0; base < total; base += stride) {
-    const int64_t t = base + lane;
-    bool rec = false, pred = false;
+  Hit *hits = hits_all + sw.hit_off;
+  int32_t *deg = deg_all + (int64_t)blockIdx.y * n;
+  int npred = 0;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (int64_t)gridDim.x * blockDim.x) {
     Hit h;
-    if (t < total) {
-      int k = 0;
-      for (int step = 32; step > 0; step >>= 1)
-        if (k + step < nr && sr[k + step].prefix <= t) k += step;
-      const int64_t idx = sr[k].lo + (t - sr[k].prefix);
-      const int64_t s = cs[idx], e = ce[idx];
-      if (s < sw.qe && sw.qs < e) {
-        pred = true;
-        // Coordinates handed to the CSR builder: mirrored back when the
-        // stored orientation differs from the query's.
-        int64_t hs = s, he = e;
-        if ((s < 0) != query_neg) {
-          hs = -e;
-          he = -(int64_t)(int32_t)s;
-        }
-        const int64_t os = hs > sw.ws ? hs : sw.ws;
-        const int64_t oe = he < sw.we ? he : sw.we;
-        const int64_t ov = oe - os;
-        h.rank = crank[idx];
-        h.v = cv[idx];
-        if (ov > 0) {
-          h.u = cu[idx];
-          h.w = weight_f32 ? __float_as_int(__fmul_rn(__ll2float_rn(ov), sw.scale))
-                           : (int32_t)ov;
-          rec = true;
-          if (count_deg) {
-            atomicAdd(&deg[h.u], 1);
-            atomicAdd(&deg[h.v], 1);
-          }
-        } else if (!count_deg) {
-          h.u = -1;
-          h.w = 0;
-          rec = true;
+    h.rank = -1;
+    h.u = -2;
+    h.v = h.w = 0;
+    int k = 0;
+    for (int step = 32; step > 0; step >>= 1)
+      if (k + step < nr && sr[k + step].prefix <= t) k += step;
+    const int64_t idx = sr[k].lo + (t - sr[k].prefix);
+    const int64_t s = cs[idx], e = ce[idx];
+    if (s < sw.qe && sw.qs < e) {
+      ++npred;
+      // Coordinates handed to the CSR builder: mirrored back when the
+      // stored orientation differs from the query's.
+      int64_t hs = s, he = e;
+      if ((s < 0) != query_neg) {
+        hs = -e;
+        he = -(int64_t)(int32_t)s;
+      }
+      const int64_t os = hs > sw.ws ? hs : sw.ws;
+      const int64_t oe = he < sw.we ? he : sw.we;
+      const int64_t ov = oe - os;
+      h.rank = crank[idx];
+      h.v = cv[idx];
+      h.u = -1;  // in the window without overlap: counts toward the hit cap only
+      if (ov > 0) {
+        h.u = cu[idx];
+        h.w = weight_f32 ? __float_as_int(__fmul_rn(__ll2float_rn(ov), sw.scale)) : (int32_t)ov;
+        if (count_deg) {
+          atomicAdd(&deg[h.u], 1);
+          atomicAdd(&deg[h.v], 1);
         }
       }
     }
-    const unsigned pmask = __ballot_sync(kFull, pred);
-    if (pmask && lane == 0) atomicAdd(&counters[3], (unsigned long long)__popc(pmask));
-    const unsigned mask = __ballot_sync(kFull, rec);
-    if (mask) {
-      unsigned long long pos0 = 0;
-      if (lane == 0) pos0 = atomicAdd(&counters[0], (unsigned long long)__popc(mask));
-      pos0 = __shfl_sync(kFull, pos0, 0);
-      if (rec) hits[pos0 + __popc(mask & ((1u << lane) - 1u))] = h;
-    }
+    hits[t] = h;
   }
+  npred = __reduce_add_sync(kFull, npred);
+  if ((threadIdx.x & 31) == 0 && npred) atomicAdd(&s_pred, npred);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_pred)
+    atomicAdd(&counters[4 * blockIdx.y + 3], (unsigned long long)s_pred);
 }
 
 // The reference query stops after max(nlists,1) hits taken in sorted order
 // (the NCLS depth-first order), i.e. it keeps the cap smallest ranks.
+// Candidates outside the window rank last (-1 is the largest unsigned rank)
+// and carry no weight, so they never displace a hit.
 __global__ void __launch_bounds__(1024)
-    k_trunc(Hit *__restrict__ hits, const unsigned long long *__restrict__ counters,
-            int64_t cap, int32_t *__restrict__ deg) {
+    k_trunc(const WinDesc *__restrict__ wins, Hit *__restrict__ hits_all, int64_t cap,
+            int32_t *__restrict__ deg_all, int32_t nodes) {
   __shared__ unsigned hist[256];
   __shared__ unsigned s_prefix, s_k;
-  const int64_t n = (int64_t)counters[0];
+  if (!wins[blockIdx.y].may_truncate) return;
+  Hit *hits = hits_all + wins[blockIdx.y].hit_off;
+  int32_t *deg = deg_all + (int64_t)blockIdx.y * nodes;
+  const int64_t n = wins[blockIdx.y].n_candidates;
   uint32_t thr = 0xFFFFFFFFu;
   if (n > cap) {
     if (threadIdx.x == 0) {
@@ -195,24 +205,30 @@ __global__ void __launch_bounds__(1024)
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan_tiles(const int32_t *__restrict__ in, int32_t n, int32_t *__restrict__ tiles) {
+    k_scan_tiles(const int32_t *__restrict__ in_all, int32_t n, int32_t *__restrict__ tiles) {
   __shared__ int wt[32];
+  const int32_t *in = in_all + (int64_t)blockIdx.y * n;
   const int64_t base = (int64_t)blockIdx.x * kScanTile + 4 * threadIdx.x;
   int s = 0;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     if (base + j < n) s += in[base + j];
   s = block_sum(s, wt);
-  if (threadIdx.x == 0) tiles[blockIdx.x] = s;
+  if (threadIdx.x == 0) tiles[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
 
+// Row pointers from the degrees (one block per tile and window; a window of
+// one tile needs no tile sums).
 __global__ void __launch_bounds__(kScanThreads)
-    k_scan_apply(int32_t *__restrict__ in, int32_t n,
-                 const int32_t *__restrict__ tiles, int32_t *__restrict__ out,
+    k_scan_apply(int32_t *__restrict__ in_all, int32_t n,
+                 const int32_t *__restrict__ tiles, int32_t *__restrict__ out_all,
                  int zero_in) {
   __shared__ int wt[32];
+  int32_t *in = in_all + (int64_t)blockIdx.y * n;
+  int32_t *out = out_all + (int64_t)blockIdx.y * (n + 1);
   int off = 0;
-  for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x) off += tiles[b];
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x)
+    off += tiles[(int64_t)blockIdx.y * gridDim.x + b];
   off = block_sum(off, wt);
   const int64_t base = (int64_t)blockIdx.x * kScanTile + 4 * threadIdx.x;
   int v[4], s = 0;
@@ -235,20 +251,28 @@ __global__ void __launch_bounds__(kScanThreads)
 }
 
 __global__ void __launch_bounds__(256)
-    k_fill(const Hit *__restrict__ hits, const unsigned long long *__restrict__ counters,
-           const int32_t *__restrict__ row_ptr, int32_t *__restrict__ cursor,
-           int2 *__restrict__ entries, int32_t *__restrict__ erank) {
-  const int64_t n = (int64_t)counters[0];
+    k_fill(const WinDesc *__restrict__ wins, const Hit *__restrict__ hits_all,
+           const int32_t *__restrict__ row_ptr_all, int32_t *__restrict__ cursor_all,
+           int2 *__restrict__ entries_all, int32_t *__restrict__ erank_all, int32_t nodes,
+           int keep_rank) {
+  const int64_t n = wins[blockIdx.y].n_candidates, hoff = wins[blockIdx.y].hit_off;
+  const Hit *hits = hits_all + hoff;
+  const int32_t *row_ptr = row_ptr_all + (int64_t)blockIdx.y * (nodes + 1);
+  int32_t *cursor = cursor_all + (int64_t)blockIdx.y * nodes;
+  int2 *entries = entries_all + 2 * hoff;
+  int32_t *erank = erank_all + 2 * hoff;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const Hit h = hits[i];
     if (h.u < 0) continue;
     const int32_t pu = row_ptr[h.u] + atomicAdd(&cursor[h.u], 1);
     entries[pu] = make_int2(h.v, h.w);
-    erank[pu] = h.rank;
     const int32_t pv = row_ptr[h.v] + atomicAdd(&cursor[h.v], 1);
     entries[pv] = make_int2(h.u, h.w);
-    erank[pv] = h.rank;
+    if (keep_rank) {
+      erank[pu] = h.rank;
+      erank[pv] = h.rank;
+    }
   }
 }
 
@@ -287,10 +311,16 @@ __device__ void merge_runs_smem(const uint64_t *key, int32_t *val, int L, int f3
 }
 
 __global__ void __launch_bounds__(32 * kRowsortWarps)
-    k_rowsort_warp(int32_t n, const int32_t *__restrict__ row_ptr,
-                   int2 *__restrict__ entries, int32_t *__restrict__ erank,
-                   unsigned long long *__restrict__ counters,
+    k_rowsort_warp(const WinDesc *__restrict__ wins, int32_t n,
+                   const int32_t *__restrict__ row_ptr_all, int2 *__restrict__ entries_all,
+                   int32_t *__restrict__ erank_all, unsigned long long *__restrict__ counters,
                    int32_t *__restrict__ long_rows, int f32) {
+  const int64_t hoff = wins[blockIdx.y].hit_off;
+  const int32_t *row_ptr = row_ptr_all + (int64_t)blockIdx.y * (n + 1);
+  int2 *entries = entries_all + 2 * hoff;
+  int32_t *erank = erank_all + 2 * hoff;
+  counters += 4 * blockIdx.y;
+  long_rows += (int64_t)blockIdx.y * n;
   __shared__ uint64_t skey[kRowsortWarps][kWarpCap];
   __shared__ int32_t sval[kRowsortWarps][kWarpCap];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -401,12 +431,21 @@ __global__ void __launch_bounds__(32 * kRowsortWarps)
 // (rank, then col) between the row segment and a scratch segment, then the
 // sequential merge.  Only reached by hub rows of FP32-weight windows.
 __global__ void __launch_bounds__(256)
-    k_rowsort_long(const int32_t *__restrict__ row_ptr, int2 *__restrict__ entries,
-                   int32_t *__restrict__ erank, int2 *__restrict__ tmp_e,
+    k_rowsort_long(const WinDesc *__restrict__ wins, int32_t n,
+                   const int32_t *__restrict__ row_ptr_all, int2 *__restrict__ entries_all,
+                   int32_t *__restrict__ erank_all, int2 *__restrict__ tmp_e,
                    int32_t *__restrict__ tmp_r,
                    const unsigned long long *__restrict__ counters,
                    const int32_t *__restrict__ long_rows, int rank_bits,
                    int col_bits, int f32) {
+  const int64_t hoff = wins[blockIdx.y].hit_off;
+  const int32_t *row_ptr = row_ptr_all + (int64_t)blockIdx.y * (n + 1);
+  int2 *entries = entries_all + 2 * hoff;
+  int32_t *erank = erank_all + 2 * hoff;
+  tmp_e += 2 * hoff;
+  tmp_r += 2 * hoff;
+  counters += 4 * blockIdx.y;
+  long_rows += (int64_t)blockIdx.y * n;
   __shared__ unsigned hist[256];
   __shared__ unsigned offs[256];
   const int64_t nl = (int64_t)counters[1];
@@ -528,30 +567,31 @@ int32_t window_scan_tiles(int32_t n_nodes) {
   return t < 1 ? 1 : t;
 }
 
-rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes,
-                                 int64_t cap_hits, int64_t n_windows,
+rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t slots,
+                                 int64_t cap_hits, bool sort_rows,
                                  const std::vector<WinDesc> &wins,
                                  const std::vector<CandRange> &ranges) {
   w.n_nodes = n_nodes;
   w.cap_hits = cap_hits < 1 ? 1 : cap_hits;
   w.cap_entries = 2 * w.cap_hits;
-  w.n_tiles = (int32_t)((n_nodes + kScanTile - 1) / kScanTile);
-  if (w.n_tiles < 1) w.n_tiles = 1;
+  w.n_tiles = window_scan_tiles(n_nodes);
+  const size_t n = (size_t)n_nodes, g = (size_t)(slots < 1 ? 1 : slots);
   RP_TRY(w.hits.alloc(sizeof(Hit) * w.cap_hits));
   // two spare pairs: the step kernel stages entry ranges with 16-byte bulk
   // copies that may read 8 bytes past the last pair
   RP_TRY(w.entries.alloc(sizeof(int2) * (w.cap_entries + 2)));
-  RP_TRY(w.erank.alloc(sizeof(int32_t) * w.cap_entries));
-  RP_TRY(w.tmp_e.alloc(sizeof(int2) * w.cap_entries));
-  RP_TRY(w.tmp_r.alloc(sizeof(int32_t) * w.cap_entries));
-  RP_TRY(w.row_ptr.alloc(sizeof(int32_t) * ((size_t)n_nodes + 1)));
-  RP_TRY(w.deg.alloc(sizeof(int32_t) * ((size_t)n_nodes + 1)));
-  RP_TRY(w.tiles.alloc(sizeof(int32_t) * (size_t)w.n_tiles));
-  RP_TRY(w.counters.alloc(sizeof(unsigned long long) * 4));
-  RP_TRY(w.long_rows.alloc(sizeof(int32_t) * ((size_t)n_nodes + 1)));
-  RP_TRY(w.win.alloc(sizeof(WinDesc) * (n_windows > 0 ? n_windows : 1)));
+  if (sort_rows) {
+    RP_TRY(w.erank.alloc(sizeof(int32_t) * w.cap_entries));
+    RP_TRY(w.tmp_e.alloc(sizeof(int2) * w.cap_entries));
+    RP_TRY(w.tmp_r.alloc(sizeof(int32_t) * w.cap_entries));
+    RP_TRY(w.long_rows.alloc(sizeof(int32_t) * g * n));
+  }
+  RP_TRY(w.row_ptr.alloc(sizeof(int32_t) * g * (n + 1)));
+  RP_TRY(w.deg.alloc(sizeof(int32_t) * g * n));
+  RP_TRY(w.tiles.alloc(sizeof(int32_t) * g * (size_t)w.n_tiles));
+  RP_TRY(w.counters.alloc(sizeof(unsigned long long) * 4 * g));
+  RP_TRY(w.win.alloc(sizeof(WinDesc) * (wins.empty() ? 1 : wins.size())));
   RP_TRY(w.ranges.alloc(sizeof(CandRange) * (ranges.empty() ? 1 : ranges.size())));
-  RP_TRY_CUDA(cudaMemset(w.deg.ptr, 0, w.deg.bytes));
   if (!wins.empty())
     RP_TRY_CUDA(cudaMemcpy(w.win.ptr, wins.data(), sizeof(WinDesc) * wins.size(),
                            cudaMemcpyHostToDevice));
@@ -561,39 +601,80 @@ rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes,
   return RP_OK;
 }
 
-void enqueue_window_build(const Graph &g, WindowWorkspace &ws, int wi,
-                          const WinDesc &desc, int64_t cap, int weight_kind,
-                          bool sort_rows, cudaStream_t st) {
-  const int32_t n = ws.n_nodes;
-  unsigned long long *ctr = ws.counters.as<unsigned long long>();
-  cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * 4, st);
-  // degrees start at zero (the previous window left its fill cursors here)
-  cudaMemsetAsync(ws.deg.ptr, 0, sizeof(int32_t) * (size_t)n, st);
-  const int f32 = weight_kind == kWeightF32;
-  k_hits<<<grid_for(desc.n_candidates, 256, 148 * 16), 256, 0, st>>>(
-      ws.win.as<WinDesc>(), wi, ws.ranges.as<CandRange>(), g.cs.as<int64_t>(),
-      g.ce.as<int64_t>(), g.cu.as<int32_t>(), g.cv.as<int32_t>(), g.crank.as<int32_t>(),
-      ws.hits.as<Hit>(), ctr, ws.deg.as<int32_t>(), f32);
-  if (desc.may_truncate)
-    k_trunc<<<1, 1024, 0, st>>>(ws.hits.as<Hit>(), ctr, cap, ws.deg.as<int32_t>());
-  k_scan_tiles<<<ws.n_tiles, kScanThreads, 0, st>>>(ws.deg.as<int32_t>(), n,
-                                                   ws.tiles.as<int32_t>());
-  k_scan_apply<<<ws.n_tiles, kScanThreads, 0, st>>>(ws.deg.as<int32_t>(), n,
-                                                   ws.tiles.as<int32_t>(),
-                                                   ws.row_ptr.as<int32_t>(), 1);
-  k_fill<<<grid_for(desc.n_candidates, 256, 148 * 8), 256, 0, st>>>(
-      ws.hits.as<Hit>(), ctr, ws.row_ptr.as<int32_t>(), ws.deg.as<int32_t>(),
-      ws.entries.as<int2>(), ws.erank.as<int32_t>());
-  if (sort_rows) {
-    k_rowsort_warp<<<grid_for(n, 32 * kRowsortWarps / 32, 148 * 16), 32 * kRowsortWarps, 0,
-                     st>>>(n, ws.row_ptr.as<int32_t>(), ws.entries.as<int2>(),
-                           ws.erank.as<int32_t>(), ctr, ws.long_rows.as<int32_t>(), f32);
-    k_rowsort_long<<<148, 256, 0, st>>>(ws.row_ptr.as<int32_t>(), ws.entries.as<int2>(),
-                                        ws.erank.as<int32_t>(), ws.tmp_e.as<int2>(),
-                                        ws.tmp_r.as<int32_t>(), ctr,
-                                        ws.long_rows.as<int32_t>(), bits_for(g.n_contacts),
-                                        bits_for(n), f32);
+// Consecutive windows whose candidates and per-node arrays fit the budget
+// form a group (at most kGroupMax windows).  A window of a small network is a
+// chain of six launches of a few microseconds each, most of it launch
+// latency: 22 us for N = 1,000, twice what the two step kernels of the window
+// take.  A group pays that chain once.  The budget keeps a group's pairs in
+// L2 between its build and its last step; the first group is smaller, since
+// no step can overlap its build.
+constexpr int64_t kGroupBytes = 32ll << 20, kFirstGroupBytes = 4ll << 20;
+constexpr int32_t kGroupMax = 256;
+
+void plan_window_groups(std::vector<WinDesc> &wins, int32_t n_nodes, bool single,
+                        std::vector<WindowGroup> &groups) {
+  groups.clear();
+  const int64_t node_bytes = 12ll * n_nodes;
+  for (int32_t w = 0; w < (int32_t)wins.size();) {
+    const int64_t budget = groups.empty() ? kFirstGroupBytes : kGroupBytes;
+    WindowGroup g;
+    g.first = w;
+    do {
+      wins[w].hit_off = g.candidates;
+      g.candidates += wins[w].n_candidates;
+      if (wins[w].n_candidates > g.max_candidates) g.max_candidates = wins[w].n_candidates;
+      g.truncate |= wins[w].may_truncate;
+      ++g.count;
+      ++w;
+    } while (!single && w < (int32_t)wins.size() && g.count < kGroupMax &&
+             48 * (g.candidates + wins[w].n_candidates) + node_bytes * (g.count + 1) <= budget);
+    groups.push_back(g);
   }
+}
+
+int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup &grp, int64_t cap,
+                         int weight_kind, bool sort_rows, cudaStream_t st) {
+  const int32_t n = ws.n_nodes;
+  const unsigned G = (unsigned)grp.count;
+  int launches = 0;
+  unsigned long long *ctr = ws.counters.as<unsigned long long>();
+  const WinDesc *wins = ws.win.as<WinDesc>() + grp.first;
+  cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * 4 * G, st);
+  // degrees start at zero (the previous group left its fill cursors here)
+  cudaMemsetAsync(ws.deg.ptr, 0, sizeof(int32_t) * (size_t)n * G, st);
+  const int f32 = weight_kind == kWeightF32;
+  const int blocks = std::max(1, 148 * 16 / (int)G);  // per window
+  k_hits<<<dim3(grid_for(grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
+      wins, ws.ranges.as<CandRange>(), g.cs.as<int64_t>(), g.ce.as<int64_t>(),
+      g.cu.as<int32_t>(), g.cv.as<int32_t>(), g.crank.as<int32_t>(), ws.hits.as<Hit>(), ctr,
+      ws.deg.as<int32_t>(), n, f32);
+  ++launches;
+  if (grp.truncate) {
+    k_trunc<<<dim3(1, G), 1024, 0, st>>>(wins, ws.hits.as<Hit>(), cap, ws.deg.as<int32_t>(), n);
+    ++launches;
+  }
+  if (ws.n_tiles > 1) {
+    k_scan_tiles<<<dim3(ws.n_tiles, G), kScanThreads, 0, st>>>(ws.deg.as<int32_t>(), n,
+                                                               ws.tiles.as<int32_t>());
+    ++launches;
+  }
+  k_scan_apply<<<dim3(ws.n_tiles, G), kScanThreads, 0, st>>>(
+      ws.deg.as<int32_t>(), n, ws.tiles.as<int32_t>(), ws.row_ptr.as<int32_t>(), 1);
+  k_fill<<<dim3(grid_for(grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
+      wins, ws.hits.as<Hit>(), ws.row_ptr.as<int32_t>(), ws.deg.as<int32_t>(),
+      ws.entries.as<int2>(), ws.erank.as<int32_t>(), n, sort_rows);
+  launches += 2;
+  if (sort_rows) {
+    k_rowsort_warp<<<dim3(grid_for(n, kRowsortWarps, blocks), G), 32 * kRowsortWarps, 0, st>>>(
+        wins, n, ws.row_ptr.as<int32_t>(), ws.entries.as<int2>(), ws.erank.as<int32_t>(), ctr,
+        ws.long_rows.as<int32_t>(), f32);
+    k_rowsort_long<<<dim3(std::max(1, 148 / (int)G), G), 256, 0, st>>>(
+        wins, n, ws.row_ptr.as<int32_t>(), ws.entries.as<int2>(), ws.erank.as<int32_t>(),
+        ws.tmp_e.as<int2>(), ws.tmp_r.as<int32_t>(), ctr, ws.long_rows.as<int32_t>(),
+        bits_for(g.n_contacts), bits_for(n), f32);
+    launches += 2;
+  }
+  return launches;
 }
 
 void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out,
@@ -602,7 +683,8 @@ void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out,
   int32_t *len = ws.deg.as<int32_t>();
   k_count_kept<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(n, ws.row_ptr.as<int32_t>(),
                                                         ws.entries.as<int2>(), len);
-  k_scan_tiles<<<ws.n_tiles, kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>());
+  if (ws.n_tiles > 1)
+    k_scan_tiles<<<ws.n_tiles, kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>());
   k_scan_apply<<<ws.n_tiles, kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>(),
                                                    row_ptr_out, 1);
   k_compact<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(n, ws.row_ptr.as<int32_t>(),

@@ -135,7 +135,11 @@ rp_status window_csr_noalloc(const Graph &g, int64_t ws, int64_t we, float scale
   if (desc.n_ranges > 0)
     RP_TRY_CUDA(cudaMemcpyAsync(w.ranges.ptr, ranges, sizeof(CandRange) * desc.n_ranges,
                                 cudaMemcpyHostToDevice, st));
-  enqueue_window_build(g, w, 0, desc, cap, weight_kind, true, st);
+  WindowGroup grp;
+  grp.count = 1;
+  grp.truncate = desc.may_truncate;
+  grp.candidates = grp.max_candidates = desc.n_candidates;
+  enqueue_window_build(g, w, grp, cap, weight_kind, true, st);
   unsigned long long hits_raw = 0;
   RP_TRY_CUDA(cudaMemcpyAsync(&hits_raw, w.counters.as<unsigned long long>() + 3,
                               sizeof(hits_raw), cudaMemcpyDeviceToHost, st));

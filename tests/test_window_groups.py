@@ -1,0 +1,52 @@
+"""Windows built in groups (one chain of launches for many consecutive
+windows): per-step replays against the oracle where the grouping has edges."""
+import numpy as np
+import pytest
+
+from replay_b200 import synthetic
+
+CASES = [
+    # 700 windows of a tiny network: more than one full group of 256, a remainder, empty windows at the end
+    dict(n=20, contacts=900, span=550 * 300, steps=700, step=300, kw=dict(transition="geometric", beta=1e-3, p_ei=0.2, p_ir=0.1)),
+    # the hit cap binds in some windows of a group and not in others
+    dict(n=30, contacts=400, span=6 * 3600, steps=24, step=900, cap=True,
+         kw=dict(transition="countdown", infect_prob=0.4, exposed_duration=900, infectious_duration=2700,
+                 resistant_duration=900)),
+    # several scan tiles per window, FP32 rows sorted in a group, two steps per window
+    dict(n=9000, contacts=40_000, span=6 * 3600, steps=12, step=1800, window=3600,
+         kw=dict(transition="countdown", infect_prob=0.4, exposed_duration=900, infectious_duration=7200,
+                 resistant_duration=900)),
+]
+
+
+def capped(net, c):
+    """Contacts whose sublist count (the reference's hit cap) is small: one long
+    contact over non-nested ones of one duration, every 16th of which holds another."""
+    k = np.arange(c["contacts"])
+    start = net["t0"] + k * (c["span"] // c["contacts"])
+    start[0], start[1::16] = net["t0"], start[:-1:16] + 1
+    end = start + 1200
+    end[0], end[1::16] = net["t0"] + c["span"] + 1300, start[1::16] + 60
+    return dict(net, start=start, end=end)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_grouped_windows_match_oracle(oracle, case):
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import replay_b200 as rb
+    c = CASES[case]
+    net = synthetic.tiny(seed=90 + case, n_nodes=c["n"], n_contacts=c["contacts"], span=c["span"], max_dur=3000)
+    if c.get("cap"):
+        net = capped(net, c)
+    kw = dict(step_size=float(c["step"]), window=c.get("window", c["step"]), start_time=net["t0"], seed=5,
+              ncls_cap=int(bool(c.get("cap"))), initial_infected=0.1)
+    g = rb.Graph.from_arrays(net["start"], net["end"], net["u"], net["v"], c["n"])
+    sim = rb.Simulation(g, M=40, iterations=c["steps"], path="batched", csr="per-step", **kw, **c["kw"])
+    mode = 0 if c["kw"]["transition"] == "countdown" else 1
+    want = oracle.run(net["start"], net["end"], net["u"], net["v"], c["n"], n_replicas=40, n_steps=c["steps"],
+                      **kw, **dict(c["kw"], transition=mode))
+    np.testing.assert_array_equal(sim.run(), want)
+    np.testing.assert_array_equal(sim.run(), want)  # the workspaces are reused
