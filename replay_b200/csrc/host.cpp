@@ -285,14 +285,14 @@ struct rp_sim {
   cudaEvent_t ev_built[2] = {nullptr, nullptr}, ev_free = nullptr, ev_join = nullptr;
   bool prebuilt = false;
   std::vector<int64_t> arena_rp_off, arena_ent_off;
-  DevBuf arena_rp, arena_ent;
+  DevBuf arena_rp, arena_ent, arena_heavy, arena_heavy_n;
+  std::vector<int64_t> arena_heavy_off;  // n_windows + 1 offsets of the heavy-row lists
   int64_t prebuilt_nnz = 0;
   // plain state
   DevBuf state, exposure;
   // batched state
-  DevBuf sa, sb, mask, evs, flag, tasks, ev, rs, init_counts;
+  DevBuf sa, sb, mask, evs, bits, tasks, ev, rs, init_counts;
   DevBuf mask2;  // countdown mode: the infectious masks alternate between steps
-  DevBuf err;  // int32: set by a kernel that gave up a bounded wait
   // batched countdown state: per-replica codes into the countdown table
   DevBuf codes, cd_tab;
   CdTable cd;
@@ -314,7 +314,7 @@ struct rp_sim {
   int64_t *text_len_host = nullptr;
   cudaEvent_t text_ev[2] = {nullptr, nullptr};
   // shared
-  DevBuf counts, beta_r, sus, classes;
+  DevBuf counts, beta_r, beta_word, sus, classes;
   StepConsts c{};
   cudaStream_t stream = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -392,6 +392,17 @@ struct rp_sim {
     return ws_of(win_group[w]).entries.as<int2>() + 2 * wins[w].hit_off;
   }
 
+  HeavyRows heavy_of(int t) const {
+    const int w = step_win[t], grp = win_group[w];
+    if (prebuilt)
+      return HeavyRows{arena_heavy.as<int32_t>() + arena_heavy_off[w],
+                       arena_heavy.as<int32_t>() + arena_heavy_off[w + 1],
+                       arena_heavy_n.as<unsigned long long>() + 4 * (int64_t)w};
+    const int64_t slot = w - groups[grp].first;
+    const int32_t *rows = ws_of(grp).long_rows.as<int32_t>() + slot * N;
+    return HeavyRows{rows, rows + N, ws_of(grp).counters.as<unsigned long long>() + 4 * slot};
+  }
+
   // Optional event marks around kernel groups (rp_sim_profile).
   struct Marks {
     std::vector<cudaEvent_t> ev;
@@ -453,7 +464,7 @@ struct rp_sim {
       if (rs.ptr && p.p_rs > 0.0f) RP_TRY_CUDA(cudaMemsetAsync(rs.ptr, 0, rs.bytes, st));
       RP_TRY_CUDA(cudaMemsetAsync(init_counts.ptr, 0, init_counts.bytes, st));
       packed_init(L, sa.as<uint32_t>(), sb.as<uint32_t>(), mask.as<uint32_t>(),
-                  flag.as<uint8_t>(), p.initial_infected, p.initial_count, net_first.as<int32_t>(),
+                  bits.as<uint32_t>(), p.initial_infected, p.initial_count, net_first.as<int32_t>(),
                   net_rows.as<int32_t>(), n_nets, c, st);
       if (cd.code_bytes)  // countdown codes from the initial-infection plane
         cd_init(L, tasks.as<PackedTask>(), sa.as<uint32_t>(), codes.ptr, cd.code_bytes,
@@ -511,16 +522,16 @@ struct rp_sim {
           mark(kMarkStep);
           k += 1;
         } else {
-          packed_infect(L, tasks.as<PackedTask>(), rp_of(t), ent_of(t), mask.as<uint32_t>(),
+          packed_infect(L, rp_of(t), ent_of(t), heavy_of(t), mask.as<uint32_t>(),
                         sa.as<uint32_t>(), sb.as<uint32_t>(), evs.as<uint32_t>(),
-                        flag.as<uint8_t>(), (uint32_t)t, step_scale[t], c, st);
+                        bits.as<uint32_t>(), (uint32_t)t, step_scale[t], c, st);
           mark(kMarkSpmv);
-          packed_flow(L, tasks.as<PackedTask>(), rp_of(t), mask.as<uint32_t>(),
-                      sa.as<uint32_t>(), sb.as<uint32_t>(), evs.as<uint32_t>(),
-                      flag.as<uint8_t>(), ev.as<unsigned long long>() + (int64_t)t * per_row,
+          packed_flow(L, mask.as<uint32_t>(), sa.as<uint32_t>(), sb.as<uint32_t>(),
+                      evs.as<uint32_t>(), bits.as<uint32_t>(),
+                      ev.as<unsigned long long>() + (int64_t)t * per_row,
                       p.p_rs > 0.0f ? rs.as<unsigned long long>() + (int64_t)t * per_row
                                     : nullptr,
-                      (uint32_t)t, c, st);
+                      net_first.as<int32_t>(), n_nets, (uint32_t)t, c, st);
           mark(kMarkStep);
           k += 2;
         }
@@ -614,12 +625,21 @@ rp_status prebuild(rp_sim &s) {
   }
   s.prebuilt_nnz = ent;
   RP_TRY(s.arena_rp.alloc(sizeof(int32_t) * (size_t)nw * ((size_t)N + 1)));
-  // two spare pairs for the step kernel's 16-byte bulk staging
-  RP_TRY(s.arena_ent.alloc(sizeof(int2) * (size_t)(ent + 2)));
+  RP_TRY(s.arena_ent.alloc(sizeof(int2) * (size_t)ent));
+  // rows of more than kHeavyPairs pairs: fewer than nnz / kHeavyPairs a window
+  s.arena_heavy_off.assign((size_t)nw + 1, 0);
+  for (int w = 0; w < nw; ++w)
+    s.arena_heavy_off[w + 1] = s.arena_heavy_off[w] + nnz[w] / kHeavyPairs + 1;
+  RP_TRY(s.arena_heavy.alloc(sizeof(int32_t) * (size_t)s.arena_heavy_off[nw]));
+  RP_TRY(s.arena_heavy_n.alloc(sizeof(unsigned long long) * 4 * (size_t)nw));
+  RP_TRY_CUDA(cudaMemsetAsync(s.arena_heavy_n.ptr, 0, s.arena_heavy_n.bytes, st));
   for (int w = 0; w < nw; ++w) {
     enqueue_window_build(*s.g, s.wsp, s.groups[w], s.cap, s.weight_kind, true, st);
     enqueue_window_compact(s.wsp, s.arena_rp.as<int32_t>() + s.arena_rp_off[w],
-                           s.arena_ent.as<int2>() + s.arena_ent_off[w], st);
+                           s.arena_ent.as<int2>() + s.arena_ent_off[w], st,
+                           s.arena_heavy.as<int32_t>() + s.arena_heavy_off[w],
+                           s.arena_heavy_off[w + 1] - s.arena_heavy_off[w],
+                           s.arena_heavy_n.as<unsigned long long>() + 4 * (int64_t)w);
   }
   RP_TRY_CUDA(cudaStreamSynchronize(st));
   return RP_OK;
@@ -706,12 +726,6 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
     }
     s.step_win[t] = (int32_t)s.wins.size() - 1;
   }
-  // per-item hint bytes pay off on windows with many pairs per row (two per
-  // hit; a window's candidates bound its hits from above): at least 4 N
-  // candidates
-  s.c.hints = 0;
-  for (const WinDesc &d : s.wins)
-    if (d.n_candidates >= 4 * (int64_t)s.N) s.c.hints = 1;
   if (max_cand > (int64_t)INT32_MAX / 2) {
     set_error("a window has %lld candidate contacts; at most 2^30 are supported",
               (long long)max_cand);
@@ -754,6 +768,12 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
   s.c.th.te = thr(p.p_ei, s.c.th.te_all);
   s.c.th.ti = thr(p.p_ir, s.c.th.ti_all);
   s.c.th.tr = thr(p.p_rs, s.c.th.tr_all);
+  s.c.th.small = ((s.c.th.te | s.c.th.ti | s.c.th.tr) >> 60) == 0;
+  for (int k = 0; k < 8; ++k) {
+    s.c.th.me[k] = (s.c.th.te >> (63 - k)) & 1 ? ~0u : 0u;
+    s.c.th.mi[k] = (s.c.th.ti >> (63 - k)) & 1 ? ~0u : 0u;
+    s.c.th.mr[k] = (s.c.th.tr >> (63 - k)) & 1 ? ~0u : 0u;
+  }
   s.c.p_ei = p.p_ei;
   s.c.p_ir = p.p_ir;
   s.c.p_rs = p.p_rs;
@@ -770,6 +790,13 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
     RP_TRY_CUDA(cudaMemcpy(s.beta_r.ptr, p.beta_per_replica, sizeof(float) * s.M,
                            cudaMemcpyHostToDevice));
     s.c.beta_r = s.beta_r.as<float>();
+    std::vector<float> mx((size_t)(s.M + 31) / 32, 0.0f);
+    for (int32_t r = 0; r < s.M; ++r)
+      mx[r >> 5] = std::fmax(mx[r >> 5], std::fabs(p.beta_per_replica[r]));
+    RP_TRY(s.beta_word.alloc(sizeof(float) * mx.size()));
+    RP_TRY_CUDA(cudaMemcpy(s.beta_word.ptr, mx.data(), sizeof(float) * mx.size(),
+                           cudaMemcpyHostToDevice));
+    s.c.beta_word = s.beta_word.as<float>();
   }
   if (p.susceptibility) {
     RP_TRY(s.sus.alloc(sizeof(float) * (size_t)s.N));
@@ -804,25 +831,19 @@ rp_status upload_tasks(rp_sim &s) {
     const int32_t f = s.h_first[net], e = f + s.h_rows[net];
     for (int32_t r0 = f; r0 < e; r0 += rpt)
       for (int32_t sl = 0; sl < s.n_slices; ++sl)
-        tasks.push_back(PackedTask{r0, std::min(r0 + rpt, e), sl, net * M, s.task_stage[net]});
+        tasks.push_back(PackedTask{r0, std::min(r0 + rpt, e), sl, net * M});
   }
   if (s.tasks.bytes < sizeof(PackedTask) * tasks.size())
     RP_TRY(s.tasks.alloc(sizeof(PackedTask) * tasks.size()));
   RP_TRY_CUDA(cudaMemcpy(s.tasks.ptr, tasks.data(), sizeof(PackedTask) * tasks.size(),
                          cudaMemcpyHostToDevice));
   s.L.n_tasks = (int32_t)tasks.size();
-  s.L.max_task_rows = 0;
-  for (const PackedTask &t : tasks)
-    s.L.max_task_rows = std::max(s.L.max_task_rows, t.row_end - t.row_begin);
   return RP_OK;
 }
 
 rp_status alloc_state(rp_sim &s) {
   const int32_t N = s.N, M = s.M, T = s.T;
   const int64_t NM = (int64_t)N * M;
-  RP_TRY(s.err.alloc(sizeof(int32_t)));
-  RP_TRY_CUDA(cudaMemset(s.err.ptr, 0, sizeof(int32_t)));
-  s.c.err = s.err.as<int32_t>();
   RP_TRY(s.counts.alloc(sizeof(int32_t) * (size_t)(T + 1) * (size_t)M * 4 * s.n_nets));
   if (s.p.record_node_states) RP_TRY(s.classes.alloc((size_t)NM));
   if (s.path == RP_PATH_PLAIN) {
@@ -840,11 +861,12 @@ rp_status alloc_state(rp_sim &s) {
   L.words = (L.vwords + 3) / 4 * 4;
   L.q4 = L.words / 4;
   L.last_mask = (M % 32) ? ((1u << (M % 32)) - 1u) : 0xFFFFFFFFu;
-  int lpr = 1;
-  while (lpr < L.q4 && lpr < 32) lpr <<= 1;
-  L.lpr = lpr;
+  L.lb = 0;
+  while ((1 << L.lb) < L.q4 && L.lb < 5) ++L.lb;
   const int32_t n_slices = (L.q4 + 31) / 32;
-  s.n_slices = n_slices;
+  s.n_slices = L.n_slices = n_slices;
+  const int32_t rows_per_word = 32 >> L.lb;
+  L.bit_words = (int64_t)((N + rows_per_word - 1) / rows_per_word) * n_slices;
   std::vector<int32_t> first, rows, size;
   if (s.net_bounds.empty()) {  // one network: rows [0, N)
     first.push_back(0);
@@ -862,15 +884,17 @@ rp_status alloc_state(rp_sim &s) {
   // default tiles: about 3 tasks per SM over the whole batch's rows (a
   // network smaller than a task is one task); rp_sim_autotune refines them
   s.task_rows.assign(s.n_nets, rows_per_task(N, n_slices));
-  s.task_stage.assign(s.n_nets, kStageDefault);
+  s.task_stage.assign(s.n_nets, 0);
   RP_TRY(packed_prepare());
   RP_TRY(cd_prepare());
   const size_t plane = sizeof(uint32_t) * (size_t)N * L.words;
   RP_TRY(s.sa.alloc(plane));
   RP_TRY(s.sb.alloc(plane));
   RP_TRY(s.mask.alloc(plane));
-  RP_TRY(s.flag.alloc(((size_t)N * L.q4 + 3) / 4 * 4));
-  if (!s.cd.code_bytes) RP_TRY(s.evs.alloc(plane));
+  if (!s.cd.code_bytes) {
+    RP_TRY(s.evs.alloc(plane));
+    RP_TRY(s.bits.alloc(sizeof(uint32_t) * 4 * (size_t)L.bit_words));
+  }
   if (s.cd.code_bytes) {
     RP_TRY(s.mask2.alloc(plane));
     RP_TRY(s.codes.alloc((size_t)s.cd.code_bytes * 32 * (size_t)N * L.words));
@@ -1004,20 +1028,6 @@ rp_status mf_capture_backward(rp_meanfield &m) {
     mf_finish(m.gpart.as<double>(), m.nblk, m.grates.as<double>(), st);
     return RP_OK;
   });
-}
-
-// Fails when a kernel of the last replay gave up a bounded wait (the flag is
-// sticky until read here).
-rp_status check_kernel_flag(rp_sim &s, cudaStream_t st) {
-  int32_t flag = 0;
-  RP_TRY_CUDA(cudaMemcpyAsync(&flag, s.err.ptr, sizeof(flag), cudaMemcpyDeviceToHost, st));
-  RP_TRY_CUDA(cudaStreamSynchronize(st));
-  if (flag) {
-    RP_TRY_CUDA(cudaMemsetAsync(s.err.ptr, 0, sizeof(int32_t), st));
-    set_error("a step kernel gave up waiting for its staged copies; results are invalid");
-    return RP_ERR_DEVICE;
-  }
-  return RP_OK;
 }
 
 // ===========================================================================
@@ -1318,7 +1328,6 @@ RP_API rp_status rp_sim_counts(rp_sim *s, int32_t *counts) {
   }
   RP_TRY_CUDA(cudaSetDevice(s->g->device));
   RP_TRY_CUDA(cudaDeviceSynchronize());
-  RP_TRY(check_kernel_flag(*s, s->stream));
   RP_TRY_CUDA(cudaMemcpy(counts, s->counts.ptr, s->counts.bytes, cudaMemcpyDeviceToHost));
   return RP_OK;
 }
@@ -1338,7 +1347,7 @@ RP_API rp_status rp_sim_run(rp_sim *s, int32_t *counts, rp_state_cb cb, void *us
   }
   RP_TRY_CUDA(cudaMemcpyAsync(counts, s->counts.ptr, s->counts.bytes, cudaMemcpyDeviceToHost,
                               s->stream));
-  RP_TRY(check_kernel_flag(*s, s->stream));
+  RP_TRY_CUDA(cudaStreamSynchronize(s->stream));
   return RP_OK;
 }
 
@@ -1383,7 +1392,7 @@ RP_API rp_status rp_sim_run_text(rp_sim *s, int32_t *counts, rp_text_cb cb, void
   RP_TRY(st);
   RP_TRY_CUDA(cudaMemcpyAsync(counts, s->counts.ptr, s->counts.bytes, cudaMemcpyDeviceToHost,
                               s->stream));
-  RP_TRY(check_kernel_flag(*s, s->stream));
+  RP_TRY_CUDA(cudaStreamSynchronize(s->stream));
   return RP_OK;
 }
 
@@ -1412,13 +1421,13 @@ RP_API rp_status rp_sim_get_info(const rp_sim *s, rp_sim_info *o) {
   o->prebuilt_nnz = s->prebuilt_nnz;
   int64_t bytes = 0;
   const DevBuf *bufs[] = {&s->arena_rp, &s->arena_ent, &s->state, &s->exposure, &s->sa,
-                          &s->sb, &s->mask, &s->mask2, &s->evs, &s->flag, &s->err,
+                          &s->sb, &s->mask, &s->mask2, &s->evs, &s->bits,
                           &s->codes, &s->cd_tab,
                           &s->tasks, &s->ev, &s->rs,
                           &s->init_counts, &s->counts, &s->beta_r, &s->sus, &s->classes,
                           &s->wsp.hits, &s->wsp.entries, &s->wsp.erank, &s->wsp.tmp_e,
                           &s->wsp.tmp_r, &s->wsp.row_ptr, &s->wsp.deg, &s->wsp.tiles,
-                          &s->wsp.long_rows};
+                          &s->wsp.long_rows, &s->arena_heavy, &s->arena_heavy_n};
   for (auto b : bufs) bytes += (int64_t)b->bytes;
   o->device_bytes = bytes;
   o->nnz_total = s->nnz_total;

@@ -7,13 +7,20 @@
 //             R (1,1)
 //   mask      infectious bits (a & ~b); k_infect reads it, then k_flow
 //             rewrites the words whose state changed
-//   evs       infection events of the step (items with events only; a
-//             per-item flag byte tells k_flow which ones)
+//   evs       infection events of the step (items with events only)
+//   bits      four bitmaps with one bit per item (item = node x 4-word column,
+//             128 replicas): act (some replica may move: E, I, waning R), inf
+//             (some may be infectious), sus (some may be susceptible), evb
+//             (infection events of this step).  act, inf and sus are supersets
+//             of the state; evb is exact.
 // The window CSR holds {col, weight} pairs (int32 contact-seconds).
 //
 // k_infect (exposure SpMM + infection draws), per row with contacts, lanes
 // over 4-word columns (the replacement of cusparseSpMM,
 // tool/gpu_cpu_temporal_sim.cu:1062, and monte_carlo_simulation, :137-159):
+//   0. one lane per row ORs the neighbours' inf bits, 4 B per contact for 32
+//      columns: only items with an infectious neighbour and susceptible
+//      replicas go on;
 //   1. inf = OR over neighbours j of mask_t[j] (16 B per lane per entry);
 //   2. exposed = inf & S; the exposed replicas of a word compare the top
 //      byte of their infection uniforms (8 bit-sliced planes, two Philox
@@ -22,14 +29,14 @@
 //      replicas at or below it compute their exact int64 exposure and
 //      P = 1 - exp(-beta_r s_i e) and finish the comparison against
 //      floor(P 2^64) (infect_event; the uniform's low 56 bits are drawn
-//      only on a tie of the top byte);
-//   3. events are OR-ed into evs and flag their item.
-// k_flow (transitions + count reduction), every (row, 4-word column):
-//   reads the planes and the row's infection events, draws the bit-sliced
+//      only on a tie of the top byte).  Rows of more than kHeavyPairs pairs
+//      sum every replica's exposure bit-sliced instead;
+//   3. events are OR-ed into evs and flag their item (evb).
+// k_flow (transitions + count reduction), every item set in act or evb:
+//   reads the planes and the item's infection events, draws the bit-sliced
 //   flow uniforms of the E, I (and waning R) replicas, 32 replicas per random
 //   plane (flow_events), applies all moves with bitwise operations, writes the
-//   planes and mask_{t+1}, and adds every transition event to per-replica
-//   counters in shared memory, flushed once per task to the step's event
+//   planes and mask_{t+1}, and adds every transition event to the step's event
 //   row; k_finalize turns initial counts + events into per-step counts.
 // Every decision uses the state at the start of the step: k_infect reads the
 // planes before k_flow rewrites them.
@@ -52,24 +59,12 @@ __device__ __forceinline__ uint32_t get4(const uint4 &v, int w) {
   return w == 0 ? v.x : (w == 1 ? v.y : (w == 2 ? v.z : v.w));
 }
 
-__device__ __forceinline__ void set4(uint4 &v, int w, uint32_t x) {
-  if (w == 0) v.x = x; else if (w == 1) v.y = x; else if (w == 2) v.z = x; else v.w = x;
-}
-
 __device__ __forceinline__ void or4(uint4 &a, const uint4 b) {
   a.x |= b.x;
   a.y |= b.y;
   a.z |= b.z;
   a.w |= b.w;
 }
-
-// Fast division of an item index by the columns of a task (ncols <= 32,
-// items < 2^27): q = umulhi(i, ceil(2^32 / d)).
-struct Div {
-  uint32_t d, mag;
-  __device__ explicit Div(uint32_t dd) : d(dd), mag(dd > 1 ? 0xFFFFFFFFu / dd + 1u : 0u) {}
-  __device__ uint32_t div(uint32_t i) const { return d > 1 ? __umulhi(i, mag) : i; }
-};
 
 __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
   int incl = v;
@@ -105,114 +100,63 @@ __device__ __forceinline__ int find_owner(const int32_t *off, int p) {
   return owner;
 }
 
-constexpr int kMaxTaskRows = 4096;  // rows of one task (host-side limit)
-
-// Per-item hint byte (item = node x 4-word column): bit 0 an infection event
-// of this step (k_infect), bit 1 replicas that may move (E, I, waning R),
-// bit 2 replicas that may be susceptible.  k_flow rewrites bits 1-2 of every
-// item from its start-of-step planes and events, as a superset of the next
-// step's state; k_infect skips the neighbours of items without bit 2 where
-// rows are long enough for the extra load to pay.  The hints are kept only
-// for graphs whose windows average at least 8 pairs per row (StepConsts
-// hints); elsewhere the extra work would not pay.
-constexpr uint8_t kFlagEvent = 1, kFlagActive = 2, kFlagSusceptible = 4;
-
-constexpr int kEntCap = kStageDefault;  // staging buffer capacity, CSR pairs
-constexpr int kEntBuf = kEntCap + 4; // a staging buffer (the copy may start one pair early)
-constexpr int kPiece = kEntBuf / 2 - 2;  // pairs per piece of a long row (a half buffer)
-constexpr long long kSpinLimit = 1ll << 22;
-
-// ---- bulk asynchronous copies (global -> this CTA's shared memory) ----------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+// Bitmap word and bit of item (row, col): rows of at most 32 columns share a
+// word (1 << lb bits per row), wider rows take one word per slice of 32
+// columns.
+__device__ __forceinline__ int64_t bit_word(int lb, int n_slices, int row, int col) {
+  return (int64_t)(row >> (5 - lb)) * n_slices + (col >> 5);
 }
-__device__ __forceinline__ void mbar_init(unsigned long long *bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)));
+__device__ __forceinline__ int bit_shift(int lb, int row, int col) {
+  return ((row & ((32 >> lb) - 1)) << lb) + (col & 31);
 }
-// Waits for the phase with the given parity to complete; false after
-// kSpinLimit polls.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t parity) {
-  const uint32_t a = smem_u32(bar);
-  for (long long i = 0; i < kSpinLimit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-// Stages pairs [k0, k1) of `ent` (k1 - k0 <= kEntBuf - 2) into `dst` with one
-// bulk copy (cp.async.bulk, no multicast) completing on `bar`; the copy
-// starts on the 16-byte boundary at or below pair k0, so pair k lands at
-// dst[k - k0 + shift].  Returns shift.  Issued by one thread.
-__device__ __forceinline__ int stage_pairs(int2 *dst, const int2 *ent, int32_t k0, int32_t k1,
-                                           unsigned long long *bar) {
-  const uintptr_t src = reinterpret_cast<uintptr_t>(ent + k0);
-  const int shift = (int)((src & 15u) >> 3);
-  const uint32_t bytes = ((uint32_t)(k1 - k0 + shift) * 8u + 15u) & ~15u;
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_u32(dst)),
-      "l"(ent + k0 - shift), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-  return shift;
-}
-__device__ __forceinline__ int pair_shift(const int2 *ent, int32_t k0) {
-  return (int)((reinterpret_cast<uintptr_t>(ent + k0) & 15u) >> 3);
+__device__ __forceinline__ uint32_t bit_of(int lb, int row, int col) {
+  return 1u << bit_shift(lb, row, col);
 }
 
-// ---------------------------------------------------------------------------
-// Per-warp queue of exposed words of k_infect (dynamic shared memory):
-// entries accumulate over rows and are decided 32 at a time.
+// ---- k_infect ---------------------------------------------------------------
+// Every warp works alone on units of consecutive rows and one slice of 32
+// columns: no block-wide step, so a warp that waits for memory or draws
+// holds up nobody, and units interleave over the whole grid.  (One task of
+// 226 rows per 256-thread block, staged by bulk copies behind mbarriers, took
+// 51 us on a step of 256 sparse networks with 17% of the items active, and a
+// network of 1,000 nodes used 32 of 148 SMs.)
 constexpr int kInfectQueue = 160;  // 31 left over + 4 words x 32 lanes of one pass
-constexpr int kWordExact = 4;      // candidates of a word (long row) for the one-pass exact test
-struct InfectQueue {
-  uint4 pl[32][2];               // the 8 random planes of each word (round scratch)
-  int32_t rloc[kInfectQueue];    // task-relative row
-  int32_t word[kInfectQueue];    // word index within the row
-  uint32_t X[kInfectQueue];      // exposed replicas of the word
-  float efmax[kInfectQueue];     // ef(e_max) of the row
-  uint32_t C[32];      // candidates after the bound test (round scratch)
-  int32_t off[32];     // warp scan offsets of the candidates
+constexpr int kUnitRows = 128;     // most rows of a unit
+
+// Per warp: the unit's rows and items, and a queue of exposed words that
+// accumulates over units and is decided 32 words at a time.
+struct InfectWarp {
+  uint4 pl[32][2];             // the 8 random planes of each word (round scratch)
+  int32_t urow[kUnitRows];     // the unit's rows with pairs (row in unit)
+  int32_t ubeg[kUnitRows];     // their first pairs
+  int32_t list[128];           // items of a batch of 32 rows: row in batch << 5 | column
+  uint32_t rmask[32];          // column masks of the batch's rows
+  int32_t row[kInfectQueue];
+  int32_t word[kInfectQueue];  // word index within the row << 6 | the row's pairs
+  int32_t beg[kInfectQueue];   // the row's first CSR pair
+  uint32_t X[kInfectQueue];    // exposed replicas of the word
+  float efmax[kInfectQueue];   // ef(e_max) of the row
+  uint16_t cl[1024];           // candidates after the bound test: lane << 5 | bit (round scratch)
   // candidates carried to the next round (fewer than 32), self-contained
-  int32_t krloc[32];
-  int32_t kwb[32];  // word << 5 | replica bit
-  uint8_t ku8[32];  // top 8 bits of the replica's uniform
-  // exact-test batch: per candidate lane, its row's first CSR pair, its
-  // word << 5 | bit, the scan offsets of the batch's (candidate, pair)
-  // products and the exposure sums
-  int32_t cbeg[32];
-  int32_t cword[32];
-  int32_t poff[32];
-  long long esum[32];
+  int32_t krow[32];
+  int32_t kwb[32];             // word << 5 | replica bit
+  int32_t kbeg[32];
+  int32_t knpr[32];
+  uint8_t ku8[32];             // top 8 bits of the replica's uniform
   int32_t n;
   int32_t nk;
 };
-
-// k_infect's dynamic shared memory, sized per launch: two staging buffers
-// and the warps' queues at fixed offsets, then the task's row pointers (max
-// task rows + 1), then a long row's per-replica exposures (int32,
-// min(32, q4) columns x 128 replicas).  Sized for the launch, so that tall
-// tasks or wide rows cost only where they occur (three CTAs per SM need at
-// most about 74 KB each).
-constexpr int kInfectQueueOff = 2 * kEntBuf * 8;
-constexpr int kInfectRpOff = kInfectQueueOff + kWarps * (int)sizeof(InfectQueue);
-__host__ __device__ constexpr int infect_acc_off(int max_rows) {
-  return (kInfectRpOff + 4 * (max_rows + 1) + 15) / 16 * 16;
-}
-__host__ __device__ constexpr int infect_smem(int q4, int max_rows) {
-  return infect_acc_off(max_rows) + (q4 < 32 ? q4 : 32) * 128 * 4;
-}
-constexpr int kInfectDynSmemMax = infect_smem(32, kMaxTaskRows);
+// Per warp, for rows of more than kHeavyPairs pairs (before the queue is used).
+struct HeavyWarp {
+  uint32_t e[32][32];  // bit k of the exposures of lane o's 32 replicas: e[k][o]
+  uint4 pl[32][2];
+  uint32_t C[32];
+  int32_t off[32];
+};
+constexpr int kInfectWarpBytes =
+    (int)((sizeof(InfectWarp) > sizeof(HeavyWarp) ? sizeof(InfectWarp) : sizeof(HeavyWarp)) + 15) /
+    16 * 16;
+constexpr int kInfectDynSmem = kWarps * kInfectWarpBytes;
 
 // Top 8 uniform bits of replica bit b from a queued word's planes.
 __device__ __forceinline__ uint32_t queued_top8(const uint4 (&q)[2], uint32_t b) {
@@ -221,25 +165,28 @@ __device__ __forceinline__ uint32_t queued_top8(const uint4 (&q)[2], uint32_t b)
   return top8_of(pl, b);
 }
 
-// What an infection decision reads besides the candidate (values, so that
-// the out-of-line word_exact_pass takes them in registers).
-struct DecideArgs {
-  const uint32_t *rk;     // Philox round keys
-  const float *beta_r;    // per-replica beta, or null
-  const float *sus;       // per-node susceptibility, or null
-  float beta, scale;
-  uint32_t roff, step;
-  int32_t words, q4, row_begin;
+// What the kernel reads and writes.
+struct InfectArgs {
+  const int32_t *row_ptr;
+  const int2 *ent;
+  const uint32_t *mask, *sa, *sb;
+  uint32_t *evs;
+  const uint32_t *infb, *susb;
+  uint32_t *evb;
+  const int32_t *heavy, *heavy_end;    // rows of more than kHeavyPairs / kHugePairs pairs (window.cu)
+  const unsigned long long *n_heavy;  // [0] heavy, [2] huge rows
+  uint32_t step;
+  float scale;
+  int32_t unit_rows, n_units;
 };
 
-// Decides candidate replica b of task-relative row orl, word `word`, from
-// its exact exposure e (contact-seconds) and its uniform's top byte u8.
-__device__ __forceinline__ void decide(const DecideArgs &d, int orl, int word, int b,
-                                       long long e, uint32_t u8, uint32_t *evs_w,
-                                       uint32_t *flag32) {
-  const int orow = d.row_begin + orl;
-  const float br = d.beta_r ? __ldg(d.beta_r + word * 32 + b) : d.beta;
-  const float bs = d.sus ? __fmul_rn(br, d.sus[orow]) : br;
+// Decides candidate replica b of (row, word) from its exact exposure e
+// (contact-seconds) and its uniform's top byte u8.
+__device__ __forceinline__ void decide(const InfectArgs &d, const StepConsts &c,
+                                       const PackedLayout &L, int row, int word, int b,
+                                       long long e, uint32_t u8) {
+  const float br = c.beta_r ? __ldg(c.beta_r + word * 32 + b) : c.beta;
+  const float bs = c.sus ? __fmul_rn(br, __ldg(c.sus + row)) : br;
   float ef = __ll2float_rn(e);
   if (d.scale != 1.0f) ef = __fmul_rn(ef, d.scale);
   const float xx = __fmul_rn(bs, ef);
@@ -247,186 +194,96 @@ __device__ __forceinline__ void decide(const DecideArgs &d, int orl, int word, i
   // P <= x: a uniform whose top byte is above x's cannot infect (no
   // exponential)
   if (xx < 1.0f && u8 > (uint32_t)(fixed64(xx) >> 56)) return;
-  const uint32_t gword = (uint32_t)word + (d.roff >> 5);
-  if (infect_event(one_minus_exp_neg(xx), u8, d.rk, (uint32_t)orow, d.step,
+  const uint32_t gword = (uint32_t)word + (c.roff >> 5);
+  if (infect_event(one_minus_exp_neg(xx), u8, c.rk, (uint32_t)row, d.step,
                    gword * 32u + (uint32_t)b)) {
-    atomicOr(&evs_w[(int64_t)orow * d.words + word], 1u << b);
-    const int64_t idx = (int64_t)orow * d.q4 + (word >> 2);
-    atomicOr(&flag32[idx >> 2], 1u << (8 * (idx & 3)));
+    atomicOr(&d.evs[(int64_t)row * L.words + word], 1u << b);
+    atomicOr(&d.evb[bit_word(L.lb, L.n_slices, row, word >> 2)], bit_of(L.lb, row, word >> 2));
   }
 }
 
-// The exact test of the queued words in `wlist` (lane o's word holds
-// candidates Cw of lane o): one pass over each word's row with lane =
-// replica, so that each pair's mask word is one broadcast load shared by all
-// the word's candidates.  For words with many candidates on rows of more
-// than 32 pairs (a dense neighbourhood, whose bound test lets most exposed
-// replicas through); on other words the per-replica test costs less.  Kept
-// out of line: the busy steps of sparse graphs rarely take it.
-__device__ __noinline__ void word_exact_pass(const InfectQueue &Q, unsigned wlist, uint32_t Cw,
-                                             int lane, const int32_t *s_rp, const int2 *s_ent,
-                                             const int2 *__restrict__ ent, bool staged, int32_t e0,
-                                             const uint32_t *mask_w, uint32_t *evs_w,
-                                             uint32_t *flag32, DecideArgs d) {
-  for (unsigned t = wlist; t; t &= t - 1) {
-    const int o = __ffs(t) - 1;
-    const uint32_t Co = __shfl_sync(kFull, Cw, o);
-    const int orl = Q.rloc[o], word = Q.word[o];
-    const int32_t kend = s_rp[orl + 1];
-    int32_t k = s_rp[orl];
-    long long e = 0;
-    for (; k + 4 <= kend; k += 4) {
-      int2 q[4];
-      uint32_t m[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) q[j] = staged ? s_ent[k + j - e0] : __ldg(ent + k + j);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) m[j] = mask_w[(int64_t)q[j].x * d.words + word];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) e += ((m[j] >> lane) & 1u) ? q[j].y : 0;
-    }
-    for (; k < kend; ++k) {
-      const int2 q0 = staged ? s_ent[k - e0] : __ldg(ent + k);
-      e += ((mask_w[(int64_t)q0.x * d.words + word] >> lane) & 1u) ? q0.y : 0;
-    }
-    if ((Co >> lane) & 1u)
-      decide(d, orl, word, lane, e, queued_top8(Q.pl[o], (uint32_t)lane), evs_w, flag32);
-  }
+// max over the word's replicas of |beta_r s_i|: every x is at most this times
+// ef(e)
+__device__ __forceinline__ float word_bs(const StepConsts &c, int row, int word) {
+  const float bs = c.beta_r ? __ldg(c.beta_word + word) : fabsf(c.beta);
+  return c.sus ? __fmul_rn(bs, fabsf(__ldg(c.sus + row))) : bs;
 }
 
-// Decides up to 32 queued exposed words: the bound test one word per lane
-// (phase 2), then the exact test of the surviving candidates: a word with
-// at least kWordExact of them in one pass over its row (phase 3a), the
-// others one replica per lane (phase 3), in full batches of 32 together with
-// the candidates carried from earlier rounds; fewer than 32 left over are
-// carried to the next round unless `drain` is set.  Events are OR-ed into
-// their words and flag their items.
-__device__ __forceinline__ void infect_round(InfectQueue &Q, int n, bool drain, int lane,
-                                             const PackedLayout &L, const PackedTask &T,
-                                             int cbase, const int32_t *s_rp, const int2 *s_ent,
-                                             const int2 *__restrict__ ent, bool staged,
-                                             int32_t e0, const float *s_bw,
-                                             const uint32_t *mask_w, uint32_t *evs_w,
-                                             uint32_t *flag32, uint32_t step, float scale,
+// Decides up to 32 queued exposed words: the bound test one word per lane,
+// then the exact test of the surviving candidates, one replica per lane, in
+// full batches of 32 together with the candidates carried from earlier
+// rounds; fewer than 32 left over are carried to the next round unless
+// `drain` is set.  Events are OR-ed into their words and flag their items.
+__device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, int lane,
+                                             const PackedLayout &L, const InfectArgs &d,
                                              const StepConsts &c) {
-  // ---- phase 2: bound test, one word per lane ----
+  // ---- bound test, one word per lane ----
   uint32_t Cw = 0;
   if (lane < n) {
-    const int orow = T.row_begin + Q.rloc[lane];
-    const int word = Q.word[lane];
+    const int row = Q.row[lane], word = Q.word[lane] >> 6;
     // every exposed replica has P <= x <= |bs_r| ef(e_max) =: B; replicas
     // whose uniform's top byte is above B's cannot infect
-    float bsmax = c.beta_r ? s_bw[word - 4 * cbase] : fabsf(c.beta);
-    if (c.sus) bsmax = __fmul_rn(bsmax, fabsf(c.sus[orow]));
-    const float B = __fmul_rn(bsmax, Q.efmax[lane]);
+    const float B = __fmul_rn(word_bs(c, row, word), Q.efmax[lane]);
     if (B > 0.0f) {
       uint32_t pl[8];
-      infect_planes(c.rk, (uint32_t)orow, step, (uint32_t)word + (c.roff >> 5), pl);
+      infect_planes(c.rk, (uint32_t)row, d.step, (uint32_t)word + (c.roff >> 5), pl);
       Cw = B >= 1.0f ? Q.X[lane] : top8_le(Q.X[lane], fixed64(B), pl);
       Q.pl[lane][0] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
       Q.pl[lane][1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
     }
   }
-  // ---- phase 3a: a word with many candidates on a row of more than 32
-  // pairs takes one pass over its row (word_exact_pass) ----
-  const unsigned wlist = __ballot_sync(
-      kFull, __popc(Cw) >= kWordExact && s_rp[Q.rloc[lane] + 1] - s_rp[Q.rloc[lane]] > 32);
-  const DecideArgs d{c.rk, c.beta_r, c.sus, c.beta, scale, c.roff, step, L.words, L.q4,
-                     T.row_begin};
-  if (wlist) word_exact_pass(Q, wlist, Cw, lane, s_rp, s_ent, ent, staged, e0, mask_w, evs_w, flag32, d);
-  if ((wlist >> lane) & 1u) Cw = 0;
-  Q.C[lane] = Cw;
   int ctotal;
-  Q.off[lane] = warp_excl_scan(__popc(Cw), lane, ctotal);
+  int pos = warp_excl_scan(__popc(Cw), lane, ctotal);
+  for (; Cw; Cw &= Cw - 1) Q.cl[pos++] = (uint16_t)(lane << 5 | (__ffs(Cw) - 1));
   __syncwarp();
-  // ---- phase 3: exact test of 32 candidates at a time ----
-  // When every candidate's row is short, each lane sums its own row.
-  // Otherwise the batch's (candidate, CSR pair) products are spread over the
-  // lanes: every pair is one independent mask-word load (a long row is
-  // shared by all 32 lanes), and the exposures sum in shared memory (exact
-  // int64).
+  // ---- exact test of 32 candidates at a time: each lane sums its own row
+  // (at most kHeavyPairs pairs), four mask words in flight ----
   const int nk = Q.nk;
   const int total = nk + ctotal;
   int base = 0;
   for (; total - base >= 32 || (drain && base < total); base += 32) {
     const int p = base + lane;
-    int orl = 0, word = 0, b = 0, npairs = 0;
-    int32_t beg = 0;
-    uint32_t u8 = 0;
     if (p < total) {
+      int row, word, b, npairs;
+      int32_t beg;
+      uint32_t u8;
       if (p < nk) {
         const int wb = Q.kwb[p];
-        orl = Q.krloc[p];
+        row = Q.krow[p];
         word = wb >> 5;
         b = wb & 31;
         u8 = Q.ku8[p];
+        beg = Q.kbeg[p];
+        npairs = Q.knpr[p];
       } else {
-        const int o = find_owner(Q.off, p - nk);
-        b = nth_set_bit(Q.C[o], p - nk - Q.off[o]);
-        orl = Q.rloc[o];
+        const int ob = Q.cl[p - nk], o = ob >> 5;
+        b = ob & 31;
+        row = Q.row[o];
         word = Q.word[o];
+        npairs = word & 63;
+        word >>= 6;
         u8 = queued_top8(Q.pl[o], (uint32_t)b);
+        beg = Q.beg[o];
       }
-      beg = s_rp[orl];
-      npairs = s_rp[orl + 1] - beg;
-    }
-    long long e = 0;
-    if (__reduce_max_sync(kFull, (unsigned)npairs) <= 32u) {
-      // short rows: each lane sums its own row (loads two pairs ahead)
-      int32_t k = beg;
-      const int32_t kend = beg + npairs;
-      for (; k + 1 < kend; k += 2) {
-        const int2 q0 = staged ? s_ent[k - e0] : __ldg(ent + k);
-        const int2 q1 = staged ? s_ent[k + 1 - e0] : __ldg(ent + k + 1);
-        const uint32_t m0 = mask_w[(int64_t)q0.x * L.words + word];
-        const uint32_t m1 = mask_w[(int64_t)q1.x * L.words + word];
-        e += ((m0 >> b) & 1u) ? q0.y : 0;
-        e += ((m1 >> b) & 1u) ? q1.y : 0;
-      }
-      if (k < kend) {
-        const int2 q0 = staged ? s_ent[k - e0] : __ldg(ent + k);
-        e += ((mask_w[(int64_t)q0.x * L.words + word] >> b) & 1u) ? q0.y : 0;
-      }
-    } else {
-    int ptotal;
-    const int poff = warp_excl_scan(npairs, lane, ptotal);
-    __syncwarp();
-    Q.poff[lane] = poff;
-    Q.cbeg[lane] = beg;
-    Q.cword[lane] = word << 5 | b;
-    Q.esum[lane] = 0;
-    __syncwarp();
-    for (int q0 = 0; q0 < ptotal; q0 += 64) {
-      int32_t pc[2], pw[2], cw[2], own[2];
+      long long e = 0;
+      for (int32_t k = 0; k < npairs; k += 4) {
+        uint32_t m[4];
+        int32_t wt[4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int q = q0 + 32 * h + lane;
-        own[h] = -1;
-        pc[h] = pw[h] = cw[h] = 0;
-        if (q < ptotal) {
-          const int o = find_owner(Q.poff, q);
-          const int32_t k = Q.cbeg[o] + (q - Q.poff[o]);
-          const int2 e = staged ? s_ent[k - e0] : __ldg(ent + k);
-          pc[h] = e.x;
-          pw[h] = e.y;
-          cw[h] = Q.cword[o];
-          own[h] = o;
+        for (int j = 0; j < 4; ++j) {
+          m[j] = 0;
+          wt[j] = 0;
+          if (k + j < npairs) {
+            const int2 q = __ldg(d.ent + beg + k + j);
+            m[j] = __ldg(d.mask + (int64_t)q.x * L.words + word);
+            wt[j] = q.y;
+          }
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e += ((m[j] >> b) & 1u) ? wt[j] : 0;
       }
-      uint32_t mw[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        mw[h] = own[h] >= 0 ? mask_w[(int64_t)pc[h] * L.words + (cw[h] >> 5)] : 0u;
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        if (own[h] >= 0 && ((mw[h] >> (cw[h] & 31)) & 1u))
-          atomicAdd(reinterpret_cast<unsigned long long *>(&Q.esum[own[h]]),
-                    (unsigned long long)(long long)pw[h]);
+      decide(d, c, L, row, word, b, e, u8);
     }
-    __syncwarp();
-    e = Q.esum[lane];
-    }
-    if (p < total) decide(d, orl, word, b, e, u8, evs_w, flag32);
   }
   __syncwarp();
   // carry the rest: slots below nk keep their entries when no batch ran
@@ -434,10 +291,11 @@ __device__ __forceinline__ void infect_round(InfectQueue &Q, int n, bool drain, 
   if (rest > 0) {
     const int p = base + lane;
     if (p < total && p >= nk) {
-      const int o = find_owner(Q.off, p - nk);
-      const int b = nth_set_bit(Q.C[o], p - nk - Q.off[o]);
-      Q.kwb[lane] = Q.word[o] << 5 | b;
-      Q.krloc[lane] = Q.rloc[o];
+      const int ob = Q.cl[p - nk], o = ob >> 5, b = ob & 31;
+      Q.kwb[lane] = (Q.word[o] >> 6) << 5 | b;
+      Q.krow[lane] = Q.row[o];
+      Q.kbeg[lane] = Q.beg[o];
+      Q.knpr[lane] = Q.word[o] & 63;
       Q.ku8[lane] = (uint8_t)queued_top8(Q.pl[o], (uint32_t)b);
     }
   }
@@ -446,342 +304,405 @@ __device__ __forceinline__ void infect_round(InfectQueue &Q, int n, bool drain, 
   __syncwarp();
 }
 
-// One item (row, 4-word column) per lane gathers the OR of the neighbours'
-// mask words (its loads issued together) and queues its exposed words;
-// infect_round decides the queue 32 words at a time, so that every lane
-// works on a dense list of words and then of candidate replicas.
-__global__ void __launch_bounds__(kThreads, 3)
-    k_infect(PackedLayout L, const PackedTask *__restrict__ tasks,
-             const int32_t *__restrict__ row_ptr, const int2 *__restrict__ ent,
-             const uint4 *__restrict__ mask_in, const uint4 *__restrict__ sa,
-             const uint4 *__restrict__ sb, uint4 *__restrict__ evs,
-             uint32_t *__restrict__ flag32, uint32_t step, float scale,
-             const __grid_constant__ StepConsts c) {
-  __shared__ float s_bw[128];  // max |beta_r| of each word of the slice
-  __shared__ uint4 s_lor[32];  // long row: OR of the neighbours' masks per column
-  __shared__ long long s_lemax;
-  __shared__ int32_t s_stage;  // the task's staging depth (CSR pairs per chunk)
-  __shared__ unsigned long long s_bar[4];  // chunk buffers 0, 1; long-row halves 0, 1
-  extern __shared__ __align__(16) unsigned char s_dyn[];
-  int2 *const s_buf0 = reinterpret_cast<int2 *>(s_dyn);  // two staging buffers of kEntBuf pairs
-  auto bufp = [&](int b) { return s_buf0 + b * kEntBuf; };
-  InfectQueue &Q = reinterpret_cast<InfectQueue *>(s_dyn + kInfectQueueOff)[threadIdx.x >> 5];
-  // the task's row pointers (rows of a task <= L.max_task_rows)
-  int32_t *const s_rp = reinterpret_cast<int32_t *>(s_dyn + kInfectRpOff);
-  // a long row's per-replica exposures (int32, ncols x 128 replicas)
-  int32_t *const s_acc = reinterpret_cast<int32_t *>(s_dyn + infect_acc_off(L.max_task_rows));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t *mask_w = reinterpret_cast<const uint32_t *>(mask_in);
-  uint32_t *evs_w = reinterpret_cast<uint32_t *>(evs);
-  const uint8_t *flag8 = reinterpret_cast<const uint8_t *>(flag32);
-  if (lane == 0) {
-    Q.n = 0;
-    Q.nk = 0;
-  }
-  if (threadIdx.x < 4) mbar_init(&s_bar[threadIdx.x]);
-  if (threadIdx.x == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  __syncthreads();
-  uint32_t cph = 0, pph = 0;  // phase parity of each chunk buffer / half barrier
-  int buf = 0;
-  // every thread waits on the same barriers in the same order; a wait that
-  // gives up raises the error flag (the host fails the run)
-  auto wait_bar = [&](int b, uint32_t &ph, int bit) {
-    const bool ready = mbar_wait(&s_bar[b], (ph >> bit) & 1u);
-    ph ^= 1u << bit;
-    if (!ready && c.err) atomicExch(c.err, 1);
-  };
-  for (int ti = blockIdx.x; ti < L.n_tasks; ti += gridDim.x) {
-    const PackedTask T = tasks[ti];
-    const int cbase = T.slice * 32;
-    const int ncols = min(32, L.q4 - cbase);
-    const Div dv((uint32_t)ncols);
-    const int nrows = T.row_end - T.row_begin;
-    for (int i = threadIdx.x; i <= nrows; i += blockDim.x) s_rp[i] = row_ptr[T.row_begin + i];
-    if (threadIdx.x == 0) s_stage = T.stage < 1 || T.stage > kEntCap ? kEntCap : T.stage;
-    if (c.beta_r)
-      for (int wl = threadIdx.x; wl < ncols * 4; wl += blockDim.x) {
-        float mx = 0.0f;
-        for (int r = 0; r < 32; ++r) {
-          const int rep = cbase * 128 + wl * 32 + r;
-          if (rep < L.m) mx = fmaxf(mx, fabsf(__ldg(c.beta_r + rep)));
-        }
-        s_bw[wl] = mx;
-      }
-    __syncthreads();
-    // chunk of rows [r0, end) of at most s_stage CSR pairs (>= 1 row; the
-    // task's staging depth, at most a buffer; read from shared memory so
-    // that it holds no register across the task)
-    auto chunk_end = [&](int r0) {
-      const int32_t stage = s_stage;
-      int lo = r0 + 1, hi = nrows;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (s_rp[mid] - s_rp[r0] <= stage) lo = mid; else hi = mid - 1;
-      }
-      return lo;
-    };
-    // the chunk's pairs go to buffer b with one bulk copy (thread 0)
-    auto stage_chunk = [&](int ra, int rb, int b) {
-      const int32_t k0 = s_rp[ra], k1 = s_rp[rb];
-      if (threadIdx.x == 0 && k1 > k0 && k1 - k0 <= kEntCap)
-        stage_pairs(bufp(b), ent, k0, k1, &s_bar[b]);
-    };
-    int r0 = 0, r1 = nrows > 0 ? chunk_end(0) : 0;
-    if (nrows > 0) stage_chunk(0, r1, buf);
-    while (r0 < nrows) {
-      const int r2 = r1 < nrows ? chunk_end(r1) : nrows;
-      if (r1 < nrows) stage_chunk(r1, r2, buf ^ 1);  // prefetch the next chunk's pairs
-      const int32_t e0 = s_rp[r0], e1 = s_rp[r1];
-      const bool staged = e1 - e0 <= kEntCap;
-      if (staged && e1 > e0) wait_bar(buf, cph, buf);
-      const int2 *s_ent = bufp(buf) + pair_shift(ent, e0);
-      // one row with more pairs than a buffer; streamed only when one of
-      // its items may hold susceptible replicas
-      const bool long_row =
-          !staged && (!c.hints ||
-                      __syncthreads_or(threadIdx.x < ncols &&
-                                       (flag8[(int64_t)(T.row_begin + r0) * L.q4 + cbase +
-                                              threadIdx.x] & kFlagSusceptible)));
-      const bool skip_row = !staged && !long_row;
-      const bool use_hint = c.hints && e1 - e0 >= 8 * (r1 - r0);  // at least 8 pairs per row
-      bool dense_done = false;
-      if (long_row) {
-        // A hub of the window graph.  Its pairs stream through the two halves
-        // of this chunk's buffer, one piece ahead; every warp takes a share
-        // of each piece (lane = column: a pair costs one 512-byte line of mask
-        // words) and, for the susceptible replicas of the row, adds the
-        // pair's contact-seconds to each infectious neighbour replica's exact
-        // exposure in shared memory.  Every exposed replica is then decided
-        // from its exposure directly (no bound test, no per-candidate scan).
-        const int64_t row = T.row_begin + r0;
-        uint4 S4 = make_uint4(0, 0, 0, 0);
-        if (lane < ncols) {
-          const uint4 a4 = sa[row * L.q4 + cbase + lane], b4 = sb[row * L.q4 + cbase + lane];
+// ---- rows of more than kHeavyPairs pairs ------------------------------------
+// Lane = one 32-replica word, 32 words (1,024 replicas) per warp.  The exact
+// exposures of a word's replicas are kept bit-sliced: s[k] holds bit k of all
+// 32 sums, and adding a pair's weight to the replicas of its mask word is a
+// ripple-carry add, three logic operations per bit of the row's total
+// whatever the number of replicas.  Afterwards a word's candidates are the
+// replicas whose uniform's top byte is at most floor(256 x') with x' >= x the
+// exposure times the next power of two above beta, compared bit-sliced; their
+// exposures are read back from the planes, so no candidate walks its row
+// again.  (Before, a word with candidates took one pass over its row with lane
+// = replica and an e_max bound near 1 let nearly every exposed replica
+// through: 7.5 ms on the first steps of the dense network, N = 5,000 and
+// M = 16,384; see k_infect for the time now.)
+__device__ __forceinline__ void sliced_add(uint32_t (&s)[32], uint32_t m, uint32_t w, int nb) {
+  uint32_t cy = 0;
 #pragma unroll
-          for (int w = 0; w < 4; ++w)
-            set4(S4, w, ~get4(a4, w) & ~get4(b4, w) & word_mask(L, 4 * (cbase + lane) + w));
-        }
-        for (int j = threadIdx.x; j < ncols * 128; j += blockDim.x) s_acc[j] = 0;
-        int2 *const half0 = bufp(buf);
-        auto half = [&](int h) { return half0 + h * (kEntBuf / 2); };
-        if (threadIdx.x < 32) s_lor[threadIdx.x] = make_uint4(0, 0, 0, 0);
-        if (threadIdx.x == 0) {
-          s_lemax = 0;
-          stage_pairs(half(0), ent, e0, min(e0 + kPiece, e1), &s_bar[2]);
-        }
-        __syncthreads();
-        uint4 linf = make_uint4(0, 0, 0, 0);
-        long long lemax = 0;
-        auto add_pair = [&](int2 q, uint4 m) {
-          m = make_uint4(m.x & S4.x, m.y & S4.y, m.z & S4.z, m.w & S4.w);
-          or4(linf, m);
+  for (int g = 0; g < 8; ++g) {
+    if (4 * g >= nb) break;
 #pragma unroll
-          for (int w = 0; w < 4; ++w)
-            for (uint32_t t = get4(m, w); t; t &= t - 1)
-              atomicAdd(&s_acc[(lane * 4 + w) * 32 + __ffs(t) - 1], q.y);
-        };
-        const int npieces = (e1 - e0 + kPiece - 1) / kPiece;
-        for (int pk = 0; pk < npieces; ++pk) {
-          const int hb = pk & 1;
-          const int32_t p0 = e0 + pk * kPiece, p1 = min(p0 + kPiece, e1);
-          if (threadIdx.x == 0 && pk + 1 < npieces)
-            stage_pairs(half(hb ^ 1), ent, p1, min(p1 + kPiece, e1), &s_bar[2 + (hb ^ 1)]);
-          wait_bar(2 + hb, pph, hb);
-          const int2 *pc = half(hb) + pair_shift(ent, p0);
-          int32_t k = p0 + warp;
-          for (; k + kWarps < p1; k += 2 * kWarps) {
-            const int2 q0 = pc[k - p0], q1 = pc[k - p0 + kWarps];
-            lemax += (long long)q0.y + q1.y;
-            if (lane < ncols) {
-              const uint4 m0 = mask_in[(int64_t)q0.x * L.q4 + cbase + lane];
-              const uint4 m1 = mask_in[(int64_t)q1.x * L.q4 + cbase + lane];
-              add_pair(q0, m0);
-              add_pair(q1, m1);
-            }
-          }
-          for (; k < p1; k += kWarps) {
-            const int2 q0 = pc[k - p0];
-            lemax += q0.y;
-            if (lane < ncols) add_pair(q0, mask_in[(int64_t)q0.x * L.q4 + cbase + lane]);
-          }
-          __syncthreads();  // the half is free to restage
-        }
-        if (lane < ncols) {
-          atomicOr(&s_lor[lane].x, linf.x);
-          atomicOr(&s_lor[lane].y, linf.y);
-          atomicOr(&s_lor[lane].z, linf.z);
-          atomicOr(&s_lor[lane].w, linf.w);
-        }
-        if (lane == 0) atomicAdd(reinterpret_cast<unsigned long long *>(&s_lemax),
-                                 (unsigned long long)lemax);
-        __syncthreads();
-        // int32 sums are exact while the row's total fits; otherwise its
-        // items take the per-candidate exact test below
-        dense_done = s_lemax <= 0x7FFFFFFFll;
-        if (dense_done) {
-          const uint32_t *lor = reinterpret_cast<const uint32_t *>(s_lor);
-          const float bs_row = c.sus ? __ldg(c.sus + row) : 1.0f;
-          for (int wl = threadIdx.x; wl < ncols * 4; wl += blockDim.x) {
-            const uint32_t X = lor[wl];  // exposed replicas of the word
-            if (!X) continue;
-            const int word = 4 * cbase + wl;
-            uint32_t pl[8];
-            infect_planes(c.rk, (uint32_t)row, step, (uint32_t)word + (c.roff >> 5), pl);
-            uint32_t ev = 0;
-            for (uint32_t t = X; t; t &= t - 1) {
-              const int b = __ffs(t) - 1;
-              const float br = c.beta_r ? __ldg(c.beta_r + word * 32 + b) : c.beta;
-              const float bs = c.sus ? __fmul_rn(br, bs_row) : br;
-              float ef = __int2float_rn(s_acc[wl * 32 + b]);
-              if (scale != 1.0f) ef = __fmul_rn(ef, scale);
-              const float xx = __fmul_rn(bs, ef);
-              if (!(xx > 0.0f)) continue;
-              const uint32_t u8 = top8_of(pl, (uint32_t)b);
-              if (xx < 1.0f && u8 > (uint32_t)(fixed64(xx) >> 56)) continue;
-              const uint32_t gword = (uint32_t)word + (c.roff >> 5);
-              if (infect_event(one_minus_exp_neg(xx), u8, c.rk, (uint32_t)row, step,
-                               gword * 32u + (uint32_t)b))
-                ev |= 1u << b;
-            }
-            if (ev) {
-              atomicOr(&evs_w[row * L.words + word], ev);
-              const int64_t idx = row * L.q4 + (word >> 2);
-              atomicOr(&flag32[idx >> 2], 1u << (8 * (idx & 3)));
-            }
-          }
-        }
-        __syncthreads();
-      }
-      const int nitems = skip_row || dense_done ? 0 : (r1 - r0) * ncols;
-      // warp-uniform passes; one pass past the items decides what is left
-      // queued (the staged pairs change with the next chunk)
-      int blk = warp * 32;  // this warp's next block of 32 items
-      // a chunk with fewer pairs than half its rows compacts its items
-      // (most of its rows have no pairs)
-      const bool sparse = 2 * (e1 - e0) < r1 - r0;
-      for (;;) {
-        // ---- phase 1a: in a sparse chunk, up to 32 items with CSR pairs
-        // from the warp's next blocks (many blocks fold into one pass; items
-        // without pairs have nothing to gather).  Their indices pass through
-        // Q.off, the rounds' scratch, which is free until the rounds ----
-        int got, it;
-        if (sparse) {
-          got = 0;
-          while (blk < nitems) {
-            const int itb = blk + lane;
-            bool has = false;
-            if (itb < nitems) {
-              const int rlb = (int)dv.div((uint32_t)itb);
-              has = s_rp[r0 + rlb + 1] > s_rp[r0 + rlb];
-            }
-            const unsigned hm = __ballot_sync(kFull, has);
-            if (got + __popc(hm) > 32) break;
-            if (has) Q.off[got + __popc(hm & ((1u << lane) - 1u))] = itb;
-            got += __popc(hm);
-            blk += kWarps * 32;
-          }
-          __syncwarp();
-          it = lane < got ? Q.off[lane] : 0;
-          __syncwarp();
-        } else {  // one block per pass
-          got = blk < nitems ? min(32, nitems - blk) : 0;
-          it = blk + lane;
-          blk += kWarps * 32;
-        }
-        const bool flushing = got == 0;
-        // ---- phase 1: gather, per lane ----
-        const bool ok = lane < got;
-        const int rl = ok ? (int)dv.div((uint32_t)it) : 0;
-        const int cc = ok ? it - rl * ncols : 0;
-        const int rloc = r0 + rl;
-        const int col = cbase + cc;
-        const int row = T.row_begin + rloc;
-        const int32_t beg = s_rp[rloc], end = s_rp[rloc + 1];
-        const int64_t idx = (int64_t)row * L.q4 + col;
-        // an item without susceptible replicas cannot be infected: on
-        // pair-heavy chunks the hint byte saves the item's whole gather
-        const int n = ok && (!use_hint || (flag8[idx] & kFlagSusceptible)) ? end - beg : 0;
-        uint32_t X[4] = {0, 0, 0, 0};
-        float efmax = 0.0f;
-        if (n > 0) {
-          const uint4 a4 = sa[idx], b4 = sb[idx];
-          const int2 *er = s_ent + (beg - e0);
-          uint4 inf = make_uint4(0, 0, 0, 0);
-          long long emax = 0;
-          int k = 0;
-          if (long_row) {  // gathered by the whole CTA above
-            inf = s_lor[cc];
-            emax = s_lemax;
-            k = n;
-          }
-          for (; k + 4 <= n; k += 4) {
-            const int2 q0 = er[k], q1 = er[k + 1], q2 = er[k + 2], q3 = er[k + 3];
-            const uint4 m0 = mask_in[(int64_t)q0.x * L.q4 + col];
-            const uint4 m1 = mask_in[(int64_t)q1.x * L.q4 + col];
-            const uint4 m2 = mask_in[(int64_t)q2.x * L.q4 + col];
-            const uint4 m3 = mask_in[(int64_t)q3.x * L.q4 + col];
-            or4(inf, m0);
-            or4(inf, m1);
-            or4(inf, m2);
-            or4(inf, m3);
-            emax += (long long)q0.y + q1.y + q2.y + q3.y;
-          }
-          for (; k < n; ++k) {
-            const int2 q0 = er[k];
-            or4(inf, mask_in[(int64_t)q0.x * L.q4 + col]);
-            emax += q0.y;
-          }
-#pragma unroll
-          for (int w = 0; w < 4; ++w)
-            X[w] = get4(inf, w) & ~get4(a4, w) & ~get4(b4, w) & word_mask(L, 4 * col + w);
-          efmax = __ll2float_rn(emax);
-          if (scale != 1.0f) efmax = __fmul_rn(efmax, scale);
-        }
-        // ---- queue the exposed words ----
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const unsigned qm = __ballot_sync(kFull, X[w] != 0u);
-          if (!qm) continue;
-          const int base = Q.n;
-          if (X[w]) {
-            const int pos = base + __popc(qm & ((1u << lane) - 1u));
-            Q.rloc[pos] = rloc;
-            Q.word[pos] = 4 * col + w;
-            Q.X[pos] = X[w];
-            Q.efmax[pos] = efmax;
-          }
-          __syncwarp();
-          if (lane == 0) Q.n = base + __popc(qm);
-          __syncwarp();
-        }
-        // ---- decide full rounds (and, past the items, the remainder and
-        // the carried candidates: the staged pairs change with the chunk) ----
-        while (Q.n >= 32 || (flushing && (Q.n > 0 || Q.nk > 0))) {
-          const int take = Q.n < 32 ? Q.n : 32;
-          infect_round(Q, take, flushing && take == Q.n, lane, L, T, cbase, s_rp, s_ent, ent,
-                       staged, e0, s_bw, mask_w, evs_w, flag32, step, scale, c);
-          const int rest = Q.n - take;
-          for (int i = lane; i < rest; i += 32) {
-            Q.rloc[i] = Q.rloc[take + i];
-            Q.word[i] = Q.word[take + i];
-            Q.X[i] = Q.X[take + i];
-            Q.efmax[i] = Q.efmax[take + i];
-          }
-          __syncwarp();
-          if (lane == 0) Q.n = rest;
-          __syncwarp();
-        }
-        if (flushing) break;
-      }
-      __syncthreads();
-      r0 = r1;
-      r1 = r2;
-      buf ^= 1;
+    for (int j = 0; j < 4; ++j) {
+      const int k = 4 * g + j;
+      const uint32_t a = ((w >> k) & 1u) ? m : 0u, t = s[k];
+      s[k] = t ^ a ^ cy;
+      cy = (t & a) | (t & cy) | (a & cy);
     }
   }
 }
 
-// ---------------------------------------------------------------------------
+struct HeavyUnit {
+  int row, w0;          // first word
+  int32_t beg, end;
+  int nb;               // bits of the row's total weight
+  uint32_t S;           // the lane's susceptible replicas
+};
+
+// Loads unit u of `rows` x nws words; false when no replica is susceptible.
+__device__ __forceinline__ bool heavy_load(HeavyUnit &h, const int32_t *list, int dir, int u,
+                                           int nws, int lane, const PackedLayout &L,
+                                           const InfectArgs &d) {
+  h.row = list[dir * (u / nws)];
+  const int ws = u % nws;
+  h.w0 = ws * 32;
+  const int word = h.w0 + lane;
+  const uint32_t sb8 = d.susb[bit_word(L.lb, L.n_slices, h.row, ws * 8)] >>
+                       bit_shift(L.lb, h.row, ws * 8);
+  if (!(sb8 & (L.lb >= 3 ? 0xFFu : (1u << (1 << L.lb)) - 1u))) return false;
+  h.beg = d.row_ptr[h.row];
+  h.end = d.row_ptr[h.row + 1];
+  h.S = 0;
+  if (word < L.vwords) {
+    const int64_t wi = (int64_t)h.row * L.words + word;
+    h.S = ~d.sa[wi] & ~d.sb[wi] & word_mask(L, word);
+  }
+  if (!__any_sync(kFull, h.S != 0u)) return false;
+  long long emax = 0;
+  for (int32_t k = h.beg + lane; k < h.end; k += 32) emax += __ldg(&d.ent[k].y);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) emax += __shfl_xor_sync(kFull, emax, o);
+  h.nb = 64 - __clzll(emax);
+  return true;
+}
+
+// Adds the pairs first, first + stride, ... of the unit's row to H.e (planes
+// of the 32 words) and returns the lane's exposed replicas.
+__device__ __forceinline__ uint32_t heavy_sum(const HeavyUnit &h, HeavyWarp &H, int first,
+                                              int stride, int lane, const PackedLayout &L,
+                                              const InfectArgs &d) {
+  uint32_t s[32];
+#pragma unroll
+  for (int k = 0; k < 32; ++k) s[k] = 0;
+  uint32_t X = 0;
+  const uint32_t *mw = d.mask + min(h.w0 + lane, L.words - 1);
+  const int nb = min(h.nb, 32);
+  for (int32_t k = h.beg + first; k < h.end; k += 4 * stride) {
+    uint32_t m[4], w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      m[j] = 0;
+      w[j] = 0;
+      if (k + j * stride < h.end) {
+        const int2 q = __ldg(d.ent + k + j * stride);
+        w[j] = (uint32_t)q.y;
+        m[j] = __ldg(mw + (int64_t)q.x * L.words);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      m[j] &= h.S;
+      X |= m[j];
+      if (h.nb <= 32 && __any_sync(kFull, m[j] != 0u)) sliced_add(s, m[j], w[j], nb);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 32; ++k)
+    if (k < nb) H.e[k][lane] = s[k];
+  return X;
+}
+
+// The candidates among the lane's exposed replicas X, their random planes and
+// the scan offsets, for heavy_decide.
+__device__ __forceinline__ void heavy_candidates(const HeavyUnit &h, HeavyWarp &H, uint32_t X,
+                                                 int lane, const PackedLayout &L,
+                                                 const InfectArgs &d, const StepConsts &c) {
+  uint32_t cand = 0;
+  if (X) {
+    const int word = h.w0 + lane;
+    uint32_t pl[8];
+    infect_planes(c.rk, (uint32_t)h.row, d.step, (uint32_t)word + (c.roff >> 5), pl);
+    H.pl[lane][0] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+    H.pl[lane][1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
+    // x <= e t (the 1.0001 covers the roundings of x), t < 2^ex
+    const float t = __fmul_rn(__fmul_rn(word_bs(c, h.row, word), d.scale), 1.0001f);
+    if (!(t < 0x1p-8f) || h.nb > 32) {
+      cand = X;
+    } else if (t > 0.0f) {
+      const int ex = (int)((__float_as_uint(t) >> 23) & 0xFFu) - 126;
+      const int p0 = -ex - 8;  // floor(256 e 2^ex) = e >> p0
+      uint32_t hi = 0;
+      for (int k = p0 + 8; k < h.nb; ++k) hi |= H.e[k][lane];
+      uint32_t lt = 0, und = X & ~hi;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int k = p0 + 7 - j;
+        const uint32_t v = k < h.nb ? H.e[k][lane] : 0u;
+        lt |= und & v & ~pl[j];
+        und &= ~(v ^ pl[j]);
+      }
+      cand = (X & hi) | lt | und;
+    }
+  }
+  H.C[lane] = cand;
+  int total;
+  H.off[lane] = warp_excl_scan(__popc(cand), lane, total);
+}
+
+// Exact decisions of H's candidates in batches first, first + stride, ...
+__device__ __forceinline__ void heavy_decide(const HeavyUnit &h, const HeavyWarp &H, int first,
+                                             int stride, int lane, const PackedLayout &L,
+                                             const InfectArgs &d, const StepConsts &c) {
+  const int total = H.off[31] + __popc(H.C[31]);
+  for (int p = 32 * first + lane; p < total; p += 32 * stride) {
+    const int o = find_owner(H.off, p);
+    const int b = nth_set_bit(H.C[o], p - H.off[o]);
+    unsigned long long e = 0;
+    if (h.nb <= 32) {
+      for (int k = 0; k < h.nb; ++k) e |= (unsigned long long)((H.e[k][o] >> b) & 1u) << k;
+    } else {  // totals beyond 2^32 contact-seconds: a plain sum
+      for (int32_t k = h.beg; k < h.end; ++k) {
+        const int2 q = __ldg(d.ent + k);
+        if ((__ldg(d.mask + (int64_t)q.x * L.words + h.w0 + o) >> b) & 1u) e += (uint32_t)q.y;
+      }
+    }
+    decide(d, c, L, h.row, h.w0 + o, b, (long long)e, queued_top8(H.pl[o], (uint32_t)b));
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 3)
+    k_infect(PackedLayout L, const __grid_constant__ InfectArgs d,
+             const __grid_constant__ StepConsts c) {
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // warps of one block are gridDim.x apart: neighbouring units go to
+  // different SMs
+  const int gw = warp * gridDim.x + blockIdx.x, tw = kWarps * gridDim.x;
+  __shared__ unsigned s_next;
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  const int n_heavy = (int)d.n_heavy[0], n_huge = (int)d.n_heavy[2];
+  if (n_heavy | n_huge) {
+    const int nws = (L.words + 31) / 32;
+    HeavyWarp &H = *reinterpret_cast<HeavyWarp *>(s_dyn + warp * kInfectWarpBytes);
+    HeavyUnit h;
+    // rows of more than kHugePairs pairs: the block's warps share the pairs,
+    // warp 0 adds their planes, and the decisions are shared again
+    for (int u = blockIdx.x; u < n_huge * nws; u += gridDim.x) {
+      if (!heavy_load(h, d.heavy_end - 1, -1, u, nws, lane, L, d)) continue;  // same for all warps
+      uint32_t X = heavy_sum(h, H, warp, kWarps, lane, L, d);
+      H.C[lane] = X;
+      __syncthreads();
+      HeavyWarp &H0 = *reinterpret_cast<HeavyWarp *>(s_dyn);
+      if (warp == 0) {
+        for (int v = 1; v < kWarps; ++v) {
+          const HeavyWarp &Hv = *reinterpret_cast<const HeavyWarp *>(s_dyn + v * kInfectWarpBytes);
+          X |= Hv.C[lane];
+          uint32_t cy = 0;
+          for (int k = 0; k < min(h.nb, 32); ++k) {
+            const uint32_t a = H0.e[k][lane], t = Hv.e[k][lane];
+            H0.e[k][lane] = a ^ t ^ cy;
+            cy = (a & t) | (a & cy) | (t & cy);
+          }
+        }
+        heavy_candidates(h, H0, X, lane, L, d, c);
+      }
+      __syncthreads();
+      heavy_decide(h, H0, warp, kWarps, lane, L, d, c);
+      __syncthreads();
+    }
+    for (int u = gw; u < n_heavy * nws; u += tw) {
+      if (!heavy_load(h, d.heavy, 1, u, nws, lane, L, d)) continue;
+      const uint32_t X = heavy_sum(h, H, 0, 1, lane, L, d);
+      if (!__any_sync(kFull, X != 0u)) continue;
+      heavy_candidates(h, H, X, lane, L, d, c);
+      __syncwarp();
+      heavy_decide(h, H, 0, 1, lane, L, d, c);
+      __syncwarp();
+    }
+  }
+
+  InfectWarp &Q = *reinterpret_cast<InfectWarp *>(s_dyn + warp * kInfectWarpBytes);
+  if (lane == 0) {
+    Q.n = 0;
+    Q.nk = 0;
+  }
+  __syncwarp();
+  // the block's units, blockIdx.x + k gridDim.x, go to its warps as they ask
+  auto next_unit = [&]() {
+    int k = 0;
+    if (lane == 0) k = (int)atomicAdd(&s_next, 1u);
+    return (int)blockIdx.x + __shfl_sync(kFull, k, 0) * (int)gridDim.x;
+  };
+  const uint4 *mask4 = reinterpret_cast<const uint4 *>(d.mask);
+  const uint4 *sa4 = reinterpret_cast<const uint4 *>(d.sa);
+  const uint4 *sb4 = reinterpret_cast<const uint4 *>(d.sb);
+  bool more = true;
+  int cbase = 0, cnt = 0;    // the current unit's first column; items listed
+  int nrows = 0, ub = 0;     // the unit's rows with pairs; the first row not yet taken
+  int lrow = 0, n = 0;       // the lane's row of the batch: pairs beg .. beg + n
+  int32_t beg = 0;
+  unsigned nz = 0;           // rows of the batch with items not yet listed
+  for (;;) {
+    if (cnt == 0 && !nz) {
+      if (ub >= nrows) {
+        const int unit = next_unit();
+        if (unit >= d.n_units) {
+          more = false;
+        } else {
+          // the next unit's rows that have pairs (longer rows were taken above)
+          const int rb = L.n_slices == 1 ? unit : unit / L.n_slices;
+          cbase = L.n_slices == 1 ? 0 : (unit - rb * L.n_slices) * 32;
+          const int r0 = rb * d.unit_rows, r1 = min(r0 + d.unit_rows, L.n_nodes);
+          nrows = ub = 0;
+          __syncwarp();
+          for (int r = r0; r < r1; r += 128) {
+            int32_t b[4], len[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int row = r + 32 * j + lane;
+              b[j] = len[j] = 0;
+              if (row < r1) {
+                b[j] = __ldg(d.row_ptr + row);
+                len[j] = __ldg(d.row_ptr + row + 1) - b[j];
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (r + 32 * j >= r1) break;
+              const bool has = len[j] > 0 && len[j] <= kHeavyPairs;
+              const unsigned hm = __ballot_sync(kFull, has);
+              if (has) {
+                const int pos = nrows + __popc(hm & ((1u << lane) - 1u));
+                Q.urow[pos] = (r + 32 * j + lane) << 6 | len[j];
+                Q.ubeg[pos] = b[j];
+              }
+              nrows += __popc(hm);
+            }
+          }
+          __syncwarp();
+          if (nrows == 0) continue;
+        }
+      }
+      // ---- phase 0: items of the next 32 rows with an infectious neighbour and
+      // susceptible replicas.  Lane = row: the OR of the neighbours' inf bits
+      // gives the row's columns at 4 B per contact, where the mask words of 32
+      // columns cost 512 B ----
+      if (more) {
+        n = 0;
+        if (ub + lane < nrows) {
+          lrow = Q.urow[ub + lane];
+          beg = Q.ubeg[ub + lane];
+          n = lrow & 63;
+          lrow >>= 6;
+        }
+        ub += 32;
+        auto row_bits = [&](const uint32_t *bits, int r) {
+          return __ldg(bits + bit_word(L.lb, L.n_slices, r, cbase)) >> bit_shift(L.lb, r, 0);
+        };
+        const int ncols = min(32, L.q4 - cbase);
+        uint32_t sus = n ? row_bits(d.susb, lrow) : 0u, m = 0;
+        sus &= ncols == 32 ? kFull : (1u << ncols) - 1u;
+        for (int k = 0; k < n; k += 4) {  // four words in flight
+          uint32_t v[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            v[j] = k + j < n ? row_bits(d.infb, __ldg(&d.ent[beg + k + j].x)) : 0u;
+          m |= v[0] | v[1] | v[2] | v[3];
+        }
+        m &= sus;
+        // few items: every lane lists its own row's; else row by row below
+        int tot;
+        int pos = warp_excl_scan(__popc(m), lane, tot);
+        if (tot <= 128) {
+          for (; m; m &= m - 1) Q.list[pos++] = lane << 5 | (__ffs(m) - 1);
+          cnt = tot;
+        } else {
+          Q.rmask[lane] = m;
+          nz = __ballot_sync(kFull, m != 0u);
+        }
+        __syncwarp();
+        if (tot == 0) continue;
+      }
+    }
+    while (cnt < 32 && nz) {
+      const int o = __ffs(nz) - 1;
+      nz &= nz - 1;
+      const uint32_t m = Q.rmask[o];
+      if ((m >> lane) & 1u) Q.list[cnt + __popc(m & ((1u << lane) - 1u))] = o << 5 | lane;
+      cnt += __popc(m);
+    }
+    __syncwarp();
+    // ---- phase 1: gather, one item per lane ----
+    const int got = min(cnt, 32);
+    cnt -= got;
+    const bool ok = lane < got;
+    const int it = ok ? Q.list[cnt + lane] : 0;
+    __syncwarp();
+    const int row = __shfl_sync(kFull, lrow, it >> 5), col = cbase + (it & 31);
+    const int32_t rbeg = __shfl_sync(kFull, beg, it >> 5);
+    const int rn = __shfl_sync(kFull, n, it >> 5);
+    uint32_t X[4] = {0, 0, 0, 0};
+    float efmax = 0.0f;
+    if (ok) {
+      const int64_t idx = (int64_t)row * L.q4 + col;
+      const uint4 a4 = __ldg(sa4 + idx), b4 = __ldg(sb4 + idx);
+      uint4 inf = make_uint4(0, 0, 0, 0);
+      long long emax = 0;
+      for (int k = 0; k < rn; k += 4) {  // four mask items in flight
+        uint4 m[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          m[j] = make_uint4(0, 0, 0, 0);
+          if (k + j < rn) {
+            const int2 q = __ldg(d.ent + rbeg + k + j);
+            m[j] = __ldg(mask4 + (int64_t)q.x * L.q4 + col);
+            emax += q.y;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) or4(inf, m[j]);
+      }
+#pragma unroll
+      for (int w = 0; w < 4; ++w)
+        X[w] = get4(inf, w) & ~get4(a4, w) & ~get4(b4, w) & word_mask(L, 4 * col + w);
+      efmax = __ll2float_rn(emax);
+      if (d.scale != 1.0f) efmax = __fmul_rn(efmax, d.scale);
+    }
+    // ---- queue the exposed words ----
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const unsigned qm = __ballot_sync(kFull, X[w] != 0u);
+      if (!qm) continue;
+      const int base = Q.n;
+      if (X[w]) {
+        const int pos = base + __popc(qm & ((1u << lane) - 1u));
+        Q.row[pos] = row;
+        Q.word[pos] = (4 * col + w) << 6 | rn;
+        Q.beg[pos] = rbeg;
+        Q.X[pos] = X[w];
+        Q.efmax[pos] = efmax;
+      }
+      __syncwarp();
+      if (lane == 0) Q.n = base + __popc(qm);
+      __syncwarp();
+    }
+    // ---- decide full rounds and, past the last unit, what is left ----
+    while (Q.n >= 32 || (!more && (Q.n > 0 || Q.nk > 0))) {
+      const int take = Q.n < 32 ? Q.n : 32;
+      infect_round(Q, take, !more && take == Q.n, lane, L, d, c);
+      const int rest = Q.n - take;
+      for (int i = lane; i < rest; i += 32) {
+        Q.row[i] = Q.row[take + i];
+        Q.word[i] = Q.word[take + i];
+        Q.beg[i] = Q.beg[take + i];
+        Q.X[i] = Q.X[take + i];
+        Q.efmax[i] = Q.efmax[take + i];
+      }
+      __syncwarp();
+      if (lane == 0) Q.n = rest;
+      __syncwarp();
+    }
+    if (!more) break;
+  }
+}
+
+// ---- k_flow -------------------------------------------------------------------
+// Transition events go straight to the step's event row with one 64-bit
+// reduction each: about 1% of the active replicas move in a step, and warps
+// that share no counters need no barrier.  (Counters in shared memory cost
+// every block a clear, a flush and two barriers per task, and tied a block's
+// warps to one network and slice.)
 __device__ __forceinline__ void count_bits(unsigned long long *s_ev, int wl, uint32_t t,
                                            unsigned long long inc) {
   while (t) {
@@ -791,272 +712,296 @@ __device__ __forceinline__ void count_bits(unsigned long long *s_ev, int wl, uin
   }
 }
 
-// Applies one word's moves; returns the new planes and counts the events.
-// Per-replica event counters of a task slice in shared memory, two 32-bit
-// words per replica (32-bit shared atomics): c0 = S->E | ->I << 16,
-// c1 = I-> | R->S << 16 (a task has at most 4,096 rows).
-__device__ __forceinline__ void count_bits32(uint32_t *s_c, int wl, uint32_t t, uint32_t inc) {
-  while (t) {
-    const int r = __ffs(t) - 1;
-    atomicAdd(&s_c[wl * 32 + r], inc);
-    t &= t - 1;
-  }
-}
+struct FlowArgs {
+  uint32_t *evs, *mask, *sa, *sb;
+  uint32_t *actb, *infb, *susb, *evb;
+  unsigned long long *ev_row, *rs_row;
+  const int32_t *net_first;  // several networks: their first rows
+  int32_t n_nets;
+  uint32_t step;
+  int32_t split;             // a unit is 1 / (1 << split) of a bitmap word
+  int32_t take;              // units a warp takes at a time (at most 32)
+  int64_t n_units;
+};
 
-__device__ __forceinline__ void apply_word(uint32_t A, uint32_t B, uint32_t evS, uint32_t f,
-                                           bool waning, const StepConsts &c,
-                                           unsigned long long *s_ev, int wl, uint32_t &na,
-                                           uint32_t &nb) {
+// Applies one word's infection events and flows (disjoint state bits) to the
+// start-of-step planes, writes what changed and counts the events.
+__device__ __forceinline__ void apply_word(const PackedLayout &L, const FlowArgs &d,
+                                           const StepConsts &c, bool waning, int row, int word,
+                                           uint32_t A, uint32_t B, uint32_t evS, uint32_t f) {
   const uint32_t E = ~A & B, I = A & ~B, Rw = waning ? (A & B) : 0u;
   const uint32_t evE = f & E, evI = f & I, evR = f & Rw;
-  uint32_t xa = A, xb = B;
+  uint32_t all = evS | evE | evI | evR;
+  if (!all) return;
+  uint32_t na = A, nb = B;
   if (c.has_exposed)
-    xb |= evS;
+    nb |= evS;
   else
-    xa |= evS;
-  xa |= evE;
-  xb &= ~evE;
+    na |= evS;
+  na |= evE;
+  nb &= ~evE;
   if (c.ir_to_s)
-    xa &= ~evI;
+    na &= ~evI;
   else
-    xb |= evI;
-  xa &= ~evR;
-  xb &= ~evR;
-  na = xa;
-  nb = xb;
-  if (evS | evE | evI | evR) {
-    uint32_t *c0 = reinterpret_cast<uint32_t *>(s_ev), *c1 = c0 + 128 * 32;
-    count_bits32(c0, wl, c.has_exposed ? evS : 0u, 1u);
-    count_bits32(c0, wl, evE | (c.has_exposed ? 0u : evS), 1u << 16);
-    count_bits32(c1, wl, evI, 1u);
-    count_bits32(c1, wl, evR, 1u << 16);
+    nb |= evI;
+  na &= ~evR;
+  nb &= ~evR;
+  const int64_t wi = (int64_t)row * L.words + word;
+  d.sa[wi] = na;
+  d.sb[wi] = nb;
+  const uint32_t mk = na & ~nb;
+  if (mk != I) {
+    d.mask[wi] = mk;
+    if (!I) atomicOr(&d.infb[bit_word(L.lb, L.n_slices, row, word >> 2)], bit_of(L.lb, row, word >> 2));
+  }
+  int net = 0;
+  if (d.n_nets > 1) {  // the row's network: last first row <= row
+    int hi = d.n_nets;
+    while (hi - net > 1) {
+      const int mid = (net + hi) >> 1;
+      if (__ldg(d.net_first + mid) <= row) net = mid; else hi = mid;
+    }
+  }
+  const int64_t base = (int64_t)net * L.m + word * 32;
+  for (; all; all &= all - 1) {
+    const uint32_t bit = all & (0u - all);
+    const int64_t rep = base + __ffs(all) - 1;
+    if (evR & bit) {
+      atomicAdd(&d.rs_row[rep], 1ull);
+    } else {
+      const int field = (evI & bit) ? 2 * kFieldBits
+                                    : (((evE & bit) || !c.has_exposed) ? kFieldBits : 0);
+      atomicAdd(&d.ev_row[rep], 1ull << field);
+    }
   }
 }
 
-// Per-warp queue of words with flow candidates (dynamic shared memory):
-// words are queued while the warp streams its items and drawn in full
-// 32-lane rounds, so sparse candidates do not leave lanes idle.
-constexpr int kFlowIPL = 4;      // items per lane per pass (loads in flight)
-constexpr int kFlowQueue = 576;  // 31 left over + 4 words x kFlowIPL items x 32 lanes (+ pad)
+// Per-warp queue of words with flow candidates or infection events (dynamic
+// shared memory): words are queued while the warp streams its items and drawn
+// in full 32-lane rounds, so sparse candidates do not leave lanes idle.  An
+// entry carries its planes: read again from global memory they miss the
+// L1 that the passes of 24 warps stream through.
+constexpr int kFlowIPL = 2;      // items per lane per pass (loads in flight)
+constexpr int kFlowQueue = 31 + 4 * kFlowIPL * 32 + 1;  // left over + one pass
 struct FlowQueue {
-  int32_t row[kFlowQueue];
-  uint16_t word[kFlowQueue];  // word index within the row
-  int32_t n;
+  uint4 q[kFlowQueue];           // row, word (kWordEvent: infection events), planes a and b
+  uint4 q2[64];                  // words that the first draw left with candidates or events
+  uint32_t cand2[64];
+  uint32_t list[32 * kFlowIPL];  // items of the next pass (see k_flow)
 };
-constexpr int kFlowDynSmem = 128 * 32 * 8 + kWarps * (int)sizeof(FlowQueue);
+constexpr int kFlowDynSmem = kWarps * (int)sizeof(FlowQueue);
+constexpr uint32_t kWordEvent = 1u << 30;
 
-// Draws the flows of queue entries [0, cnt) (cnt <= 32, one per lane) and
-// writes the words: infection events and flows act on disjoint state bits,
-// so both are applied here from the start-of-step planes.
-__device__ __forceinline__ void flow_round(const FlowQueue &Q, int base, int cnt, int lane,
-                                           bool waning, const StepConsts &c, uint32_t step,
-                                           unsigned long long *s_ev, uint32_t *sa_w,
-                                           uint32_t *sb_w, uint32_t *mask_w, uint32_t *evs_w,
-                                           int words, int cbase) {
-  if (lane < cnt) {
-    const int q = base + lane;
-    const int row = Q.row[q], word = Q.word[q];
-    const int64_t wi = (int64_t)row * words + word;
-    const uint32_t A = sa_w[wi], B = sb_w[wi], ev = evs_w[wi];
-    if (ev) evs_w[wi] = 0u;
-    const uint32_t E = ~A & B, I = A & ~B, R = waning ? (A & B) : 0u;
-    const uint32_t f =
-        flow_events(E, I, R, c.th, c.rk, (uint32_t)row, step, (uint32_t)word + (c.roff >> 5));
-    uint32_t na, nb;
-    apply_word(A, B, ev, f, waning, c, s_ev, word - 4 * cbase, na, nb);
-    if (na != A || nb != B) {
-      sa_w[wi] = na;
-      sb_w[wi] = nb;
-      mask_w[wi] = na & ~nb;
-    }
-  }
-}
-
-// Streams the items of each task: infection events of words without flow
-// candidates are applied on the spot, words with candidates are queued.
+// Streams the active items (act | evb, 32 items per bitmap word), units of
+// the bitmap interleaved over all blocks and handed to a block's warps as they
+// ask; words with flow candidates or infection events are queued.
+// Loading an item also brings its act, inf and sus bits up to date with the
+// planes it found; moves made afterwards only set bits (inf, on a word's first
+// infectious replica), so a bit may stay set one step too long and is never
+// missing.
 __global__ void __launch_bounds__(kThreads, 3)
-    k_flow(PackedLayout L, const PackedTask *__restrict__ tasks,
-           const int32_t *__restrict__ row_ptr, uint4 *__restrict__ evs,
-           uint4 *__restrict__ mask, uint4 *__restrict__ sa, uint4 *__restrict__ sb,
-           uint8_t *__restrict__ flag, unsigned long long *__restrict__ ev_row,
-           unsigned long long *__restrict__ rs_row, uint32_t step, StepConsts c) {
+    k_flow(PackedLayout L, const __grid_constant__ FlowArgs d, const __grid_constant__ StepConsts c) {
   extern __shared__ __align__(16) unsigned char s_dynf[];
-  // 4 x 16-bit event counters per replica of the slice
-  unsigned long long *s_ev = reinterpret_cast<unsigned long long *>(s_dynf);
-  FlowQueue &Q = reinterpret_cast<FlowQueue *>(s_dynf + 128 * 32 * 8)[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  FlowQueue &Q = reinterpret_cast<FlowQueue *>(s_dynf)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   const bool waning = c.th.tr_all || c.th.tr != 0;
-  uint32_t *sa_w = reinterpret_cast<uint32_t *>(sa);
-  uint32_t *sb_w = reinterpret_cast<uint32_t *>(sb);
-  uint32_t *mask_w = reinterpret_cast<uint32_t *>(mask);
-  for (int ti = blockIdx.x; ti < L.n_tasks; ti += gridDim.x) {
-    const PackedTask T = tasks[ti];
-    const int cbase = T.slice * 32;
-    const int ncols = min(32, L.q4 - cbase);
-    const Div dv((uint32_t)ncols);
-    const int nrows = T.row_end - T.row_begin;
-    {  // the task's counters: two 32-bit words for each of its ncols x 128 replicas
-      uint32_t *c0 = reinterpret_cast<uint32_t *>(s_ev);
-      for (int j = threadIdx.x; j < ncols * 128; j += blockDim.x) {
-        c0[j] = 0;
-        c0[128 * 32 + j] = 0;
+  __shared__ unsigned s_next;  // the block's units, blockIdx.x + k gridDim.x, taken so far
+  if (threadIdx.x == 0) s_next = 0;
+  __syncthreads();
+  const uint4 *sa4 = reinterpret_cast<const uint4 *>(d.sa);
+  const uint4 *sb4 = reinterpret_cast<const uint4 *>(d.sb);
+  const uint4 *evs4 = reinterpret_cast<const uint4 *>(d.evs);
+  // the lane's unit of the current block: its bitmap word and bits
+  int64_t wi = 0;
+  bool more = true;
+  int wrow = 0, wcol = 0;     // first row and column of the lane's word
+  uint32_t aw = 0, ew = 0, iw = 0, sw = 0;
+  unsigned nz = 0;            // lanes with items not yet listed
+  int got = 0, n1 = 0, n2 = 0;  // items listed; words queued; words left by the first draw
+  const bool certain = c.th.te_all || c.th.ti_all || c.th.tr_all;
+  // warp-uniform passes of kFlowIPL items per lane, all loads issued first;
+  // candidate words are queued, and full rounds of 32 decided after the pass
+  // (one pass past the items decides the rest; one call site of the draws
+  // keeps the kernel small)
+  for (;;) {
+    while (!nz && !got && more) {
+      unsigned k = 0;
+      if (lane == 0) k = atomicAdd(&s_next, (unsigned)d.take);
+      k = __shfl_sync(kFull, k, 0);
+      more = blockIdx.x + (int64_t)(k + d.take) * gridDim.x < d.n_units;
+      const int64_t u = blockIdx.x + (int64_t)(k + lane) * gridDim.x;
+      aw = ew = 0;
+      if (lane < d.take && u < d.n_units) {
+        wi = u >> d.split;
+        const int len = 32 >> d.split;
+        const uint32_t own = (kFull >> (32 - len)) << (len * (int)(u & ((1 << d.split) - 1)));
+        aw = d.actb[wi] & own;
+        ew = d.evb[wi] & own;
+        if (aw | ew) {
+          iw = d.infb[wi];
+          sw = d.susb[wi];
+          const int64_t wr = L.n_slices == 1 ? wi : wi / L.n_slices;
+          wrow = (int)wr << (5 - L.lb);
+          wcol = (int)(wi - wr * L.n_slices) * 32;
+        }
+        if (ew) atomicAnd(&d.evb[wi], ~own);
+      }
+      // few items: every lane lists its own word's; else word by word below
+      int tot;
+      int pos = warp_excl_scan(__popc(aw | ew), lane, tot);
+      if (tot <= 32 * kFlowIPL) {
+        for (uint32_t t = aw | ew; t; t &= t - 1) {
+          const int b = __ffs(t) - 1;
+          Q.list[pos++] = (uint32_t)(lane << 5 | b) | ((aw >> b) & 1u) << 31 |
+                          ((ew >> b) & 1u) << 30 | ((iw >> b) & 1u) << 29 |
+                          ((sw >> b) & 1u) << 28;
+        }
+        got = tot;
+      } else {
+        nz = __ballot_sync(kFull, (aw | ew) != 0u);
       }
     }
-    if (lane == 0) Q.n = 0;
-    __syncthreads();
-    const int nitems = nrows * ncols;
-    uint32_t *evs_w = reinterpret_cast<uint32_t *>(evs);
-    // warp-uniform passes of kFlowIPL items per lane, all loads issued
-    // first; candidate words are queued, and full rounds of 32 decided after
-    // the pass (one pass past the items decides the rest; one call site of
-    // flow_round keeps the kernel small)
-    for (int it0 = warp * 32 * kFlowIPL;; it0 += kWarps * 32 * kFlowIPL) {
-      const bool flushing = it0 >= nitems;
-      int rl[kFlowIPL], cl[kFlowIPL];
-      bool in[kFlowIPL];
-      uint8_t st[kFlowIPL];
-      uint4 a4[kFlowIPL], b4[kFlowIPL];
+    while (nz && got <= 32 * (kFlowIPL - 1)) {
+      const int o = __ffs(nz) - 1;
+      nz &= nz - 1;
+      const uint32_t a = __shfl_sync(kFull, aw, o), e = __shfl_sync(kFull, ew, o);
+      const uint32_t i1 = __shfl_sync(kFull, iw, o), s1 = __shfl_sync(kFull, sw, o);
+      const uint32_t w = a | e;
+      if ((w >> lane) & 1u)
+        Q.list[got + __popc(w & ((1u << lane) - 1u))] =
+            (uint32_t)(o << 5 | lane) | ((a >> lane) & 1u) << 31 | ((e >> lane) & 1u) << 30 |
+            ((i1 >> lane) & 1u) << 29 | ((s1 >> lane) & 1u) << 28;
+      got += __popc(w);
+    }
+    __syncwarp();
+    const bool flushing = got == 0;
+    if (flushing && n1 == 0 && n2 == 0) break;
+    int rl[kFlowIPL], cl[kFlowIPL];
+    uint32_t st[kFlowIPL];
+    uint4 a4[kFlowIPL], b4[kFlowIPL];
 #pragma unroll
-      for (int h = 0; h < kFlowIPL; ++h) {
-        const int itv = it0 + 32 * h + lane;
-        in[h] = itv < nitems;
-        rl[h] = in[h] ? (int)dv.div((uint32_t)itv) : 0;
-        cl[h] = in[h] ? itv - rl[h] * ncols : 0;
-        const int64_t idx = (int64_t)(T.row_begin + rl[h]) * L.q4 + cbase + cl[h];
-        a4[h] = b4[h] = make_uint4(0, 0, 0, 0);
-        st[h] = 0;
-        if (in[h]) {
-          st[h] = flag[idx];
-          a4[h] = sa[idx];
-          b4[h] = sb[idx];
-        }
+    for (int h = 0; h < kFlowIPL; ++h) {
+      st[h] = 0;
+      rl[h] = cl[h] = 0;
+      a4[h] = b4[h] = make_uint4(0, 0, 0, 0);
+      if (32 * h >= got) continue;  // warp-uniform, as below
+      const bool in = 32 * h + lane < got;
+      if (in) st[h] = Q.list[32 * h + lane];
+      const int o = (st[h] >> 5) & 31, bit = st[h] & 31;
+      rl[h] = __shfl_sync(kFull, wrow, o) + (bit >> L.lb);
+      cl[h] = __shfl_sync(kFull, wcol, o) + (bit & ((1 << L.lb) - 1));
+      if (in) {
+        const int64_t idx = (int64_t)rl[h] * L.q4 + cl[h];
+        a4[h] = sa4[idx];
+        b4[h] = sb4[idx];
       }
-      // quiet items (every replica susceptible, or recovered without waning,
-      // and no infection event) need no work: skip them a warp at a time
-      bool busy = false;
-      uint32_t cm[kFlowIPL];
-      int cnt = 0;
+    }
 #pragma unroll
-      for (int h = 0; h < kFlowIPL; ++h) {
-        cm[h] = 0;
+    for (int h = 0; h < kFlowIPL; ++h) {
+      if (32 * h >= got) continue;
+      uint32_t cm = 0, evm = 0, s4 = 0, i4 = 0, r4 = 0;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {  // padding replicas are S: no replica mask needed
-          const uint32_t A = get4(a4[h], w), B = get4(b4[h], w);
-          if ((waning ? (A | B) : (A ^ B)) != 0u) cm[h] |= 1u << w;
+      for (int w = 0; w < 4; ++w) {  // padding replicas are S: no replica mask needed
+        const uint32_t A = get4(a4[h], w), B = get4(b4[h], w);
+        if ((waning ? (A | B) : (A ^ B)) != 0u) cm |= 1u << w;
+        i4 |= A & ~B;
+        r4 |= A & B;
+        // padding replicas are S, so only a row's last item needs the mask
+        const uint32_t S = ~(A | B);
+        s4 |= 4 * cl[h] + 4 > L.vwords ? S & word_mask(L, 4 * cl[h] + w) : S;
+      }
+      // S now, or back to S this step (waning R, or I -> S)
+      if (waning) s4 |= r4;
+      if (c.ir_to_s) s4 |= i4;
+      // words with infection events join the queue (they need no draw)
+      if ((st[h] >> 30) & 1u) {
+        const uint4 e4 = evs4[(int64_t)rl[h] * L.q4 + cl[h]];
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+          if (get4(e4, w)) evm |= 1u << w;
+        cm |= evm;
+      }
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const unsigned qm = __ballot_sync(kFull, (cm >> w) & 1u);
+        if (!qm) continue;
+        if ((cm >> w) & 1u)
+          Q.q[n1 + __popc(qm & ((1u << lane) - 1u))] =
+              make_uint4((uint32_t)rl[h],
+                         (uint32_t)(4 * cl[h] + w) | ((evm >> w) & 1u ? kWordEvent : 0u),
+                         get4(a4[h], w), get4(b4[h], w));
+        n1 += __popc(qm);
+      }
+      const uint32_t now = (cm ? 8u : 0u) | ((st[h] >> 28) & 4u) |
+                           (i4 ? 2u : 0u) | (s4 ? 1u : 0u);
+      const uint32_t diff = st[h] >> 28 ? now ^ (st[h] >> 28) : 0u;  // the list entry is in use
+      if (diff) {
+        const int64_t bw = bit_word(L.lb, L.n_slices, rl[h], cl[h]);
+        const uint32_t bit = bit_of(L.lb, rl[h], cl[h]);
+        if (diff & 8u) atomicXor(&d.actb[bw], bit);
+        if (diff & 2u) atomicXor(&d.infb[bw], bit);
+        if (diff & 1u) atomicXor(&d.susb[bw], bit);
+      }
+    }
+    got = 0;
+    __syncwarp();  // bits are cleared before a round of this warp may set them
+    // Two rounds of draws, 32 words each.  With every rate below 1/16 the first
+    // draw (planes 0-3) leaves one candidate in 16, and a word without any and
+    // without infection events is done: no second draw, no write.  The words
+    // left are collected again, so that the second round's lanes are full too.
+    for (;;) {
+      const bool first = n1 >= 32 || (flushing && n1 > 0);
+      if (first) {
+        const int take = min(n1, 32);
+        n1 -= take;
+        uint4 q = make_uint4(0, 0, 0, 0);
+        bool keep = false;
+        uint32_t cand = 0;
+        if (lane < take) {
+          q = Q.q[n1 + lane];
+          cand = flow_candidates(~q.z & q.w, q.z & ~q.w, waning ? (q.z & q.w) : 0u, c.th);
+          if (c.th.small && cand)
+            cand = flow_top(cand, c.rk, q.x, d.step, (q.y & ~kWordEvent) + (c.roff >> 5));
+          keep = cand || q.y >= kWordEvent || certain;
         }
-        cnt += __popc(cm[h]);
-        busy |= (st[h] & kFlagEvent) != 0 || cm[h] != 0;
-        // next step's hint byte, from this step's planes and events: a
-        // superset of the items with susceptible replicas (and of those
-        // that can move: E, I, waning R, or newly infected)
-        if (c.hints && in[h]) {
-          // E, I or waning R (the words of cm), or an infection event
-          const bool act = (st[h] & kFlagEvent) != 0 || cm[h] != 0u;
-          uint32_t s4 = 0;
-#pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            const uint32_t A = get4(a4[h], w), B = get4(b4[h], w);
-            // S now, or back to S this step (waning R, or I -> S); padding
-            // replicas are S, so only a row's last item needs the mask
-            uint32_t sw = (~A & ~B) | (waning ? (A & B) : 0u) | (c.ir_to_s ? (A & ~B) : 0u);
-            if (4 * (cbase + cl[h]) + 4 > L.vwords) sw &= word_mask(L, 4 * (cbase + cl[h]) + w);
-            s4 |= sw;
+        const unsigned km = __ballot_sync(kFull, keep);
+        if (keep) {
+          const int at = n2 + __popc(km & ((1u << lane) - 1u));
+          Q.q2[at] = q;
+          Q.cand2[at] = cand;
+        }
+        n2 += __popc(km);
+        __syncwarp();
+      }
+      if (n2 >= 32 || (flushing && !first && n2 > 0)) {
+        const int take = min(n2, 32);
+        n2 -= take;
+        if (lane < take) {
+          const uint4 q = Q.q2[n2 + lane];
+          const uint32_t cand = Q.cand2[n2 + lane], A = q.z, B = q.w;
+          const int row = (int)q.x, word = (int)(q.y & ~kWordEvent);
+          uint32_t ev = 0;
+          if (q.y >= kWordEvent) {
+            const int64_t qi = (int64_t)row * L.words + word;
+            ev = d.evs[qi];
+            d.evs[qi] = 0u;
           }
-          const uint8_t nb = (uint8_t)((act ? kFlagActive : 0) | (s4 ? kFlagSusceptible : 0));
-          if (nb != st[h]) flag[(int64_t)(T.row_begin + rl[h]) * L.q4 + cbase + cl[h]] = nb;
-        }
-      }
-      if (!flushing && !__any_sync(kFull, busy)) continue;
-      // infection events: words without flow candidates are applied here;
-      // the queued words' events are read (and cleared) by their round
-#pragma unroll
-      for (int h = 0; h < kFlowIPL; ++h) {
-        if (!(st[h] & kFlagEvent)) continue;
-        const int64_t idx = (int64_t)(T.row_begin + rl[h]) * L.q4 + cbase + cl[h];
-        const uint4 e4 = evs[idx];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const uint32_t ev = get4(e4, w);
-          if (!ev || ((cm[h] >> w) & 1u)) continue;
-          const int word = 4 * (cbase + cl[h]) + w;
-          const int64_t wi = (int64_t)(T.row_begin + rl[h]) * L.words + word;
-          uint32_t na, nb;
-          apply_word(get4(a4[h], w), get4(b4[h], w), ev, 0u, waning, c, s_ev, 4 * cl[h] + w, na,
-                     nb);
-          sa_w[wi] = na;
-          sb_w[wi] = nb;
-          mask_w[wi] = na & ~nb;
-          evs_w[wi] = 0u;
-        }
-      }
-      // queue the candidate words of the pass (one scan)
-      int total;
-      int pos = warp_excl_scan(cnt, lane, total);
-      if (total > 0) {  // warp-uniform
-        pos += Q.n;
-        // one iteration per candidate word of the lane (most lanes have none)
-        uint32_t all = 0;
-#pragma unroll
-        for (int h = 0; h < kFlowIPL; ++h) all |= cm[h] << (4 * h);
-        while (all) {
-          const int bit = __ffs(all) - 1;
-          all &= all - 1;
-          const int h = bit >> 2;
-          int r = rl[0], cc = cl[0];
-#pragma unroll
-          for (int hh = 1; hh < kFlowIPL; ++hh)
-            if (h == hh) {
-              r = rl[hh];
-              cc = cl[hh];
-            }
-          Q.row[pos] = T.row_begin + r;
-          Q.word[pos] = (uint16_t)(4 * (cbase + cc) + (bit & 3));
-          ++pos;
+          const uint32_t E = ~A & B, I = A & ~B, R = waning ? (A & B) : 0u;
+          uint32_t f = certain ? flow_sure(E, I, R, c.th) : 0u;
+          if (cand)
+            f |= flow_rest(cand, E, I, R, c.th, c.rk, (uint32_t)row, d.step,
+                           (uint32_t)word + (c.roff >> 5));
+          apply_word(L, d, c, waning, row, word, A, B, ev, f);
         }
         __syncwarp();
+      } else if (!first) {
+        break;
       }
-      const int n = Q.n + total;
-      int start = 0;
-      for (; n - start >= 32 || (flushing && n - start > 0); start += 32)
-        flow_round(Q, start, min(32, n - start), lane, waning, c, step, s_ev, sa_w, sb_w, mask_w,
-                   evs_w, L.words, cbase);
-      __syncwarp();
-      const int rest = max(n - start, 0);
-      if (start > 0 && rest > 0) {  // move the remainder (< 32 words) to the front
-        const int q = start + lane;
-        int32_t r0 = 0;
-        uint16_t w0 = 0;
-        if (lane < rest) {
-          r0 = Q.row[q];
-          w0 = Q.word[q];
-        }
-        __syncwarp();
-        if (lane < rest) {
-          Q.row[lane] = r0;
-          Q.word[lane] = w0;
-        }
-      }
-      __syncwarp();
-      if (lane == 0) Q.n = rest;
-      __syncwarp();
-      if (flushing) break;
     }
-    __syncthreads();
-    for (int j = threadIdx.x; j < ncols * 128; j += blockDim.x) {
-      const uint32_t *c0 = reinterpret_cast<const uint32_t *>(s_ev), *c1 = c0 + 128 * 32;
-      const unsigned long long v = (unsigned long long)c0[j] | ((unsigned long long)c1[j] << 32);
-      if (!v) continue;
-      const int rep = cbase * 128 + j;
-      if (rep >= L.m) continue;
-      const unsigned long long f16 = 0xFFFFull;
-      const unsigned long long g = (v & f16) | (((v >> 16) & f16) << kFieldBits) |
-                                   (((v >> 32) & f16) << (2 * kFieldBits));
-      if (g) atomicAdd(&ev_row[T.count_base + rep], g);
-      if (rs_row && (v >> 48)) atomicAdd(&rs_row[T.count_base + rep], v >> 48);
-    }
-    __syncthreads();
+    if (flushing) break;
   }
 }
+
 // Full E/I/R counts of the planes (initial state): one shared atomic per
 // set bit, E | I << 21 | R << 42 per replica.
 __global__ void __launch_bounds__(kThreads)
@@ -1152,24 +1097,37 @@ __global__ void k_mask_from_planes(int64_t total, const uint32_t *__restrict__ s
     mask[i] = sa[i] & ~sb[i];
 }
 
-// Hint bytes of every item from the initial planes (kFlagActive: E, I or
-// waning R replicas; kFlagSusceptible: S replicas).
-__global__ void k_flag_from_planes(PackedLayout L, const uint4 *__restrict__ sa,
-                                   const uint4 *__restrict__ sb, uint8_t *__restrict__ flag,
-                                   bool waning) {
-  const int64_t total = (int64_t)L.n_nodes * L.q4;
+// The bitmaps from the initial planes: one thread per bit.
+__global__ void __launch_bounds__(256)
+    k_bits_from_planes(PackedLayout L, const uint4 *__restrict__ sa, const uint4 *__restrict__ sb,
+                       uint32_t *__restrict__ actb, uint32_t *__restrict__ infb,
+                       uint32_t *__restrict__ susb, uint32_t *__restrict__ evb, bool waning) {
+  const int64_t total = L.bit_words * 32;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const uint4 a4 = sa[i], b4 = sb[i];
-    const int col = (int)(i % L.q4);
-    bool act = false, sus = false;
+    const int64_t wi = i >> 5;
+    const int bit = (int)(i & 31), slice = (int)(wi % L.n_slices);
+    const int64_t row = ((wi / L.n_slices) << (5 - L.lb)) + (bit >> L.lb);
+    const int col = slice * 32 + (bit & ((1 << L.lb) - 1));
+    bool act = false, inf = false, sus = false;
+    if (row < L.n_nodes && col < L.q4) {
+      const uint4 a4 = sa[row * L.q4 + col], b4 = sb[row * L.q4 + col];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const uint32_t A = get4(a4, w), B = get4(b4, w), vm = word_mask(L, 4 * col + w);
-      act |= (((A ^ B) | (waning ? (A & B) : 0u)) & vm) != 0u;
-      sus |= ((~A & ~B) & vm) != 0u;
+      for (int w = 0; w < 4; ++w) {
+        const uint32_t A = get4(a4, w), B = get4(b4, w), vm = word_mask(L, 4 * col + w);
+        act |= (((A ^ B) | (waning ? (A & B) : 0u)) & vm) != 0u;
+        inf |= (A & ~B & vm) != 0u;
+        sus |= ((~A & ~B) & vm) != 0u;
+      }
     }
-    flag[i] = (uint8_t)((act ? kFlagActive : 0) | (sus ? kFlagSusceptible : 0));
+    const uint32_t a = __ballot_sync(kFull, act), f = __ballot_sync(kFull, inf),
+                   s = __ballot_sync(kFull, sus);
+    if ((i & 31) == 0) {
+      actb[wi] = a;
+      infb[wi] = f;
+      susb[wi] = s;
+      evb[wi] = 0u;
+    }
   }
 }
 
@@ -1246,17 +1204,16 @@ int task_grid(int n_tasks, int per_sm) {
 }  // namespace
 
 rp_status packed_prepare() {
-  cudaError_t e = cudaFuncSetAttribute(k_flow, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kFlowDynSmem);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_flow)");
-  e = cudaFuncSetAttribute(k_infect, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kInfectDynSmemMax);
+  cudaError_t e = cudaFuncSetAttribute(k_infect, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kInfectDynSmem);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_infect)");
+  e = cudaFuncSetAttribute(k_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlowDynSmem);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_flow)");
   return RP_OK;
 }
 
 void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb, uint32_t *mask,
-                 uint8_t *flag, float p0, int32_t k_exact, const int32_t *net_first_row,
+                 uint32_t *bits, float p0, int32_t k_exact, const int32_t *net_first_row,
                  const int32_t *net_rows, int32_t n_nets, const StepConsts &c,
                  cudaStream_t st) {
   const int64_t total = (int64_t)L.n_nodes * L.words;
@@ -1267,38 +1224,80 @@ void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb, uint32_t *ma
                                                                 n_nets, k_exact, c);
     k_mask_from_planes<<<1184, 256, 0, st>>>(total, sa, sb, mask);
   }
-  cudaMemsetAsync(flag, 0, ((size_t)L.n_nodes * L.q4 + 3) / 4 * 4, st);
-  k_flag_from_planes<<<1184, 256, 0, st>>>(L, reinterpret_cast<const uint4 *>(sa),
-                                           reinterpret_cast<const uint4 *>(sb), flag,
-                                           c.th.tr_all || c.th.tr != 0);
+  if (bits)
+    k_bits_from_planes<<<1184, 256, 0, st>>>(
+        L, reinterpret_cast<const uint4 *>(sa), reinterpret_cast<const uint4 *>(sb), bits,
+        bits + L.bit_words, bits + 2 * L.bit_words, bits + 3 * L.bit_words,
+        c.th.tr_all || c.th.tr != 0);
 }
 
-void packed_step(const PackedLayout &L, const PackedTask *tasks, const int32_t *row_ptr,
-                 const int2 *entries, uint32_t *mask, uint32_t *sa, uint32_t *sb, uint32_t *evs,
-                 uint8_t *flag, unsigned long long *ev_row, unsigned long long *rs_row,
-                 uint32_t step, float scale, const StepConsts &c, cudaStream_t st) {
-  packed_infect(L, tasks, row_ptr, entries, mask, sa, sb, evs, flag, step, scale, c, st);
-  packed_flow(L, tasks, row_ptr, mask, sa, sb, evs, flag, ev_row, rs_row, step, c, st);
+// Blocks for `units` warp-sized units: one warp each over all SMs first, then
+// up to the three resident blocks of each SM.
+static int unit_grid(int64_t units) {
+  return (int)(units < 1 ? 1 : (units < 148 * 3 ? units : 148 * 3));
 }
 
-void packed_infect(const PackedLayout &L, const PackedTask *tasks, const int32_t *row_ptr,
-                   const int2 *entries, const uint32_t *mask, const uint32_t *sa,
-                   const uint32_t *sb, uint32_t *evs, uint8_t *flag, uint32_t step, float scale,
+void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
+                   const HeavyRows &heavy, const uint32_t *mask, const uint32_t *sa,
+                   const uint32_t *sb, uint32_t *evs, uint32_t *bits, uint32_t step, float scale,
                    const StepConsts &c, cudaStream_t st) {
-  k_infect<<<task_grid(L.n_tasks, 3), kThreads, infect_smem(L.q4, L.max_task_rows), st>>>(
-      L, tasks, row_ptr, entries, reinterpret_cast<const uint4 *>(mask),
-      reinterpret_cast<const uint4 *>(sa), reinterpret_cast<const uint4 *>(sb),
-      reinterpret_cast<uint4 *>(evs), reinterpret_cast<uint32_t *>(flag), step, scale, c);
+  InfectArgs d{};
+  d.row_ptr = row_ptr;
+  d.ent = entries;
+  d.mask = mask;
+  d.sa = sa;
+  d.sb = sb;
+  d.evs = evs;
+  d.infb = bits + L.bit_words;
+  d.susb = bits + 2 * L.bit_words;
+  d.evb = bits + 3 * L.bit_words;
+  d.heavy = heavy.rows;
+  d.heavy_end = heavy.end;
+  d.n_heavy = heavy.counts;
+  d.step = step;
+  d.scale = scale;
+  // 8 rows per unit, so that a block's warps end together; fewer (down to 8
+  // items, one round of words) where blocks would have none, more where every
+  // warp has many: a unit's row pointers are loaded together, and sparse rows
+  // fold into batches of 32
+  d.unit_rows = 8;
+  const int64_t warps = 148 * 3 * kWarps;
+  auto units = [&](int rows) { return (int64_t)((L.n_nodes + rows - 1) / rows) * L.n_slices; };
+  while (d.unit_rows > 1 && units(d.unit_rows) * 2 < warps && (int64_t)d.unit_rows * L.q4 > 8)
+    d.unit_rows >>= 1;
+  while (d.unit_rows < kUnitRows && (units(2 * d.unit_rows) >= 4 * warps ||
+                                     (int64_t)d.unit_rows * L.q4 < 8))
+    d.unit_rows *= 2;
+  d.n_units = (int32_t)units(d.unit_rows);
+  k_infect<<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
 }
 
-void packed_flow(const PackedLayout &L, const PackedTask *tasks, const int32_t *row_ptr,
-                 uint32_t *mask, uint32_t *sa, uint32_t *sb, const uint32_t *evs, uint8_t *flag,
-                 unsigned long long *ev_row, unsigned long long *rs_row, uint32_t step,
-                 const StepConsts &c, cudaStream_t st) {
-  k_flow<<<task_grid(L.n_tasks, 3), kThreads, kFlowDynSmem, st>>>(
-      L, tasks, row_ptr, reinterpret_cast<uint4 *>(const_cast<uint32_t *>(evs)),
-      reinterpret_cast<uint4 *>(mask), reinterpret_cast<uint4 *>(sa),
-      reinterpret_cast<uint4 *>(sb), flag, ev_row, rs_row, step, c);
+void packed_flow(const PackedLayout &L, uint32_t *mask, uint32_t *sa, uint32_t *sb, uint32_t *evs,
+                 uint32_t *bits, unsigned long long *ev_row, unsigned long long *rs_row,
+                 const int32_t *net_first, int32_t n_nets, uint32_t step, const StepConsts &c,
+                 cudaStream_t st) {
+  FlowArgs d{};
+  d.evs = evs;
+  d.mask = mask;
+  d.sa = sa;
+  d.sb = sb;
+  d.actb = bits;
+  d.infb = bits + L.bit_words;
+  d.susb = bits + 2 * L.bit_words;
+  d.evb = bits + 3 * L.bit_words;
+  d.ev_row = ev_row;
+  d.rs_row = rs_row;
+  d.net_first = net_first;
+  d.n_nets = n_nets;
+  d.step = step;
+  // a small bitmap is cut finer: 8 items of 128 replicas are one full round
+  d.split = 0;
+  while (d.split < 2 && (L.bit_words << (d.split + 1)) <= 148 * 3 * kWarps) ++d.split;
+  d.n_units = L.bit_words << d.split;
+  // units of a warp's block: up to 32, fewer so that a block's warps end together
+  d.take = 1;
+  while (d.take < 32 && d.n_units > (int64_t)148 * 3 * kWarps * 4 * d.take) d.take *= 2;
+  k_flow<<<unit_grid(d.n_units), kThreads, kFlowDynSmem, st>>>(L, d, c);
 }
 
 void packed_count(const PackedLayout &L, const PackedTask *tasks, const uint32_t *sa,

@@ -151,46 +151,83 @@ __device__ __forceinline__ float one_minus_exp_neg(float x) {
 // floor(p 2^64); p >= 1 is a certain event, p <= 0 none.
 // Flow events of the replicas selected by E, I, R (disjoint masks of one
 // 32-replica word of `node`): replica r moves iff its bit-sliced uniform is
-// below its state's threshold.  All 32 replicas are compared at once, one
-// random plane per bit, stopping when every candidate is decided (about
-// log2(candidates) + 2 planes).  Returns the event mask.
+// below its state's threshold.  All 32 replicas are compared at once; the
+// first 8 planes decide all but 1 in 256 candidates, further planes are drawn
+// only while some replica is undecided.  Returns the event mask.
+//
+// The 8-plane comparison runs from the least significant plane up, with one
+// majority per plane: `less` keeps its value where uniform and threshold bits
+// agree and becomes the threshold's bit where they differ, which is
+// maj(~u, less, t).  The thresholds' bits come as masks from the constant bank
+// (FlowThresholds); taken bit by bit from the 64-bit thresholds they cost more
+// instructions than the two Philox calls.
+__device__ __forceinline__ uint32_t maj_not(uint32_t u, uint32_t less, uint32_t t) {
+  return (~u & (less | t)) | (less & t);
+}
+// Replicas whose threshold is 1 (they move without a draw).
+__device__ __forceinline__ uint32_t flow_sure(uint32_t E, uint32_t I, uint32_t R,
+                                              const FlowThresholds &th) {
+  return (th.te_all ? E : 0u) | (th.ti_all ? I : 0u) | (th.tr_all ? R : 0u);
+}
+// Planes 0-3 where every threshold is below 1/16 (th.small): the replicas of
+// `cand` whose top four uniform bits are 0; the others do not move.
+__device__ __forceinline__ uint32_t flow_top(uint32_t cand, const uint32_t *rk, uint32_t node,
+                                             uint32_t step, uint32_t word) {
+  uint32_t x[4];
+  philox4x32_10_rk(node, step, word, 0u, rk, x);
+  return cand & ~(x[0] | x[1] | x[2] | x[3]);
+}
+// Events among the candidates `cand` (those flow_top left, with th.small).
+__device__ __forceinline__ uint32_t flow_rest(uint32_t cand, uint32_t E, uint32_t I, uint32_t R,
+                                              const FlowThresholds &th, const uint32_t *rk,
+                                              uint32_t node, uint32_t step, uint32_t word) {
+  const uint32_t e2 = E & cand, i2 = I & cand, r2 = R & cand;
+  uint32_t x[4], less = 0, same = cand;
+  philox4x32_10_rk(node, step, word, 1u << 4, rk, x);
+#pragma unroll
+  for (int k = 7; k >= 4; --k) {
+    const uint32_t t = (e2 & th.me[k]) | (i2 & th.mi[k]) | (r2 & th.mr[k]);
+    less = maj_not(x[k - 4], less, t);
+    same &= ~(t ^ x[k - 4]);
+  }
+  if (!th.small) {
+    philox4x32_10_rk(node, step, word, 0u, rk, x);
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+      const uint32_t t = (e2 & th.me[k]) | (i2 & th.mi[k]) | (r2 & th.mr[k]);
+      less = maj_not(x[k], less, t);
+      same &= ~(t ^ x[k]);
+    }
+  }
+  uint32_t lt = less & cand;
+#pragma unroll 1
+  for (int j = 2; j < 16 && same != 0u; ++j) {
+    philox4x32_10_rk(node, step, word, (uint32_t)j << 4, rk, x);
+    const int sh = 60 - 4 * j;
+    const uint32_t ce = (uint32_t)(th.te >> sh), ci = (uint32_t)(th.ti >> sh),
+                   cr = (uint32_t)(th.tr >> sh);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t t = (((ce >> (3 - q)) & 1u) ? e2 : 0u) | (((ci >> (3 - q)) & 1u) ? i2 : 0u) |
+                         (((cr >> (3 - q)) & 1u) ? r2 : 0u);
+      lt |= same & t & ~x[q];
+      same &= ~(t ^ x[q]);
+    }
+  }
+  return lt;
+}
+// Candidates of a word: those whose threshold is neither 0 nor 1.
+__device__ __forceinline__ uint32_t flow_candidates(uint32_t E, uint32_t I, uint32_t R,
+                                                    const FlowThresholds &th) {
+  return (th.te == 0 ? 0u : E) | (th.ti == 0 ? 0u : I) | (th.tr == 0 ? 0u : R);
+}
 __device__ __forceinline__ uint32_t flow_events(uint32_t E, uint32_t I, uint32_t R,
                                                 const FlowThresholds &th, const uint32_t *rk,
                                                 uint32_t node, uint32_t step, uint32_t word) {
-  uint32_t lt = (th.te_all ? E : 0u) | (th.ti_all ? I : 0u) | (th.tr_all ? R : 0u);
-  const uint32_t e2 = (th.te_all || th.te == 0) ? 0u : E;
-  const uint32_t i2 = (th.ti_all || th.ti == 0) ? 0u : I;
-  const uint32_t r2 = (th.tr_all || th.tr == 0) ? 0u : R;
-  uint32_t und = e2 | i2 | r2;
-  if (und == 0u) return lt;  // every candidate's threshold is 0 or 1: no draw
-  // one random call decides 4 planes for all 32 replicas of the word
-  auto planes = [&](const uint32_t (&x)[4], int j) {
-    const int sh = 60 - 4 * j;
-    const uint32_t ce = (uint32_t)(th.te >> sh) & 0xFu;
-    const uint32_t ci = (uint32_t)(th.ti >> sh) & 0xFu;
-    const uint32_t cr = (uint32_t)(th.tr >> sh) & 0xFu;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint32_t b = 3 - q;
-      const uint32_t T = (((ce >> b) & 1u) ? e2 : 0u) | (((ci >> b) & 1u) ? i2 : 0u) |
-                         (((cr >> b) & 1u) ? r2 : 0u);
-      const uint32_t w = x[q];
-      lt |= und & T & ~w;
-      und &= ~(T ^ w);
-    }
-  };
-  // the first two calls (8 planes) run together, unconditionally; later
-  // planes only while some replica is undecided
-  uint32_t x0[4], x1[4];
-  philox4x32_10_rk_x2(node, step, word, 0u, 1u << 4, rk, x0, x1);
-  planes(x0, 0);
-  planes(x1, 1);
-  for (int j = 2; j < 16 && und != 0u; ++j) {
-    uint32_t x[4];
-    philox4x32_10_rk(node, step, word, (uint32_t)j << 4, rk, x);
-    planes(x, j);
-  }
-  return lt;
+  uint32_t cand = flow_candidates(E, I, R, th);
+  const uint32_t sure = flow_sure(E, I, R, th);
+  if (cand && th.small) cand = flow_top(cand, rk, node, step, word);
+  return cand ? sure | flow_rest(cand, E, I, R, th, rk, node, step, word) : sure;
 }
 
 // floor(p 2^64) for 0 < p < 1 (exact: p 2^64 is exact in float, then
@@ -219,7 +256,7 @@ __device__ __forceinline__ void infect_planes(const uint32_t *rk, uint32_t node,
 __device__ __forceinline__ uint32_t top8_of(const uint32_t pl[8], uint32_t b) {
   uint32_t u = 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) u = (u << 1) | ((pl[k] >> b) & 1u);
+  for (int k = 0; k < 8; ++k) u = __funnelshift_l(pl[k] << (31u - b), u, 1);
   return u;
 }
 
@@ -228,14 +265,11 @@ __device__ __forceinline__ uint32_t top8_of(const uint32_t pl[8], uint32_t b) {
 __device__ __forceinline__ uint32_t top8_le(uint32_t cand, unsigned long long T,
                                             const uint32_t pl[8]) {
   const uint32_t t8 = (uint32_t)(T >> 56);
-  uint32_t lt = 0, und = cand;
+  uint32_t le = 0xFFFFFFFFu;  // equal bits below: at most
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const uint32_t t = ((t8 >> (7 - k)) & 1u) ? 0xFFFFFFFFu : 0u;
-    lt |= und & t & ~pl[k];
-    und &= ~(t ^ pl[k]);
-  }
-  return lt | und;
+  for (int k = 7; k >= 0; --k)
+    le = maj_not(pl[k], le, (uint32_t)((int32_t)(t8 << (24 + k)) >> 31));
+  return cand & le;
 }
 
 // Low 56 bits of the infection uniform of (global) replica `replica`.

@@ -15,6 +15,8 @@ namespace rp {
 struct FlowThresholds {
   unsigned long long te, ti, tr;
   int te_all, ti_all, tr_all;
+  int small;                     // every threshold's top four bits are 0
+  uint32_t me[8], mi[8], mr[8];  // their top 8 bits as masks, most significant first
 };
 
 // ---- errors ---------------------------------------------------------------
@@ -239,6 +241,15 @@ struct Hit {
   int32_t w;     // int32 seconds or float bits
 };
 
+// Rows with many pairs, listed while a window's row pointers are written:
+// rows of more than kHeavyPairs pairs from the front of the list, of more than
+// kHugePairs pairs from its end; counts[0] and counts[2] of them.
+constexpr int32_t kHeavyPairs = 32, kHugePairs = 512;
+struct HeavyRows {
+  const int32_t *rows, *end;
+  const unsigned long long *counts;
+};
+
 struct WindowWorkspace {
   int32_t n_nodes = 0;
   int64_t cap_hits = 0, cap_entries = 0;
@@ -252,8 +263,8 @@ struct WindowWorkspace {
   DevBuf row_ptr;   // int32[G][n+1]
   DevBuf deg;       // int32[G][n] degree, then fill cursor
   DevBuf tiles;     // int32[G][n_tiles]
-  DevBuf counters;  // u64[G][4]: spare, long rows, spare, predicate hits
-  DevBuf long_rows; // int32[G][n]
+  DevBuf counters;  // u64[G][4]: heavy rows, long rows, huge rows, predicate hits
+  DevBuf long_rows; // int32[G][n]: heavy rows (unsorted rows) or rows to sort in a block
   DevBuf win;       // WinDesc[n_windows]
   DevBuf ranges;    // CandRange[...]
 };
@@ -302,9 +313,12 @@ enum WeightKind { kWeightF32 = 0, kWeightI32 = 1 };
 int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup &grp, int64_t cap,
                          int weight_kind, bool sort_rows, cudaStream_t st);
 // Compacts the sorted, merged CSR in ws (slot 0) into (row_ptr_out, entries_out):
-// drops merged-away entries.  tmp_rows: int32[n+1] scratch.
-void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out,
-                            int2 *entries_out, cudaStream_t st);
+// drops merged-away entries.  With `heavy` (a list of heavy_cap rows) the rows
+// with many pairs are listed, their counts (4 words, zeroed by the caller) in
+// heavy_counts.
+void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out, int2 *entries_out,
+                            cudaStream_t st, int32_t *heavy = nullptr, int64_t heavy_cap = 0,
+                            unsigned long long *heavy_counts = nullptr);
 
 // ---- kernels of the step loop -------------------------------------------------
 struct StepConsts {
@@ -318,10 +332,9 @@ struct StepConsts {
   int32_t has_exposed, ir_to_s;
   float beta;
   const float *beta_r;  // device, may be null
+  const float *beta_word;  // device, with beta_r: max |beta_r| of each 32-replica word
   const float *sus;     // device, may be null
   uint32_t roff;        // replica offset of the stream layout (multiple of 32)
-  int32_t *err;         // device flag set by a kernel that gave up a bounded wait
-  int32_t hints;        // batched path: keep and use the per-item hint bytes
 };
 
 // Plain path (column-major N x M state, per-replica SpMV + elementwise).
@@ -345,9 +358,7 @@ struct PackedTask {
   int32_t row_begin, row_end;  // rows of one network
   int32_t slice;               // 32 four-word columns (128 words) per slice
   int32_t count_base;          // index of replica 0 of this network in counts
-  int32_t stage;               // k_infect: CSR pairs staged per chunk (<= 768)
 };
-constexpr int32_t kStageDefault = 768;  // k_infect's staging buffer, in pairs
 struct PackedLayout {
   int32_t n_nodes;
   int32_t words;      // words per node row, padded to a multiple of 4
@@ -355,27 +366,30 @@ struct PackedLayout {
   int32_t q4;         // four-word columns per row (words / 4)
   int32_t m;          // replicas per network
   uint32_t last_mask; // valid bits of word vwords - 1
-  int32_t lpr;        // lanes per row (power of 2, <= 32)
+  int32_t lb;         // bitmap bits per row: 1 << lb, the power of 2 >= min(q4, 32)
+  int32_t n_slices;   // slices of 32 four-word columns
+  int64_t bit_words;  // words of one item bitmap (packed.cu)
   int32_t n_tasks;
-  int32_t max_task_rows;  // rows of the tallest task
 };
 rp_status packed_prepare();  // kernel attributes, once per device
+// `bits`: the four item bitmaps (act, inf, sus, evb), or null (countdown mode).
+// `bits`: the four item bitmaps (act, inf, sus, evb), or null (countdown mode).
 void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb,
-                 uint32_t *mask, uint8_t *flag, float p0, int32_t k_exact,
+                 uint32_t *mask, uint32_t *bits, float p0, int32_t k_exact,
                  const int32_t *net_first_row, const int32_t *net_rows,
                  int32_t n_nets, const StepConsts &c, cudaStream_t st);
 // One step: exposure + infection draws (k_infect), then transitions, counts
 // and the next infectious mask (k_flow).
-void packed_infect(const PackedLayout &L, const PackedTask *tasks,
-                   const int32_t *row_ptr, const int2 *entries,
-                   const uint32_t *mask, const uint32_t *sa, const uint32_t *sb,
-                   uint32_t *evs, uint8_t *flag, uint32_t step, float scale,
+void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
+                   const HeavyRows &heavy, const uint32_t *mask, const uint32_t *sa,
+                   const uint32_t *sb, uint32_t *evs, uint32_t *bits, uint32_t step, float scale,
                    const StepConsts &c, cudaStream_t st);
-void packed_flow(const PackedLayout &L, const PackedTask *tasks,
-                 const int32_t *row_ptr, uint32_t *mask, uint32_t *sa,
-                 uint32_t *sb, const uint32_t *evs, uint8_t *flag,
-                 unsigned long long *ev_row, unsigned long long *rs_row,
-                 uint32_t step, const StepConsts &c, cudaStream_t st);
+// net_first: first row of each of several networks (their counts follow one
+// another in ev_row and rs_row).
+void packed_flow(const PackedLayout &L, uint32_t *mask, uint32_t *sa, uint32_t *sb, uint32_t *evs,
+                 uint32_t *bits, unsigned long long *ev_row, unsigned long long *rs_row,
+                 const int32_t *net_first, int32_t n_nets, uint32_t step, const StepConsts &c,
+                 cudaStream_t st);
 // Batched countdown mode (countdown.cu): per-replica codes into the host's
 // countdown table (next | class << 16 | infectious << 18), 1 or 2 bytes each.
 rp_status cd_prepare();

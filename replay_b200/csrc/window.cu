@@ -222,7 +222,8 @@ __global__ void __launch_bounds__(kScanThreads)
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_apply(int32_t *__restrict__ in_all, int32_t n,
                  const int32_t *__restrict__ tiles, int32_t *__restrict__ out_all,
-                 int zero_in) {
+                 int zero_in, int32_t *__restrict__ heavy_all, int64_t heavy_cap,
+                 unsigned long long *__restrict__ heavy_counts) {
   __shared__ int wt[32];
   int32_t *in = in_all + (int64_t)blockIdx.y * n;
   int32_t *out = out_all + (int64_t)blockIdx.y * (n + 1);
@@ -244,6 +245,13 @@ __global__ void __launch_bounds__(kScanThreads)
     if (base + j < n) {
       out[base + j] = ex;
       if (zero_in) in[base + j] = 0;
+      if (heavy_all && v[j] > kHeavyPairs) {  // the step kernel's list of long rows
+        int32_t *list = heavy_all + (int64_t)blockIdx.y * heavy_cap;
+        unsigned long long *cnt = heavy_counts + 4 * blockIdx.y;
+        const bool huge = v[j] > kHugePairs;
+        const int64_t at = (int64_t)atomicAdd(&cnt[huge ? 2 : 0], 1ull);
+        list[huge ? heavy_cap - 1 - at : at] = (int32_t)(base + j);
+      }
     }
     ex += v[j];
   }
@@ -584,8 +592,8 @@ rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t sl
     RP_TRY(w.erank.alloc(sizeof(int32_t) * w.cap_entries));
     RP_TRY(w.tmp_e.alloc(sizeof(int2) * w.cap_entries));
     RP_TRY(w.tmp_r.alloc(sizeof(int32_t) * w.cap_entries));
-    RP_TRY(w.long_rows.alloc(sizeof(int32_t) * g * n));
   }
+  RP_TRY(w.long_rows.alloc(sizeof(int32_t) * g * n));
   RP_TRY(w.row_ptr.alloc(sizeof(int32_t) * g * (n + 1)));
   RP_TRY(w.deg.alloc(sizeof(int32_t) * g * n));
   RP_TRY(w.tiles.alloc(sizeof(int32_t) * g * (size_t)w.n_tiles));
@@ -614,7 +622,7 @@ constexpr int32_t kGroupMax = 256;
 void plan_window_groups(std::vector<WinDesc> &wins, int32_t n_nodes, bool single,
                         std::vector<WindowGroup> &groups) {
   groups.clear();
-  const int64_t node_bytes = 12ll * n_nodes;
+  const int64_t node_bytes = 12ll * n_nodes;  // degrees, row pointers, long rows
   for (int32_t w = 0; w < (int32_t)wins.size();) {
     const int64_t budget = groups.empty() ? kFirstGroupBytes : kGroupBytes;
     WindowGroup g;
@@ -659,7 +667,8 @@ int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup 
     ++launches;
   }
   k_scan_apply<<<dim3(ws.n_tiles, G), kScanThreads, 0, st>>>(
-      ws.deg.as<int32_t>(), n, ws.tiles.as<int32_t>(), ws.row_ptr.as<int32_t>(), 1);
+      ws.deg.as<int32_t>(), n, ws.tiles.as<int32_t>(), ws.row_ptr.as<int32_t>(), 1,
+      sort_rows ? nullptr : ws.long_rows.as<int32_t>(), n, ctr);
   k_fill<<<dim3(grid_for(grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
       wins, ws.hits.as<Hit>(), ws.row_ptr.as<int32_t>(), ws.deg.as<int32_t>(),
       ws.entries.as<int2>(), ws.erank.as<int32_t>(), n, sort_rows);
@@ -677,8 +686,9 @@ int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup 
   return launches;
 }
 
-void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out,
-                            int2 *entries_out, cudaStream_t st) {
+void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out, int2 *entries_out,
+                            cudaStream_t st, int32_t *heavy, int64_t heavy_cap,
+                            unsigned long long *heavy_counts) {
   const int32_t n = ws.n_nodes;
   int32_t *len = ws.deg.as<int32_t>();
   k_count_kept<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(n, ws.row_ptr.as<int32_t>(),
@@ -686,7 +696,8 @@ void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out,
   if (ws.n_tiles > 1)
     k_scan_tiles<<<ws.n_tiles, kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>());
   k_scan_apply<<<ws.n_tiles, kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>(),
-                                                   row_ptr_out, 1);
+                                                   row_ptr_out, 1, heavy, heavy_cap,
+                                                   heavy_counts);
   k_compact<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(n, ws.row_ptr.as<int32_t>(),
                                                      ws.entries.as<int2>(), row_ptr_out,
                                                      entries_out);
