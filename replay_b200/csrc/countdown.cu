@@ -1,4 +1,8 @@
-// Batched path, countdown mode: the reference's own transition rules
+// Batched path, countdown mode: the reference's own transition rules as codes
+// into a table, for replays too large for the sets of replicas further down
+// (those are the usual form: k_cd_flow here, k_infect<true> in packed.cu).
+//
+// The reference's own transition rules
 // (initialize_countdown_vector, generate_infectious_vector,
 // compute_infection_probability, monte_carlo_simulation and
 // update_countdown_vector, tool/gpu_cpu_temporal_sim.cu:73-176) for every
@@ -304,6 +308,243 @@ __global__ void __launch_bounds__(kCdThreads)
   }
 }
 
+// ---- the rule as changes of state at fixed ages -----------------------------------
+// A replica infected in step t enters the same states at the same ages, so
+// the host lists the ages at which the summary class, the infectious flag or
+// the susceptibility change (a handful), and the replicas infected in step t
+// stay together as one bit plane of a ring until the last change.  A step
+// touches only the words of the sets that change in it, 32 replicas at a time,
+// where a code per replica had to be read, looked up and written for every
+// replica: 747 us a step on N = 1,000, M = 10,000 with half of all replicas
+// changing class together, 48 us now (k_infect<true> 8-43, k_cd_flow 20).
+//
+// One warp takes up to 32 rows and 32 words (1,024 replicas, 8 items of a
+// row's bitmap): lane = row finds the rows with members, then lane = word applies
+// the changes row by row.  Class changes are counted in vertical counters
+// (bit k of 32 counts per word), expanded once per unit: the half of 10^7
+// replicas that change class together would otherwise be 5 * 10^6 reductions.
+struct CdFlowArgs {
+  CdSources src;
+  uint32_t *busy, *mask, *ca, *cb, *infb, *susb;
+  unsigned long long *ev_row;
+  const int32_t *net_first;
+  int32_t n_nets, n_groups;
+  int32_t unit_rows;  // at most 32
+  int64_t n_units;
+};
+constexpr int kVertical = 4;  // sources with vertical counters
+constexpr int kVPlanes = 6;   // counts up to 32 rows
+
+__device__ __forceinline__ unsigned long long class_step(int from, int to) {
+  return cls_enc((uint32_t)to, 21) - cls_enc((uint32_t)from, 21);
+}
+
+__global__ void __launch_bounds__(kCdThreads, 3)
+    k_cd_flow(PackedLayout L, const __grid_constant__ CdFlowArgs d) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t tw = (int64_t)gridDim.x * kCdWarps;
+  for (int64_t unit = (int64_t)warp * gridDim.x + blockIdx.x; unit < d.n_units; unit += tw) {
+    const int r0 = (int)(unit / d.n_groups) * d.unit_rows, g = (int)(unit % d.n_groups);
+    const int r1 = min(r0 + d.unit_rows, L.n_nodes);
+    // ---- lane = row: which sources have members in the row's 8 items ----
+    const int row = r0 + lane, col = g * 8;
+    const int64_t bw = (int64_t)(row >> (5 - L.lb)) * L.n_slices + (col >> 5);
+    const int sh = ((row & ((32 >> L.lb) - 1)) << L.lb) + (col & 31);
+    const uint32_t im = L.lb >= 3 ? 0xFFu : (1u << (1 << L.lb)) - 1u;
+    unsigned fl[kCdSources], any = 0;
+#pragma unroll
+    for (int j = 0; j < kCdSources; ++j) {
+      fl[j] = 0;
+      if (j >= d.src.n) continue;
+      uint32_t v = 0;
+      if (row < r1) v = (d.src.s[j].bits[bw] >> sh) & im;
+      if (v && d.src.s[j].clear) atomicAnd(&d.src.s[j].bits[bw], ~(v << sh));
+      fl[j] = __ballot_sync(kFull, v != 0u);
+      any |= fl[j];
+    }
+    if (!any) continue;
+    uint32_t oi = 0, os = 0;
+    if (row < r1) {
+      oi = (d.infb[bw] >> sh) & im;
+      os = (d.susb[bw] >> sh) & im;
+    }
+    // ---- lane = word ----
+    const int word = g * 32 + lane;
+    const bool in = word < L.words;
+    const uint32_t vm = in ? word_mask(L, word) : 0u;
+    const bool vertical = d.n_nets == 1 && __popc(any) >= 6;
+    uint32_t vc[kVertical][kVPlanes];
+#pragma unroll
+    for (int j = 0; j < kVertical; ++j)
+#pragma unroll
+      for (int k = 0; k < kVPlanes; ++k) vc[j][k] = 0;
+    // the next row's words are loaded while a row is worked on
+    uint32_t nb = 0, nmk = 0, nm[kCdSources];
+    auto load = [&](int o) {
+      const int64_t wi = (int64_t)(r0 + o) * L.words + word;
+      if (in) {
+        nb = d.busy[wi];
+        nmk = d.mask[wi];
+      }
+#pragma unroll
+      for (int j = 0; j < kCdSources; ++j)
+        nm[j] = j < d.src.n && ((fl[j] >> o) & 1u) && in ? d.src.s[j].plane[wi] : 0u;
+    };
+    load(__ffs(any) - 1);
+    for (unsigned rows = any; rows; rows &= rows - 1) {
+      const int o = __ffs(rows) - 1;
+      const int64_t wi = (int64_t)(r0 + o) * L.words + word;
+      uint32_t b = nb, mk = nmk, m[kCdSources];
+#pragma unroll
+      for (int j = 0; j < kCdSources; ++j) m[j] = nm[j];
+      if (rows & (rows - 1)) load(__ffs(rows & (rows - 1)) - 1);
+      const uint32_t b0 = b, mk0 = mk;
+      int64_t base = 0;
+      if (!vertical) {
+        int net = 0;
+        if (d.n_nets > 1) {  // the row's network: last first row <= row
+          int hi = d.n_nets;
+          while (hi - net > 1) {
+            const int mid = (net + hi) >> 1;
+            if (__ldg(d.net_first + mid) <= r0 + o) net = mid; else hi = mid;
+          }
+        }
+        base = (int64_t)net * L.m + word * 32;
+      }
+#pragma unroll
+      for (int j = 0; j < kCdSources; ++j) {
+        if (j >= d.src.n || !m[j]) continue;
+        const CdSource &s = d.src.s[j];
+        b = s.busy ? b | m[j] : b & ~m[j];
+        mk = s.infectious ? mk | m[j] : mk & ~m[j];
+        if (s.clear) s.plane[wi] = 0u;
+        if (d.ca && s.from != s.to) {  // class planes: S 00, E 01, I 10, R 11
+          d.ca[wi] = (s.to & 2) ? d.ca[wi] | m[j] : d.ca[wi] & ~m[j];
+          d.cb[wi] = (s.to & 1) ? d.cb[wi] | m[j] : d.cb[wi] & ~m[j];
+        }
+        if (s.from == s.to) continue;
+        if (vertical && j < kVertical) {
+          uint32_t cy = m[j];
+#pragma unroll
+          for (int k = 0; k < kVPlanes; ++k) {
+            const uint32_t t = vc[j < kVertical ? j : 0][k];
+            vc[j < kVertical ? j : 0][k] = t ^ cy;
+            cy &= t;
+          }
+        } else {
+          if (vertical) base = word * 32;
+          for (uint32_t t = m[j]; t; t &= t - 1)
+            atomicAdd(&d.ev_row[base + __ffs(t) - 1], class_step(s.from, s.to));
+        }
+      }
+      if (b != b0) d.busy[wi] = b;
+      if (mk != mk0) d.mask[wi] = mk;
+      // the row's inf and sus bits, exact: an item is four lanes
+      const unsigned wi4 = __ballot_sync(kFull, mk != 0u);
+      const unsigned ws4 = __ballot_sync(kFull, (~b & vm) != 0u);
+      const uint32_t ni = __ballot_sync(kFull, lane < 8 && ((wi4 >> (4 * lane & 31)) & 15u)) & im;
+      const uint32_t ns = __ballot_sync(kFull, lane < 8 && ((ws4 >> (4 * lane & 31)) & 15u)) & im;
+      if (lane == o) {
+        if (ni != oi) atomicXor(&d.infb[bw], (ni ^ oi) << sh);
+        if (ns != os) atomicXor(&d.susb[bw], (ns ^ os) << sh);
+      }
+    }
+    if (!vertical) continue;
+    uint32_t used = 0;
+#pragma unroll
+    for (int j = 0; j < kVertical; ++j)
+#pragma unroll
+      for (int k = 0; k < kVPlanes; ++k) used |= vc[j][k];
+    // word by word, lane = replica: 32 neighbouring reductions
+    for (unsigned w = __ballot_sync(kFull, used != 0u); w; w &= w - 1) {
+      const int o = __ffs(w) - 1;
+      unsigned long long gsum = 0;
+#pragma unroll
+      for (int j = 0; j < kVertical; ++j) {
+        if (j >= d.src.n) continue;
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int k = 0; k < kVPlanes; ++k)
+          cnt |= ((__shfl_sync(kFull, vc[j][k], o) >> lane) & 1u) << k;
+        gsum += cnt * class_step(d.src.s[j].from, d.src.s[j].to);
+      }
+      if (gsum) atomicAdd(&d.ev_row[(g * 32 + o) * 32 + lane], gsum);
+    }
+  }
+}
+
+// The same changes on rows of fewer than 32 words: a row would fill a few
+// lanes only, so a warp takes 8 items of the bitmap, four lanes each, and
+// counts every change directly.  (Row by row, N = 5,000 with 64 replicas took
+// about 14 us a step: up to 32 rows in turn per warp, 4 of 32 lanes at work.)
+__global__ void __launch_bounds__(kCdThreads, 3)
+    k_cd_flow_narrow(PackedLayout L, const __grid_constant__ CdFlowArgs d) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t tw = (int64_t)gridDim.x * kCdWarps;
+  for (int64_t unit = (int64_t)warp * gridDim.x + blockIdx.x; unit < d.n_units; unit += tw) {
+    const int64_t bw = unit >> 2;
+    const int bit = (int)(unit & 3) * 8 + (lane >> 2);  // the lane's item
+    uint32_t fl[kCdSources], any = 0;
+#pragma unroll
+    for (int j = 0; j < kCdSources; ++j) fl[j] = j < d.src.n ? d.src.s[j].bits[bw] : 0u;
+#pragma unroll
+    for (int j = 0; j < kCdSources; ++j) {
+      fl[j] = (fl[j] >> bit) & 1u;
+      any |= fl[j];
+    }
+    if (!__any_sync(kFull, any != 0u)) continue;
+    const int row = (int)(bw << (5 - L.lb)) + (bit >> L.lb);
+    const int word = (bit & ((1 << L.lb) - 1)) * 4 + (lane & 3);
+    const int64_t wi = (int64_t)row * L.words + word;
+    uint32_t b = 0, mk = 0, oi = 0, os = 0, m[kCdSources];
+    if (any) {
+      b = d.busy[wi];
+      mk = d.mask[wi];
+      oi = (d.infb[bw] >> bit) & 1u;
+      os = (d.susb[bw] >> bit) & 1u;
+    }
+#pragma unroll
+    for (int j = 0; j < kCdSources; ++j) m[j] = fl[j] ? d.src.s[j].plane[wi] : 0u;
+    const uint32_t b0 = b, mk0 = mk;
+    int64_t base = word * 32;
+    if (any && d.n_nets > 1) {  // the row's network: last first row <= row
+      int net = 0, hi = d.n_nets;
+      while (hi - net > 1) {
+        const int mid = (net + hi) >> 1;
+        if (__ldg(d.net_first + mid) <= row) net = mid; else hi = mid;
+      }
+      base += (int64_t)net * L.m;
+    }
+#pragma unroll
+    for (int j = 0; j < kCdSources; ++j) {
+      if (j >= d.src.n) continue;
+      const CdSource &s = d.src.s[j];
+      if (fl[j] && s.clear && (lane & 3) == 0) atomicAnd(&s.bits[bw], ~(1u << bit));
+      if (!m[j]) continue;
+      b = s.busy ? b | m[j] : b & ~m[j];
+      mk = s.infectious ? mk | m[j] : mk & ~m[j];
+      if (s.clear) s.plane[wi] = 0u;
+      if (s.from == s.to) continue;
+      if (d.ca) {  // class planes: S 00, E 01, I 10, R 11
+        d.ca[wi] = (s.to & 2) ? d.ca[wi] | m[j] : d.ca[wi] & ~m[j];
+        d.cb[wi] = (s.to & 1) ? d.cb[wi] | m[j] : d.cb[wi] & ~m[j];
+      }
+      for (uint32_t t = m[j]; t; t &= t - 1)
+        atomicAdd(&d.ev_row[base + __ffs(t) - 1], class_step(s.from, s.to));
+    }
+    if (b != b0) d.busy[wi] = b;
+    if (mk != mk0) d.mask[wi] = mk;
+    // the items' inf and sus bits, exact
+    const unsigned wi4 = __ballot_sync(kFull, mk != 0u);
+    const unsigned ws4 = __ballot_sync(kFull, any && (~b & word_mask(L, word)) != 0u);
+    if (any && (lane & 3) == 0) {
+      const uint32_t ni = ((wi4 >> lane) & 15u) != 0u, ns = ((ws4 >> lane) & 15u) != 0u;
+      if (ni != oi) atomicXor(&d.infb[bw], 1u << bit);
+      if (ns != os) atomicXor(&d.susb[bw], 1u << bit);
+    }
+  }
+}
+
 // counts[t][net][r][4] (E, I, R, S) from the initial counts and the per-step
 // signed class deltas.
 __global__ void k_cd_finalize(const unsigned long long *__restrict__ init,
@@ -397,6 +638,36 @@ void cd_step(const PackedLayout &L, const PackedTask *tasks, const int32_t *row_
     k_cd_step<uint16_t><<<g, kCdThreads, smem, st>>>(L, tasks, row_ptr, entries, mask_in, mask_out,
                                                      static_cast<uint16_t *>(codes), tab, n_codes,
                                                      infect_code, ev_row, step, c);
+}
+
+void cd_flow(const PackedLayout &L, const CdSources &src, uint32_t *busy, uint32_t *mask,
+             uint32_t *ca, uint32_t *cb, uint32_t *infb, uint32_t *susb,
+             unsigned long long *ev_row, const int32_t *net_first, int32_t n_nets,
+             cudaStream_t st) {
+  if (src.n == 0) return;
+  CdFlowArgs d{};
+  d.src = src;
+  d.busy = busy;
+  d.mask = mask;
+  d.ca = ca;
+  d.cb = cb;
+  d.infb = infb;
+  d.susb = susb;
+  d.ev_row = ev_row;
+  d.net_first = net_first;
+  d.n_nets = n_nets;
+  const bool narrow = L.words < 32;
+  d.n_groups = (L.words + 31) / 32;
+  // 32 rows per unit, fewer (down to 8) where warps would have no unit
+  d.unit_rows = 32;
+  auto units = [&](int rows) { return (int64_t)((L.n_nodes + rows - 1) / rows) * d.n_groups; };
+  while (d.unit_rows > 8 && units(d.unit_rows) < 1024) d.unit_rows >>= 1;
+  d.n_units = narrow ? 4 * L.bit_words : units(d.unit_rows);
+  const int grid = (int)(d.n_units < 148 * 3 ? d.n_units : 148 * 3);
+  if (narrow)
+    k_cd_flow_narrow<<<grid, kCdThreads, 0, st>>>(L, d);
+  else
+    k_cd_flow<<<grid, kCdThreads, 0, st>>>(L, d);
 }
 
 void cd_finalize(const unsigned long long *init, const unsigned long long *ev, int32_t steps,

@@ -240,6 +240,28 @@ void build_cd_table(const rp_params &p, CdTable &t) {
   t.code_bytes = t.tab.size() <= 256 ? 1 : (t.tab.size() <= 65536 ? 2 : 0);
 }
 
+// The same countdowns as changes of state: at `age` steps after the infection
+// (age 0: in the step itself) or, for the initially infected, at the end of
+// step `age` - 1 (age 0: the initial state).
+struct CdChange {
+  int32_t age, from, to, infectious, busy;
+};
+
+std::vector<CdChange> cd_changes(const CdTable &t, uint32_t code, int32_t n_ages) {
+  std::vector<CdChange> out;
+  uint32_t cls = 0, inf = 0, busy = 0;
+  for (int32_t age = 0; age < n_ages; ++age) {
+    const uint32_t e = t.tab[code];
+    const uint32_t ncls = (e >> 16) & 3u, ninf = (e >> 18) & 1u, nbusy = code != 0;
+    if (ncls != cls || ninf != inf || nbusy != busy)
+      out.push_back(CdChange{age, (int32_t)cls, (int32_t)ncls, (int32_t)ninf, (int32_t)nbusy});
+    cls = ncls, inf = ninf, busy = nbusy;
+    if (code == 0) break;  // susceptible: the next change is an infection
+    code = e & 0xFFFFu;
+  }
+  return out;
+}
+
 int resolve_path(const rp_params &p) {
   if (p.path != RP_PATH_AUTO) return p.path;
   if (p.transition == RP_TRANSITION_GEOMETRIC) return RP_PATH_BATCHED;
@@ -293,7 +315,13 @@ struct rp_sim {
   // batched state
   DevBuf sa, sb, mask, evs, bits, tasks, ev, rs, init_counts;
   DevBuf mask2;  // countdown mode: the infectious masks alternate between steps
-  // batched countdown state: per-replica codes into the countdown table
+  // batched countdown state: the sets of replicas infected in the last
+  // ring_slots steps (bit planes and item bitmaps), sb the replicas that are
+  // not susceptible, sa the initially infected ...
+  std::vector<CdChange> cd_inf, cd_init_ch;
+  int32_t ring_slots = 0;  // 0: codes
+  DevBuf ring, ring_bits, class_a, class_b;
+  // ... or, where the sets would not fit, per-replica codes into the table
   DevBuf codes, cd_tab;
   CdTable cd;
   PackedLayout L{};
@@ -421,6 +449,65 @@ struct rp_sim {
   };
   enum { kMarkStart = 0, kMarkOther = 1, kMarkBuild = 2, kMarkSpmv = 3, kMarkStep = 4 };
 
+  // ---- countdown rule with sets of replicas per infection step ----
+  uint32_t *ring_plane(int32_t t) const {
+    return ring.as<uint32_t>() + (int64_t)(t % ring_slots) * N * L.words;
+  }
+  uint32_t *ring_bit(int32_t t) const {  // slots, then: initial set, inf, sus
+    return ring_bits.as<uint32_t>() + (int64_t)(t % ring_slots) * L.bit_words;
+  }
+  uint32_t *init_bits() const { return ring_bits.as<uint32_t>() + ring_slots * L.bit_words; }
+  uint32_t *inf_bits() const { return init_bits() + L.bit_words; }
+  uint32_t *sus_bits() const { return init_bits() + 2 * L.bit_words; }
+  static CdSource source(const CdChange &ch, uint32_t *plane, uint32_t *bits, bool last) {
+    return CdSource{plane, bits, last, ch.from, ch.to, ch.infectious, ch.busy};
+  }
+  void ring_flow(const CdSources &src, unsigned long long *row, cudaStream_t st) {
+    cd_flow(L, src, sb.as<uint32_t>(), mask.as<uint32_t>(), class_a.as<uint32_t>(),
+            class_b.as<uint32_t>(), inf_bits(), sus_bits(), row, net_first.as<int32_t>(), n_nets,
+            st);
+  }
+  // Initial state from the initial-infection plane sa.
+  rp_status ring_init(cudaStream_t st, int &k) {
+    RP_TRY_CUDA(cudaMemsetAsync(ring.ptr, 0, ring.bytes, st));
+    RP_TRY_CUDA(cudaMemsetAsync(ring_bits.ptr, 0, ring_bits.bytes, st));
+    // no infectious replica, every item susceptible (bits without an item are
+    // never asked for)
+    RP_TRY_CUDA(cudaMemsetAsync(mask.ptr, 0, mask.bytes, st));
+    RP_TRY_CUDA(cudaMemsetAsync(sus_bits(), 0xFF, sizeof(uint32_t) * L.bit_words, st));
+    if (class_a.ptr) {
+      RP_TRY_CUDA(cudaMemsetAsync(class_a.ptr, 0, class_a.bytes, st));
+      RP_TRY_CUDA(cudaMemsetAsync(class_b.ptr, 0, class_b.bytes, st));
+    }
+    cd_bits(L, sa.as<uint32_t>(), init_bits(), st);
+    CdSources src{};
+    if (!cd_init_ch.empty() && cd_init_ch[0].age == 0)
+      src.s[src.n++] = source(cd_init_ch[0], sa.as<uint32_t>(), init_bits(), false);
+    ring_flow(src, init_counts.as<unsigned long long>(), st);
+    k += 1 + (src.n > 0);
+    return RP_OK;
+  }
+  template <typename Mark>
+  int ring_step(int32_t t, cudaStream_t st, Mark &mark) {
+    int k = 0;
+    CdSources src{};
+    for (const CdChange &ch : cd_inf)  // a set's last change frees its slot
+      if (ch.age <= t)
+        src.s[src.n++] = source(ch, ring_plane(t - ch.age), ring_bit(t - ch.age),
+                                ch.age == cd_inf.back().age);
+    for (const CdChange &ch : cd_init_ch)
+      if (ch.age == t + 1) src.s[src.n++] = source(ch, sa.as<uint32_t>(), init_bits(), false);
+    if (!cd_inf.empty()) {
+      cd_infect(L, rp_of(t), ent_of(t), mask.as<uint32_t>(), sb.as<uint32_t>(), ring_plane(t),
+                inf_bits(), sus_bits(), ring_bit(t), (uint32_t)t, c, st);
+      ++k;
+    }
+    mark(kMarkSpmv);
+    ring_flow(src, ev.as<unsigned long long>() + (int64_t)t * n_nets * M, st);
+    mark(kMarkStep);
+    return k + (src.n > 0);
+  }
+
   // Enqueues one whole replay.  With `cb`, per-step node states are copied
   // out and handed to the callback (not capturable).
   rp_status enqueue(cudaStream_t st, rp_state_cb cb, void *user, int *n_kernels,
@@ -435,7 +522,10 @@ struct rp_sim {
     if (cb && !text_cb) host_states.resize((size_t)N * M);
     auto emit_states = [&](int32_t step_index, int64_t tstamp) -> rp_status {
       if (!cb && !text_cb) return RP_OK;
-      if (path == RP_PATH_BATCHED && cd.code_bytes)
+      if (path == RP_PATH_BATCHED && ring_slots)
+        packed_classify(L, class_a.as<uint32_t>(), class_b.as<uint32_t>(), classes.as<uint8_t>(),
+                        st);
+      else if (path == RP_PATH_BATCHED && cd.code_bytes)
         cd_classify(L, codes.ptr, cd.code_bytes, cd_tab.as<uint32_t>(), classes.as<uint8_t>(),
                     st);
       else if (path == RP_PATH_BATCHED)
@@ -466,7 +556,9 @@ struct rp_sim {
       packed_init(L, sa.as<uint32_t>(), sb.as<uint32_t>(), mask.as<uint32_t>(),
                   bits.as<uint32_t>(), p.initial_infected, p.initial_count, net_first.as<int32_t>(),
                   net_rows.as<int32_t>(), n_nets, c, st);
-      if (cd.code_bytes)  // countdown codes from the initial-infection plane
+      if (ring_slots) {
+        RP_TRY(ring_init(st, k));
+      } else if (cd.code_bytes)  // countdown codes from the initial-infection plane
         cd_init(L, tasks.as<PackedTask>(), sa.as<uint32_t>(), codes.ptr, cd.code_bytes,
                 mask.as<uint32_t>(), cd_tab.as<uint32_t>(), cd.init_code,
                 init_counts.as<unsigned long long>(), st);
@@ -511,7 +603,9 @@ struct rp_sim {
         mark(kMarkStep);
         k += 2;
       } else {
-        if (cd.code_bytes) {
+        if (ring_slots) {
+          k += ring_step(t, st, mark);
+        } else if (cd.code_bytes) {
           // countdown codes: the infectious masks alternate, step t reads
           // buffer t & 1 and writes every word of the other
           const uint32_t *m_in = (t & 1) ? mask2.as<uint32_t>() : mask.as<uint32_t>();
@@ -841,6 +935,8 @@ rp_status upload_tasks(rp_sim &s) {
   return RP_OK;
 }
 
+constexpr int64_t kRingBytes = 16ll << 30;
+
 rp_status alloc_state(rp_sim &s) {
   const int32_t N = s.N, M = s.M, T = s.T;
   const int64_t NM = (int64_t)N * M;
@@ -896,6 +992,23 @@ rp_status alloc_state(rp_sim &s) {
     RP_TRY(s.bits.alloc(sizeof(uint32_t) * 4 * (size_t)L.bit_words));
   }
   if (s.cd.code_bytes) {
+    // the sets of replicas per infection step, as long as an age may still
+    // change: at most kRingBytes, else (or without the memory) codes
+    s.cd_inf = s.cd.infect_code ? cd_changes(s.cd, s.cd.infect_code, T) : std::vector<CdChange>();
+    s.cd_init_ch =
+        s.cd.init_code ? cd_changes(s.cd, s.cd.init_code, T + 1) : std::vector<CdChange>();
+    const int32_t slots = s.cd_inf.empty() ? 1 : s.cd_inf.back().age + 1;
+    if ((int64_t)plane * slots <= kRingBytes && (int)s.cd_inf.size() < kCdSources &&
+        s.ring.alloc(plane * slots) == RP_OK) {
+      s.ring_slots = slots;
+      RP_TRY(s.ring_bits.alloc(sizeof(uint32_t) * (size_t)L.bit_words * (slots + 3)));
+      if (s.p.record_node_states) {
+        RP_TRY(s.class_a.alloc(plane));
+        RP_TRY(s.class_b.alloc(plane));
+      }
+    }
+  }
+  if (s.cd.code_bytes && !s.ring_slots) {
     RP_TRY(s.mask2.alloc(plane));
     RP_TRY(s.codes.alloc((size_t)s.cd.code_bytes * 32 * (size_t)N * L.words));
     RP_TRY(s.cd_tab.alloc(sizeof(uint32_t) * s.cd.tab.size()));
@@ -1422,7 +1535,7 @@ RP_API rp_status rp_sim_get_info(const rp_sim *s, rp_sim_info *o) {
   int64_t bytes = 0;
   const DevBuf *bufs[] = {&s->arena_rp, &s->arena_ent, &s->state, &s->exposure, &s->sa,
                           &s->sb, &s->mask, &s->mask2, &s->evs, &s->bits,
-                          &s->codes, &s->cd_tab,
+                          &s->codes, &s->cd_tab, &s->ring, &s->ring_bits, &s->class_a, &s->class_b,
                           &s->tasks, &s->ev, &s->rs,
                           &s->init_counts, &s->counts, &s->beta_r, &s->sus, &s->classes,
                           &s->wsp.hits, &s->wsp.entries, &s->wsp.erank, &s->wsp.tmp_e,

@@ -127,15 +127,16 @@ constexpr int kUnitRows = 128;     // most rows of a unit
 // accumulates over units and is decided 32 words at a time.
 struct InfectWarp {
   uint4 pl[32][2];             // the 8 random planes of each word (round scratch)
-  int32_t urow[kUnitRows];     // the unit's rows with pairs (row in unit)
+  int32_t urow[kUnitRows];     // the unit's rows with pairs: row in unit | pairs << 7
   int32_t ubeg[kUnitRows];     // their first pairs
   int32_t list[128];           // items of a batch of 32 rows: row in batch << 5 | column
   uint32_t rmask[32];          // column masks of the batch's rows
   int32_t row[kInfectQueue];
-  int32_t word[kInfectQueue];  // word index within the row << 6 | the row's pairs
-  int32_t beg[kInfectQueue];   // the row's first CSR pair
+  int32_t word[kInfectQueue];  // word index within the row
+  int32_t beg[kInfectQueue];   // the row's first CSR pair and pairs
+  int32_t npr[kInfectQueue];
   uint32_t X[kInfectQueue];    // exposed replicas of the word
-  float efmax[kInfectQueue];   // ef(e_max) of the row
+  float efmax[kInfectQueue];   // ef(e_max) of the row (countdown rule: x_max, or kSure)
   uint16_t cl[1024];           // candidates after the bound test: lane << 5 | bit (round scratch)
   // candidates carried to the next round (fewer than 32), self-contained
   int32_t krow[32];
@@ -209,35 +210,124 @@ __device__ __forceinline__ float word_bs(const StepConsts &c, int row, int word)
   return c.sus ? __fmul_rn(bs, fabsf(__ldg(c.sus + row))) : bs;
 }
 
+// ---- countdown rule -----------------------------------------------------------
+// The reference's rule on the same gather (countdown.cu holds the rest): the
+// exposed replicas draw the plain path's uniforms (Philox counter (node, step,
+// replica / 4, 3), output replica % 4, on the 24-bit grid) and are candidates
+// when u < x_max = -log(1 - p) * (e_max / 3600), e_max the in-order FP32 sum
+// of the row's weights (every in-order sum of a subset is at most the full
+// one, and P <= x).  Candidates add their infectious neighbours' weights one
+// by one in CSR order, as Eigen's row-major product does, and infect iff P > u.
+// Where the row's smallest weight alone gives x >= 87, P is 1 whatever the
+// exposure: those replicas infect iff u < 1, without a sum.
+constexpr float kSure = -1.0f;
+__device__ __forceinline__ float countdown_x(const StepConsts &c, float e) {
+  return __fmul_rn(c.neg_log_base, __fdiv_rn(e, 3600.0f));
+}
+__device__ __forceinline__ void set_events(const InfectArgs &d, const PackedLayout &L, int row,
+                                           int word, uint32_t ev) {
+  atomicOr(&d.evs[(int64_t)row * L.words + word], ev);
+  atomicOr(&d.evb[bit_word(L.lb, L.n_slices, row, word >> 2)], bit_of(L.lb, row, word >> 2));
+}
+__device__ __forceinline__ void countdown_decide(const InfectArgs &d, const StepConsts &c,
+                                                 const PackedLayout &L, int row, int word, int b,
+                                                 float e) {
+  uint32_t x[4];
+  philox4x32_10_rk((uint32_t)row, d.step, (uint32_t)(word * 8 + (b >> 2)) + (c.roff >> 2),
+                   kStreamInfect, c.rk, x);
+  const uint32_t xb = (b & 2) ? ((b & 1) ? x[3] : x[2]) : ((b & 1) ? x[1] : x[0]);
+  if (one_minus_exp_neg(countdown_x(c, e)) > unit24(xb)) set_events(d, L, row, word, 1u << b);
+}
+// Candidates of the round's words into Q.cl; returns their number.  One lane
+// takes one quad of replicas with an exposed member (a draw covers a quad), so
+// that sparse words share the draws; the events of sure words are set here.
+__device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int n, int lane,
+                                                    const InfectArgs &d, const StepConsts &c,
+                                                    const PackedLayout &L) {
+  uint16_t *quads = reinterpret_cast<uint16_t *>(Q.pl[0]);  // lane << 3 | quad, at most 256
+  uint32_t *events = reinterpret_cast<uint32_t *>(Q.pl[16]);  // of the sure words
+  const uint32_t X = lane < n ? Q.X[lane] : 0u;
+  int nq = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const bool has = ((X >> (4 * q)) & 15u) != 0u;
+    const unsigned hm = __ballot_sync(kFull, has);
+    if (has) quads[nq + __popc(hm & ((1u << lane) - 1u))] = (uint16_t)(lane << 3 | q);
+    nq += __popc(hm);
+  }
+  events[lane] = 0;
+  __syncwarp();
+  int total = 0;
+  for (int p = lane; p - lane < nq; p += 32) {
+    uint32_t m = 0;
+    int o = 0, q = 0;
+    if (p < nq) {
+      o = quads[p] >> 3;
+      q = quads[p] & 7;
+      const int row = Q.row[o], word = Q.word[o];
+      const bool sure = Q.efmax[o] == kSure;
+      const float lim = sure ? 1.0f : Q.efmax[o];
+      // u = k 2^-24 < lim with k = (x >> 8) + 1, as x <= (K << 8) - 1 for the
+      // largest such k
+      const uint32_t K = !(lim > 0.0f) ? 0u
+                         : lim > 1.0f ? 1u << 24
+                                      : (uint32_t)ceilf(__fmul_rn(lim, 0x1p24f)) - 1u;
+      const uint32_t last = (K << 8) - 1u;
+      uint32_t x[4];
+      philox4x32_10_rk((uint32_t)row, d.step, (uint32_t)(word * 8 + q) + (c.roff >> 2),
+                       kStreamInfect, c.rk, x);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) m |= x[k] <= last ? 1u << k : 0u;
+      m = K ? m & Q.X[o] >> (4 * q) : 0u;
+      if (sure) {
+        if (m) atomicOr(&events[o], m << (4 * q));
+        m = 0;
+      }
+    }
+    int sum;
+    int at = total + warp_excl_scan(__popc(m), lane, sum);
+    for (; m; m &= m - 1) Q.cl[at++] = (uint16_t)(o << 5 | 4 * q + __ffs(m) - 1);
+    total += sum;
+  }
+  __syncwarp();
+  if (events[lane]) set_events(d, L, Q.row[lane], Q.word[lane], events[lane]);
+  return total;
+}
+
 // Decides up to 32 queued exposed words: the bound test one word per lane,
 // then the exact test of the surviving candidates, one replica per lane, in
 // full batches of 32 together with the candidates carried from earlier
 // rounds; fewer than 32 left over are carried to the next round unless
 // `drain` is set.  Events are OR-ed into their words and flag their items.
+template <bool kCountdown>
 __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, int lane,
                                              const PackedLayout &L, const InfectArgs &d,
                                              const StepConsts &c) {
   // ---- bound test, one word per lane ----
-  uint32_t Cw = 0;
-  if (lane < n) {
-    const int row = Q.row[lane], word = Q.word[lane] >> 6;
-    // every exposed replica has P <= x <= |bs_r| ef(e_max) =: B; replicas
-    // whose uniform's top byte is above B's cannot infect
-    const float B = __fmul_rn(word_bs(c, row, word), Q.efmax[lane]);
-    if (B > 0.0f) {
-      uint32_t pl[8];
-      infect_planes(c.rk, (uint32_t)row, d.step, (uint32_t)word + (c.roff >> 5), pl);
-      Cw = B >= 1.0f ? Q.X[lane] : top8_le(Q.X[lane], fixed64(B), pl);
-      Q.pl[lane][0] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-      Q.pl[lane][1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
-    }
-  }
   int ctotal;
-  int pos = warp_excl_scan(__popc(Cw), lane, ctotal);
-  for (; Cw; Cw &= Cw - 1) Q.cl[pos++] = (uint16_t)(lane << 5 | (__ffs(Cw) - 1));
+  if constexpr (kCountdown) {
+    ctotal = countdown_candidates(Q, n, lane, d, c, L);
+  } else {
+    uint32_t Cw = 0;
+    if (lane < n) {
+      const int row = Q.row[lane], word = Q.word[lane];
+      // every exposed replica has P <= x <= |bs_r| ef(e_max) =: B; replicas
+      // whose uniform's top byte is above B's cannot infect
+      const float B = __fmul_rn(word_bs(c, row, word), Q.efmax[lane]);
+      if (B > 0.0f) {
+        uint32_t pl[8];
+        infect_planes(c.rk, (uint32_t)row, d.step, (uint32_t)word + (c.roff >> 5), pl);
+        Cw = B >= 1.0f ? Q.X[lane] : top8_le(Q.X[lane], fixed64(B), pl);
+        Q.pl[lane][0] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+        Q.pl[lane][1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
+      }
+    }
+    int pos = warp_excl_scan(__popc(Cw), lane, ctotal);
+    for (; Cw; Cw &= Cw - 1) Q.cl[pos++] = (uint16_t)(lane << 5 | (__ffs(Cw) - 1));
+  }
   __syncwarp();
-  // ---- exact test of 32 candidates at a time: each lane sums its own row
-  // (at most kHeavyPairs pairs), four mask words in flight ----
+  // ---- exact test of 32 candidates at a time: each lane sums its own row in
+  // CSR order, four mask words in flight ----
   const int nk = Q.nk;
   const int total = nk + ctotal;
   int base = 0;
@@ -246,13 +336,13 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, i
     if (p < total) {
       int row, word, b, npairs;
       int32_t beg;
-      uint32_t u8;
+      uint32_t u8 = 0;
       if (p < nk) {
         const int wb = Q.kwb[p];
         row = Q.krow[p];
         word = wb >> 5;
         b = wb & 31;
-        u8 = Q.ku8[p];
+        if (!kCountdown) u8 = Q.ku8[p];
         beg = Q.kbeg[p];
         npairs = Q.knpr[p];
       } else {
@@ -260,12 +350,12 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, i
         b = ob & 31;
         row = Q.row[o];
         word = Q.word[o];
-        npairs = word & 63;
-        word >>= 6;
-        u8 = queued_top8(Q.pl[o], (uint32_t)b);
+        npairs = Q.npr[o];
+        if (!kCountdown) u8 = queued_top8(Q.pl[o], (uint32_t)b);
         beg = Q.beg[o];
       }
       long long e = 0;
+      float ef = 0.0f;
       for (int32_t k = 0; k < npairs; k += 4) {
         uint32_t m[4];
         int32_t wt[4];
@@ -280,9 +370,18 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, i
           }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) e += ((m[j] >> b) & 1u) ? wt[j] : 0;
+        for (int j = 0; j < 4; ++j) {
+          if (kCountdown) {
+            if ((m[j] >> b) & 1u) ef = __fadd_rn(ef, __int_as_float(wt[j]));
+          } else {
+            e += ((m[j] >> b) & 1u) ? wt[j] : 0;
+          }
+        }
       }
-      decide(d, c, L, row, word, b, e, u8);
+      if (kCountdown)
+        countdown_decide(d, c, L, row, word, b, ef);
+      else
+        decide(d, c, L, row, word, b, e, u8);
     }
   }
   __syncwarp();
@@ -292,11 +391,11 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, i
     const int p = base + lane;
     if (p < total && p >= nk) {
       const int ob = Q.cl[p - nk], o = ob >> 5, b = ob & 31;
-      Q.kwb[lane] = (Q.word[o] >> 6) << 5 | b;
+      Q.kwb[lane] = Q.word[o] << 5 | b;
       Q.krow[lane] = Q.row[o];
       Q.kbeg[lane] = Q.beg[o];
-      Q.knpr[lane] = Q.word[o] & 63;
-      Q.ku8[lane] = (uint8_t)queued_top8(Q.pl[o], (uint32_t)b);
+      Q.knpr[lane] = Q.npr[o];
+      if (!kCountdown) Q.ku8[lane] = (uint8_t)queued_top8(Q.pl[o], (uint32_t)b);
     }
   }
   __syncwarp();
@@ -460,6 +559,7 @@ __device__ __forceinline__ void heavy_decide(const HeavyUnit &h, const HeavyWarp
   }
 }
 
+template <bool kCountdown>
 __global__ void __launch_bounds__(kThreads, 3)
     k_infect(PackedLayout L, const __grid_constant__ InfectArgs d,
              const __grid_constant__ StepConsts c) {
@@ -471,8 +571,12 @@ __global__ void __launch_bounds__(kThreads, 3)
   __shared__ unsigned s_next;
   if (threadIdx.x == 0) s_next = 0;
   __syncthreads();
-  const int n_heavy = (int)d.n_heavy[0], n_huge = (int)d.n_heavy[2];
-  if (n_heavy | n_huge) {
+  int n_heavy = 0, n_huge = 0;
+  if (!kCountdown) {  // the countdown rule's FP32 sums have an order
+    n_heavy = (int)d.n_heavy[0];
+    n_huge = (int)d.n_heavy[2];
+  }
+  if (!kCountdown && (n_heavy | n_huge)) {
     const int nws = (L.words + 31) / 32;
     HeavyWarp &H = *reinterpret_cast<HeavyWarp *>(s_dyn + warp * kInfectWarpBytes);
     HeavyUnit h;
@@ -529,6 +633,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   const uint4 *sb4 = reinterpret_cast<const uint4 *>(d.sb);
   bool more = true;
   int cbase = 0, cnt = 0;    // the current unit's first column; items listed
+  int r0 = 0;                // the unit's first row
   int nrows = 0, ub = 0;     // the unit's rows with pairs; the first row not yet taken
   int lrow = 0, n = 0;       // the lane's row of the batch: pairs beg .. beg + n
   int32_t beg = 0;
@@ -543,7 +648,8 @@ __global__ void __launch_bounds__(kThreads, 3)
           // the next unit's rows that have pairs (longer rows were taken above)
           const int rb = L.n_slices == 1 ? unit : unit / L.n_slices;
           cbase = L.n_slices == 1 ? 0 : (unit - rb * L.n_slices) * 32;
-          const int r0 = rb * d.unit_rows, r1 = min(r0 + d.unit_rows, L.n_nodes);
+          r0 = rb * d.unit_rows;
+          const int r1 = min(r0 + d.unit_rows, L.n_nodes);
           nrows = ub = 0;
           __syncwarp();
           for (int r = r0; r < r1; r += 128) {
@@ -560,11 +666,11 @@ __global__ void __launch_bounds__(kThreads, 3)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               if (r + 32 * j >= r1) break;
-              const bool has = len[j] > 0 && len[j] <= kHeavyPairs;
+              const bool has = len[j] > 0 && (kCountdown || len[j] <= kHeavyPairs);
               const unsigned hm = __ballot_sync(kFull, has);
               if (has) {
                 const int pos = nrows + __popc(hm & ((1u << lane) - 1u));
-                Q.urow[pos] = (r + 32 * j + lane) << 6 | len[j];
+                Q.urow[pos] = (r - r0 + 32 * j + lane) | len[j] << 7;
                 Q.ubeg[pos] = b[j];
               }
               nrows += __popc(hm);
@@ -583,8 +689,8 @@ __global__ void __launch_bounds__(kThreads, 3)
         if (ub + lane < nrows) {
           lrow = Q.urow[ub + lane];
           beg = Q.ubeg[ub + lane];
-          n = lrow & 63;
-          lrow >>= 6;
+          n = lrow >> 7;
+          lrow = r0 + (lrow & 127);
         }
         ub += 32;
         auto row_bits = [&](const uint32_t *bits, int r) {
@@ -593,13 +699,22 @@ __global__ void __launch_bounds__(kThreads, 3)
         const int ncols = min(32, L.q4 - cbase);
         uint32_t sus = n ? row_bits(d.susb, lrow) : 0u, m = 0;
         sus &= ncols == 32 ? kFull : (1u << ncols) - 1u;
-        for (int k = 0; k < n; k += 4) {  // four words in flight
+        for (int k = 0; k < n && (!kCountdown || n <= 32); k += 4) {  // four words in flight
           uint32_t v[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             v[j] = k + j < n ? row_bits(d.infb, __ldg(&d.ent[beg + k + j].x)) : 0u;
           m |= v[0] | v[1] | v[2] | v[3];
         }
+        if (kCountdown)  // longer rows are shared by the warp
+          for (unsigned big = __ballot_sync(kFull, n > 32); big; big &= big - 1) {
+            const int o = __ffs(big) - 1;
+            const int32_t ob = __shfl_sync(kFull, beg, o), on = __shfl_sync(kFull, n, o);
+            uint32_t om = 0;
+            for (int k = lane; k < on; k += 32) om |= row_bits(d.infb, __ldg(&d.ent[ob + k].x));
+            om = __reduce_or_sync(kFull, om);
+            if (lane == o) m = om;
+          }
         m &= sus;
         // few items: every lane lists its own row's; else row by row below
         int tot;
@@ -636,9 +751,11 @@ __global__ void __launch_bounds__(kThreads, 3)
     float efmax = 0.0f;
     if (ok) {
       const int64_t idx = (int64_t)row * L.q4 + col;
-      const uint4 a4 = __ldg(sa4 + idx), b4 = __ldg(sb4 + idx);
+      // countdown rule: one plane, the replicas that are not susceptible
+      const uint4 a4 = __ldg(sa4 + idx), b4 = kCountdown ? a4 : __ldg(sb4 + idx);
       uint4 inf = make_uint4(0, 0, 0, 0);
       long long emax = 0;
+      float fmax = 0.0f, wmin = 3e38f;  // countdown rule: in-order sum, smallest weight
       for (int k = 0; k < rn; k += 4) {  // four mask items in flight
         uint4 m[4];
 #pragma unroll
@@ -647,7 +764,13 @@ __global__ void __launch_bounds__(kThreads, 3)
           if (k + j < rn) {
             const int2 q = __ldg(d.ent + rbeg + k + j);
             m[j] = __ldg(mask4 + (int64_t)q.x * L.q4 + col);
-            emax += q.y;
+            if (kCountdown) {
+              const float wt = __int_as_float(q.y);
+              fmax = __fadd_rn(fmax, wt);
+              if (wt > 0.0f) wmin = fminf(wmin, wt);  // duplicates merged away weigh 0
+            } else {
+              emax += q.y;
+            }
           }
         }
 #pragma unroll
@@ -656,8 +779,12 @@ __global__ void __launch_bounds__(kThreads, 3)
 #pragma unroll
       for (int w = 0; w < 4; ++w)
         X[w] = get4(inf, w) & ~get4(a4, w) & ~get4(b4, w) & word_mask(L, 4 * col + w);
-      efmax = __ll2float_rn(emax);
-      if (d.scale != 1.0f) efmax = __fmul_rn(efmax, d.scale);
+      if (kCountdown) {
+        efmax = countdown_x(c, wmin) >= 87.0f ? kSure : countdown_x(c, fmax);
+      } else {
+        efmax = __ll2float_rn(emax);
+        if (d.scale != 1.0f) efmax = __fmul_rn(efmax, d.scale);
+      }
     }
     // ---- queue the exposed words ----
 #pragma unroll
@@ -668,8 +795,9 @@ __global__ void __launch_bounds__(kThreads, 3)
       if (X[w]) {
         const int pos = base + __popc(qm & ((1u << lane) - 1u));
         Q.row[pos] = row;
-        Q.word[pos] = (4 * col + w) << 6 | rn;
+        Q.word[pos] = 4 * col + w;
         Q.beg[pos] = rbeg;
+        Q.npr[pos] = rn;
         Q.X[pos] = X[w];
         Q.efmax[pos] = efmax;
       }
@@ -680,12 +808,13 @@ __global__ void __launch_bounds__(kThreads, 3)
     // ---- decide full rounds and, past the last unit, what is left ----
     while (Q.n >= 32 || (!more && (Q.n > 0 || Q.nk > 0))) {
       const int take = Q.n < 32 ? Q.n : 32;
-      infect_round(Q, take, !more && take == Q.n, lane, L, d, c);
+      infect_round<kCountdown>(Q, take, !more && take == Q.n, lane, L, d, c);
       const int rest = Q.n - take;
       for (int i = lane; i < rest; i += 32) {
         Q.row[i] = Q.row[take + i];
         Q.word[i] = Q.word[take + i];
         Q.beg[i] = Q.beg[take + i];
+        Q.npr[i] = Q.npr[take + i];
         Q.X[i] = Q.X[take + i];
         Q.efmax[i] = Q.efmax[take + i];
       }
@@ -1097,6 +1226,26 @@ __global__ void k_mask_from_planes(int64_t total, const uint32_t *__restrict__ s
     mask[i] = sa[i] & ~sb[i];
 }
 
+// Bit of every item whose words hold a set bit (one thread per bit).
+__global__ void __launch_bounds__(256)
+    k_bits_of(PackedLayout L, const uint4 *__restrict__ plane, uint32_t *__restrict__ bits) {
+  const int64_t total = L.bit_words * 32;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t wi = i >> 5;
+    const int bit = (int)(i & 31), slice = (int)(wi % L.n_slices);
+    const int64_t row = ((wi / L.n_slices) << (5 - L.lb)) + (bit >> L.lb);
+    const int col = slice * 32 + (bit & ((1 << L.lb) - 1));
+    bool set = false;
+    if (row < L.n_nodes && col < L.q4) {
+      const uint4 v = plane[row * L.q4 + col];
+      set = (v.x | v.y | v.z | v.w) != 0u;
+    }
+    const uint32_t m = __ballot_sync(kFull, set);
+    if ((i & 31) == 0) bits[wi] = m;
+  }
+}
+
 // The bitmaps from the initial planes: one thread per bit.
 __global__ void __launch_bounds__(256)
     k_bits_from_planes(PackedLayout L, const uint4 *__restrict__ sa, const uint4 *__restrict__ sb,
@@ -1204,8 +1353,11 @@ int task_grid(int n_tasks, int per_sm) {
 }  // namespace
 
 rp_status packed_prepare() {
-  cudaError_t e = cudaFuncSetAttribute(k_infect, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kInfectDynSmem);
+  cudaError_t e = cudaFuncSetAttribute(
+      k_infect<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfectDynSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_infect<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kInfectDynSmem);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_infect)");
   e = cudaFuncSetAttribute(k_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlowDynSmem);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_flow)");
@@ -1231,10 +1383,30 @@ void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb, uint32_t *ma
         c.th.tr_all || c.th.tr != 0);
 }
 
+void cd_bits(const PackedLayout &L, const uint32_t *plane, uint32_t *bits, cudaStream_t st) {
+  k_bits_of<<<1184, 256, 0, st>>>(L, reinterpret_cast<const uint4 *>(plane), bits);
+}
+
 // Blocks for `units` warp-sized units: one warp each over all SMs first, then
 // up to the three resident blocks of each SM.
 static int unit_grid(int64_t units) {
   return (int)(units < 1 ? 1 : (units < 148 * 3 ? units : 148 * 3));
+}
+
+// 8 rows per unit, so that a block's warps end together; fewer (down to 8
+// items, one round of words) where blocks would have none, more where every
+// warp has many: a unit's row pointers are loaded together, and sparse rows
+// fold into batches of 32.
+static void set_infect_units(const PackedLayout &L, InfectArgs &d) {
+  d.unit_rows = 8;
+  const int64_t warps = 148 * 3 * kWarps;
+  auto units = [&](int rows) { return (int64_t)((L.n_nodes + rows - 1) / rows) * L.n_slices; };
+  while (d.unit_rows > 1 && units(d.unit_rows) * 2 < warps && (int64_t)d.unit_rows * L.q4 > 8)
+    d.unit_rows >>= 1;
+  while (d.unit_rows < kUnitRows && (units(2 * d.unit_rows) >= 4 * warps ||
+                                     (int64_t)d.unit_rows * L.q4 < 8))
+    d.unit_rows *= 2;
+  d.n_units = (int32_t)units(d.unit_rows);
 }
 
 void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
@@ -1256,20 +1428,26 @@ void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *en
   d.n_heavy = heavy.counts;
   d.step = step;
   d.scale = scale;
-  // 8 rows per unit, so that a block's warps end together; fewer (down to 8
-  // items, one round of words) where blocks would have none, more where every
-  // warp has many: a unit's row pointers are loaded together, and sparse rows
-  // fold into batches of 32
-  d.unit_rows = 8;
-  const int64_t warps = 148 * 3 * kWarps;
-  auto units = [&](int rows) { return (int64_t)((L.n_nodes + rows - 1) / rows) * L.n_slices; };
-  while (d.unit_rows > 1 && units(d.unit_rows) * 2 < warps && (int64_t)d.unit_rows * L.q4 > 8)
-    d.unit_rows >>= 1;
-  while (d.unit_rows < kUnitRows && (units(2 * d.unit_rows) >= 4 * warps ||
-                                     (int64_t)d.unit_rows * L.q4 < 8))
-    d.unit_rows *= 2;
-  d.n_units = (int32_t)units(d.unit_rows);
-  k_infect<<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
+  set_infect_units(L, d);
+  k_infect<false><<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
+}
+
+void cd_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
+               const uint32_t *mask, const uint32_t *busy, uint32_t *evs, const uint32_t *infb,
+               const uint32_t *susb, uint32_t *evb, uint32_t step, const StepConsts &c,
+               cudaStream_t st) {
+  InfectArgs d{};
+  d.row_ptr = row_ptr;
+  d.ent = entries;
+  d.mask = mask;
+  d.sa = busy;
+  d.evs = evs;
+  d.infb = infb;
+  d.susb = susb;
+  d.evb = evb;
+  d.step = step;
+  set_infect_units(L, d);
+  k_infect<true><<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
 }
 
 void packed_flow(const PackedLayout &L, uint32_t *mask, uint32_t *sa, uint32_t *sb, uint32_t *evs,

@@ -390,8 +390,34 @@ void packed_flow(const PackedLayout &L, uint32_t *mask, uint32_t *sa, uint32_t *
                  uint32_t *bits, unsigned long long *ev_row, unsigned long long *rs_row,
                  const int32_t *net_first, int32_t n_nets, uint32_t step, const StepConsts &c,
                  cudaStream_t st);
-// Batched countdown mode (countdown.cu): per-replica codes into the host's
-// countdown table (next | class << 16 | infectious << 18), 1 or 2 bytes each.
+// Batched countdown mode (countdown.cu) as changes of state at fixed ages: a
+// source is a set of replicas (a bit plane and its item bitmap) that enters
+// one summary class from another in this step.
+struct CdSource {
+  uint32_t *plane, *bits;
+  int32_t clear;           // the set is not needed after this change
+  int32_t from, to;        // summary classes (0 S, 1 E, 2 I, 3 R)
+  int32_t infectious;      // from this change on
+  int32_t busy;            // 0: susceptible from this change on
+};
+constexpr int kCdSources = 8;
+struct CdSources {
+  CdSource s[kCdSources];
+  int32_t n;
+};
+void cd_bits(const PackedLayout &L, const uint32_t *plane, uint32_t *bits, cudaStream_t st);
+void cd_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
+               const uint32_t *mask, const uint32_t *busy, uint32_t *evs, const uint32_t *infb,
+               const uint32_t *susb, uint32_t *evb, uint32_t step, const StepConsts &c,
+               cudaStream_t st);
+// ca, cb: class planes (packed_classify's), or null.
+void cd_flow(const PackedLayout &L, const CdSources &src, uint32_t *busy, uint32_t *mask,
+             uint32_t *ca, uint32_t *cb, uint32_t *infb, uint32_t *susb,
+             unsigned long long *ev_row, const int32_t *net_first, int32_t n_nets,
+             cudaStream_t st);
+// The same rule with per-replica codes into the host's countdown table (next |
+// class << 16 | infectious << 18), 1 or 2 bytes each: for replays whose sets
+// of replicas per age would not fit.
 rp_status cd_prepare();
 void cd_init(const PackedLayout &L, const PackedTask *tasks, const uint32_t *infected,
              void *codes, int code_bytes, uint32_t *mask, const uint32_t *tab,
