@@ -658,19 +658,23 @@ struct rp_sim {
 };
 
 // Mean-field replay: the schedule and prebuilt window CSRs of a geometric
-// simulation, FP32 probability planes, checkpoints every K steps.
+// simulation, FP32 probability planes; the forward keeps every state for the
+// adjoint where they fit in kMfKeepBytes (a third of the adjoint's time was
+// recomputing them), else checkpoints every K steps.
+constexpr int64_t kMfKeepBytes = 4ll << 30;
 struct rp_meanfield {
   ParkGuard park;  // destroyed last (see rp_sim)
   rp_sim base;
-  int32_t N = 0, T = 0, K = 24, nblk = 0, n_ckpt = 0;
+  int32_t N = 0, T = 0, K = 24, nwarp = 0, n_ckpt = 0;
+  bool keep = false;           // ckpt holds x_0 .. x_T, seg_q and seg_e every step
   MfRates rates{};
   bool have_forward = false, has_sus = false;
   DevBuf ckpt;                 // n_ckpt x 4N: x_0, x_K, x_2K, ...
   DevBuf xa, xb;               // 4N ping-pong
   DevBuf seg_x, seg_q, seg_e;  // recomputed segment: K x 4N, K x N, K x N
-  DevBuf inc_part;             // T x blocks incidence partials
+  DevBuf inc_part;             // T x warps incidence partials
   DevBuf a0, a1, z0, z1;       // adjoint ping-pong (4N), coupling terms (N)
-  DevBuf gpart;                // blocks x 4 FP64 scalar-gradient partials
+  DevBuf gpart;                // warps x 4 FP64 scalar-gradient partials
   DevBuf sus;                  // copy of the forward's susceptibility (ones when none)
   DevBuf ones;                 // N x 1.0f
   DevBuf d_rates;              // MfRates read by the kernels
@@ -1069,35 +1073,43 @@ rp_status mf_capture(rp_meanfield &m, cudaGraphExec_t &exec, F body) {
   return RP_OK;
 }
 
-// The forward over every step from ckpt[0]: states ping-pong in xa/xb,
-// checkpoints every K steps, per-step incidence into m.inc.
+// The forward over every step from ckpt[0]: every state kept, or states
+// ping-ponging in xa/xb with checkpoints every K steps; per-step incidence
+// into m.inc.
 rp_status mf_capture_forward(rp_meanfield &m) {
   const int32_t N = m.N, T = m.T;
   const size_t plane = sizeof(float) * 4 * (size_t)N;
   float *ck = m.ckpt.as<float>();
   float *pp[2] = {m.xa.as<float>(), m.xb.as<float>()};
-  m.final_x = T > 0 ? pp[(T - 1) & 1] : ck;
+  m.final_x = m.keep ? ck + (size_t)T * 4 * N : (T > 0 ? pp[(T - 1) & 1] : ck);
   return mf_capture(m, m.fwd, [&](cudaStream_t st) -> rp_status {
     const float *x = ck;
+    bool after_kernel = false;
     for (int32_t t = 0; t < T; ++t) {
-      float *nxt = pp[t & 1];
+      float *nxt = m.keep ? ck + (size_t)(t + 1) * 4 * N : pp[t & 1];
       mf_step(m.base.rp_of(t), m.base.ent_of(t), N, m.base.step_scale[t],
-              m.d_rates.as<MfRates>(), m.sus.as<float>(), x, nxt, nullptr, nullptr,
-              m.inc_part.as<float>() + (size_t)t * m.nblk, st);
-      if ((t + 1) % m.K == 0 && t + 1 < T)
+              m.d_rates.as<MfRates>(), m.sus.as<float>(), x, nxt,
+              m.keep ? m.seg_q.as<float>() + (size_t)t * N : nullptr,
+              m.keep ? m.seg_e.as<float>() + (size_t)t * N : nullptr,
+              m.inc_part.as<float>() + (size_t)t * m.nwarp, after_kernel, st);
+      after_kernel = true;
+      if (!m.keep && (t + 1) % m.K == 0 && t + 1 < T) {
         RP_TRY_CUDA(cudaMemcpyAsync(ck + (size_t)((t + 1) / m.K) * 4 * N, nxt, plane,
                                     cudaMemcpyDeviceToDevice, st));
+        after_kernel = false;
+      }
       x = nxt;
     }
-    mf_incidence(m.inc_part.as<float>(), m.nblk, T, m.inc.as<float>(), st);
+    mf_incidence(m.inc_part.as<float>(), m.nwarp, T, m.inc.as<float>(), st);
     return RP_OK;
   });
 }
 
 // The adjoint from y = a0 (dL/dx_T) and m.ginc (dL/dincidence) back to
 // dL/dx_0 (gx0), with dL/ds (gsus) and the FP64 rate gradients (grates):
-// per checkpoint segment the states, exp(-beta s e) and scaled exposures
-// are recomputed, then one kernel per reverse step.
+// where the forward kept no states, those of a checkpoint segment are
+// recomputed with exp(-beta s e) and the scaled exposures; then one kernel per
+// reverse step.
 rp_status mf_capture_backward(rp_meanfield &m) {
   const int32_t N = m.N, T = m.T, K = m.K;
   const size_t plane = sizeof(float) * 4 * (size_t)N;
@@ -1113,16 +1125,20 @@ rp_status mf_capture_backward(rp_meanfield &m) {
     float *sx = m.seg_x.as<float>(), *sq = m.seg_q.as<float>(), *se = m.seg_e.as<float>();
     // x of step t within the recomputed segment starting at c0
     auto seg_state = [&](int32_t c0, int32_t t) -> const float * {
+      if (m.keep) return ck + (size_t)t * 4 * N;
       return t == c0 ? ck + (size_t)(c0 / K) * 4 * N : sx + (size_t)(t - c0) * 4 * N;
     };
+    bool after_kernel = false;
     for (int32_t t = T - 1; t >= 0; --t) {
-      const int32_t c0 = (t / K) * K;
-      if (t == T - 1 || t == c0 + K - 1) {
+      const int32_t c0 = m.keep ? 0 : (t / K) * K;
+      if (!m.keep && (t == T - 1 || t == c0 + K - 1)) {
         for (int32_t u = c0; u <= t; ++u) {
           float *xo = u + 1 <= t ? sx + (size_t)(u + 1 - c0) * 4 * N : m.xa.as<float>();
+          // the first rewrites a segment that the previous kernel reads
           mf_step(m.base.rp_of(u), m.base.ent_of(u), N, m.base.step_scale[u], r, sus,
                   seg_state(c0, u), xo, sq + (size_t)(u - c0) * N, se + (size_t)(u - c0) * N,
-                  m.inc_part.as<float>() + (size_t)u * m.nblk, st);
+                  m.inc_part.as<float>() + (size_t)u * m.nwarp, after_kernel, st);
+          after_kernel = true;
         }
       }
       const bool couple = t + 1 < T;
@@ -1130,15 +1146,17 @@ rp_status mf_capture_backward(rp_meanfield &m) {
                  couple ? m.base.ent_of(t + 1) : nullptr, z[(t + 1) & 1], a[ai],
                  seg_state(c0, t), sq + (size_t)(t - c0) * N, se + (size_t)(t - c0) * N,
                  m.ginc.as<float>(), t, m.base.step_scale[t], r, sus, a[ai ^ 1], z[t & 1],
-                 m.gsus.as<float>(), m.gpart.as<double>(), st);
+                 m.gsus.as<float>(), m.gpart.as<double>(), m.keep, after_kernel, st);
+      after_kernel = true;
       ai ^= 1;
     }
     if (T > 0)
       mf_adjoint(N, m.base.rp_of(0), m.base.ent_of(0), z[0], a[ai], nullptr, nullptr, nullptr,
-                 nullptr, 0, 1.0f, r, sus, m.gx0.as<float>(), nullptr, nullptr, nullptr, st);
+                 nullptr, 0, 1.0f, r, sus, m.gx0.as<float>(), nullptr, nullptr, nullptr, false,
+                 true, st);
     else
       RP_TRY_CUDA(cudaMemcpyAsync(m.gx0.ptr, a[ai], plane, cudaMemcpyDeviceToDevice, st));
-    mf_finish(m.gpart.as<double>(), m.nblk, m.grates.as<double>(), st);
+    mf_finish(m.gpart.as<double>(), m.nwarp, m.grates.as<double>(), st);
     return RP_OK;
   });
 }
@@ -1788,21 +1806,29 @@ RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
   m->N = N;
   m->T = T;
   m->K = checkpoint_every < (T > 0 ? T : 1) ? checkpoint_every : (T > 0 ? T : 1);
-  m->nblk = mf_blocks(N);
-  m->n_ckpt = T > 0 ? (T + m->K - 1) / m->K : 1;
+  m->nwarp = mf_warps(N);
   const size_t plane = sizeof(float) * 4 * (size_t)N;
-  RP_TRY(m->ckpt.alloc(plane * m->n_ckpt));
-  RP_TRY(m->xa.alloc(plane));
-  RP_TRY(m->xb.alloc(plane));
-  RP_TRY(m->seg_x.alloc(plane * m->K));
-  RP_TRY(m->seg_q.alloc(sizeof(float) * (size_t)N * m->K));
-  RP_TRY(m->seg_e.alloc(sizeof(float) * (size_t)N * m->K));
-  RP_TRY(m->inc_part.alloc(sizeof(float) * (size_t)m->nblk * (T > 0 ? T : 1)));
+  const size_t per_step = sizeof(float) * (size_t)N;
+  // every state, exp(-beta s e) and exposure of the forward, or checkpoints
+  m->keep = (int64_t)(plane * ((size_t)T + 1) + 2 * per_step * T) <= kMfKeepBytes &&
+            m->ckpt.alloc(plane * ((size_t)T + 1)) == RP_OK &&
+            m->seg_q.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
+            m->seg_e.alloc(per_step * (T > 0 ? T : 1)) == RP_OK;
+  if (!m->keep) {
+    m->n_ckpt = T > 0 ? (T + m->K - 1) / m->K : 1;
+    RP_TRY(m->ckpt.alloc(plane * m->n_ckpt));
+    RP_TRY(m->xa.alloc(plane));
+    RP_TRY(m->xb.alloc(plane));
+    RP_TRY(m->seg_x.alloc(plane * m->K));
+    RP_TRY(m->seg_q.alloc(per_step * m->K));
+    RP_TRY(m->seg_e.alloc(per_step * m->K));
+  }
+  RP_TRY(m->inc_part.alloc(sizeof(float) * (size_t)m->nwarp * (T > 0 ? T : 1)));
   RP_TRY(m->a0.alloc(plane));
   RP_TRY(m->a1.alloc(plane));
   RP_TRY(m->z0.alloc(sizeof(float) * (size_t)N));
   RP_TRY(m->z1.alloc(sizeof(float) * (size_t)N));
-  RP_TRY(m->gpart.alloc(sizeof(double) * 4 * (size_t)m->nblk));
+  RP_TRY(m->gpart.alloc(sizeof(double) * 4 * (size_t)m->nwarp));
   RP_TRY(m->sus.alloc(sizeof(float) * (size_t)N));
   RP_TRY(m->ones.alloc(sizeof(float) * (size_t)N));
   {
