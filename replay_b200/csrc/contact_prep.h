@@ -1,5 +1,6 @@
-// Host preparation of caller-given contact arrays before the device index
-// build (rp_graph_from_arrays): endpoints ordered u <= v (the reference's
+// Preparation of caller-given contact arrays on the host, the reference of the
+// device pass that rp_graph_from_arrays runs (k_endpoints in ingest.cu; not part
+// of the library): endpoints ordered u <= v (the reference's
 // pair packing, tool/temporal_contact_matrix.c:80-90), range checks, and the
 // number of distinct nodes that appear.  Header-only so that a host-side
 // test can compile it without the CUDA runtime.

@@ -544,53 +544,4 @@ rp_status parse_contact_file(const char *path, ParsedContacts &out) {
   return RP_OK;
 }
 
-// ---------------------------------------------------------------------------
-static int64_t sat_sub(int64_t a, int64_t b) {  // a - b, b >= 0, saturating
-  if (a < INT64_MIN + b) return INT64_MIN;
-  return a - b;
-}
-
-int32_t plan_window_ranges(const Graph &g, int64_t ws, int64_t we, float scale, int64_t cap,
-                           CandRange *ranges, WinDesc &out) {
-  out.ws = ws;
-  out.we = we;
-  out.scale = scale;
-  // The reference mirrors a query whose start is negative (intervaldb.c:437-444).
-  if (ws < 0) {
-    out.qs = -we;
-    out.qe = -ws;
-  } else {
-    out.qs = ws;
-    out.qe = we;
-  }
-  out.range_off = 0;
-  out.hit_off = 0;
-  out.n_ranges = 0;
-  out.n_candidates = 0;
-  for (int c = 0; c < kClasses; ++c) {
-    const int64_t b0 = g.class_off[c], b1 = g.class_off[c + 1];
-    if (b1 <= b0) continue;
-    // candidates: stored start in (qs - 2^c, qe)
-    const int64_t span = c >= 63 ? INT64_MAX : ((int64_t)1 << c);
-    const int64_t lo_key = sat_sub(out.qs, span);  // start > lo_key
-    auto first = g.h_cs.begin() + b0, last = g.h_cs.begin() + b1;
-    auto lo = std::upper_bound(first, last, lo_key);
-    auto hi = std::lower_bound(lo, last, out.qe);
-    const int64_t count = hi - lo;
-    if (count <= 0) continue;
-    ranges[out.n_ranges++] = CandRange{(int64_t)(lo - g.h_cs.begin()), count, out.n_candidates};
-    out.n_candidates += count;
-  }
-  out.may_truncate = out.n_candidates > cap ? 1 : 0;
-  return out.n_ranges;
-}
-
-void plan_window(const Graph &g, int64_t ws, int64_t we, float scale,
-                 int64_t cap, std::vector<CandRange> &ranges, WinDesc &out) {
-  CandRange r[kClasses];
-  const int32_t n = plan_window_ranges(g, ws, we, scale, cap, r, out);
-  out.range_off = (int32_t)ranges.size();
-  ranges.insert(ranges.end(), r, r + n);
-}
-
 }  // namespace rp

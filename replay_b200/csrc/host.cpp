@@ -18,7 +18,6 @@
 #include <thread>
 #include <vector>
 
-#include "contact_prep.h"
 #include "rp_internal.h"
 
 namespace rp {
@@ -813,17 +812,18 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
   RP_TRY(make_schedule(p, s.step_ws, s.step_scale, s.step_ts));
   s.cap = p.ncls_cap ? (g.nlists > 0 ? g.nlists : 1) : INT64_MAX;
   s.step_win.resize(s.T);
-  int64_t max_cand = 0;
+  std::vector<int64_t> starts;
+  std::vector<float> scales;
   for (int32_t t = 0; t < s.T; ++t) {
     if (t == 0 || s.step_ws[t] != s.step_ws[t - 1]) {
-      WinDesc d{};
-      plan_window(g, s.step_ws[t], s.step_ws[t] + p.window, s.step_scale[t], s.cap, s.ranges,
-                  d);
-      s.wins.push_back(d);
-      if (d.n_candidates > max_cand) max_cand = d.n_candidates;
+      starts.push_back(s.step_ws[t]);
+      scales.push_back(s.step_scale[t]);
     }
-    s.step_win[t] = (int32_t)s.wins.size() - 1;
+    s.step_win[t] = (int32_t)starts.size() - 1;
   }
+  RP_TRY(plan_windows(g, starts, p.window, scales, s.cap, s.ranges, s.wins));
+  int64_t max_cand = 0;
+  for (const WinDesc &d : s.wins) max_cand = std::max(max_cand, d.n_candidates);
   if (max_cand > (int64_t)INT32_MAX / 2) {
     set_error("a window has %lld candidate contacts; at most 2^30 are supported",
               (long long)max_cand);
@@ -1198,7 +1198,8 @@ RP_API rp_status rp_graph_load_text(const char *path, int device, rp_graph **out
   h->g.n_malformed = pc.n_malformed;
   h->prep_ms = ms_since(t0);
   const auto t1 = std::chrono::steady_clock::now();
-  RP_TRY(graph_build_device(h->g, pc.start, pc.end, pc.u, pc.v, pc.n, pc.n_nodes));
+  int64_t bad = -1;
+  RP_TRY(graph_build_device(h->g, pc.start, pc.end, pc.u, pc.v, pc.n, pc.n_nodes, false, &bad));
   RP_TRY_CUDA(cudaDeviceSynchronize());
   h->build_ms = ms_since(t1);
   *out = h.release();
@@ -1238,21 +1239,24 @@ RP_API rp_status rp_graph_from_arrays(const int64_t *start, const int64_t *end,
   }
   *out = nullptr;
   const auto t0 = std::chrono::steady_clock::now();
-  std::vector<int32_t> uu(n_contacts), vv(n_contacts);
-  int32_t n_index = 0;
-  const int threads = (int)std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
-  const int64_t bad = prep_contacts(u, v, n_contacts, n_nodes, uu.data(), vv.data(), &n_index,
-                                    threads);
+  std::unique_ptr<rp_graph> h(new rp_graph());
+  h->g.device = device;
+  h->prep_ms = ms_since(t0);
+  const auto t1 = std::chrono::steady_clock::now();
+  // the endpoints are ordered, checked and counted on the device; without one,
+  // an argument error still comes before the device error
+  int64_t bad = -1;
+  const rp_status st =
+      graph_build_device(h->g, start, end, u, v, n_contacts, n_nodes, true, &bad);
+  if (st == RP_ERR_CUDA) {
+    for (int64_t k = 0; k < n_contacts && bad < 0; ++k)
+      if (u[k] < 0 || v[k] < 0 || u[k] >= n_nodes || v[k] >= n_nodes) bad = k;
+  }
   if (bad >= 0) {
     set_error("contact %lld joins node outside [0, %d)", (long long)bad, n_nodes);
     return RP_ERR_ARG;
   }
-  std::unique_ptr<rp_graph> h(new rp_graph());
-  h->g.device = device;
-  h->g.n_index = n_index;
-  h->prep_ms = ms_since(t0);
-  const auto t1 = std::chrono::steady_clock::now();
-  RP_TRY(graph_build_device(h->g, start, end, uu.data(), vv.data(), n_contacts, n_nodes));
+  RP_TRY(st);
   RP_TRY_CUDA(cudaDeviceSynchronize());
   h->build_ms = ms_since(t1);
   *out = h.release();
@@ -1297,9 +1301,9 @@ RP_API rp_status rp_window_csr(rp_graph *h, int64_t ws, int64_t we, float scale,
   }
   RP_TRY_CUDA(cudaSetDevice(g.device));
   const int64_t cap = ncls_cap ? (g.nlists > 0 ? g.nlists : 1) : INT64_MAX;
-  std::vector<WinDesc> wins(1);
+  std::vector<WinDesc> wins;
   std::vector<CandRange> ranges;
-  plan_window(g, ws, we, scale, cap, ranges, wins[0]);
+  RP_TRY(plan_windows(g, {ws}, we - ws, {scale}, cap, ranges, wins));
   WindowWorkspace w;
   std::vector<WindowGroup> one;
   plan_window_groups(wins, g.n_nodes, true, one);

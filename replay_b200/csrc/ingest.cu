@@ -15,7 +15,7 @@
 //      maximum end was first reached -- a prefix scan;
 //   4. duration classes (class 0: duration <= 1, class c: (2^(c-1), 2^c]),
 //      a stable partition: one more radix pass on the class.
-// The host keeps only the class-ordered starts (window planning).
+// Window queries are planned on the device, too (k_plan).
 #include <algorithm>
 
 #include "rp_internal.h"
@@ -213,57 +213,186 @@ __global__ void k_gather(const T *__restrict__ src, const uint32_t *__restrict__
 
 struct MaxFirst {  // running maximum end and the first index reaching it
   int64_t v;
-  int64_t at;
+  int64_t at;  // -1: nothing before
 };
-__device__ __forceinline__ MaxFirst combine(MaxFirst a, MaxFirst b) { return b.v > a.v ? b : a; }
-
-constexpr int kNestChunk = 4096;
-
-__global__ void __launch_bounds__(256)
-    k_nest_chunks(const int64_t *__restrict__ se, int64_t n, MaxFirst *__restrict__ agg) {
-  // sequential per chunk is enough here: one thread per chunk
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t b = c * kNestChunk;
-  if (b >= n) return;
-  const int64_t e = min(n, b + kNestChunk);
-  MaxFirst m{se[b], b};
-  for (int64_t i = b + 1; i < e; ++i) m = combine(m, MaxFirst{se[i], i});
-  agg[c] = m;
+// b follows a.
+__device__ __forceinline__ MaxFirst combine(MaxFirst a, MaxFirst b) {
+  return a.at < 0 || (b.at >= 0 && b.v > a.v) ? b : a;
+}
+__device__ __forceinline__ MaxFirst shfl_up(MaxFirst m, int o) {
+  return MaxFirst{__shfl_up_sync(0xFFFFFFFFu, m.v, o), __shfl_up_sync(0xFFFFFFFFu, m.at, o)};
+}
+// Inclusive scan of one value per thread in thread order; the last thread's
+// is the block's total.
+__device__ __forceinline__ MaxFirst block_scan(MaxFirst m, MaxFirst *ws) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const MaxFirst y = shfl_up(m, o);
+    if (lane >= o) m = combine(y, m);
+  }
+  if (lane == 31) ws[warp] = m;
+  __syncthreads();
+  if (warp == 0) {
+    MaxFirst w = lane < (int)(blockDim.x >> 5) ? ws[lane] : MaxFirst{0, -1};
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const MaxFirst y = shfl_up(w, o);
+      if (lane >= o) w = combine(y, w);
+    }
+    ws[lane] = w;
+  }
+  __syncthreads();
+  if (warp > 0) m = combine(ws[warp - 1], m);
+  __syncthreads();
+  return m;
 }
 
-__global__ void k_nest_prefix(MaxFirst *__restrict__ agg, int64_t n_chunks) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  MaxFirst run{INT64_MIN, -1};
-  for (int64_t c = 0; c < n_chunks; ++c) {
+// One block per chunk, 16 contacts per thread.  (One thread per chunk walked
+// its 4,096 contacts one load after another: 0.6 + 2.4 ms for the two passes at
+// 1.4M contacts; 0.08 + 0.26 ms now at 20M.)
+constexpr int kNestItems = 16, kNestThreads = 256;
+constexpr int kNestChunk = kNestItems * kNestThreads;
+
+__device__ __forceinline__ MaxFirst thread_max(const int64_t *__restrict__ se, int64_t b,
+                                               int64_t e) {
+  MaxFirst m{0, -1};
+#pragma unroll 4
+  for (int64_t i = b; i < e; ++i) m = combine(m, MaxFirst{se[i], i});
+  return m;
+}
+
+__global__ void __launch_bounds__(kNestThreads)
+    k_nest_chunks(const int64_t *__restrict__ se, int64_t n, MaxFirst *__restrict__ agg) {
+  __shared__ MaxFirst ws[32];
+  const int64_t b = (int64_t)blockIdx.x * kNestChunk + threadIdx.x * kNestItems;
+  const MaxFirst m = block_scan(thread_max(se, b, min(n, b + kNestItems)), ws);
+  if (threadIdx.x == blockDim.x - 1) agg[blockIdx.x] = m;
+}
+
+// Exclusive scan of the chunks' maxima (one block).
+__global__ void __launch_bounds__(1024)
+    k_nest_prefix(MaxFirst *__restrict__ agg, int64_t n_chunks) {
+  __shared__ MaxFirst ws[32];
+  __shared__ MaxFirst s_last[1024];
+  const int64_t per = (n_chunks + blockDim.x - 1) / blockDim.x;
+  const int64_t b = threadIdx.x * per, e = min(n_chunks, b + per);
+  MaxFirst m{0, -1};
+  for (int64_t c = b; c < e; ++c) m = combine(m, agg[c]);
+  s_last[threadIdx.x] = block_scan(m, ws);
+  __syncthreads();
+  MaxFirst run = threadIdx.x ? s_last[threadIdx.x - 1] : MaxFirst{0, -1};
+  for (int64_t c = b; c < e; ++c) {
     const MaxFirst v = agg[c];
-    agg[c] = run;  // exclusive
-    run = c == 0 ? v : combine(run, v);
+    agg[c] = run;
+    run = combine(run, v);
   }
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kNestThreads)
     k_nest_count(const int64_t *__restrict__ ss, const int64_t *__restrict__ se, int64_t n,
                  const MaxFirst *__restrict__ agg, unsigned long long *__restrict__ counters) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t b = c * kNestChunk;
-  if (b >= n) return;
-  const int64_t e = min(n, b + kNestChunk);
-  MaxFirst run = agg[c];
-  unsigned long long top = 0, parents = 0;
+  __shared__ MaxFirst ws[32];
+  __shared__ MaxFirst s_last[kNestThreads];
+  const int64_t b = (int64_t)blockIdx.x * kNestChunk + threadIdx.x * kNestItems;
+  const int64_t e = min(n, b + kNestItems);
+  s_last[threadIdx.x] = block_scan(thread_max(se, b, e), ws);
+  __syncthreads();
+  MaxFirst run = agg[blockIdx.x];
+  if (threadIdx.x) run = combine(run, s_last[threadIdx.x - 1]);
+  int64_t root_start = run.at >= 0 && b < e ? ss[run.at] : 0;
+  unsigned top = 0, parents = 0;
   for (int64_t i = b; i < e; ++i) {
-    // i is top-level iff outside the chain root R = run.at (none for i = 0)
-    bool is_top = run.at < 0;
-    if (!is_top) {
-      const int64_t r = run.at;
-      is_top = se[i] > se[r] || (se[i] == se[r] && ss[i] == ss[r]);
-    }
-    top += is_top;
+    const int64_t s0 = ss[i], e0 = se[i];
+    // i is top-level iff outside the chain root run.at (none for i = 0)
+    top += run.at < 0 || e0 > run.v || (e0 == run.v && s0 == root_start);
     // i has a child iff i+1 is not outside i
-    if (i + 1 < n) parents += !(se[i + 1] > se[i] || (se[i + 1] == se[i] && ss[i + 1] == ss[i]));
-    run = run.at < 0 ? MaxFirst{se[i], i} : combine(run, MaxFirst{se[i], i});
+    if (i + 1 < n) parents += !(se[i + 1] > e0 || (se[i + 1] == e0 && ss[i + 1] == s0));
+    if (run.at < 0 || e0 > run.v) {
+      run = MaxFirst{e0, i};
+      root_start = s0;
+    }
   }
-  atomicAdd(&counters[0], top);
-  atomicAdd(&counters[1], parents);
+  top = __reduce_add_sync(0xFFFFFFFFu, top);
+  parents = __reduce_add_sync(0xFFFFFFFFu, parents);
+  if ((threadIdx.x & 31) == 0) {
+    if (top) atomicAdd(&counters[0], (unsigned long long)top);
+    if (parents) atomicAdd(&counters[1], (unsigned long long)parents);
+  }
+}
+
+// Endpoints as the caller gave them: ordered u <= v (the reference's pair
+// packing, tool/temporal_contact_matrix.c:80-90), nodes that appear marked,
+// and the first contact with an endpoint outside [0, n_nodes).
+__global__ void __launch_bounds__(256)
+    k_endpoints(int32_t *__restrict__ u, int32_t *__restrict__ v, int64_t n, int32_t n_nodes,
+                uint8_t *__restrict__ seen, unsigned long long *__restrict__ bad) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t a = u[i], b = v[i];
+    if ((uint32_t)a >= (uint32_t)n_nodes || (uint32_t)b >= (uint32_t)n_nodes) {
+      atomicMin(bad, (unsigned long long)i);
+      continue;
+    }
+    if (a > b) {
+      u[i] = b;
+      v[i] = a;
+    }
+    if (!seen[a]) seen[a] = 1;
+    if (!seen[b]) seen[b] = 1;
+  }
+}
+__global__ void __launch_bounds__(256)
+    k_count_seen(const uint8_t *__restrict__ seen, int32_t n_nodes,
+                 unsigned long long *__restrict__ count) {
+  unsigned c = 0;
+  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x)
+    c += seen[i];
+  c = __reduce_add_sync(0xFFFFFFFFu, c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
+}
+
+// ---- window planning ----------------------------------------------------------
+// One thread per (window, class in use): the candidates of the query are the
+// class's starts in (qs - 2^c, qe).  (On the host this needed a copy of every
+// start: 160 MB for 20M contacts.)
+struct PlanArgs {
+  int64_t off[kClasses + 1];
+  int32_t used[kClasses];
+  int32_t n_used;
+  const int64_t *ws;   // window starts, or null: the one window ws0
+  int64_t ws0, length;
+  int32_t n_windows;
+};
+// The reference mirrors a query whose start is negative (intervaldb.c:437-444).
+__host__ __device__ inline void query_of(int64_t ws, int64_t we, int64_t &qs, int64_t &qe) {
+  qs = ws < 0 ? -we : ws;
+  qe = ws < 0 ? -ws : we;
+}
+__global__ void __launch_bounds__(128)
+    k_plan(const __grid_constant__ PlanArgs a, const int64_t *__restrict__ cs,
+           int64_t *__restrict__ lo_out, int64_t *__restrict__ count_out) {
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= (int64_t)a.n_windows * a.n_used) return;
+  const int64_t ws = a.ws ? a.ws[j / a.n_used] : a.ws0;
+  const int c = a.used[j % a.n_used];
+  int64_t qs, qe;
+  query_of(ws, ws + a.length, qs, qe);
+  const int64_t span = c >= 63 ? INT64_MAX : ((int64_t)1 << c);
+  const int64_t lo_key = qs < INT64_MIN + span ? INT64_MIN : qs - span;  // start > lo_key
+  int64_t lo = a.off[c], end = a.off[c + 1], hi = end;
+  while (lo < hi) {  // first start > lo_key
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (cs[mid] > lo_key) hi = mid; else lo = mid + 1;
+  }
+  int64_t h = lo;
+  hi = end;
+  while (h < hi) {  // first start >= qe
+    const int64_t mid = h + (hi - h) / 2;
+    if (cs[mid] >= qe) hi = mid; else h = mid + 1;
+  }
+  lo_out[j] = lo;
+  count_out[j] = h - lo;
 }
 
 // duration class keys (sorted order) and per-class counts
@@ -326,7 +455,9 @@ rp_status radix_sort(DevBuf &key, DevBuf &val, DevBuf &k2, DevBuf &v2, int64_t n
 }  // namespace
 
 rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end, const int32_t *u,
-                             const int32_t *v, int64_t n, int32_t n_nodes) {
+                             const int32_t *v, int64_t n, int32_t n_nodes, bool raw,
+                             int64_t *bad) {
+  *bad = -1;
   g.n_nodes = n_nodes;
   g.n_contacts = n;
   if (n > (int64_t)INT32_MAX) {
@@ -342,12 +473,11 @@ rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
   RP_TRY(g.cu.alloc(sizeof(int32_t) * n));
   RP_TRY(g.cv.alloc(sizeof(int32_t) * n));
   RP_TRY(g.crank.alloc(sizeof(int32_t) * n));
-  g.h_cs.clear();
   if (n == 0) return RP_OK;
   cudaStream_t st = nullptr;
   // the scratch below is kept for the next build once the stream is idle
   ParkGuard park;
-  DevBuf s, e, uu, vv, key, val, k2, v2, counts, offs, sums, mm, ctr, agg, ss, se, su, sv;
+  DevBuf s, e, uu, vv, key, val, k2, v2, counts, offs, sums, mm, ctr, agg, ss, se, su, sv, seen;
   RP_TRY(s.alloc(sizeof(int64_t) * n));
   RP_TRY(e.alloc(sizeof(int64_t) * n));
   RP_TRY(uu.alloc(sizeof(int32_t) * n));
@@ -358,14 +488,31 @@ rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
   RP_TRY_CUDA(cudaMemcpyAsync(vv.ptr, v, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
 
   // 1. stored coordinates and the key ranges
-  RP_TRY(mm.alloc(sizeof(unsigned long long) * 4));
-  const unsigned long long init[4] = {~0ull, 0ull, ~0ull, 0ull};
+  // (and, for endpoints from a caller, their order, range and number)
+  RP_TRY(mm.alloc(sizeof(unsigned long long) * 6));
+  const unsigned long long init[6] = {~0ull, 0ull, ~0ull, 0ull, ~0ull, 0ull};
   RP_TRY_CUDA(cudaMemcpyAsync(mm.ptr, init, sizeof(init), cudaMemcpyHostToDevice, st));
   k_store_coords<<<grid_of(n, 256), 256, 0, st>>>(s.as<int64_t>(), e.as<int64_t>(), n,
                                                   mm.as<unsigned long long>());
-  unsigned long long hmm[4];
+  if (raw) {
+    RP_TRY(seen.alloc((size_t)n_nodes));
+    RP_TRY_CUDA(cudaMemsetAsync(seen.ptr, 0, (size_t)n_nodes, st));
+    k_endpoints<<<grid_of(n, 256), 256, 0, st>>>(uu.as<int32_t>(), vv.as<int32_t>(), n, n_nodes,
+                                                 seen.as<uint8_t>(),
+                                                 mm.as<unsigned long long>() + 4);
+    k_count_seen<<<grid_of(n_nodes, 256), 256, 0, st>>>(seen.as<uint8_t>(), n_nodes,
+                                                        mm.as<unsigned long long>() + 5);
+  }
+  unsigned long long hmm[6];
   RP_TRY_CUDA(cudaMemcpyAsync(hmm, mm.ptr, sizeof(hmm), cudaMemcpyDeviceToHost, st));
   RP_TRY_CUDA(cudaStreamSynchronize(st));
+  if (raw) {
+    if (hmm[4] != ~0ull) {
+      *bad = (int64_t)hmm[4];
+      return RP_OK;  // the caller reports it
+    }
+    g.n_index = (int32_t)hmm[5];
+  }
   const int64_t smin = (int64_t)(hmm[0] ^ 0x8000000000000000ull);
   const int64_t smax = (int64_t)(hmm[1] ^ 0x8000000000000000ull);
   const int64_t emin = (int64_t)(hmm[2] ^ 0x8000000000000000ull);
@@ -417,10 +564,10 @@ rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
   RP_TRY(agg.alloc(sizeof(MaxFirst) * n_chunks));
   RP_TRY(ctr.alloc(sizeof(unsigned long long) * (2 + kClasses)));
   RP_TRY_CUDA(cudaMemsetAsync(ctr.ptr, 0, ctr.bytes, st));
-  const int nb = (int)((n_chunks + 255) / 256);
-  k_nest_chunks<<<nb, 256, 0, st>>>(se.as<int64_t>(), n, agg.as<MaxFirst>());
-  k_nest_prefix<<<1, 32, 0, st>>>(agg.as<MaxFirst>(), n_chunks);
-  k_nest_count<<<nb, 256, 0, st>>>(ss.as<int64_t>(), se.as<int64_t>(), n, agg.as<MaxFirst>(),
+  const int nb = (int)n_chunks;
+  k_nest_chunks<<<nb, kNestThreads, 0, st>>>(se.as<int64_t>(), n, agg.as<MaxFirst>());
+  k_nest_prefix<<<1, 1024, 0, st>>>(agg.as<MaxFirst>(), n_chunks);
+  k_nest_count<<<nb, kNestThreads, 0, st>>>(ss.as<int64_t>(), se.as<int64_t>(), n, agg.as<MaxFirst>(),
                                    ctr.as<unsigned long long>());
 
   // 4. stable partition by duration class; class c's rank in (start, end)
@@ -439,9 +586,6 @@ rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
 
   unsigned long long hc[2 + kClasses];
   RP_TRY_CUDA(cudaMemcpyAsync(hc, ctr.ptr, sizeof(hc), cudaMemcpyDeviceToHost, st));
-  g.h_cs.resize(n);
-  RP_TRY_CUDA(cudaMemcpyAsync(g.h_cs.data(), g.cs.ptr, sizeof(int64_t) * n, cudaMemcpyDeviceToHost,
-                              st));
   RP_TRY_CUDA(cudaStreamSynchronize(st));
   park.arm();
   g.nlists = ((int64_t)hc[0] - 1) + (int64_t)hc[1];
@@ -449,6 +593,88 @@ rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
     g.class_off[c + 1] = g.class_off[c] + (int64_t)hc[2 + c];
     g.n_classes_used += hc[2 + c] > 0;
   }
+  return RP_OK;
+}
+
+namespace {
+PlanArgs plan_args(const Graph &g, int64_t length) {
+  PlanArgs a{};
+  for (int c = 0; c <= kClasses; ++c) a.off[c] = g.class_off[c];
+  for (int c = 0; c < kClasses; ++c)
+    if (g.class_off[c + 1] > g.class_off[c]) a.used[a.n_used++] = c;
+  a.length = length;
+  return a;
+}
+// The window's candidate ranges (at most kClasses, to `ranges`) from k_plan's
+// answers for the classes in use.
+void window_desc(int64_t ws, int64_t we, float scale, int64_t cap, int32_t n_used,
+                 const int64_t *lo, const int64_t *count, CandRange *ranges, WinDesc &out) {
+  out = WinDesc{};
+  out.ws = ws;
+  out.we = we;
+  out.scale = scale;
+  query_of(ws, we, out.qs, out.qe);
+  for (int32_t c = 0; c < n_used; ++c) {
+    if (count[c] <= 0) continue;
+    ranges[out.n_ranges++] = CandRange{lo[c], count[c], out.n_candidates};
+    out.n_candidates += count[c];
+  }
+  out.may_truncate = out.n_candidates > cap ? 1 : 0;
+}
+}  // namespace
+
+rp_status plan_windows(const Graph &g, const std::vector<int64_t> &ws, int64_t length,
+                       const std::vector<float> &scale, int64_t cap,
+                       std::vector<CandRange> &ranges, std::vector<WinDesc> &wins) {
+  PlanArgs a = plan_args(g, length);
+  const size_t W = ws.size(), n = W * (size_t)a.n_used;
+  std::vector<int64_t> out(2 * n);
+  if (n > 0) {
+    cudaStream_t st = nullptr;
+    ParkGuard park;
+    DevBuf d_ws, d_out;
+    RP_TRY(d_ws.alloc(sizeof(int64_t) * W));
+    RP_TRY(d_out.alloc(sizeof(int64_t) * 2 * n));
+    RP_TRY_CUDA(cudaMemcpyAsync(d_ws.ptr, ws.data(), sizeof(int64_t) * W, cudaMemcpyHostToDevice,
+                                st));
+    a.ws = d_ws.as<int64_t>();
+    a.n_windows = (int32_t)W;
+    k_plan<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(a, g.cs.as<int64_t>(),
+                                                        d_out.as<int64_t>(),
+                                                        d_out.as<int64_t>() + n);
+    RP_TRY_CUDA(cudaGetLastError());
+    RP_TRY_CUDA(cudaMemcpyAsync(out.data(), d_out.ptr, sizeof(int64_t) * 2 * n,
+                                cudaMemcpyDeviceToHost, st));
+    RP_TRY_CUDA(cudaStreamSynchronize(st));
+    park.arm();
+  }
+  CandRange r[kClasses];
+  for (size_t w = 0; w < W; ++w) {
+    WinDesc d;
+    const size_t at = w * (size_t)a.n_used;
+    window_desc(ws[w], ws[w] + length, scale[w], cap, a.n_used, out.data() + at,
+                out.data() + n + at, r, d);
+    d.range_off = (int32_t)ranges.size();
+    ranges.insert(ranges.end(), r, r + d.n_ranges);
+    wins.push_back(d);
+  }
+  return RP_OK;
+}
+
+rp_status plan_window_noalloc(const Graph &g, int64_t ws, int64_t we, float scale, int64_t cap,
+                              int64_t *scratch, CandRange *ranges, WinDesc &out,
+                              cudaStream_t st) {
+  PlanArgs a = plan_args(g, we - ws);
+  int64_t got[2 * kClasses];
+  if (a.n_used > 0) {
+    a.ws0 = ws;
+    a.n_windows = 1;
+    k_plan<<<1, 128, 0, st>>>(a, g.cs.as<int64_t>(), scratch, scratch + kClasses);
+    RP_TRY_CUDA(cudaGetLastError());
+    RP_TRY_CUDA(cudaMemcpyAsync(got, scratch, sizeof(got), cudaMemcpyDeviceToHost, st));
+    RP_TRY_CUDA(cudaStreamSynchronize(st));
+  }
+  window_desc(ws, we, scale, cap, a.n_used, got, got + kClasses, ranges, out);
   return RP_OK;
 }
 

@@ -195,7 +195,6 @@ struct Graph {
   int64_t t_min = 0, t_max = 0;
   int32_t n_classes_used = 0;
   std::vector<int64_t> class_off;  // kClasses + 1 offsets
-  std::vector<int64_t> h_cs;       // class-ordered stored starts
   DevBuf cs, ce;                   // int64 stored start / end, class order
   DevBuf cu, cv;                   // int32 endpoints (u <= v)
   DevBuf crank;                    // int32 position in (start asc, end desc) order
@@ -220,18 +219,26 @@ struct ParsedContacts {
   void release() { start = end = nullptr, u = v = nullptr; }  // ownership passed on
 };
 rp_status parse_contact_file(const char *path, ParsedContacts &out);
-// Builds the device interval index of n contacts given in host memory
-// (u[k] <= v[k]); ingest.cu.
+// Builds the device interval index of n contacts given in host memory;
+// ingest.cu.  `raw`: the endpoints come as the caller gave them; they are
+// ordered (u <= v), checked and counted (g.n_index) on the device, and *bad is
+// the first contact with an endpoint outside [0, n_nodes), or -1.
 rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
-                             const int32_t *u, const int32_t *v, int64_t n, int32_t n_nodes);
+                             const int32_t *u, const int32_t *v, int64_t n, int32_t n_nodes,
+                             bool raw, int64_t *bad);
 
-// Plans the query of one window: candidate ranges appended to `ranges`.
-// Candidate ranges of window [ws, we) (at most kClasses, written to `ranges`,
-// range_off = 0); returns their number.  plan_window appends them to a list.
-int32_t plan_window_ranges(const Graph &g, int64_t ws, int64_t we, float scale, int64_t cap,
-                           CandRange *ranges, WinDesc &out);
-void plan_window(const Graph &g, int64_t ws, int64_t we, float scale,
-                 int64_t cap, std::vector<CandRange> &ranges, WinDesc &out);
+// Plans the queries of the windows [ws[k], ws[k] + length): candidate ranges
+// appended to `ranges`, one WinDesc each to `wins`.  The binary searches run
+// on the device (ingest.cu).
+rp_status plan_windows(const Graph &g, const std::vector<int64_t> &ws, int64_t length,
+                       const std::vector<float> &scale, int64_t cap,
+                       std::vector<CandRange> &ranges, std::vector<WinDesc> &wins);
+// One window with caller-owned scratch (kPlanBytes on the device); ranges
+// holds kClasses entries.  Synchronizes st.
+constexpr size_t kPlanBytes = sizeof(int64_t) * 2 * kClasses;
+rp_status plan_window_noalloc(const Graph &g, int64_t ws, int64_t we, float scale, int64_t cap,
+                              int64_t *scratch, CandRange *ranges, WinDesc &out,
+                              cudaStream_t st);
 
 // ---- window builder ----------------------------------------------------------
 struct Hit {

@@ -44,7 +44,8 @@ constexpr size_t kTilesOff = kLongOff + kNodeBytes;
 constexpr size_t kCtrOff = kTilesOff + align256(sizeof(int32_t) * kNoAllocMaxTiles);
 constexpr size_t kWinOff = kCtrOff + align256(sizeof(unsigned long long) * 4);
 constexpr size_t kRangeOff = kWinOff + align256(sizeof(WinDesc));
-constexpr size_t kScratchBytes = kRangeOff + align256(sizeof(CandRange) * kClasses);  // ~8.8 MB
+constexpr size_t kPlanOff = kRangeOff + align256(sizeof(CandRange) * kClasses);
+constexpr size_t kScratchBytes = kPlanOff + align256(kPlanBytes);  // ~8.8 MB
 
 static __device__ __align__(256) unsigned char g_window_scratch[kScratchBytes];
 
@@ -97,7 +98,8 @@ rp_status window_csr_noalloc(const Graph &g, int64_t ws, int64_t we, float scale
   const int64_t cap = ncls_cap ? (g.nlists > 0 ? g.nlists : 1) : INT64_MAX;
   CandRange ranges[kClasses];
   WinDesc desc{};
-  plan_window_ranges(g, ws, we, scale, cap, ranges, desc);
+  RP_TRY(plan_window_noalloc(g, ws, we, scale, cap, reinterpret_cast<int64_t *>(base + kPlanOff),
+                             ranges, desc, st));
   if (desc.n_candidates > kNoAllocMaxCandidates) {
     set_error("window [%lld, %lld) scans %lld candidate contacts; the allocation-free window "
               "build takes at most %lld", (long long)ws, (long long)we,
