@@ -16,7 +16,8 @@
  * is a thread-safe cache of device blocks: freeing a graph, simulation or
  * mean-field handle synchronizes the device and keeps its blocks (up to
  * 8 GiB per device) for the next handle instead of returning them with
- * cudaFree; rp_release_cached_memory() returns them.
+ * cudaFree, and large copies keep their pinned staging buffers (at most
+ * 64 MB); rp_release_cached_memory() returns both.
  */
 #ifndef REPLAY_H
 #define REPLAY_H
@@ -50,7 +51,8 @@ RP_API const char *rp_last_error(void);
 /* Library version string. */
 RP_API const char *rp_version(void);
 /* Returns every device block kept from freed handles to the driver
- * (cudaFree), on every device.  No reference counterpart. */
+ * (cudaFree), on every device, and the pinned staging buffers.  No reference
+ * counterpart. */
 RP_API void rp_release_cached_memory(void);
 
 /* ------------------------------------------------------------------------ */

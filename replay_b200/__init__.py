@@ -221,8 +221,9 @@ class Simulation:
             return flat.reshape(self.T + 1, self.M, 4)
         return flat.reshape(self.T + 1, self.n_networks, self.M, 4)
 
-    def _zeros(self):
-        return np.zeros((self.T + 1) * (self.n_networks or 1) * self.M * 4, np.int32)
+    def _counts(self):
+        # written whole by the library
+        return np.empty((self.T + 1) * (self.n_networks or 1) * self.M * 4, np.int32)
 
     @property
     def info(self):
@@ -236,7 +237,7 @@ class Simulation:
 
         node_states: optional callable(step_index, timestamp, states[M, N])
         (requires record_node_states=True)."""
-        counts = self._zeros()
+        counts = self._counts()
         if node_states is not None:
             def _cb(user, step_index, ts, states, n, m):
                 arr = np.ctypeslib.as_array(states, shape=(m * n,)).reshape(m, n).copy()
@@ -262,7 +263,7 @@ class Simulation:
         """Runs the replay with node-state CSV lines formatted on the GPU;
         write(step_index, timestamp, data: bytes) receives them in chunks of
         whole lines (requires record_node_states=True).  Returns counts."""
-        counts = self._zeros()
+        counts = self._counts()
 
         def _cb(user, step_index, ts, text, n):
             return int(bool(write(step_index, ts, C.string_at(text, n))))
@@ -287,7 +288,7 @@ class Simulation:
         check(lib().rp_sim_enqueue(self._h, C.c_void_p(stream) if stream else None))
 
     def counts(self):
-        counts = self._zeros()
+        counts = self._counts()
         check(lib().rp_sim_counts(self._h, _ptr(counts)))
         return self._shape(counts)
 

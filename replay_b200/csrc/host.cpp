@@ -1168,7 +1168,10 @@ extern "C" {
 
 RP_API const char *rp_last_error(void) { return g_err; }
 RP_API const char *rp_version(void) { return "replay-b200 0.1 (sm_100a)"; }
-RP_API void rp_release_cached_memory(void) { cache_trim(-1); }
+RP_API void rp_release_cached_memory(void) {
+  cache_trim(-1);
+  release_slots();
+}
 
 RP_API rp_status rp_graph_load_text(const char *path, int device, rp_graph **out) {
   if (!path || !out) {
@@ -1463,7 +1466,7 @@ RP_API rp_status rp_sim_counts(rp_sim *s, int32_t *counts) {
   }
   RP_TRY_CUDA(cudaSetDevice(s->g->device));
   RP_TRY_CUDA(cudaDeviceSynchronize());
-  RP_TRY_CUDA(cudaMemcpy(counts, s->counts.ptr, s->counts.bytes, cudaMemcpyDeviceToHost));
+  RP_TRY(download(s->g->device, counts, s->counts.ptr, s->counts.bytes));
   return RP_OK;
 }
 
@@ -1480,9 +1483,9 @@ RP_API rp_status rp_sim_run(rp_sim *s, int32_t *counts, rp_state_cb cb, void *us
   } else {
     RP_TRY(s->enqueue(s->stream, nullptr, nullptr, nullptr));
   }
-  RP_TRY_CUDA(cudaMemcpyAsync(counts, s->counts.ptr, s->counts.bytes, cudaMemcpyDeviceToHost,
-                              s->stream));
+  touch_pages(counts, s->counts.bytes);
   RP_TRY_CUDA(cudaStreamSynchronize(s->stream));
+  RP_TRY(download(s->g->device, counts, s->counts.ptr, s->counts.bytes));
   return RP_OK;
 }
 
@@ -1525,9 +1528,9 @@ RP_API rp_status rp_sim_run_text(rp_sim *s, int32_t *counts, rp_text_cb cb, void
   s->text_cb = nullptr;
   s->text_user = nullptr;
   RP_TRY(st);
-  RP_TRY_CUDA(cudaMemcpyAsync(counts, s->counts.ptr, s->counts.bytes, cudaMemcpyDeviceToHost,
-                              s->stream));
+  touch_pages(counts, s->counts.bytes);
   RP_TRY_CUDA(cudaStreamSynchronize(s->stream));
+  RP_TRY(download(s->g->device, counts, s->counts.ptr, s->counts.bytes));
   return RP_OK;
 }
 

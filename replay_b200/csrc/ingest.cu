@@ -482,10 +482,11 @@ rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
   RP_TRY(e.alloc(sizeof(int64_t) * n));
   RP_TRY(uu.alloc(sizeof(int32_t) * n));
   RP_TRY(vv.alloc(sizeof(int32_t) * n));
-  RP_TRY_CUDA(cudaMemcpyAsync(s.ptr, start, sizeof(int64_t) * n, cudaMemcpyHostToDevice, st));
-  RP_TRY_CUDA(cudaMemcpyAsync(e.ptr, end, sizeof(int64_t) * n, cudaMemcpyHostToDevice, st));
-  RP_TRY_CUDA(cudaMemcpyAsync(uu.ptr, u, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
-  RP_TRY_CUDA(cudaMemcpyAsync(vv.ptr, v, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
+  const HostPart parts[4] = {{s.ptr, start, sizeof(int64_t) * (size_t)n},
+                             {e.ptr, end, sizeof(int64_t) * (size_t)n},
+                             {uu.ptr, u, sizeof(int32_t) * (size_t)n},
+                             {vv.ptr, v, sizeof(int32_t) * (size_t)n}};
+  RP_TRY(upload(g.device, parts, 4));
 
   // 1. stored coordinates and the key ranges
   // (and, for endpoints from a caller, their order, range and number)

@@ -153,6 +153,17 @@ struct DevBuf {
   }
 };
 
+// ---- large copies between pageable host memory and the device (transfer.cpp) ----
+struct HostPart {
+  void *dev;
+  const void *host;
+  size_t bytes;
+};
+rp_status upload(int device, const HostPart *parts, int n);
+rp_status download(int device, void *host, const void *dev, size_t n);
+void touch_pages(void *host, size_t n);
+void release_slots();
+
 // ---- interval index -----------------------------------------------------------
 // Contacts live in "stored coordinates" (the reference interval database's
 // orientation rule, see graph.cpp) and are partitioned into duration classes:
