@@ -302,6 +302,7 @@ struct rp_sim {
   // workspace while group g's steps run
   WindowWorkspace wsp2;
   bool overlap = false;
+  bool sparse = false;  // windows list their rows with pairs
   cudaStream_t side = nullptr;
   cudaEvent_t ev_built[2] = {nullptr, nullptr}, ev_free = nullptr, ev_join = nullptr;
   bool prebuilt = false;
@@ -428,6 +429,16 @@ struct rp_sim {
     const int64_t slot = w - groups[grp].first;
     const int32_t *rows = ws_of(grp).long_rows.as<int32_t>() + slot * N;
     return HeavyRows{rows, rows + N, ws_of(grp).counters.as<unsigned long long>() + 4 * slot};
+  }
+
+  RowList rows_of(int t) const {
+    if (!sparse) return RowList{};
+    const int w = step_win[t], grp = win_group[w];
+    const WindowWorkspace &ws = ws_of(grp);
+    return RowList{ws.rows.as<int32_t>() + 2 * wins[w].hit_off,
+                   ws.span.as<int2>() + 2 * wins[w].hit_off,
+                   ws.counters.as<unsigned long long>() + 4 * (int64_t)(w - groups[grp].first),
+                   std::min<int64_t>(2 * wins[w].n_candidates, N)};
   }
 
   // Optional event marks around kernel groups (rp_sim_profile).
@@ -615,7 +626,7 @@ struct rp_sim {
           mark(kMarkStep);
           k += 1;
         } else {
-          packed_infect(L, rp_of(t), ent_of(t), heavy_of(t), mask.as<uint32_t>(),
+          packed_infect(L, rp_of(t), ent_of(t), rows_of(t), heavy_of(t), mask.as<uint32_t>(),
                         sa.as<uint32_t>(), sb.as<uint32_t>(), evs.as<uint32_t>(),
                         bits.as<uint32_t>(), (uint32_t)t, step_scale[t], c, st);
           mark(kMarkSpmv);
@@ -751,7 +762,7 @@ rp_status sim_window_workspace(rp_sim &s, WindowWorkspace &w) {
     hits = std::max(hits, g.candidates);
   }
   const bool sorted = s.weight_kind == kWeightF32 || s.p.csr_mode == RP_CSR_PREBUILT;
-  return window_workspace_alloc(w, s.N, slots, hits, sorted, s.wins, s.ranges);
+  return window_workspace_alloc(w, s.N, slots, hits, sorted, s.sparse, s.wins, s.ranges);
 }
 
 rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
@@ -830,7 +841,11 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
     return RP_ERR_RANGE;
   }
   const bool prebuilt = p.csr_mode == RP_CSR_PREBUILT;
-  plan_window_groups(s.wins, s.N, prebuilt, s.groups);
+  bool truncate = false;
+  for (const WinDesc &d : s.wins) truncate |= d.may_truncate != 0;
+  s.sparse = !prebuilt && !truncate && s.path == RP_PATH_BATCHED &&
+             s.weight_kind == kWeightI32 && sparse_windows(max_cand, s.N);
+  plan_window_groups(s.wins, s.N, prebuilt, s.sparse, s.groups);
   s.win_group.resize(s.wins.size());
   for (size_t k = 0; k < s.groups.size(); ++k)
     for (int32_t w = 0; w < s.groups[k].count; ++w) s.win_group[s.groups[k].first + w] = (int32_t)k;
@@ -1309,8 +1324,8 @@ RP_API rp_status rp_window_csr(rp_graph *h, int64_t ws, int64_t we, float scale,
   RP_TRY(plan_windows(g, {ws}, we - ws, {scale}, cap, ranges, wins));
   WindowWorkspace w;
   std::vector<WindowGroup> one;
-  plan_window_groups(wins, g.n_nodes, true, one);
-  RP_TRY(window_workspace_alloc(w, g.n_nodes, 1, wins[0].n_candidates, true, wins, ranges));
+  plan_window_groups(wins, g.n_nodes, true, false, one);
+  RP_TRY(window_workspace_alloc(w, g.n_nodes, 1, wins[0].n_candidates, true, false, wins, ranges));
   DevBuf out_rp, out_ent;
   RP_TRY(out_rp.alloc(sizeof(int32_t) * ((size_t)g.n_nodes + 1)));
   RP_TRY(out_ent.alloc(sizeof(int2) * (size_t)w.cap_entries));

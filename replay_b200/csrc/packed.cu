@@ -127,7 +127,8 @@ constexpr int kUnitRows = 128;     // most rows of a unit
 // accumulates over units and is decided 32 words at a time.
 struct InfectWarp {
   uint4 pl[32][2];             // the 8 random planes of each word (round scratch)
-  int32_t urow[kUnitRows];     // the unit's rows with pairs: row in unit | pairs << 7
+  int32_t urow[kUnitRows];     // the unit's rows with pairs: row (or list entry) in unit |
+                               // pairs << 7
   int32_t ubeg[kUnitRows];     // their first pairs
   int32_t list[128];           // items of a batch of 32 rows: row in batch << 5 | column
   uint32_t rmask[32];          // column masks of the batch's rows
@@ -158,6 +159,7 @@ constexpr int kInfectWarpBytes =
     (int)((sizeof(InfectWarp) > sizeof(HeavyWarp) ? sizeof(InfectWarp) : sizeof(HeavyWarp)) + 15) /
     16 * 16;
 constexpr int kInfectDynSmem = kWarps * kInfectWarpBytes;
+static_assert(3 * (kInfectDynSmem + 1024 + 64) <= 228 * 1024, "three blocks per SM");
 
 // Top 8 uniform bits of replica bit b from a queued word's planes.
 __device__ __forceinline__ uint32_t queued_top8(const uint4 (&q)[2], uint32_t b) {
@@ -176,9 +178,10 @@ struct InfectArgs {
   uint32_t *evb;
   const int32_t *heavy, *heavy_end;    // rows of more than kHeavyPairs / kHugePairs pairs (window.cu)
   const unsigned long long *n_heavy;  // [0] heavy, [2] huge rows
+  RowList list;                        // sparse window: rows with pairs
   uint32_t step;
   float scale;
-  int32_t unit_rows, n_units;
+  int32_t unit_rows, n_units;          // sparse: units follow from the list's length
 };
 
 // Decides candidate replica b of (row, word) from its exact exposure e
@@ -443,14 +446,21 @@ __device__ __forceinline__ bool heavy_load(HeavyUnit &h, const int32_t *list, in
                                            int nws, int lane, const PackedLayout &L,
                                            const InfectArgs &d) {
   h.row = list[dir * (u / nws)];
+  if (d.list.rows) {  // sparse window: an entry of its row list
+    const int2 sp = __ldg(d.list.span + h.row);
+    h.beg = sp.x;
+    h.end = sp.x + sp.y;
+    h.row = __ldg(d.list.rows + h.row);
+  } else {
+    h.beg = d.row_ptr[h.row];
+    h.end = d.row_ptr[h.row + 1];
+  }
   const int ws = u % nws;
   h.w0 = ws * 32;
   const int word = h.w0 + lane;
   const uint32_t sb8 = d.susb[bit_word(L.lb, L.n_slices, h.row, ws * 8)] >>
                        bit_shift(L.lb, h.row, ws * 8);
   if (!(sb8 & (L.lb >= 3 ? 0xFFu : (1u << (1 << L.lb)) - 1u))) return false;
-  h.beg = d.row_ptr[h.row];
-  h.end = d.row_ptr[h.row + 1];
   h.S = 0;
   if (word < L.vwords) {
     const int64_t wi = (int64_t)h.row * L.words + word;
@@ -622,6 +632,9 @@ __global__ void __launch_bounds__(kThreads, 3)
     Q.nk = 0;
   }
   __syncwarp();
+  const int n_rows = d.list.rows ? (int)d.list.counts[1] : L.n_nodes;
+  const int n_units =
+      d.list.rows ? (n_rows + d.unit_rows - 1) / d.unit_rows * L.n_slices : d.n_units;
   // the block's units, blockIdx.x + k gridDim.x, go to its warps as they ask
   auto next_unit = [&]() {
     int k = 0;
@@ -642,14 +655,14 @@ __global__ void __launch_bounds__(kThreads, 3)
     if (cnt == 0 && !nz) {
       if (ub >= nrows) {
         const int unit = next_unit();
-        if (unit >= d.n_units) {
+        if (unit >= n_units) {
           more = false;
         } else {
           // the next unit's rows that have pairs (longer rows were taken above)
           const int rb = L.n_slices == 1 ? unit : unit / L.n_slices;
           cbase = L.n_slices == 1 ? 0 : (unit - rb * L.n_slices) * 32;
           r0 = rb * d.unit_rows;
-          const int r1 = min(r0 + d.unit_rows, L.n_nodes);
+          const int r1 = min(r0 + d.unit_rows, n_rows);
           nrows = ub = 0;
           __syncwarp();
           for (int r = r0; r < r1; r += 128) {
@@ -659,8 +672,14 @@ __global__ void __launch_bounds__(kThreads, 3)
               const int row = r + 32 * j + lane;
               b[j] = len[j] = 0;
               if (row < r1) {
-                b[j] = __ldg(d.row_ptr + row);
-                len[j] = __ldg(d.row_ptr + row + 1) - b[j];
+                if (d.list.rows) {
+                  const int2 sp = __ldg(d.list.span + row);
+                  b[j] = sp.x;
+                  len[j] = sp.y;
+                } else {
+                  b[j] = __ldg(d.row_ptr + row);
+                  len[j] = __ldg(d.row_ptr + row + 1) - b[j];
+                }
               }
             }
 #pragma unroll
@@ -691,6 +710,7 @@ __global__ void __launch_bounds__(kThreads, 3)
           beg = Q.ubeg[ub + lane];
           n = lrow >> 7;
           lrow = r0 + (lrow & 127);
+          if (d.list.rows) lrow = __ldg(d.list.rows + lrow);
         }
         ub += 32;
         auto row_bits = [&](const uint32_t *bits, int r) {
@@ -1111,9 +1131,9 @@ __global__ void __launch_bounds__(kThreads, 3)
           const int row = (int)q.x, word = (int)(q.y & ~kWordEvent);
           uint32_t ev = 0;
           if (q.y >= kWordEvent) {
-            const int64_t qi = (int64_t)row * L.words + word;
-            ev = d.evs[qi];
-            d.evs[qi] = 0u;
+            // one exchange: a load and a store of a sector that k_infect's
+            // atomics left cost 21 us a step on the replica sweep
+            ev = atomicExch(&d.evs[(int64_t)row * L.words + word], 0u);
           }
           const uint32_t E = ~A & B, I = A & ~B, R = waning ? (A & B) : 0u;
           uint32_t f = certain ? flow_sure(E, I, R, c.th) : 0u;
@@ -1397,10 +1417,10 @@ static int unit_grid(int64_t units) {
 // items, one round of words) where blocks would have none, more where every
 // warp has many: a unit's row pointers are loaded together, and sparse rows
 // fold into batches of 32.
-static void set_infect_units(const PackedLayout &L, InfectArgs &d) {
+static void set_infect_units(const PackedLayout &L, int64_t n_rows, InfectArgs &d) {
   d.unit_rows = 8;
   const int64_t warps = 148 * 3 * kWarps;
-  auto units = [&](int rows) { return (int64_t)((L.n_nodes + rows - 1) / rows) * L.n_slices; };
+  auto units = [&](int rows) { return (n_rows + rows - 1) / rows * L.n_slices; };
   while (d.unit_rows > 1 && units(d.unit_rows) * 2 < warps && (int64_t)d.unit_rows * L.q4 > 8)
     d.unit_rows >>= 1;
   while (d.unit_rows < kUnitRows && (units(2 * d.unit_rows) >= 4 * warps ||
@@ -1410,9 +1430,9 @@ static void set_infect_units(const PackedLayout &L, InfectArgs &d) {
 }
 
 void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
-                   const HeavyRows &heavy, const uint32_t *mask, const uint32_t *sa,
-                   const uint32_t *sb, uint32_t *evs, uint32_t *bits, uint32_t step, float scale,
-                   const StepConsts &c, cudaStream_t st) {
+                   const RowList &list, const HeavyRows &heavy, const uint32_t *mask,
+                   const uint32_t *sa, const uint32_t *sb, uint32_t *evs, uint32_t *bits,
+                   uint32_t step, float scale, const StepConsts &c, cudaStream_t st) {
   InfectArgs d{};
   d.row_ptr = row_ptr;
   d.ent = entries;
@@ -1426,9 +1446,10 @@ void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *en
   d.heavy = heavy.rows;
   d.heavy_end = heavy.end;
   d.n_heavy = heavy.counts;
+  d.list = list;
   d.step = step;
   d.scale = scale;
-  set_infect_units(L, d);
+  set_infect_units(L, list.rows ? list.bound : L.n_nodes, d);
   k_infect<false><<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
 }
 
@@ -1446,7 +1467,7 @@ void cd_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entrie
   d.susb = susb;
   d.evb = evb;
   d.step = step;
-  set_infect_units(L, d);
+  set_infect_units(L, L.n_nodes, d);
   k_infect<true><<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
 }
 

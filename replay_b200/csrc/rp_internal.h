@@ -261,15 +261,27 @@ struct Hit {
 
 // Rows with many pairs, listed while a window's row pointers are written:
 // rows of more than kHeavyPairs pairs from the front of the list, of more than
-// kHugePairs pairs from its end; counts[0] and counts[2] of them.
+// kHugePairs pairs from its end; counts[0] and counts[2] of them.  A sparse
+// window lists entries of its RowList.
 constexpr int32_t kHeavyPairs = 32, kHugePairs = 512;
 struct HeavyRows {
   const int32_t *rows, *end;
   const unsigned long long *counts;
 };
+// The rows of a sparse window that have pairs, in any order (WindowWorkspace
+// with sparse set), or null: every row by its row pointers.
+struct RowList {
+  const int32_t *rows;       // counts[1] of them
+  const int2 *span;          // {first pair, pairs}
+  const unsigned long long *counts;
+  int64_t bound;             // at most so many rows
+};
 
 struct WindowWorkspace {
   int32_t n_nodes = 0;
+  // Windows with pairs in few rows: only those rows are counted, placed and
+  // listed, so that a window costs its contacts and not its nodes.
+  bool sparse = false;
   int64_t cap_hits = 0, cap_entries = 0;
   int32_t n_tiles = 0;
   // a group of windows, slot after slot (WindowGroup); G slots
@@ -279,9 +291,14 @@ struct WindowWorkspace {
   DevBuf tmp_e;     // int2[cap_entries]  radix ping-pong for hub rows
   DevBuf tmp_r;     // int32[cap_entries]
   DevBuf row_ptr;   // int32[G][n+1]
-  DevBuf deg;       // int32[G][n] degree, then fill cursor
+  DevBuf deg;       // int32[G][n] degrees, counted down to zero while pairs are placed
   DevBuf tiles;     // int32[G][n_tiles]
-  DevBuf counters;  // u64[G][4]: heavy rows, long rows, huge rows, predicate hits
+  DevBuf hpos;      // int2[cap_hits], sparse: a hit's positions in its two rows
+  DevBuf rows;      // int32[cap_entries], sparse: rows with pairs
+  DevBuf span;      // int2[cap_entries], sparse: their first pairs and pairs
+  DevBuf placed;    // u64[G], sparse: pairs placed so far
+  DevBuf counters;  // u64[G][4]: heavy rows, long rows (sparse: listed rows), huge rows,
+                    // predicate hits
   DevBuf long_rows; // int32[G][n]: heavy rows (unsorted rows) or rows to sort in a block
   DevBuf win;       // WinDesc[n_windows]
   DevBuf ranges;    // CandRange[...]
@@ -289,13 +306,18 @@ struct WindowWorkspace {
 
 // Room for any group of at most `slots` windows and `cap_hits` candidates.
 rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t slots,
-                                 int64_t cap_hits, bool sort_rows,
+                                 int64_t cap_hits, bool sort_rows, bool sparse,
                                  const std::vector<WinDesc> &wins,
                                  const std::vector<CandRange> &ranges);
 // Splits the windows into groups (`single`: one window each) and places each
 // window's hits in its group's list.
-void plan_window_groups(std::vector<WinDesc> &wins, int32_t n_nodes, bool single,
+void plan_window_groups(std::vector<WinDesc> &wins, int32_t n_nodes, bool single, bool sparse,
                         std::vector<WindowGroup> &groups);
+// Whether windows of at most max_candidates contacts on n_nodes rows are built
+// sparse: fewer than one row in four has pairs then.
+inline bool sparse_windows(int64_t max_candidates, int32_t n_nodes) {
+  return 8 * max_candidates < n_nodes;
+}
 
 // ---- mean-field replay (meanfield.cu) ----
 struct MfRates {
@@ -403,7 +425,7 @@ void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb,
 // One step: exposure + infection draws (k_infect), then transitions, counts
 // and the next infectious mask (k_flow).
 void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
-                   const HeavyRows &heavy, const uint32_t *mask, const uint32_t *sa,
+                   const RowList &list, const HeavyRows &heavy, const uint32_t *mask, const uint32_t *sa,
                    const uint32_t *sb, uint32_t *evs, uint32_t *bits, uint32_t step, float scale,
                    const StepConsts &c, cudaStream_t st);
 // net_first: first row of each of several networks (their counts follow one

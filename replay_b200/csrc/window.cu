@@ -10,7 +10,7 @@
 //   k_hits      candidates of the duration-class index -> hit list (+degrees)
 //   k_trunc     only when the reference's hit cap can bind: keep the cap
 //               smallest ranks (radix select), then count degrees
-//   k_scan_*    degrees -> row_ptr (exclusive scan), cursors reset
+//   k_scan_*    degrees -> row_ptr (exclusive scan)
 //   k_fill      hits -> row segments {col, weight} + rank
 //   k_rowsort_* rows ordered by (col, rank), duplicates merged in rank order
 #include <algorithm>
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(256)
            const int32_t *__restrict__ cu, const int32_t *__restrict__ cv,
            const int32_t *__restrict__ crank, Hit *__restrict__ hits_all,
            unsigned long long *__restrict__ counters, int32_t *__restrict__ deg_all, int32_t n,
-           int weight_f32) {
+           int weight_f32, int2 *__restrict__ hpos_all, int32_t *__restrict__ rows_all) {
   __shared__ CandRange sr[kClasses];
   __shared__ WinDesc sw;
   __shared__ int s_pred;
@@ -103,42 +103,66 @@ __global__ void __launch_bounds__(256)
   Hit *hits = hits_all + sw.hit_off;
   int32_t *deg = deg_all + (int64_t)blockIdx.y * n;
   int npred = 0;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  // warp-uniform trip count (the list of a sparse window is appended per warp)
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; base < total;
+       base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = base + lane;
+    bool new_u = false, new_v = false;
     Hit h;
     h.rank = -1;
     h.u = -2;
     h.v = h.w = 0;
-    int k = 0;
-    for (int step = 32; step > 0; step >>= 1)
-      if (k + step < nr && sr[k + step].prefix <= t) k += step;
-    const int64_t idx = sr[k].lo + (t - sr[k].prefix);
-    const int64_t s = cs[idx], e = ce[idx];
-    if (s < sw.qe && sw.qs < e) {
-      ++npred;
-      // Coordinates handed to the CSR builder: mirrored back when the
-      // stored orientation differs from the query's.
-      int64_t hs = s, he = e;
-      if ((s < 0) != query_neg) {
-        hs = -e;
-        he = -(int64_t)(int32_t)s;
-      }
-      const int64_t os = hs > sw.ws ? hs : sw.ws;
-      const int64_t oe = he < sw.we ? he : sw.we;
-      const int64_t ov = oe - os;
-      h.rank = crank[idx];
-      h.v = cv[idx];
-      h.u = -1;  // in the window without overlap: counts toward the hit cap only
-      if (ov > 0) {
-        h.u = cu[idx];
-        h.w = weight_f32 ? __float_as_int(__fmul_rn(__ll2float_rn(ov), sw.scale)) : (int32_t)ov;
-        if (count_deg) {
-          atomicAdd(&deg[h.u], 1);
-          atomicAdd(&deg[h.v], 1);
+    if (t < total) {
+      int k = 0;
+      for (int step = 32; step > 0; step >>= 1)
+        if (k + step < nr && sr[k + step].prefix <= t) k += step;
+      const int64_t idx = sr[k].lo + (t - sr[k].prefix);
+      const int64_t s = cs[idx], e = ce[idx];
+      if (s < sw.qe && sw.qs < e) {
+        ++npred;
+        // Coordinates handed to the CSR builder: mirrored back when the
+        // stored orientation differs from the query's.
+        int64_t hs = s, he = e;
+        if ((s < 0) != query_neg) {
+          hs = -e;
+          he = -(int64_t)(int32_t)s;
+        }
+        const int64_t os = hs > sw.ws ? hs : sw.ws;
+        const int64_t oe = he < sw.we ? he : sw.we;
+        const int64_t ov = oe - os;
+        h.rank = crank[idx];
+        h.v = cv[idx];
+        h.u = -1;  // in the window without overlap: counts toward the hit cap only
+        if (ov > 0) {
+          h.u = cu[idx];
+          h.w = weight_f32 ? __float_as_int(__fmul_rn(__ll2float_rn(ov), sw.scale)) : (int32_t)ov;
+          if (rows_all) {  // sparse window: the first pair of a row lists it
+            const int pu = atomicAdd(&deg[h.u], 1), pv = atomicAdd(&deg[h.v], 1);
+            hpos_all[sw.hit_off + t] = make_int2(pu, pv);
+            new_u = pu == 0;
+            new_v = pv == 0;
+          } else if (count_deg) {
+            atomicAdd(&deg[h.u], 1);
+            atomicAdd(&deg[h.v], 1);
+          }
         }
       }
+      hits[t] = h;
     }
-    hits[t] = h;
+    if (rows_all) {
+      const unsigned mu = __ballot_sync(kFull, new_u), mv = __ballot_sync(kFull, new_v);
+      if (mu | mv) {
+        unsigned long long at = 0;
+        if (lane == 0)
+          at = atomicAdd(&counters[4 * blockIdx.y + 1],
+                         (unsigned long long)(__popc(mu) + __popc(mv)));
+        int32_t *rows = rows_all + 2 * sw.hit_off + __shfl_sync(kFull, at, 0);
+        const unsigned below = (1u << lane) - 1u;
+        if (new_u) rows[__popc(mu & below)] = h.u;
+        if (new_v) rows[__popc(mu) + __popc(mv & below)] = h.v;
+      }
+    }
   }
   npred = __reduce_add_sync(kFull, npred);
   if ((threadIdx.x & 31) == 0 && npred) atomicAdd(&s_pred, npred);
@@ -258,6 +282,70 @@ __global__ void __launch_bounds__(kScanThreads)
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == blockDim.x - 1) out[n] = off + total;
 }
 
+// Sparse window: places the listed rows' pairs in list order (one reduction per
+// block), lists the long rows, and leaves every degree zero again.
+__global__ void __launch_bounds__(256)
+    k_place_rows(const WinDesc *__restrict__ wins, int32_t *__restrict__ deg_all,
+                 const int32_t *__restrict__ rows_all, int2 *__restrict__ span_all,
+                 int32_t *__restrict__ row_ptr_all, unsigned long long *__restrict__ placed,
+                 unsigned long long *__restrict__ counters, int32_t *__restrict__ heavy_all,
+                 int32_t n) {
+  __shared__ int wt[32];
+  __shared__ unsigned long long s_base;
+  const int64_t hoff = 2 * wins[blockIdx.y].hit_off;
+  const int32_t *rows = rows_all + hoff;
+  int2 *span = span_all + hoff;
+  int32_t *deg = deg_all + (int64_t)blockIdx.y * n;
+  int32_t *row_ptr = row_ptr_all + (int64_t)blockIdx.y * (n + 1);
+  unsigned long long *cnt = counters + 4 * blockIdx.y;
+  const int64_t m = (int64_t)cnt[1];
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < m;
+       base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t j = base + threadIdx.x;
+    int32_t row = 0;
+    int d = 0;
+    if (j < m) {
+      row = rows[j];
+      // one exchange: a load and a store of the sector that the atomics of
+      // k_hits left took 118 us for 7 windows of 146,000 rows, this 30
+      d = atomicExch(&deg[row], 0);
+    }
+    int total;
+    const int off = block_excl_scan(d, wt, total);
+    if (threadIdx.x == 0) s_base = atomicAdd(&placed[blockIdx.y], (unsigned long long)total);
+    __syncthreads();
+    if (j < m) {
+      const int32_t beg = (int32_t)s_base + off;
+      row_ptr[row] = beg;
+      span[j] = make_int2(beg, d);
+      if (d > kHeavyPairs) {
+        int32_t *list = heavy_all + (int64_t)blockIdx.y * n;
+        const bool huge = d > kHugePairs;
+        const int64_t at = (int64_t)atomicAdd(&cnt[huge ? 2 : 0], 1ull);
+        list[huge ? n - 1 - at : at] = (int32_t)j;  // by list entry: the row's end is there
+      }
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256)
+    k_fill_sparse(const WinDesc *__restrict__ wins, const Hit *__restrict__ hits_all,
+                  const int2 *__restrict__ hpos_all, const int32_t *__restrict__ row_ptr_all,
+                  int2 *__restrict__ entries_all, int32_t nodes) {
+  const int64_t n = wins[blockIdx.y].n_candidates, hoff = wins[blockIdx.y].hit_off;
+  const int32_t *row_ptr = row_ptr_all + (int64_t)blockIdx.y * (nodes + 1);
+  int2 *entries = entries_all + 2 * hoff;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const Hit h = hits_all[hoff + i];
+    if (h.u < 0) continue;
+    const int2 p = hpos_all[hoff + i];
+    entries[row_ptr[h.u] + p.x] = make_int2(h.v, h.w);
+    entries[row_ptr[h.v] + p.y] = make_int2(h.u, h.w);
+  }
+}
+
 __global__ void __launch_bounds__(256)
     k_fill(const WinDesc *__restrict__ wins, const Hit *__restrict__ hits_all,
            const int32_t *__restrict__ row_ptr_all, int32_t *__restrict__ cursor_all,
@@ -273,9 +361,10 @@ __global__ void __launch_bounds__(256)
        i += (int64_t)gridDim.x * blockDim.x) {
     const Hit h = hits[i];
     if (h.u < 0) continue;
-    const int32_t pu = row_ptr[h.u] + atomicAdd(&cursor[h.u], 1);
+    // the degrees count down to the zeros that the next window starts from
+    const int32_t pu = row_ptr[h.u] + atomicSub(&cursor[h.u], 1) - 1;
     entries[pu] = make_int2(h.v, h.w);
-    const int32_t pv = row_ptr[h.v] + atomicAdd(&cursor[h.v], 1);
+    const int32_t pv = row_ptr[h.v] + atomicSub(&cursor[h.v], 1) - 1;
     entries[pv] = make_int2(h.u, h.w);
     if (keep_rank) {
       erank[pu] = h.rank;
@@ -576,10 +665,11 @@ int32_t window_scan_tiles(int32_t n_nodes) {
 }
 
 rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t slots,
-                                 int64_t cap_hits, bool sort_rows,
+                                 int64_t cap_hits, bool sort_rows, bool sparse,
                                  const std::vector<WinDesc> &wins,
                                  const std::vector<CandRange> &ranges) {
   w.n_nodes = n_nodes;
+  w.sparse = sparse;
   w.cap_hits = cap_hits < 1 ? 1 : cap_hits;
   w.cap_entries = 2 * w.cap_hits;
   w.n_tiles = window_scan_tiles(n_nodes);
@@ -598,6 +688,13 @@ rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t sl
   RP_TRY(w.deg.alloc(sizeof(int32_t) * g * n));
   RP_TRY(w.tiles.alloc(sizeof(int32_t) * g * (size_t)w.n_tiles));
   RP_TRY(w.counters.alloc(sizeof(unsigned long long) * 4 * g));
+  RP_TRY_CUDA(cudaMemset(w.deg.ptr, 0, w.deg.bytes));  // every build leaves them zero
+  if (sparse) {
+    RP_TRY(w.hpos.alloc(sizeof(int2) * w.cap_hits));
+    RP_TRY(w.rows.alloc(sizeof(int32_t) * w.cap_entries));
+    RP_TRY(w.span.alloc(sizeof(int2) * w.cap_entries));
+    RP_TRY(w.placed.alloc(sizeof(unsigned long long) * g));
+  }
   RP_TRY(w.win.alloc(sizeof(WinDesc) * (wins.empty() ? 1 : wins.size())));
   RP_TRY(w.ranges.alloc(sizeof(CandRange) * (ranges.empty() ? 1 : ranges.size())));
   if (!wins.empty())
@@ -615,16 +712,20 @@ rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t sl
 // latency: 22 us for N = 1,000, twice what the two step kernels of the window
 // take.  A group pays that chain once.  The budget keeps a group's pairs in
 // L2 between its build and its last step; the first group is smaller, since
-// no step can overlap its build.
+// no step can overlap its build.  Sparse windows touch few of their per-node
+// arrays, so their budget is a matter of memory: at 2.6M nodes and 75,000
+// contacts a window built alone took 31 us, in groups of eight 7 us.
 constexpr int64_t kGroupBytes = 32ll << 20, kFirstGroupBytes = 4ll << 20;
+constexpr int64_t kSparseGroupBytes = 256ll << 20;
 constexpr int32_t kGroupMax = 256;
 
-void plan_window_groups(std::vector<WinDesc> &wins, int32_t n_nodes, bool single,
+void plan_window_groups(std::vector<WinDesc> &wins, int32_t n_nodes, bool single, bool sparse,
                         std::vector<WindowGroup> &groups) {
   groups.clear();
   const int64_t node_bytes = 12ll * n_nodes;  // degrees, row pointers, long rows
   for (int32_t w = 0; w < (int32_t)wins.size();) {
-    const int64_t budget = groups.empty() ? kFirstGroupBytes : kGroupBytes;
+    const int64_t budget = groups.empty() ? kFirstGroupBytes
+                                          : (sparse ? kSparseGroupBytes : kGroupBytes);
     WindowGroup g;
     g.first = w;
     do {
@@ -648,15 +749,27 @@ int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup 
   unsigned long long *ctr = ws.counters.as<unsigned long long>();
   const WinDesc *wins = ws.win.as<WinDesc>() + grp.first;
   cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * 4 * G, st);
-  // degrees start at zero (the previous group left its fill cursors here)
-  cudaMemsetAsync(ws.deg.ptr, 0, sizeof(int32_t) * (size_t)n * G, st);
+  if (ws.sparse) cudaMemsetAsync(ws.placed.ptr, 0, sizeof(unsigned long long) * G, st);
   const int f32 = weight_kind == kWeightF32;
   const int blocks = std::max(1, 148 * 16 / (int)G);  // per window
   k_hits<<<dim3(grid_for(grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
       wins, ws.ranges.as<CandRange>(), g.cs.as<int64_t>(), g.ce.as<int64_t>(),
       g.cu.as<int32_t>(), g.cv.as<int32_t>(), g.crank.as<int32_t>(), ws.hits.as<Hit>(), ctr,
-      ws.deg.as<int32_t>(), n, f32);
+      ws.deg.as<int32_t>(), n, f32, ws.sparse ? ws.hpos.as<int2>() : nullptr,
+      ws.sparse ? ws.rows.as<int32_t>() : nullptr);
   ++launches;
+  if (ws.sparse) {
+    // every row pass below would touch n rows: 45 us a window at 2.6M nodes and
+    // 75,000 contacts, 15 us this way
+    k_place_rows<<<dim3(grid_for(2 * grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
+        wins, ws.deg.as<int32_t>(), ws.rows.as<int32_t>(), ws.span.as<int2>(),
+        ws.row_ptr.as<int32_t>(), ws.placed.as<unsigned long long>(), ctr,
+        ws.long_rows.as<int32_t>(), n);
+    k_fill_sparse<<<dim3(grid_for(grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
+        wins, ws.hits.as<Hit>(), ws.hpos.as<int2>(), ws.row_ptr.as<int32_t>(),
+        ws.entries.as<int2>(), n);
+    return launches + 2;
+  }
   if (grp.truncate) {
     k_trunc<<<dim3(1, G), 1024, 0, st>>>(wins, ws.hits.as<Hit>(), cap, ws.deg.as<int32_t>(), n);
     ++launches;
@@ -667,7 +780,7 @@ int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup 
     ++launches;
   }
   k_scan_apply<<<dim3(ws.n_tiles, G), kScanThreads, 0, st>>>(
-      ws.deg.as<int32_t>(), n, ws.tiles.as<int32_t>(), ws.row_ptr.as<int32_t>(), 1,
+      ws.deg.as<int32_t>(), n, ws.tiles.as<int32_t>(), ws.row_ptr.as<int32_t>(), 0,
       sort_rows ? nullptr : ws.long_rows.as<int32_t>(), n, ctr);
   k_fill<<<dim3(grid_for(grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
       wins, ws.hits.as<Hit>(), ws.row_ptr.as<int32_t>(), ws.deg.as<int32_t>(),

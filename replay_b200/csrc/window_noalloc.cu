@@ -130,9 +130,10 @@ rp_status window_csr_noalloc(const Graph &g, int64_t ws, int64_t we, float scale
   w.win.borrow(base + kWinOff, sizeof(WinDesc));
   w.ranges.borrow(base + kRangeOff, sizeof(CandRange) * kClasses);
 
-  // The builder zeroes its hit counters and degree cursors itself; the
-  // window descriptor and candidate ranges are uploaded from the stack
+  // The builder zeroes its hit counters and expects zero degrees (a call that
+  // failed on the way may have left others here); the window descriptor and candidate ranges are uploaded from the stack
   // (pageable source: the copy is staged before cudaMemcpyAsync returns).
+  RP_TRY_CUDA(cudaMemsetAsync(w.deg.ptr, 0, w.deg.bytes, st));
   RP_TRY_CUDA(cudaMemcpyAsync(w.win.ptr, &desc, sizeof(WinDesc), cudaMemcpyHostToDevice, st));
   if (desc.n_ranges > 0)
     RP_TRY_CUDA(cudaMemcpyAsync(w.ranges.ptr, ranges, sizeof(CandRange) * desc.n_ranges,

@@ -50,3 +50,37 @@ def test_grouped_windows_match_oracle(oracle, case):
                       **kw, **dict(c["kw"], transition=mode))
     np.testing.assert_array_equal(sim.run(), want)
     np.testing.assert_array_equal(sim.run(), want)  # the workspaces are reused
+
+
+# fewer than one row in eight with a contact per window: windows that list their rows, alone and in a batch,
+# with a hub row above 32 and above 512 pairs, windows without contacts, two steps per window
+@pytest.mark.gpu
+@pytest.mark.parametrize("nodes,hub,window,networks", [(5000, 0, 900, 1), (9000, 40, 900, 3), (40_000, 700, 1800, 1)])
+def test_sparse_windows_match_oracle(oracle, nodes, hub, window, networks):
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import replay_b200 as rb
+    rng = np.random.default_rng(hub)
+    first = np.array([0, nodes // 3, nodes // 2, nodes][:networks] + [nodes], np.int32)
+    t0, m = synthetic.EPOCH_2000, 4 * nodes // 10
+    start = t0 + rng.integers(0, 20 * 900, m)
+    net = rng.integers(0, networks, m)
+    lo, hi = first[net].astype(np.int64), first[net + 1].astype(np.int64)
+    u = (lo + rng.integers(0, 1 << 30, m) % (hi - lo - 1)).astype(np.int32)
+    v = (u + 1).astype(np.int32)
+    if hub:  # node 3 meets `hub` others in one window
+        start = np.concatenate([start, np.full(hub, t0 + 5 * 900 + 10)])
+        u = np.concatenate([u, np.full(hub, 3, np.int32)])
+        v = np.concatenate([v, 10 + np.arange(hub, dtype=np.int32)])
+    end = start + rng.integers(1, 800, len(start))
+    kw = dict(step_size=900.0, window=window, start_time=t0, seed=3, ncls_cap=0, beta=2e-3, p_ei=0.2, p_ir=0.05,
+              initial_infected=0.2)
+    g = rb.Graph.from_arrays(start, end, u, v, nodes)
+    batch = {"networks": first} if networks > 1 else {}
+    sim = rb.Simulation(g, M=70, iterations=24, transition="geometric", path="batched", csr="per-step", **batch, **kw)
+    if networks > 1:
+        batch = {"net_first": first}
+    want = oracle.run(start, end, u, v, nodes, n_replicas=70, n_steps=24, transition=1, **batch, **kw)
+    np.testing.assert_array_equal(sim.run(), want)
+    np.testing.assert_array_equal(sim.run(), want)
