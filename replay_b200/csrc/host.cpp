@@ -881,7 +881,8 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
   s.c.th.te = thr(p.p_ei, s.c.th.te_all);
   s.c.th.ti = thr(p.p_ir, s.c.th.ti_all);
   s.c.th.tr = thr(p.p_rs, s.c.th.tr_all);
-  s.c.th.small = ((s.c.th.te | s.c.th.ti | s.c.th.tr) >> 60) == 0;
+  const unsigned long long any = s.c.th.te | s.c.th.ti | s.c.th.tr;
+  s.c.th.lead = (any >> 56) == 0 ? 8 : ((any >> 60) == 0 ? 4 : 0);
   for (int k = 0; k < 8; ++k) {
     s.c.th.me[k] = (s.c.th.te >> (63 - k)) & 1 ? ~0u : 0u;
     s.c.th.mi[k] = (s.c.th.ti >> (63 - k)) & 1 ? ~0u : 0u;

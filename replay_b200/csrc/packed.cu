@@ -418,7 +418,9 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, i
 // again.  (Before, a word with candidates took one pass over its row with lane
 // = replica and an e_max bound near 1 let nearly every exposed replica
 // through: 7.5 ms on the first steps of the dense network, N = 5,000 and
-// M = 16,384; see k_infect for the time now.)
+// M = 16,384, 0.15-0.49 ms now.  The line at 48 pairs and the block-wide line
+// at 256: 216 us a step there; 48/128 222, 32/128 224, 63/192 222, 32/512 242,
+// 16/512 261.)
 __device__ __forceinline__ void sliced_add(uint32_t (&s)[32], uint32_t m, uint32_t w, int nb) {
   uint32_t cy = 0;
 #pragma unroll
@@ -486,10 +488,10 @@ __device__ __forceinline__ uint32_t heavy_sum(const HeavyUnit &h, HeavyWarp &H, 
   uint32_t X = 0;
   const uint32_t *mw = d.mask + min(h.w0 + lane, L.words - 1);
   const int nb = min(h.nb, 32);
-  for (int32_t k = h.beg + first; k < h.end; k += 4 * stride) {
-    uint32_t m[4], w[4];
+  for (int32_t k = h.beg + first; k < h.end; k += 2 * stride) {
+    uint32_t m[2], w[2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j) {
       m[j] = 0;
       w[j] = 0;
       if (k + j * stride < h.end) {
@@ -499,7 +501,7 @@ __device__ __forceinline__ uint32_t heavy_sum(const HeavyUnit &h, HeavyWarp &H, 
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j) {
       m[j] &= h.S;
       X |= m[j];
       if (h.nb <= 32 && __any_sync(kFull, m[j] != 0u)) sliced_add(s, m[j], w[j], nb);
@@ -590,39 +592,39 @@ __global__ void __launch_bounds__(kThreads, 3)
     const int nws = (L.words + 31) / 32;
     HeavyWarp &H = *reinterpret_cast<HeavyWarp *>(s_dyn + warp * kInfectWarpBytes);
     HeavyUnit h;
-    // rows of more than kHugePairs pairs: the block's warps share the pairs,
-    // warp 0 adds their planes, and the decisions are shared again
-    for (int u = blockIdx.x; u < n_huge * nws; u += gridDim.x) {
-      if (!heavy_load(h, d.heavy_end - 1, -1, u, nws, lane, L, d)) continue;  // same for all warps
-      uint32_t X = heavy_sum(h, H, warp, kWarps, lane, L, d);
-      H.C[lane] = X;
-      __syncthreads();
-      HeavyWarp &H0 = *reinterpret_cast<HeavyWarp *>(s_dyn);
-      if (warp == 0) {
-        for (int v = 1; v < kWarps; ++v) {
+    // Rows of more than kHugePairs pairs first: the block's warps share the
+    // pairs, warp 0 adds their planes, and the decisions are shared again.
+    // Then one warp per unit.  (One loop for both: a second copy of the
+    // unrolled sums costs more in instruction fetches than the tests here.)
+    bool huge = n_huge > 0;
+    for (int u = huge ? (int)blockIdx.x : gw;; u += huge ? (int)gridDim.x : tw) {
+      if (huge && u >= n_huge * nws) {  // the same for all warps of the block
+        huge = false;
+        u = gw;
+      }
+      if (!huge && u >= n_heavy * nws) break;
+      if (!heavy_load(h, huge ? d.heavy_end - 1 : d.heavy, huge ? -1 : 1, u, nws, lane, L, d))
+        continue;
+      uint32_t X = heavy_sum(h, H, huge ? warp : 0, huge ? kWarps : 1, lane, L, d);
+      HeavyWarp &Hd = huge ? *reinterpret_cast<HeavyWarp *>(s_dyn) : H;
+      if (huge) {
+        H.C[lane] = X;
+        __syncthreads();
+        for (int v = 1; v < kWarps && warp == 0; ++v) {
           const HeavyWarp &Hv = *reinterpret_cast<const HeavyWarp *>(s_dyn + v * kInfectWarpBytes);
           X |= Hv.C[lane];
           uint32_t cy = 0;
           for (int k = 0; k < min(h.nb, 32); ++k) {
-            const uint32_t a = H0.e[k][lane], t = Hv.e[k][lane];
-            H0.e[k][lane] = a ^ t ^ cy;
+            const uint32_t a = H.e[k][lane], t = Hv.e[k][lane];
+            H.e[k][lane] = a ^ t ^ cy;
             cy = (a & t) | (a & cy) | (t & cy);
           }
         }
-        heavy_candidates(h, H0, X, lane, L, d, c);
       }
-      __syncthreads();
-      heavy_decide(h, H0, warp, kWarps, lane, L, d, c);
-      __syncthreads();
-    }
-    for (int u = gw; u < n_heavy * nws; u += tw) {
-      if (!heavy_load(h, d.heavy, 1, u, nws, lane, L, d)) continue;
-      const uint32_t X = heavy_sum(h, H, 0, 1, lane, L, d);
-      if (!__any_sync(kFull, X != 0u)) continue;
-      heavy_candidates(h, H, X, lane, L, d, c);
-      __syncwarp();
-      heavy_decide(h, H, 0, 1, lane, L, d, c);
-      __syncwarp();
+      if (!huge || warp == 0) heavy_candidates(h, Hd, X, lane, L, d, c);
+      if (huge) __syncthreads(); else __syncwarp();
+      heavy_decide(h, Hd, huge ? warp : 0, huge ? kWarps : 1, lane, L, d, c);
+      if (huge) __syncthreads(); else __syncwarp();
     }
   }
 
@@ -1094,10 +1096,11 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
     got = 0;
     __syncwarp();  // bits are cleared before a round of this warp may set them
-    // Two rounds of draws, 32 words each.  With every rate below 1/16 the first
-    // draw (planes 0-3) leaves one candidate in 16, and a word without any and
-    // without infection events is done: no second draw, no write.  The words
-    // left are collected again, so that the second round's lanes are full too.
+    // Two rounds of draws, 32 words each.  With every rate below 1/16 (1/256)
+    // the first round (planes 0-3, or 0-7) leaves one candidate in 16 (256),
+    // and a word without any and without infection events is done: no second
+    // draw, no write.  The words left are collected again, so that the second
+    // round's lanes are full too.
     for (;;) {
       const bool first = n1 >= 32 || (flushing && n1 > 0);
       if (first) {
@@ -1109,8 +1112,8 @@ __global__ void __launch_bounds__(kThreads, 3)
         if (lane < take) {
           q = Q.q[n1 + lane];
           cand = flow_candidates(~q.z & q.w, q.z & ~q.w, waning ? (q.z & q.w) : 0u, c.th);
-          if (c.th.small && cand)
-            cand = flow_top(cand, c.rk, q.x, d.step, (q.y & ~kWordEvent) + (c.roff >> 5));
+          if (c.th.lead && cand)
+            cand = flow_top(cand, c.th, c.rk, q.x, d.step, (q.y & ~kWordEvent) + (c.roff >> 5));
           keep = cand || q.y >= kWordEvent || certain;
         }
         const unsigned km = __ballot_sync(kFull, keep);

@@ -169,28 +169,36 @@ __device__ __forceinline__ uint32_t flow_sure(uint32_t E, uint32_t I, uint32_t R
                                               const FlowThresholds &th) {
   return (th.te_all ? E : 0u) | (th.ti_all ? I : 0u) | (th.tr_all ? R : 0u);
 }
-// Planes 0-3 where every threshold is below 1/16 (th.small): the replicas of
-// `cand` whose top four uniform bits are 0; the others do not move.
-__device__ __forceinline__ uint32_t flow_top(uint32_t cand, const uint32_t *rk, uint32_t node,
-                                             uint32_t step, uint32_t word) {
-  uint32_t x[4];
-  philox4x32_10_rk(node, step, word, 0u, rk, x);
+// The first th.lead planes (4, or 8) where every threshold has zeros: the
+// replicas of `cand` whose uniform has them, too; the others do not move.
+__device__ __forceinline__ uint32_t flow_top(uint32_t cand, const FlowThresholds &th,
+                                             const uint32_t *rk, uint32_t node, uint32_t step,
+                                             uint32_t word) {
+  uint32_t x[8];
+  if (th.lead >= 8) {
+    philox4x32_10_rk_x2(node, step, word, 0u, 1u << 4, rk, x, x + 4);
+    cand &= ~(x[4] | x[5] | x[6] | x[7]);
+  } else {
+    philox4x32_10_rk(node, step, word, 0u, rk, x);
+  }
   return cand & ~(x[0] | x[1] | x[2] | x[3]);
 }
-// Events among the candidates `cand` (those flow_top left, with th.small).
+// Events among the candidates `cand` (those flow_top left, with th.lead > 0).
 __device__ __forceinline__ uint32_t flow_rest(uint32_t cand, uint32_t E, uint32_t I, uint32_t R,
                                               const FlowThresholds &th, const uint32_t *rk,
                                               uint32_t node, uint32_t step, uint32_t word) {
   const uint32_t e2 = E & cand, i2 = I & cand, r2 = R & cand;
   uint32_t x[4], less = 0, same = cand;
-  philox4x32_10_rk(node, step, word, 1u << 4, rk, x);
+  if (th.lead < 8) {
+    philox4x32_10_rk(node, step, word, 1u << 4, rk, x);
 #pragma unroll
-  for (int k = 7; k >= 4; --k) {
-    const uint32_t t = (e2 & th.me[k]) | (i2 & th.mi[k]) | (r2 & th.mr[k]);
-    less = maj_not(x[k - 4], less, t);
-    same &= ~(t ^ x[k - 4]);
+    for (int k = 7; k >= 4; --k) {
+      const uint32_t t = (e2 & th.me[k]) | (i2 & th.mi[k]) | (r2 & th.mr[k]);
+      less = maj_not(x[k - 4], less, t);
+      same &= ~(t ^ x[k - 4]);
+    }
   }
-  if (!th.small) {
+  if (th.lead < 4) {
     philox4x32_10_rk(node, step, word, 0u, rk, x);
 #pragma unroll
     for (int k = 3; k >= 0; --k) {
@@ -226,7 +234,7 @@ __device__ __forceinline__ uint32_t flow_events(uint32_t E, uint32_t I, uint32_t
                                                 uint32_t node, uint32_t step, uint32_t word) {
   uint32_t cand = flow_candidates(E, I, R, th);
   const uint32_t sure = flow_sure(E, I, R, th);
-  if (cand && th.small) cand = flow_top(cand, rk, node, step, word);
+  if (cand && th.lead) cand = flow_top(cand, th, rk, node, step, word);
   return cand ? sure | flow_rest(cand, E, I, R, th, rk, node, step, word) : sure;
 }
 

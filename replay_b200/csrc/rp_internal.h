@@ -15,7 +15,7 @@ namespace rp {
 struct FlowThresholds {
   unsigned long long te, ti, tr;
   int te_all, ti_all, tr_all;
-  int small;                     // every threshold's top four bits are 0
+  int lead;                      // every threshold's first 8, 4 or 0 bits are 0
   uint32_t me[8], mi[8], mr[8];  // their top 8 bits as masks, most significant first
 };
 
@@ -263,7 +263,7 @@ struct Hit {
 // rows of more than kHeavyPairs pairs from the front of the list, of more than
 // kHugePairs pairs from its end; counts[0] and counts[2] of them.  A sparse
 // window lists entries of its RowList.
-constexpr int32_t kHeavyPairs = 32, kHugePairs = 512;
+constexpr int32_t kHeavyPairs = 48, kHugePairs = 256;
 struct HeavyRows {
   const int32_t *rows, *end;
   const unsigned long long *counts;

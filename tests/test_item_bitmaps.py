@@ -1,7 +1,7 @@
 """The batched geometric step by active items (bitmaps of 128-replica items)
 and its paths for rows with many contacts, against the oracle at the sizes
 where the layout changes: columns per row around the powers of two and the
-32-column slices, rows around 32 and 512 pairs, replicas that return to
+32-column slices, rows around 48 and 256 pairs, replicas that return to
 susceptible, certain and impossible transitions."""
 import numpy as np
 import pytest
@@ -39,6 +39,7 @@ RULES = [
     dict(p_ir=1.0, has_exposed=False, ir_to_s=True, initial_infected=0.1),  # certain I -> S
     dict(p_ei=0.0, p_ir=0.03, initial_infected=0.1),                  # E never leaves
     dict(p_ir=0.02, has_exposed=False, p_rs=0.01, initial_infected=0.9),    # few susceptibles left
+    dict(p_ei=0.0038, p_ir=0.002, p_rs=0.003, initial_infected=0.4),  # every rate below 1/256
 ]
 
 
@@ -69,7 +70,7 @@ def hubs(degrees, n):
 @pytest.mark.parametrize("replicas", [40, 1100, 4200])
 def test_rows_with_many_pairs(oracle, replicas, csr):
     n = 1500
-    net = hubs([31, 32, 33, 64, 511, 512, 513, 900, 1300], n)
+    net = hubs([47, 48, 49, 64, 255, 256, 257, 512, 900, 1300], n)
     beta = np.geomspace(1e-8, 3e-3, replicas).astype(np.float32)
     _check(oracle, net, n, csr=csr, M=replicas, iterations=4, beta_per_replica=beta, p_ei=0.3, p_ir=0.05,
            initial_infected=0.05)

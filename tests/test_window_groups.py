@@ -53,9 +53,9 @@ def test_grouped_windows_match_oracle(oracle, case):
 
 
 # fewer than one row in eight with a contact per window: windows that list their rows, alone and in a batch,
-# with a hub row above 32 and above 512 pairs, windows without contacts, two steps per window
+# with a hub row above 48 and above 256 pairs, windows without contacts, two steps per window
 @pytest.mark.gpu
-@pytest.mark.parametrize("nodes,hub,window,networks", [(5000, 0, 900, 1), (9000, 40, 900, 3), (40_000, 700, 1800, 1)])
+@pytest.mark.parametrize("nodes,hub,window,networks", [(5000, 0, 900, 1), (9000, 60, 900, 3), (40_000, 700, 1800, 1)])
 def test_sparse_windows_match_oracle(oracle, nodes, hub, window, networks):
     import torch
     if not torch.cuda.is_available():
