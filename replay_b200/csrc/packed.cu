@@ -132,12 +132,9 @@ struct InfectWarp {
   int32_t ubeg[kUnitRows];     // their first pairs
   int32_t list[128];           // items of a batch of 32 rows: row in batch << 5 | column
   uint32_t rmask[32];          // column masks of the batch's rows
-  int32_t row[kInfectQueue];
-  int32_t word[kInfectQueue];  // word index within the row
-  int32_t beg[kInfectQueue];   // the row's first CSR pair and pairs
-  int32_t npr[kInfectQueue];
-  uint32_t X[kInfectQueue];    // exposed replicas of the word
-  float efmax[kInfectQueue];   // ef(e_max) of the row (countdown rule: x_max, or kSure)
+  uint4 q[kInfectQueue];       // row, word in the row, exposed replicas, ef(e_max) of the row
+                               // (countdown rule: x_max, or kSure)
+  int2 span[kInfectQueue];     // the row's first CSR pair and pairs
   uint16_t cl[1024];           // candidates after the bound test: lane << 5 | bit (round scratch)
   // candidates carried to the next round (fewer than 32), self-contained
   int32_t krow[32];
@@ -145,7 +142,6 @@ struct InfectWarp {
   int32_t kbeg[32];
   int32_t knpr[32];
   uint8_t ku8[32];             // top 8 bits of the replica's uniform
-  int32_t n;
   int32_t nk;
 };
 // Per warp, for rows of more than kHeavyPairs pairs (before the queue is used).
@@ -197,7 +193,7 @@ __device__ __forceinline__ void decide(const InfectArgs &d, const StepConsts &c,
   if (!(xx > 0.0f)) return;
   // P <= x: a uniform whose top byte is above x's cannot infect (no
   // exponential)
-  if (xx < 1.0f && u8 > (uint32_t)(fixed64(xx) >> 56)) return;
+  if (xx < 1.0f && u8 > fixed8(xx)) return;
   const uint32_t gword = (uint32_t)word + (c.roff >> 5);
   if (infect_event(one_minus_exp_neg(xx), u8, c.rk, (uint32_t)row, d.step,
                    gword * 32u + (uint32_t)b)) {
@@ -244,12 +240,12 @@ __device__ __forceinline__ void countdown_decide(const InfectArgs &d, const Step
 // Candidates of the round's words into Q.cl; returns their number.  One lane
 // takes one quad of replicas with an exposed member (a draw covers a quad), so
 // that sparse words share the draws; the events of sure words are set here.
-__device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int n, int lane,
+__device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int at0, int n, int lane,
                                                     const InfectArgs &d, const StepConsts &c,
                                                     const PackedLayout &L) {
   uint16_t *quads = reinterpret_cast<uint16_t *>(Q.pl[0]);  // lane << 3 | quad, at most 256
   uint32_t *events = reinterpret_cast<uint32_t *>(Q.pl[16]);  // of the sure words
-  const uint32_t X = lane < n ? Q.X[lane] : 0u;
+  const uint32_t X = lane < n ? Q.q[at0 + lane].z : 0u;
   int nq = 0;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
@@ -267,9 +263,10 @@ __device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int n, int la
     if (p < nq) {
       o = quads[p] >> 3;
       q = quads[p] & 7;
-      const int row = Q.row[o], word = Q.word[o];
-      const bool sure = Q.efmax[o] == kSure;
-      const float lim = sure ? 1.0f : Q.efmax[o];
+      const uint4 w4 = Q.q[at0 + o];
+      const int row = (int)w4.x, word = (int)w4.y;
+      const bool sure = __uint_as_float(w4.w) == kSure;
+      const float lim = sure ? 1.0f : __uint_as_float(w4.w);
       // u = k 2^-24 < lim with k = (x >> 8) + 1, as x <= (K << 8) - 1 for the
       // largest such k
       const uint32_t K = !(lim > 0.0f) ? 0u
@@ -281,7 +278,7 @@ __device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int n, int la
                        kStreamInfect, c.rk, x);
 #pragma unroll
       for (int k = 0; k < 4; ++k) m |= x[k] <= last ? 1u << k : 0u;
-      m = K ? m & Q.X[o] >> (4 * q) : 0u;
+      m = K ? m & w4.z >> (4 * q) : 0u;
       if (sure) {
         if (m) atomicOr(&events[o], m << (4 * q));
         m = 0;
@@ -293,34 +290,38 @@ __device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int n, int la
     total += sum;
   }
   __syncwarp();
-  if (events[lane]) set_events(d, L, Q.row[lane], Q.word[lane], events[lane]);
+  if (events[lane]) {
+    const uint4 w4 = Q.q[at0 + lane];
+    set_events(d, L, (int)w4.x, (int)w4.y, events[lane]);
+  }
   return total;
 }
 
-// Decides up to 32 queued exposed words: the bound test one word per lane,
+// Decides the n <= 32 queued exposed words from at0: the bound test one word per lane,
 // then the exact test of the surviving candidates, one replica per lane, in
 // full batches of 32 together with the candidates carried from earlier
 // rounds; fewer than 32 left over are carried to the next round unless
 // `drain` is set.  Events are OR-ed into their words and flag their items.
 template <bool kCountdown>
-__device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, int lane,
+__device__ __forceinline__ void infect_round(InfectWarp &Q, int at0, int n, bool drain, int lane,
                                              const PackedLayout &L, const InfectArgs &d,
                                              const StepConsts &c) {
   // ---- bound test, one word per lane ----
   int ctotal;
   if constexpr (kCountdown) {
-    ctotal = countdown_candidates(Q, n, lane, d, c, L);
+    ctotal = countdown_candidates(Q, at0, n, lane, d, c, L);
   } else {
     uint32_t Cw = 0;
     if (lane < n) {
-      const int row = Q.row[lane], word = Q.word[lane];
+      const uint4 q = Q.q[at0 + lane];
+      const int row = (int)q.x, word = (int)q.y;
       // every exposed replica has P <= x <= |bs_r| ef(e_max) =: B; replicas
       // whose uniform's top byte is above B's cannot infect
-      const float B = __fmul_rn(word_bs(c, row, word), Q.efmax[lane]);
+      const float B = __fmul_rn(word_bs(c, row, word), __uint_as_float(q.w));
       if (B > 0.0f) {
         uint32_t pl[8];
         infect_planes(c.rk, (uint32_t)row, d.step, (uint32_t)word + (c.roff >> 5), pl);
-        Cw = B >= 1.0f ? Q.X[lane] : top8_le(Q.X[lane], fixed64(B), pl);
+        Cw = B >= 1.0f ? q.z : top8_le(q.z, fixed8(B), pl);
         Q.pl[lane][0] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
         Q.pl[lane][1] = make_uint4(pl[4], pl[5], pl[6], pl[7]);
       }
@@ -351,11 +352,13 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, i
       } else {
         const int ob = Q.cl[p - nk], o = ob >> 5;
         b = ob & 31;
-        row = Q.row[o];
-        word = Q.word[o];
-        npairs = Q.npr[o];
+        const uint2 rw = *reinterpret_cast<const uint2 *>(&Q.q[at0 + o]);
+        const int2 sp = Q.span[at0 + o];
+        row = (int)rw.x;
+        word = (int)rw.y;
+        npairs = sp.y;
         if (!kCountdown) u8 = queued_top8(Q.pl[o], (uint32_t)b);
-        beg = Q.beg[o];
+        beg = sp.x;
       }
       long long e = 0;
       float ef = 0.0f;
@@ -394,10 +397,11 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int n, bool drain, i
     const int p = base + lane;
     if (p < total && p >= nk) {
       const int ob = Q.cl[p - nk], o = ob >> 5, b = ob & 31;
-      Q.kwb[lane] = Q.word[o] << 5 | b;
-      Q.krow[lane] = Q.row[o];
-      Q.kbeg[lane] = Q.beg[o];
-      Q.knpr[lane] = Q.npr[o];
+      const int2 sp = Q.span[at0 + o];
+      Q.kwb[lane] = (int)Q.q[at0 + o].y << 5 | b;
+      Q.krow[lane] = (int)Q.q[at0 + o].x;
+      Q.kbeg[lane] = sp.x;
+      Q.knpr[lane] = sp.y;
       if (!kCountdown) Q.ku8[lane] = (uint8_t)queued_top8(Q.pl[o], (uint32_t)b);
     }
   }
@@ -629,11 +633,9 @@ __global__ void __launch_bounds__(kThreads, 3)
   }
 
   InfectWarp &Q = *reinterpret_cast<InfectWarp *>(s_dyn + warp * kInfectWarpBytes);
-  if (lane == 0) {
-    Q.n = 0;
-    Q.nk = 0;
-  }
+  if (lane == 0) Q.nk = 0;
   __syncwarp();
+  int nq = 0;  // queued words
   const int n_rows = d.list.rows ? (int)d.list.counts[1] : L.n_nodes;
   const int n_units =
       d.list.rows ? (n_rows + d.unit_rows - 1) / d.unit_rows * L.n_slices : d.n_units;
@@ -812,37 +814,20 @@ __global__ void __launch_bounds__(kThreads, 3)
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       const unsigned qm = __ballot_sync(kFull, X[w] != 0u);
-      if (!qm) continue;
-      const int base = Q.n;
       if (X[w]) {
-        const int pos = base + __popc(qm & ((1u << lane) - 1u));
-        Q.row[pos] = row;
-        Q.word[pos] = 4 * col + w;
-        Q.beg[pos] = rbeg;
-        Q.npr[pos] = rn;
-        Q.X[pos] = X[w];
-        Q.efmax[pos] = efmax;
+        const int pos = nq + __popc(qm & ((1u << lane) - 1u));
+        Q.q[pos] = make_uint4((uint32_t)row, (uint32_t)(4 * col + w), X[w], __float_as_uint(efmax));
+        Q.span[pos] = make_int2(rbeg, rn);
       }
-      __syncwarp();
-      if (lane == 0) Q.n = base + __popc(qm);
-      __syncwarp();
+      nq += __popc(qm);
     }
-    // ---- decide full rounds and, past the last unit, what is left ----
-    while (Q.n >= 32 || (!more && (Q.n > 0 || Q.nk > 0))) {
-      const int take = Q.n < 32 ? Q.n : 32;
-      infect_round<kCountdown>(Q, take, !more && take == Q.n, lane, L, d, c);
-      const int rest = Q.n - take;
-      for (int i = lane; i < rest; i += 32) {
-        Q.row[i] = Q.row[take + i];
-        Q.word[i] = Q.word[take + i];
-        Q.beg[i] = Q.beg[take + i];
-        Q.npr[i] = Q.npr[take + i];
-        Q.X[i] = Q.X[take + i];
-        Q.efmax[i] = Q.efmax[take + i];
-      }
-      __syncwarp();
-      if (lane == 0) Q.n = rest;
-      __syncwarp();
+    __syncwarp();
+    // ---- decide full rounds, the last queued words first, and what is left
+    // past the last unit ----
+    while (nq >= 32 || (!more && (nq > 0 || Q.nk > 0))) {
+      const int take = min(nq, 32);
+      nq -= take;
+      infect_round<kCountdown>(Q, nq, take, !more && nq == 0, lane, L, d, c);
     }
     if (!more) break;
   }

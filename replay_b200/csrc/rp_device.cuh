@@ -244,6 +244,12 @@ __device__ __forceinline__ unsigned long long fixed64(float p) {
   return __float2ull_rz(__fmul_rn(p, 0x1p64f));
 }
 
+// Its top 8 bits (exact: p 2^8 is exact in float; one conversion to 32 bits
+// instead of one to 64).
+__device__ __forceinline__ uint32_t fixed8(float p) {
+  return __float2uint_rz(__fmul_rn(p, 256.0f));
+}
+
 // Geometric infection uniform U_r of replica r, 64 bits, compared with
 // floor(P 2^64).  Its top 8 bits are bit-sliced: bit k (k = 0 is 2^-1) is bit
 // r % 32 of output k % 4 of counter (node, step, r / 32, 4 | (k / 4) << 4),
@@ -268,15 +274,19 @@ __device__ __forceinline__ uint32_t top8_of(const uint32_t pl[8], uint32_t b) {
   return u;
 }
 
-// Replicas of `cand` whose top 8 uniform bits are at most T's: a superset of
-// those with U < T.
-__device__ __forceinline__ uint32_t top8_le(uint32_t cand, unsigned long long T,
-                                            const uint32_t pl[8]) {
-  const uint32_t t8 = (uint32_t)(T >> 56);
+// Replicas of `cand` whose top 8 uniform bits are at most t8 (< 256): with t8
+// the top byte of a threshold, a superset of those below it.
+__device__ __forceinline__ uint32_t top8_le(uint32_t cand, uint32_t t8, const uint32_t pl[8]) {
+  // bits 7..4 and 3..0 of t8 as the sign bits of four bytes each, from which
+  // one byte permute makes a mask
+  const uint32_t hi = t8 * 0x08040201u, lo = (t8 << 4) * 0x08040201u;
   uint32_t le = 0xFFFFFFFFu;  // equal bits below: at most
 #pragma unroll
-  for (int k = 7; k >= 0; --k)
-    le = maj_not(pl[k], le, (uint32_t)((int32_t)(t8 << (24 + k)) >> 31));
+  for (int k = 7; k >= 0; --k) {
+    uint32_t t;  // the byte's sign, replicated
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(t) : "r"(k < 4 ? hi : lo), "r"(0x8888 + 0x1111 * (k & 3)));
+    le = maj_not(pl[k], le, t);
+  }
   return cand & le;
 }
 
@@ -294,10 +304,9 @@ __device__ __forceinline__ bool infect_event(float P, uint32_t u8, const uint32_
                                              uint32_t node, uint32_t step, uint32_t replica) {
   if (!(P > 0.0f)) return false;
   if (P >= 1.0f) return true;
-  const unsigned long long T = fixed64(P);
-  const uint32_t t8 = (uint32_t)(T >> 56);
+  const uint32_t t8 = fixed8(P);
   if (u8 != t8) return u8 < t8;
-  return infect_tail56(rk, node, step, replica) < (T & 0x00FFFFFFFFFFFFFFull);
+  return infect_tail56(rk, node, step, replica) < (fixed64(P) & 0x00FFFFFFFFFFFFFFull);
 }
 
 // Countdown arithmetic of the reference (int op float, truncated back to
