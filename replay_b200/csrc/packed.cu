@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   // warps of one block are gridDim.x apart: neighbouring units go to
   // different SMs
   const int gw = warp * gridDim.x + blockIdx.x, tw = kWarps * gridDim.x;
-  __shared__ unsigned s_next;
+  __shared__ unsigned s_next;  // the block's units handed out so far
   if (threadIdx.x == 0) s_next = 0;
   __syncthreads();
   int n_heavy = 0, n_huge = 0;
@@ -639,12 +639,15 @@ __global__ void __launch_bounds__(kThreads, 3)
   const int n_rows = d.list.rows ? (int)d.list.counts[1] : L.n_nodes;
   const int n_units =
       d.list.rows ? (n_rows + d.unit_rows - 1) / d.unit_rows * L.n_slices : d.n_units;
-  // the block's units, blockIdx.x + k gridDim.x, go to its warps as they ask
+  // the block's units, blockIdx.x + k gridDim.x, go to its warps as they ask;
+  // warps that arrive together (no rows taken above) start with one each
+  const bool own_first = !(n_heavy | n_huge);
   auto next_unit = [&]() {
     int k = 0;
-    if (lane == 0) k = (int)atomicAdd(&s_next, 1u);
+    if (lane == 0) k = (int)atomicAdd(&s_next, 1u) + (own_first ? kWarps : 0);
     return (int)blockIdx.x + __shfl_sync(kFull, k, 0) * (int)gridDim.x;
   };
+  int unit = -1;
   const uint4 *mask4 = reinterpret_cast<const uint4 *>(d.mask);
   const uint4 *sa4 = reinterpret_cast<const uint4 *>(d.sa);
   const uint4 *sb4 = reinterpret_cast<const uint4 *>(d.sb);
@@ -658,7 +661,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   for (;;) {
     if (cnt == 0 && !nz) {
       if (ub >= nrows) {
-        const int unit = next_unit();
+        unit = unit < 0 && own_first ? gw : next_unit();
         if (unit >= n_units) {
           more = false;
         } else {
@@ -942,14 +945,15 @@ __global__ void __launch_bounds__(kThreads, 3)
   const int lane = threadIdx.x & 31;
   const bool waning = c.th.tr_all || c.th.tr != 0;
   __shared__ unsigned s_next;  // the block's units, blockIdx.x + k gridDim.x, taken so far
-  if (threadIdx.x == 0) s_next = 0;
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_next = kWarps * d.take;
   __syncthreads();
   const uint4 *sa4 = reinterpret_cast<const uint4 *>(d.sa);
   const uint4 *sb4 = reinterpret_cast<const uint4 *>(d.sb);
   const uint4 *evs4 = reinterpret_cast<const uint4 *>(d.evs);
   // the lane's unit of the current block: its bitmap word and bits
   int64_t wi = 0;
-  bool more = true;
+  bool more = true, first = true;  // a warp's first block of units is its own
   int wrow = 0, wcol = 0;     // first row and column of the lane's word
   uint32_t aw = 0, ew = 0, iw = 0, sw = 0;
   unsigned nz = 0;            // lanes with items not yet listed
@@ -961,9 +965,12 @@ __global__ void __launch_bounds__(kThreads, 3)
   // keeps the kernel small)
   for (;;) {
     while (!nz && !got && more) {
-      unsigned k = 0;
-      if (lane == 0) k = atomicAdd(&s_next, (unsigned)d.take);
-      k = __shfl_sync(kFull, k, 0);
+      unsigned k = (unsigned)(warp * d.take);
+      if (!first) {
+        if (lane == 0) k = atomicAdd(&s_next, (unsigned)d.take);
+        k = __shfl_sync(kFull, k, 0);
+      }
+      first = false;
       more = blockIdx.x + (int64_t)(k + d.take) * gridDim.x < d.n_units;
       const int64_t u = blockIdx.x + (int64_t)(k + lane) * gridDim.x;
       aw = ew = 0;
@@ -973,9 +980,9 @@ __global__ void __launch_bounds__(kThreads, 3)
         const uint32_t own = (kFull >> (32 - len)) << (len * (int)(u & ((1 << d.split) - 1)));
         aw = d.actb[wi] & own;
         ew = d.evb[wi] & own;
+        iw = d.infb[wi];
+        sw = d.susb[wi];
         if (aw | ew) {
-          iw = d.infb[wi];
-          sw = d.susb[wi];
           const int64_t wr = L.n_slices == 1 ? wi : wi / L.n_slices;
           wrow = (int)wr << (5 - L.lb);
           wcol = (int)(wi - wr * L.n_slices) * 32;
@@ -1014,12 +1021,12 @@ __global__ void __launch_bounds__(kThreads, 3)
     if (flushing && n1 == 0 && n2 == 0) break;
     int rl[kFlowIPL], cl[kFlowIPL];
     uint32_t st[kFlowIPL];
-    uint4 a4[kFlowIPL], b4[kFlowIPL];
+    uint4 a4[kFlowIPL], b4[kFlowIPL], e4[kFlowIPL];
 #pragma unroll
     for (int h = 0; h < kFlowIPL; ++h) {
       st[h] = 0;
       rl[h] = cl[h] = 0;
-      a4[h] = b4[h] = make_uint4(0, 0, 0, 0);
+      a4[h] = b4[h] = e4[h] = make_uint4(0, 0, 0, 0);
       if (32 * h >= got) continue;  // warp-uniform, as below
       const bool in = 32 * h + lane < got;
       if (in) st[h] = Q.list[32 * h + lane];
@@ -1030,6 +1037,7 @@ __global__ void __launch_bounds__(kThreads, 3)
         const int64_t idx = (int64_t)rl[h] * L.q4 + cl[h];
         a4[h] = sa4[idx];
         b4[h] = sb4[idx];
+        if ((st[h] >> 30) & 1u) e4[h] = evs4[idx];
       }
     }
 #pragma unroll
@@ -1050,13 +1058,10 @@ __global__ void __launch_bounds__(kThreads, 3)
       if (waning) s4 |= r4;
       if (c.ir_to_s) s4 |= i4;
       // words with infection events join the queue (they need no draw)
-      if ((st[h] >> 30) & 1u) {
-        const uint4 e4 = evs4[(int64_t)rl[h] * L.q4 + cl[h]];
 #pragma unroll
-        for (int w = 0; w < 4; ++w)
-          if (get4(e4, w)) evm |= 1u << w;
-        cm |= evm;
-      }
+      for (int w = 0; w < 4; ++w)
+        if (get4(e4[h], w)) evm |= 1u << w;
+      cm |= evm;
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const unsigned qm = __ballot_sync(kFull, (cm >> w) & 1u);
@@ -1087,8 +1092,8 @@ __global__ void __launch_bounds__(kThreads, 3)
     // draw, no write.  The words left are collected again, so that the second
     // round's lanes are full too.
     for (;;) {
-      const bool first = n1 >= 32 || (flushing && n1 > 0);
-      if (first) {
+      const bool draw = n1 >= 32 || (flushing && n1 > 0);
+      if (draw) {
         const int take = min(n1, 32);
         n1 -= take;
         uint4 q = make_uint4(0, 0, 0, 0);
@@ -1110,7 +1115,7 @@ __global__ void __launch_bounds__(kThreads, 3)
         n2 += __popc(km);
         __syncwarp();
       }
-      if (n2 >= 32 || (flushing && !first && n2 > 0)) {
+      if (n2 >= 32 || (flushing && !draw && n2 > 0)) {
         const int take = min(n2, 32);
         n2 -= take;
         if (lane < take) {
@@ -1131,7 +1136,7 @@ __global__ void __launch_bounds__(kThreads, 3)
           apply_word(L, d, c, waning, row, word, A, B, ev, f);
         }
         __syncwarp();
-      } else if (!first) {
+      } else if (!draw) {
         break;
       }
     }
@@ -1411,8 +1416,9 @@ static void set_infect_units(const PackedLayout &L, int64_t n_rows, InfectArgs &
   auto units = [&](int rows) { return (n_rows + rows - 1) / rows * L.n_slices; };
   while (d.unit_rows > 1 && units(d.unit_rows) * 2 < warps && (int64_t)d.unit_rows * L.q4 > 8)
     d.unit_rows >>= 1;
-  while (d.unit_rows < kUnitRows && (units(2 * d.unit_rows) >= 4 * warps ||
-                                     (int64_t)d.unit_rows * L.q4 < 8))
+  while (d.unit_rows < kUnitRows &&
+         (units(2 * d.unit_rows) >= 4 * warps || (int64_t)d.unit_rows * L.q4 < 8 ||
+          ((int64_t)d.unit_rows * L.q4 < 32 && units(2 * d.unit_rows) >= warps)))
     d.unit_rows *= 2;
   d.n_units = (int32_t)units(d.unit_rows);
 }
