@@ -356,12 +356,16 @@ enum WeightKind { kWeightF32 = 0, kWeightI32 = 1 };
 // weight 0).
 int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup &grp, int64_t cap,
                          int weight_kind, bool sort_rows, cudaStream_t st);
-// Compacts the sorted, merged CSR in ws (slot 0) into (row_ptr_out, entries_out):
-// drops merged-away entries.  With `heavy` (a list of heavy_cap rows) the rows
-// with many pairs are listed, their counts (4 words, zeroed by the caller) in
+// Compacts the sorted, merged CSRs of the group in ws: row pointers to
+// row_ptr_out (n + 1 per window), pairs (merged-away entries dropped) to
+// entries_out + entries_off[window] (device offsets; null: one window, at
+// entries_out; without entries_out only the row pointers are made).  With
+// `heavy` the rows with many pairs are listed from heavy_off[window] up to the
+// next window's, their counts (4 words a window, zeroed by the caller) in
 // heavy_counts.
-void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out, int2 *entries_out,
-                            cudaStream_t st, int32_t *heavy = nullptr, int64_t heavy_cap = 0,
+void enqueue_window_compact(WindowWorkspace &ws, const WindowGroup &grp, int32_t *row_ptr_out,
+                            int2 *entries_out, const int64_t *entries_off, cudaStream_t st,
+                            int32_t *heavy = nullptr, const int64_t *heavy_off = nullptr,
                             unsigned long long *heavy_counts = nullptr);
 
 // ---- kernels of the step loop -------------------------------------------------

@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(kScanThreads)
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_apply(int32_t *__restrict__ in_all, int32_t n,
                  const int32_t *__restrict__ tiles, int32_t *__restrict__ out_all,
-                 int zero_in, int32_t *__restrict__ heavy_all, int64_t heavy_cap,
-                 unsigned long long *__restrict__ heavy_counts) {
+                 int zero_in, int32_t *__restrict__ heavy_all,
+                 const int64_t *__restrict__ heavy_off, unsigned long long *__restrict__ heavy_counts) {
   __shared__ int wt[32];
   int32_t *in = in_all + (int64_t)blockIdx.y * n;
   int32_t *out = out_all + (int64_t)blockIdx.y * (n + 1);
@@ -270,11 +270,13 @@ __global__ void __launch_bounds__(kScanThreads)
       out[base + j] = ex;
       if (zero_in) in[base + j] = 0;
       if (heavy_all && v[j] > kHeavyPairs) {  // the step kernel's list of long rows
-        int32_t *list = heavy_all + (int64_t)blockIdx.y * heavy_cap;
+        // the window's list: at heavy_off (n_windows + 1 offsets), or n rows a slot
+        const int64_t lo = heavy_off ? heavy_off[blockIdx.y] : (int64_t)blockIdx.y * n;
+        const int64_t hi = heavy_off ? heavy_off[blockIdx.y + 1] : lo + n;
         unsigned long long *cnt = heavy_counts + 4 * blockIdx.y;
         const bool huge = v[j] > kHugePairs;
         const int64_t at = (int64_t)atomicAdd(&cnt[huge ? 2 : 0], 1ull);
-        list[huge ? heavy_cap - 1 - at : at] = (int32_t)(base + j);
+        heavy_all[huge ? hi - 1 - at : lo + at] = (int32_t)(base + j);
       }
     }
     ex += v[j];
@@ -621,8 +623,12 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void k_count_kept(int32_t n, const int32_t *__restrict__ row_ptr,
-                             const int2 *__restrict__ entries, int32_t *__restrict__ len) {
+__global__ void k_count_kept(const WinDesc *__restrict__ wins, int32_t n,
+                             const int32_t *__restrict__ row_ptr_all,
+                             const int2 *__restrict__ entries_all, int32_t *__restrict__ len_all) {
+  const int32_t *row_ptr = row_ptr_all + (int64_t)blockIdx.y * (n + 1);
+  const int2 *entries = entries_all + 2 * wins[blockIdx.y].hit_off;
+  int32_t *len = len_all + (int64_t)blockIdx.y * n;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (int64_t)gridDim.x * blockDim.x) {
     int c = 0;
@@ -631,9 +637,16 @@ __global__ void k_count_kept(int32_t n, const int32_t *__restrict__ row_ptr,
   }
 }
 
-__global__ void k_compact(int32_t n, const int32_t *__restrict__ row_ptr,
-                          const int2 *__restrict__ entries,
-                          const int32_t *__restrict__ out_ptr, int2 *__restrict__ out) {
+// out_off: where each window's pairs go (null: one window, at out).
+__global__ void k_compact(const WinDesc *__restrict__ wins, int32_t n,
+                          const int32_t *__restrict__ row_ptr_all,
+                          const int2 *__restrict__ entries_all,
+                          const int32_t *__restrict__ out_ptr_all,
+                          const int64_t *__restrict__ out_off, int2 *__restrict__ out) {
+  const int32_t *row_ptr = row_ptr_all + (int64_t)blockIdx.y * (n + 1);
+  const int32_t *out_ptr = out_ptr_all + (int64_t)blockIdx.y * (n + 1);
+  const int2 *entries = entries_all + 2 * wins[blockIdx.y].hit_off;
+  if (out_off) out += out_off[blockIdx.y];
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n;
        r += (int64_t)gridDim.x * blockDim.x) {
     int32_t o = out_ptr[r];
@@ -781,7 +794,7 @@ int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup 
   }
   k_scan_apply<<<dim3(ws.n_tiles, G), kScanThreads, 0, st>>>(
       ws.deg.as<int32_t>(), n, ws.tiles.as<int32_t>(), ws.row_ptr.as<int32_t>(), 0,
-      sort_rows ? nullptr : ws.long_rows.as<int32_t>(), n, ctr);
+      sort_rows ? nullptr : ws.long_rows.as<int32_t>(), nullptr, ctr);
   k_fill<<<dim3(grid_for(grp.max_candidates, 256, blocks), G), 256, 0, st>>>(
       wins, ws.hits.as<Hit>(), ws.row_ptr.as<int32_t>(), ws.deg.as<int32_t>(),
       ws.entries.as<int2>(), ws.erank.as<int32_t>(), n, sort_rows);
@@ -799,21 +812,23 @@ int enqueue_window_build(const Graph &g, WindowWorkspace &ws, const WindowGroup 
   return launches;
 }
 
-void enqueue_window_compact(WindowWorkspace &ws, int32_t *row_ptr_out, int2 *entries_out,
-                            cudaStream_t st, int32_t *heavy, int64_t heavy_cap,
+void enqueue_window_compact(WindowWorkspace &ws, const WindowGroup &grp, int32_t *row_ptr_out,
+                            int2 *entries_out, const int64_t *entries_off, cudaStream_t st,
+                            int32_t *heavy, const int64_t *heavy_off,
                             unsigned long long *heavy_counts) {
   const int32_t n = ws.n_nodes;
+  const unsigned G = (unsigned)grp.count;
+  const WinDesc *wins = ws.win.as<WinDesc>() + grp.first;
   int32_t *len = ws.deg.as<int32_t>();
-  k_count_kept<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(n, ws.row_ptr.as<int32_t>(),
-                                                        ws.entries.as<int2>(), len);
+  const dim3 grid(grid_for(n, 256, std::max(1, 148 * 8 / (int)G)), G);
+  k_count_kept<<<grid, 256, 0, st>>>(wins, n, ws.row_ptr.as<int32_t>(), ws.entries.as<int2>(), len);
   if (ws.n_tiles > 1)
-    k_scan_tiles<<<ws.n_tiles, kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>());
-  k_scan_apply<<<ws.n_tiles, kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>(),
-                                                   row_ptr_out, 1, heavy, heavy_cap,
-                                                   heavy_counts);
-  k_compact<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(n, ws.row_ptr.as<int32_t>(),
-                                                     ws.entries.as<int2>(), row_ptr_out,
-                                                     entries_out);
+    k_scan_tiles<<<dim3(ws.n_tiles, G), kScanThreads, 0, st>>>(len, n, ws.tiles.as<int32_t>());
+  k_scan_apply<<<dim3(ws.n_tiles, G), kScanThreads, 0, st>>>(
+      len, n, ws.tiles.as<int32_t>(), row_ptr_out, 1, heavy, heavy_off, heavy_counts);
+  if (entries_out)
+    k_compact<<<grid, 256, 0, st>>>(wins, n, ws.row_ptr.as<int32_t>(), ws.entries.as<int2>(),
+                                    row_ptr_out, entries_off, entries_out);
 }
 
 }  // namespace rp

@@ -148,7 +148,7 @@ rp_status window_csr_noalloc(const Graph &g, int64_t ws, int64_t we, float scale
                               sizeof(hits_raw), cudaMemcpyDeviceToHost, st));
   // compacted pairs go to tmp_e (free once the rows are sorted), the row
   // pointers straight to the caller
-  enqueue_window_compact(w, d_row_ptr, w.tmp_e.as<int2>(), st);
+  enqueue_window_compact(w, grp, d_row_ptr, w.tmp_e.as<int2>(), nullptr, st);
   int32_t total = 0;
   RP_TRY_CUDA(cudaMemcpyAsync(&total, d_row_ptr + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   RP_TRY_CUDA(cudaStreamSynchronize(st));

@@ -84,3 +84,54 @@ def test_sparse_windows_match_oracle(oracle, nodes, hub, window, networks):
     want = oracle.run(start, end, u, v, nodes, n_replicas=70, n_steps=24, transition=1, **batch, **kw)
     np.testing.assert_array_equal(sim.run(), want)
     np.testing.assert_array_equal(sim.run(), want)
+
+
+# prebuilt windows: grouped, empty ones among them, several windows' lists of heavy rows in one arena
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", range(len(CASES)))
+def test_prebuilt_windows_match_oracle(oracle, case):
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import replay_b200 as rb
+    c = CASES[case]
+    net = synthetic.tiny(seed=70 + case, n_nodes=c["n"], n_contacts=c["contacts"], span=c["span"], max_dur=3000)
+    if c.get("cap"):
+        net = capped(net, c)
+    net["u"][::3] = 0  # a hub
+    net["v"][::3] = 1 + net["v"][::3] % (c["n"] - 1)
+    kw = dict(step_size=float(c["step"]), window=c.get("window", c["step"]), start_time=net["t0"], seed=5,
+              ncls_cap=int(bool(c.get("cap"))), initial_infected=0.1)
+    g = rb.Graph.from_arrays(net["start"], net["end"], net["u"], net["v"], c["n"])
+    sim = rb.Simulation(g, M=40, iterations=c["steps"], path="batched", csr="prebuilt", **kw, **c["kw"])
+    mode = 0 if c["kw"]["transition"] == "countdown" else 1
+    want = oracle.run(net["start"], net["end"], net["u"], net["v"], c["n"], n_replicas=40, n_steps=c["steps"],
+                      **kw, **dict(c["kw"], transition=mode))
+    np.testing.assert_array_equal(sim.run(), want)
+
+
+# candidates for more than 1 GB of pairs: the arena is sized by a first pass over the windows
+@pytest.mark.gpu
+def test_prebuilt_arena_sized_by_a_first_pass():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import replay_b200 as rb
+    rng = np.random.default_rng(8)
+    n, m, t0 = 2000, 3_000_000, synthetic.EPOCH_2000
+    start = t0 - m + np.arange(m)
+    end = start + m + 86_400 + 3600
+    u = rng.integers(0, n, m).astype(np.int32)
+    v = ((u + rng.integers(1, n, m)) % n).astype(np.int32)
+    kw = dict(M=32, iterations=24, step_size=3600.0, window=3600, start_time=t0, seed=4, ncls_cap=0, beta=1e-8,
+              p_ei=0.2, p_ir=0.1, initial_infected=0.1, transition="geometric", path="batched")
+    g = rb.Graph.from_arrays(start, end, u, v, n)
+    runs = {}
+    for csr in ("per-step", "prebuilt"):
+        sim = rb.Simulation(g, csr=csr, **kw)
+        runs[csr] = sim.run()
+        nnz = sim.info["nnz_total"]
+    pairs = len(np.unique(np.minimum(u, v).astype(np.int64) * n + np.maximum(u, v)))
+    assert nnz == 24 * 2 * pairs  # every contact spans every window
+    np.testing.assert_array_equal(runs["prebuilt"], runs["per-step"])
+    assert runs["prebuilt"][-1, :, 3].max() < n
