@@ -676,6 +676,8 @@ struct rp_meanfield {
   ParkGuard park;  // destroyed last (see rp_sim)
   rp_sim base;
   int32_t N = 0, T = 0, K = 24, nwarp = 0, n_ckpt = 0;
+  bool cluster = false;        // one cluster runs all steps (mf_forward_cluster)
+  DevBuf steps;                // T MfStep
   bool keep = false;           // ckpt holds x_0 .. x_T, seg_q and seg_e every step
   MfRates rates{};
   bool have_forward = false, has_sus = false;
@@ -1123,7 +1125,10 @@ rp_status mf_capture_forward(rp_meanfield &m) {
   return mf_capture(m, m.fwd, [&](cudaStream_t st) -> rp_status {
     const float *x = ck;
     bool after_kernel = false;
-    for (int32_t t = 0; t < T; ++t) {
+    if (m.cluster)
+      mf_forward_cluster(m.steps.as<MfStep>(), T, N, m.d_rates.as<MfRates>(), m.sus.as<float>(),
+                         ck, m.seg_q.as<float>(), m.seg_e.as<float>(), m.inc_part.as<float>(), st);
+    for (int32_t t = 0; t < T && !m.cluster; ++t) {
       float *nxt = m.keep ? ck + (size_t)(t + 1) * 4 * N : pp[t & 1];
       mf_step(m.base.rp_of(t), m.base.ent_of(t), N, m.base.step_scale[t],
               m.d_rates.as<MfRates>(), m.sus.as<float>(), x, nxt,
@@ -1154,6 +1159,13 @@ rp_status mf_capture_backward(rp_meanfield &m) {
   return mf_capture(m, m.bwd, [&](cudaStream_t st) -> rp_status {
     const float *sus = m.sus.as<float>();
     const MfRates *r = m.d_rates.as<MfRates>();
+    if (m.cluster) {
+      mf_reverse_cluster(m.steps.as<MfStep>(), T, N, r, sus, m.a0.as<float>(), m.ckpt.as<float>(),
+                         m.seg_q.as<float>(), m.seg_e.as<float>(), m.ginc.as<float>(),
+                         m.gx0.as<float>(), m.gsus.as<float>(), m.gpart.as<double>(), st);
+      mf_finish(m.gpart.as<double>(), m.nwarp, m.grates.as<double>(), st);
+      return RP_OK;
+    }
     RP_TRY_CUDA(cudaMemsetAsync(m.gpart.ptr, 0, m.gpart.bytes, st));
     RP_TRY_CUDA(cudaMemsetAsync(m.gsus.ptr, 0, sizeof(float) * (size_t)N, st));
     float *a[2] = {m.a0.as<float>(), m.a1.as<float>()};
@@ -1857,6 +1869,14 @@ RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
     RP_TRY(m->seg_x.alloc(plane * m->K));
     RP_TRY(m->seg_q.alloc(per_step * m->K));
     RP_TRY(m->seg_e.alloc(per_step * m->K));
+  }
+  m->cluster = m->keep && T > 0 && N <= kMfClusterNodes;
+  if (m->cluster) {
+    std::vector<MfStep> steps((size_t)T);
+    for (int32_t t = 0; t < T; ++t) steps[t] = MfStep{b.rp_of(t), b.ent_of(t), b.step_scale[t]};
+    RP_TRY(m->steps.alloc(sizeof(MfStep) * (size_t)T));
+    RP_TRY_CUDA(cudaMemcpy(m->steps.ptr, steps.data(), sizeof(MfStep) * (size_t)T,
+                           cudaMemcpyHostToDevice));
   }
   RP_TRY(m->inc_part.alloc(sizeof(float) * (size_t)m->nwarp * (T > 0 ? T : 1)));
   RP_TRY(m->a0.alloc(plane));

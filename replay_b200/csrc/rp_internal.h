@@ -337,6 +337,22 @@ void mf_adjoint(int32_t n, const int32_t *rp_c, const int2 *ent_c, const float *
                 const float *ginc, int32_t tl, float scale, const MfRates *r, const float *sus,
                 float *a_out, float *z_out, float *gsus, double *gpart, bool early,
                 bool after_kernel, cudaStream_t st);
+// A whole forward, or adjoint, by one thread block cluster: up to
+// kMfClusterNodes nodes, at least one step, every state kept (states holds
+// x_0 .. x_T, q and e a plane per step).
+constexpr int32_t kMfClusterNodes = 4096;
+struct MfStep {
+  const int32_t *row_ptr;
+  const int2 *entries;
+  float scale;
+};
+void mf_forward_cluster(const MfStep *steps, int32_t n_steps, int32_t n, const MfRates *r,
+                        const float *sus, float *states, float *q, float *e, float *inc_part,
+                        cudaStream_t st);
+void mf_reverse_cluster(const MfStep *steps, int32_t n_steps, int32_t n, const MfRates *r,
+                        const float *sus, const float *a_in, const float *states, const float *q,
+                        const float *e, const float *ginc, float *gx0, float *gsus, double *gpart,
+                        cudaStream_t st);
 void mf_finish(const double *gpart, int32_t nwarp, double *out, cudaStream_t st);
 
 // ---- node-state text (text.cu) ----
