@@ -336,8 +336,7 @@ struct rp_sim {
   rp_text_cb text_cb = nullptr;
   void *text_user = nullptr;
   int32_t text_rows = 0;  // replica rows per text chunk
-  int64_t node_digits = 0;
-  DevBuf text_dev[2], text_rowlen, text_rowoff;
+  DevBuf text_dev[2], text_seglen, text_segoff;
   char *text_host[2] = {nullptr, nullptr};
   int64_t *text_len_host = nullptr;
   cudaEvent_t text_ev[2] = {nullptr, nullptr};
@@ -377,10 +376,11 @@ struct rp_sim {
     for (int32_t r0 = 0, k = 0; r0 < M; r0 += text_rows, ++k) {
       const int32_t r1 = std::min(M, r0 + text_rows);
       const int b = k & 1;
-      enqueue_states_text(classes.as<uint8_t>(), N, r0, r1, ts, node_digits,
-                          text_rowlen.as<int64_t>(), text_rowoff.as<int64_t>(),
+      enqueue_states_text(classes.as<uint8_t>(), N, r0, r1, ts,
+                          text_seglen.as<int64_t>(), text_segoff.as<int64_t>(),
                           text_dev[b].as<char>(), st);
-      RP_TRY_CUDA(cudaMemcpyAsync(text_len_host + b, text_rowoff.as<int64_t>() + (r1 - r0),
+      RP_TRY_CUDA(cudaMemcpyAsync(text_len_host + b,
+                                  text_segoff.as<int64_t>() + (r1 - r0) * text_segments(N),
                                   sizeof(int64_t), cudaMemcpyDeviceToHost, st));
       if (prev >= 0) {
         RP_TRY_CUDA(cudaEventSynchronize(text_ev[prev]));
@@ -1550,17 +1550,9 @@ RP_API rp_status rp_sim_run_text(rp_sim *s, int32_t *counts, rp_text_cb cb, void
       RP_TRY_CUDA(cudaEventCreateWithFlags(&s->text_ev[b], cudaEventDisableTiming));
     }
     RP_TRY_CUDA(cudaMallocHost(&s->text_len_host, 2 * sizeof(int64_t)));
-    RP_TRY(s->text_rowlen.alloc(sizeof(int64_t) * (size_t)s->text_rows));
-    RP_TRY(s->text_rowoff.alloc(sizeof(int64_t) * ((size_t)s->text_rows + 1)));
-    int64_t d = 0;
-    for (int64_t i = 0, p10 = 10, nd = 1; i < s->N; ++i) {
-      if (i == p10) {
-        p10 *= 10;
-        ++nd;
-      }
-      d += nd;
-    }
-    s->node_digits = d;
+    const size_t segs = (size_t)(s->text_rows * text_segments(s->N));
+    RP_TRY(s->text_seglen.alloc(sizeof(int64_t) * segs));
+    RP_TRY(s->text_segoff.alloc(sizeof(int64_t) * (segs + 1)));
   }
   s->text_cb = cb;
   s->text_user = user;

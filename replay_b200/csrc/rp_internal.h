@@ -357,8 +357,9 @@ void mf_finish(const double *gpart, int32_t nwarp, double *out, cudaStream_t st)
 
 // ---- node-state text (text.cu) ----
 int64_t text_line_bound(int32_t n_nodes);  // bytes of one line at most
+int64_t text_segments(int32_t n_nodes);    // segments of one replica's lines
 void enqueue_states_text(const uint8_t *cls, int32_t n, int32_t r0, int32_t r1, int64_t ts,
-                         int64_t node_digits, int64_t *rowlen, int64_t *rowoff, char *out,
+                         int64_t *seglen, int64_t *segoff, char *out,
                          cudaStream_t st);
 
 // Scan tiles the window builder uses for n_nodes rows.

@@ -54,3 +54,20 @@ def test_device_text_equals_host_formatting_across_chunks(rb):
     for k, (st, ts) in enumerate(zip(states, times)):
         want = "".join(f"{ts},{r},{i},{STATE_NAMES[s]}\n" for r in range(st.shape[0]) for i, s in enumerate(st[r]))
         assert b"".join(chunks[k]).decode() == want
+
+
+# rows of one line, around one segment of 256 lines, and of several; timestamps that gain a digit or have a sign
+@pytest.mark.parametrize("nodes,replicas,first", [(2, 33, 999_999_000), (255, 1, 999_998_300), (256, 12, -2000),
+                                                  (257, 40, 0), (1100, 101, 946_684_800)])
+def test_lines_of_segments(rb, nodes, replicas, first):
+    net = synthetic.tiny(seed=92, n_nodes=nodes, n_contacts=20 * nodes, span=2 * 3600)
+    shift = first - net["t0"]
+    g = rb.Graph.from_arrays(net["start"] + shift, net["end"] + shift, net["u"], net["v"], nodes)
+    kw = dict(M=replicas, iterations=3, step_size=900.0, window=900, start_time=first, seed=2,
+              transition="geometric", beta=8e-4, p_ei=0.3, p_ir=0.2, initial_infected=0.3, record_node_states=True)
+    want = {}
+    rb.Simulation(g, **kw).run(node_states=lambda k, ts, st: want.setdefault(k, "".join(
+        f"{ts},{r},{i},{STATE_NAMES[s]}\n" for r in range(st.shape[0]) for i, s in enumerate(st[r]))) and 0)
+    got = {}
+    rb.Simulation(g, **kw).run_text(lambda k, ts, data: got.setdefault(k, []).append(data) and 0)
+    assert {k: b"".join(v).decode() for k, v in got.items()} == want
