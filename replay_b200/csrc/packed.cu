@@ -122,6 +122,13 @@ __device__ __forceinline__ uint32_t bit_of(int lb, int row, int col) {
 // network of 1,000 nodes used 32 of 148 SMs.)
 constexpr int kInfectQueue = 160;  // 31 left over + 4 words x 32 lanes of one pass
 constexpr int kUnitRows = 128;     // most rows of a unit
+// Items are listed by the lanes, each in a loop over its own bits, or by the
+// warp, row by row (word by word): the first takes as many turns as the fullest
+// lane has items, the second one a row.  With the lanes always listing where
+// their items fit, a unit of one full word took 32 turns of one lane: 32.4 us a
+// step for N = 20,011, M = 1,001, 28.2 with this line (1 and 4 turns a row:
+// 28.2), N = 5,000 with hubs and M = 16,384 193 and 185, N = 1,000 12.2 and 11.3.
+constexpr int kListTurns = 2;
 
 // Per warp: the unit's rows and items, and a queue of exposed words that
 // accumulates over units and is decided 32 words at a time.
@@ -743,18 +750,22 @@ __global__ void __launch_bounds__(kThreads, 3)
             if (lane == o) m = om;
           }
         m &= sus;
-        // few items: every lane lists its own row's; else row by row below
-        int tot;
-        int pos = warp_excl_scan(__popc(m), lane, tot);
-        if (tot <= 128) {
-          for (; m; m &= m - 1) Q.list[pos++] = lane << 5 | (__ffs(m) - 1);
-          cnt = tot;
-        } else {
-          Q.rmask[lane] = m;
-          nz = __ballot_sync(kFull, m != 0u);
+        // few items on many rows: every lane lists its own row's; else row by
+        // row below, which takes about as long for a row as two turns of the
+        // lanes' loop
+        nz = __ballot_sync(kFull, m != 0u);
+        if (!nz) continue;
+        if (__reduce_max_sync(kFull, __popc(m)) <= kListTurns * __popc(nz)) {
+          int tot;
+          int pos = warp_excl_scan(__popc(m), lane, tot);
+          if (tot <= 128) {
+            for (; m; m &= m - 1) Q.list[pos++] = lane << 5 | (__ffs(m) - 1);
+            cnt = tot;
+            nz = 0;
+          }
         }
+        if (nz) Q.rmask[lane] = m;
         __syncwarp();
-        if (tot == 0) continue;
       }
     }
     while (cnt < 32 && nz) {
@@ -989,19 +1000,22 @@ __global__ void __launch_bounds__(kThreads, 3)
         }
         if (ew) atomicAnd(&d.evb[wi], ~own);
       }
-      // few items: every lane lists its own word's; else word by word below
-      int tot;
-      int pos = warp_excl_scan(__popc(aw | ew), lane, tot);
-      if (tot <= 32 * kFlowIPL) {
-        for (uint32_t t = aw | ew; t; t &= t - 1) {
-          const int b = __ffs(t) - 1;
-          Q.list[pos++] = (uint32_t)(lane << 5 | b) | ((aw >> b) & 1u) << 31 |
-                          ((ew >> b) & 1u) << 30 | ((iw >> b) & 1u) << 29 |
-                          ((sw >> b) & 1u) << 28;
+      // few items in many words: every lane lists its own word's; else word by
+      // word below (one word of 32 items is one turn there, 32 here)
+      nz = __ballot_sync(kFull, (aw | ew) != 0u);
+      if (nz && __reduce_max_sync(kFull, __popc(aw | ew)) <= kListTurns * __popc(nz)) {
+        int tot;
+        int pos = warp_excl_scan(__popc(aw | ew), lane, tot);
+        if (tot <= 32 * kFlowIPL) {
+          for (uint32_t t = aw | ew; t; t &= t - 1) {
+            const int b = __ffs(t) - 1;
+            Q.list[pos++] = (uint32_t)(lane << 5 | b) | ((aw >> b) & 1u) << 31 |
+                            ((ew >> b) & 1u) << 30 | ((iw >> b) & 1u) << 29 |
+                            ((sw >> b) & 1u) << 28;
+          }
+          got = tot;
+          nz = 0;
         }
-        got = tot;
-      } else {
-        nz = __ballot_sync(kFull, (aw | ew) != 0u);
       }
     }
     while (nz && got <= 32 * (kFlowIPL - 1)) {
