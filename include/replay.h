@@ -43,7 +43,7 @@ typedef enum {
   RP_ERR_NOMEM = 4,  /* host or device allocation failed */
   RP_ERR_CUDA = 5,   /* CUDA runtime error */
   RP_ERR_RANGE = 6,  /* size or time arithmetic out of range */
-  RP_ERR_DEVICE = 7  /* a kernel raised its error flag */
+  RP_ERR_DEVICE = 7  /* a kernel raised an error flag (no kernel has one now) */
 } rp_status;
 
 /* Message for the last failed call on this thread ("" if none). */
@@ -304,9 +304,11 @@ RP_API rp_status rp_sim_profile_steps(rp_sim *s, float *step_ms);
 /* Tile autotuner of the batched path (no reference counterpart).  Networks
  * are bucketed by size (floor(log2 nodes)); for each bucket, largest first,
  * the task height (rows of one task: 32..4096) and then the staging depth
- * (CSR pairs the exposure kernel stages per chunk: 192, 384 or the default
- * 768) are chosen by timing the replay's first `probe_steps` steps with
- * CUDA events, keeping a candidate only when it is 2% faster.  The
+ * (192, 384 or the default) are chosen by timing the replay's first
+ * `probe_steps` steps with CUDA events, keeping a candidate only when it is
+ * 2% faster.  The step kernels split their work by themselves: the height
+ * tiles the initial counts and the countdown code table (rings of more than
+ * 16 GB), the staging depth has no effect and is kept for its callers.  The
  * simulation keeps the tuned tiles (and re-captures its CUDA graph); results
  * are unchanged by tiling.  Not for simulations created with
  * record_node_states. */

@@ -249,9 +249,10 @@ class Simulation:
         return self._shape(counts)
 
     def autotune(self, probe_steps=48):
-        """Chooses the batched path's task height and staging depth per
-        network-size bucket by timing the first probe_steps steps; returns
-        the tuner's report (0 = default kept)."""
+        """Chooses the batched path's task height per network-size bucket
+        (the initial counts and the countdown code table are tiled by it) by
+        timing the first probe_steps steps; returns the tuner's report
+        (0 = default kept)."""
         r = _lib.TuneResult()
         check(lib().rp_sim_autotune(self._h, int(probe_steps), C.byref(r)))
         nb = r.n_buckets

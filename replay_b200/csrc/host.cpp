@@ -330,7 +330,8 @@ struct rp_sim {
   std::vector<int32_t> net_bounds;  // n_nets + 1 node offsets (empty: one network)
   std::vector<int32_t> h_first, h_rows;  // per network: first row, rows
   std::vector<int32_t> task_rows;        // per network: rows of one task
-  std::vector<int32_t> task_stage;       // per network: CSR pairs staged per chunk
+  std::vector<int32_t> task_stage;       // per network: the tuner's staging depths (no kernel
+                                         // stages pairs any more)
   int32_t n_slices = 1;
   // node-state text mode (rp_sim_run_text)
   rp_text_cb text_cb = nullptr;
@@ -945,10 +946,9 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
   return RP_OK;
 }
 
-// Rows per batched task: about one wave of CTAs (148 SMs x 3), between 32
-// and 4,096 rows (a task stages its row pointers in shared memory).  Sparse
-// batches of many networks reach the cap: there a task is a short chain of
-// global round trips, and fewer, taller tasks shorten the step.
+// Rows per task of the kernels that tile rows by blocks (the initial counts
+// and the countdown code table): about one wave of CTAs (148 SMs x 3), between
+// 32 and 4,096 rows.
 constexpr int64_t kTaskRowsDefaultMax = 4096;
 int32_t rows_per_task(int32_t n_rows, int32_t n_slices) {
   const int64_t target_tasks = 148 * 3;

@@ -429,9 +429,9 @@ __device__ __forceinline__ void infect_round(InfectWarp &Q, int at0, int n, bool
 // again.  (Before, a word with candidates took one pass over its row with lane
 // = replica and an e_max bound near 1 let nearly every exposed replica
 // through: 7.5 ms on the first steps of the dense network, N = 5,000 and
-// M = 16,384, 0.15-0.49 ms now.  The line at 48 pairs and the block-wide line
-// at 256: 216 us a step there; 48/128 222, 32/128 224, 63/192 222, 32/512 242,
-// 16/512 261.)
+// M = 16,384, 0.15-0.44 ms now.  The line at 48 pairs and the block-wide line
+// at 256, chosen when a step took 216 us there (185 now): 48/128 222, 32/128
+// 224, 63/192 222, 32/512 242, 16/512 261.)
 __device__ __forceinline__ void sliced_add(uint32_t (&s)[32], uint32_t m, uint32_t w, int nb) {
   uint32_t cy = 0;
 #pragma unroll

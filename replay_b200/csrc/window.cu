@@ -688,9 +688,7 @@ rp_status window_workspace_alloc(WindowWorkspace &w, int32_t n_nodes, int32_t sl
   w.n_tiles = window_scan_tiles(n_nodes);
   const size_t n = (size_t)n_nodes, g = (size_t)(slots < 1 ? 1 : slots);
   RP_TRY(w.hits.alloc(sizeof(Hit) * w.cap_hits));
-  // two spare pairs: the step kernel stages entry ranges with 16-byte bulk
-  // copies that may read 8 bytes past the last pair
-  RP_TRY(w.entries.alloc(sizeof(int2) * (w.cap_entries + 2)));
+  RP_TRY(w.entries.alloc(sizeof(int2) * w.cap_entries));
   if (sort_rows) {
     RP_TRY(w.erank.alloc(sizeof(int32_t) * w.cap_entries));
     RP_TRY(w.tmp_e.alloc(sizeof(int2) * w.cap_entries));
