@@ -42,6 +42,7 @@
 // planes before k_flow rewrites them.
 #include "rp_device.cuh"
 #include "rp_internal.h"
+#include "unit_rows.h"
 
 namespace rp {
 namespace {
@@ -121,7 +122,6 @@ __device__ __forceinline__ uint32_t bit_of(int lb, int row, int col) {
 // 51 us on a step of 256 sparse networks with 17% of the items active, and a
 // network of 1,000 nodes used 32 of 148 SMs.)
 constexpr int kInfectQueue = 160;  // 31 left over + 4 words x 32 lanes of one pass
-constexpr int kUnitRows = 128;     // most rows of a unit
 // Items are listed by the lanes, each in a loop over its own bits, or by the
 // warp, row by row (word by word): the first takes as many turns as the fullest
 // lane has items, the second one a row.  With the lanes always listing where
@@ -134,9 +134,7 @@ constexpr int kListTurns = 2;
 // accumulates over units and is decided 32 words at a time.
 struct InfectWarp {
   uint4 pl[32][2];             // the 8 random planes of each word (round scratch)
-  int32_t urow[kUnitRows];     // the unit's rows with pairs: row (or list entry) in unit |
-                               // pairs << 7
-  int32_t ubeg[kUnitRows];     // their first pairs
+  UnitRows u;                  // the unit's rows with pairs
   int32_t list[128];           // items of a batch of 32 rows: row in batch << 5 | column
   uint32_t rmask[32];          // column masks of the batch's rows
   uint4 q[kInfectQueue];       // row, word in the row, exposed replicas, ef(e_max) of the row
@@ -702,9 +700,8 @@ __global__ void __launch_bounds__(kThreads, 3)
               const bool has = len[j] > 0 && (kCountdown || len[j] <= kHeavyPairs);
               const unsigned hm = __ballot_sync(kFull, has);
               if (has) {
-                const int pos = nrows + __popc(hm & ((1u << lane) - 1u));
-                Q.urow[pos] = (r - r0 + 32 * j + lane) | len[j] << 7;
-                Q.ubeg[pos] = b[j];
+                Q.u.put(nrows + __popc(hm & ((1u << lane) - 1u)), r - r0 + 32 * j + lane, b[j],
+                        len[j]);
               }
               nrows += __popc(hm);
             }
@@ -720,10 +717,9 @@ __global__ void __launch_bounds__(kThreads, 3)
       if (more) {
         n = 0;
         if (ub + lane < nrows) {
-          lrow = Q.urow[ub + lane];
-          beg = Q.ubeg[ub + lane];
-          n = lrow >> 7;
-          lrow = r0 + (lrow & 127);
+          lrow = r0 + Q.u.row[ub + lane];
+          beg = Q.u.beg[ub + lane];
+          n = Q.u.len[ub + lane];
           if (d.list.rows) lrow = __ldg(d.list.rows + lrow);
         }
         ub += 32;
