@@ -346,7 +346,9 @@ __global__ void __launch_bounds__(256)
     k_count_seen(const uint8_t *__restrict__ seen, int32_t n_nodes,
                  unsigned long long *__restrict__ count) {
   unsigned c = 0;
-  for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x)
+  // 64 bits: close below 2^31 nodes the last stride passes the largest int32
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes;
+       i += (int64_t)gridDim.x * blockDim.x)
     c += seen[i];
   c = __reduce_add_sync(0xFFFFFFFFu, c);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
