@@ -1297,11 +1297,11 @@ RP_API rp_status rp_graph_from_arrays(const int64_t *start, const int64_t *end,
   h->prep_ms = ms_since(t0);
   const auto t1 = std::chrono::steady_clock::now();
   // the endpoints are ordered, checked and counted on the device; without one,
-  // an argument error still comes before the device error
+  // or without the memory for it, an argument error still comes first
   int64_t bad = -1;
   const rp_status st =
       graph_build_device(h->g, start, end, u, v, n_contacts, n_nodes, true, &bad);
-  if (st == RP_ERR_CUDA) {
+  if (st != RP_OK) {
     for (int64_t k = 0; k < n_contacts && bad < 0; ++k)
       if (u[k] < 0 || v[k] < 0 || u[k] >= n_nodes || v[k] >= n_nodes) bad = k;
   }
