@@ -666,6 +666,20 @@ struct rp_sim {
     if (n_kernels) *n_kernels = k;
     return RP_OK;
   }
+
+  // One replay enqueued step by step on the simulation's stream.  A run that
+  // ends early (a callback's abort, an error) leaves the build of the next
+  // windows on the side stream: it is waited for here, since the next run's
+  // first build, on the main stream, may use the same workspace, and counts into
+  // degrees that every build finds and leaves zero.
+  rp_status run_eager(rp_state_cb cb, void *user, int *n_kernels = nullptr, Marks *mk = nullptr) {
+    const rp_status st = enqueue(stream, cb, user, n_kernels, mk);
+    if (st != RP_OK) {
+      if (side) cudaStreamSynchronize(side);
+      cudaStreamSynchronize(stream);
+    }
+    return st;
+  }
 };
 
 // Mean-field replay: the schedule and prebuilt window CSRs of a geometric
@@ -1517,11 +1531,11 @@ RP_API rp_status rp_sim_run(rp_sim *s, int32_t *counts, rp_state_cb cb, void *us
   }
   RP_TRY_CUDA(cudaSetDevice(s->g->device));
   if (s->p.record_node_states && cb) {
-    RP_TRY(s->enqueue(s->stream, cb, user, nullptr));
+    RP_TRY(s->run_eager(cb, user));
   } else if (s->exec) {
     RP_TRY_CUDA(cudaGraphLaunch(s->exec, s->stream));
   } else {
-    RP_TRY(s->enqueue(s->stream, nullptr, nullptr, nullptr));
+    RP_TRY(s->run_eager(nullptr, nullptr));
   }
   touch_pages(counts, s->counts.bytes);
   RP_TRY_CUDA(cudaStreamSynchronize(s->stream));
@@ -1556,7 +1570,7 @@ RP_API rp_status rp_sim_run_text(rp_sim *s, int32_t *counts, rp_text_cb cb, void
   }
   s->text_cb = cb;
   s->text_user = user;
-  rp_status st = s->enqueue(s->stream, nullptr, nullptr, nullptr);
+  rp_status st = s->run_eager(nullptr, nullptr);
   s->text_cb = nullptr;
   s->text_user = nullptr;
   RP_TRY(st);
@@ -1618,7 +1632,7 @@ RP_API rp_status rp_sim_profile(rp_sim *s, rp_profile *out) {
   rp_sim::Marks mk;
   mk.st = s->stream;
   int nk = 0;
-  RP_TRY(s->enqueue(s->stream, nullptr, nullptr, &nk, &mk));
+  RP_TRY(s->run_eager(nullptr, nullptr, &nk, &mk));
   RP_TRY_CUDA(cudaStreamSynchronize(s->stream));
   memset(out, 0, sizeof(*out));
   for (size_t i = 1; i < mk.ev.size(); ++i) {
@@ -1646,7 +1660,7 @@ RP_API rp_status rp_sim_profile_steps(rp_sim *s, float *step_ms) {
   rp_sim::Marks mk;
   mk.st = s->stream;
   int nk = 0;
-  RP_TRY(s->enqueue(s->stream, nullptr, nullptr, &nk, &mk));
+  RP_TRY(s->run_eager(nullptr, nullptr, &nk, &mk));
   RP_TRY_CUDA(cudaStreamSynchronize(s->stream));
   int t = 0;
   for (size_t i = 1; i < mk.ev.size(); ++i) {
@@ -1718,7 +1732,7 @@ RP_API rp_status rp_sim_autotune(rp_sim *s, int32_t probe_steps, rp_tune_result 
     rp_status st = RP_OK;
     for (int rep = 0; rep < 2 && st == RP_OK; ++rep) {
       if (rep == 1) cudaEventRecord(e0, s->stream);
-      st = s->enqueue(s->stream, nullptr, nullptr, nullptr);
+      st = s->run_eager(nullptr, nullptr);
     }
     s->T = T_full;
     RP_TRY(st);
