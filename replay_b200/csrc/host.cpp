@@ -75,6 +75,10 @@ void *cache_take(int device, size_t n, size_t *cap) {
 }
 
 void cache_put(int device, void *p, size_t cap) {
+  if (cap > kCacheBytes) {  // would push every other block out and go itself
+    free_on(device, p);
+    return;
+  }
   std::vector<KeptBlock> evict;
   {
     std::lock_guard<std::mutex> lk(g_cache_mu);

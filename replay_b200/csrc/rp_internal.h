@@ -41,8 +41,8 @@ rp_status cuda_fail(cudaError_t e, const char *what);
 // buffers (ParkGuard) after synchronizing the device; DevBuf::alloc takes
 // the smallest kept block of the current device that fits (at most twice
 // the request); a failing cudaMalloc returns that device's kept blocks and
-// retries.  At most kCacheBytes stay kept per device (the oldest go first);
-// rp_release_cached_memory returns them all.
+// retries.  At most kCacheBytes stay kept per device (the oldest go first; a
+// larger block is freed); rp_release_cached_memory returns them all.
 constexpr size_t kCacheBytes = size_t(8) << 30;
 void *cache_take(int device, size_t n, size_t *cap);
 void cache_put(int device, void *p, size_t cap);
