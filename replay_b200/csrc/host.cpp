@@ -1607,15 +1607,14 @@ RP_API rp_status rp_sim_get_info(const rp_sim *s, rp_sim_info *o) {
   for (auto &w : s->wins) mc = w.n_candidates > mc ? w.n_candidates : mc;
   o->max_candidates = mc;
   o->prebuilt_nnz = s->prebuilt_nnz;
-  int64_t bytes = 0;
-  const DevBuf *bufs[] = {&s->arena_rp, &s->arena_ent, &s->state, &s->exposure, &s->sa,
-                          &s->sb, &s->mask, &s->mask2, &s->evs, &s->bits,
-                          &s->codes, &s->cd_tab, &s->ring, &s->ring_bits, &s->class_a, &s->class_b,
-                          &s->tasks, &s->ev, &s->rs,
-                          &s->init_counts, &s->counts, &s->beta_r, &s->sus, &s->classes,
-                          &s->wsp.hits, &s->wsp.entries, &s->wsp.erank, &s->wsp.tmp_e,
-                          &s->wsp.tmp_r, &s->wsp.row_ptr, &s->wsp.deg, &s->wsp.tiles,
-                          &s->wsp.long_rows, &s->arena_heavy, &s->arena_heavy_n};
+  int64_t bytes = s->wsp.bytes() + s->wsp2.bytes();
+  const DevBuf *bufs[] = {&s->arena_rp, &s->arena_ent, &s->arena_heavy, &s->arena_heavy_n,
+                          &s->state, &s->exposure, &s->sa, &s->sb, &s->mask, &s->mask2, &s->evs,
+                          &s->bits, &s->codes, &s->cd_tab, &s->ring, &s->ring_bits, &s->class_a,
+                          &s->class_b, &s->tasks, &s->ev, &s->rs, &s->init_counts, &s->net_size,
+                          &s->net_first, &s->net_rows, &s->text_dev[0], &s->text_dev[1],
+                          &s->text_seglen, &s->text_segoff, &s->counts, &s->beta_r, &s->beta_word,
+                          &s->sus, &s->classes};
   for (auto b : bufs) bytes += (int64_t)b->bytes;
   o->device_bytes = bytes;
   o->nnz_total = s->nnz_total;

@@ -302,6 +302,13 @@ struct WindowWorkspace {
   DevBuf long_rows; // int32[G][n]: heavy rows (unsorted rows) or rows to sort in a block
   DevBuf win;       // WinDesc[n_windows]
   DevBuf ranges;    // CandRange[...]
+  int64_t bytes() const {
+    int64_t b = 0;
+    for (const DevBuf *d : {&hits, &entries, &erank, &tmp_e, &tmp_r, &row_ptr, &deg, &tiles, &hpos,
+                            &rows, &span, &placed, &counters, &long_rows, &win, &ranges})
+      b += (int64_t)d->bytes;
+    return b;
+  }
 };
 
 // Room for any group of at most `slots` windows and `cap_hits` candidates.
