@@ -483,7 +483,7 @@ struct rp_sim {
             st);
   }
   // Initial state from the initial-infection plane sa.
-  rp_status ring_init(cudaStream_t st, int &k) {
+  rp_status ring_init(cudaStream_t st, int &launches) {
     RP_TRY_CUDA(cudaMemsetAsync(ring.ptr, 0, ring.bytes, st));
     RP_TRY_CUDA(cudaMemsetAsync(ring_bits.ptr, 0, ring_bits.bytes, st));
     // no infectious replica, every item susceptible (bits without an item are
@@ -499,7 +499,7 @@ struct rp_sim {
     if (!cd_init_ch.empty() && cd_init_ch[0].age == 0)
       src.s[src.n++] = source(cd_init_ch[0], sa.as<uint32_t>(), init_bits(), false);
     ring_flow(src, init_counts.as<unsigned long long>(), st);
-    k += 1 + (src.n > 0);
+    launches += 1 + (src.n > 0);
     return RP_OK;
   }
   template <typename Mark>
@@ -568,19 +568,19 @@ struct rp_sim {
       if (evs.ptr) RP_TRY_CUDA(cudaMemsetAsync(evs.ptr, 0, evs.bytes, st));
       if (rs.ptr && p.p_rs > 0.0f) RP_TRY_CUDA(cudaMemsetAsync(rs.ptr, 0, rs.bytes, st));
       RP_TRY_CUDA(cudaMemsetAsync(init_counts.ptr, 0, init_counts.bytes, st));
-      packed_init(L, sa.as<uint32_t>(), sb.as<uint32_t>(), mask.as<uint32_t>(),
-                  bits.as<uint32_t>(), p.initial_infected, p.initial_count, net_first.as<int32_t>(),
-                  net_rows.as<int32_t>(), n_nets, c, st);
-      if (ring_slots) {
+      k += packed_init(L, sa.as<uint32_t>(), sb.as<uint32_t>(), mask.as<uint32_t>(),
+                       bits.as<uint32_t>(), p.initial_infected, p.initial_count,
+                       net_first.as<int32_t>(), net_rows.as<int32_t>(), n_nets, c, st);
+      if (ring_slots)
         RP_TRY(ring_init(st, k));
-      } else if (cd.code_bytes)  // countdown codes from the initial-infection plane
+      else if (cd.code_bytes)  // countdown codes from the initial-infection plane
         cd_init(L, tasks.as<PackedTask>(), sa.as<uint32_t>(), codes.ptr, cd.code_bytes,
                 mask.as<uint32_t>(), cd_tab.as<uint32_t>(), cd.init_code,
                 init_counts.as<unsigned long long>(), st);
       else
         packed_count(L, tasks.as<PackedTask>(), sa.as<uint32_t>(), sb.as<uint32_t>(),
                      init_counts.as<unsigned long long>(), st);
-      k += 2 + 2 * (p.initial_count > 0);
+      k += !ring_slots;
     }
     mark(kMarkOther);
     RP_TRY(emit_states(0, p.start_time));

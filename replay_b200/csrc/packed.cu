@@ -1387,10 +1387,10 @@ rp_status packed_prepare() {
   return RP_OK;
 }
 
-void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb, uint32_t *mask,
-                 uint32_t *bits, float p0, int32_t k_exact, const int32_t *net_first_row,
-                 const int32_t *net_rows, int32_t n_nets, const StepConsts &c,
-                 cudaStream_t st) {
+int packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb, uint32_t *mask,
+                uint32_t *bits, float p0, int32_t k_exact, const int32_t *net_first_row,
+                const int32_t *net_rows, int32_t n_nets, const StepConsts &c,
+                cudaStream_t st) {
   const int64_t total = (int64_t)L.n_nodes * L.words;
   k_packed_init<<<1184, 256, 0, st>>>(L, sa, sb, mask, k_exact > 0 ? 0.0f : p0, c);
   if (k_exact > 0) {
@@ -1404,6 +1404,7 @@ void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb, uint32_t *ma
         L, reinterpret_cast<const uint4 *>(sa), reinterpret_cast<const uint4 *>(sb), bits,
         bits + L.bit_words, bits + 2 * L.bit_words, bits + 3 * L.bit_words,
         c.th.tr_all || c.th.tr != 0);
+  return 1 + (k_exact > 0 ? 2 : 0) + (bits ? 1 : 0);
 }
 
 void cd_bits(const PackedLayout &L, const uint32_t *plane, uint32_t *bits, cudaStream_t st) {

@@ -445,11 +445,11 @@ struct PackedLayout {
 };
 rp_status packed_prepare();  // kernel attributes, once per device
 // `bits`: the four item bitmaps (act, inf, sus, evb), or null (countdown mode).
-// `bits`: the four item bitmaps (act, inf, sus, evb), or null (countdown mode).
-void packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb,
-                 uint32_t *mask, uint32_t *bits, float p0, int32_t k_exact,
-                 const int32_t *net_first_row, const int32_t *net_rows,
-                 int32_t n_nets, const StepConsts &c, cudaStream_t st);
+// Returns the kernels launched.
+int packed_init(const PackedLayout &L, uint32_t *sa, uint32_t *sb,
+                uint32_t *mask, uint32_t *bits, float p0, int32_t k_exact,
+                const int32_t *net_first_row, const int32_t *net_rows,
+                int32_t n_nets, const StepConsts &c, cudaStream_t st);
 // One step: exposure + infection draws (k_infect), then transitions, counts
 // and the next infectious mask (k_flow).
 void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
