@@ -323,6 +323,7 @@ struct rp_sim {
   // ring_slots steps (bit planes and item bitmaps), sb the replicas that are
   // not susceptible, sa the initially infected ...
   std::vector<CdChange> cd_inf, cd_init_ch;
+  int64_t set_bytes = 0;   // most bytes of these sets
   int32_t ring_slots = 0;  // 0: codes
   DevBuf ring, ring_bits, class_a, class_b;
   // ... or, where the sets would not fit, per-replica codes into the table
@@ -997,6 +998,7 @@ rp_status upload_tasks(rp_sim &s) {
   return RP_OK;
 }
 
+// Most bytes of the countdown rule's sets.
 constexpr int64_t kRingBytes = 16ll << 30;
 
 rp_status alloc_state(rp_sim &s) {
@@ -1055,12 +1057,12 @@ rp_status alloc_state(rp_sim &s) {
   }
   if (s.cd.code_bytes) {
     // the sets of replicas per infection step, as long as an age may still
-    // change: at most kRingBytes, else (or without the memory) codes
+    // change: at most set_bytes, else (or without the memory) codes
     s.cd_inf = s.cd.infect_code ? cd_changes(s.cd, s.cd.infect_code, T) : std::vector<CdChange>();
     s.cd_init_ch =
         s.cd.init_code ? cd_changes(s.cd, s.cd.init_code, T + 1) : std::vector<CdChange>();
     const int32_t slots = s.cd_inf.empty() ? 1 : s.cd_inf.back().age + 1;
-    if ((int64_t)plane * slots <= kRingBytes && (int)s.cd_inf.size() < kCdSources &&
+    if ((int64_t)plane * slots <= s.set_bytes && (int)s.cd_inf.size() < kCdSources &&
         s.ring.alloc(plane * slots) == RP_OK) {
       s.ring_slots = slots;
       RP_TRY(s.ring_bits.alloc(sizeof(uint32_t) * (size_t)L.bit_words * (slots + 3)));
@@ -1434,6 +1436,12 @@ RP_API rp_status rp_sim_create(const rp_graph *h, const rp_params *p, rp_sim **o
 RP_API rp_status rp_sim_create_batch(const rp_graph *h, const rp_params *p,
                                      const int32_t *net_first, int32_t n_networks,
                                      rp_sim **out) {
+  return rp_sim_create_bounded(h, p, net_first, n_networks, kRingBytes, out);
+}
+
+RP_API rp_status rp_sim_create_bounded(const rp_graph *h, const rp_params *p,
+                                       const int32_t *net_first, int32_t n_networks,
+                                       int64_t set_bytes, rp_sim **out) {
   if (!h || !p || !out) {
     set_error("null argument");
     return RP_ERR_ARG;
@@ -1445,6 +1453,7 @@ RP_API rp_status rp_sim_create_batch(const rp_graph *h, const rp_params *p,
   }
   *out = nullptr;
   std::unique_ptr<rp_sim> s(new rp_sim());
+  s->set_bytes = set_bytes;
   if (net_first) {
     const int32_t N = h->g.n_nodes;
     if (n_networks < 1 || net_first[0] != 0 || net_first[n_networks] != N) {

@@ -523,6 +523,13 @@ void plain_spmv_f32_raw(const int32_t *row_ptr, const int32_t *col,
 
 }  // namespace rp
 
+// rp_sim_create_batch with another bound on the bytes of the countdown rule's
+// sets (0: the code table), so that a test can take the code table, the form of
+// replays too large for the sets, at sizes that an oracle can follow.
+extern "C" RP_API rp_status rp_sim_create_bounded(const rp_graph *g, const rp_params *p,
+                                                  const int32_t *net_first, int32_t n_networks,
+                                                  int64_t set_bytes, rp_sim **out);
+
 struct rp_graph {
   rp::ParkGuard park;  // destroyed after g: its blocks are kept for reuse
   rp::Graph g;
