@@ -1055,30 +1055,6 @@ rp_status alloc_state(rp_sim &s) {
     RP_TRY(s.evs.alloc(plane));
     RP_TRY(s.bits.alloc(sizeof(uint32_t) * 4 * (size_t)L.bit_words));
   }
-  if (s.cd.code_bytes) {
-    // the sets of replicas per infection step, as long as an age may still
-    // change: at most set_bytes, else (or without the memory) codes
-    s.cd_inf = s.cd.infect_code ? cd_changes(s.cd, s.cd.infect_code, T) : std::vector<CdChange>();
-    s.cd_init_ch =
-        s.cd.init_code ? cd_changes(s.cd, s.cd.init_code, T + 1) : std::vector<CdChange>();
-    const int32_t slots = s.cd_inf.empty() ? 1 : s.cd_inf.back().age + 1;
-    if ((int64_t)plane * slots <= s.set_bytes && (int)s.cd_inf.size() < kCdSources &&
-        s.ring.alloc(plane * slots) == RP_OK) {
-      s.ring_slots = slots;
-      RP_TRY(s.ring_bits.alloc(sizeof(uint32_t) * (size_t)L.bit_words * (slots + 3)));
-      if (s.p.record_node_states) {
-        RP_TRY(s.class_a.alloc(plane));
-        RP_TRY(s.class_b.alloc(plane));
-      }
-    }
-  }
-  if (s.cd.code_bytes && !s.ring_slots) {
-    RP_TRY(s.mask2.alloc(plane));
-    RP_TRY(s.codes.alloc((size_t)s.cd.code_bytes * 32 * (size_t)N * L.words));
-    RP_TRY(s.cd_tab.alloc(sizeof(uint32_t) * s.cd.tab.size()));
-    RP_TRY_CUDA(cudaMemcpy(s.cd_tab.ptr, s.cd.tab.data(), sizeof(uint32_t) * s.cd.tab.size(),
-                           cudaMemcpyHostToDevice));
-  }
   RP_TRY(upload_tasks(s));
   const size_t per_row = (size_t)s.n_nets * M;
   RP_TRY(s.ev.alloc(sizeof(unsigned long long) * per_row * (size_t)(T > 0 ? T : 1)));
@@ -1093,6 +1069,55 @@ rp_status alloc_state(rp_sim &s) {
   RP_TRY_CUDA(cudaMemcpy(s.net_rows.ptr, rows.data(), sizeof(int32_t) * rows.size(),
                          cudaMemcpyHostToDevice));
   RP_TRY_CUDA(cudaMemcpy(s.net_size.ptr, size.data(), sizeof(int32_t) * size.size(),
+                         cudaMemcpyHostToDevice));
+  return RP_OK;
+}
+
+// What a handle leaves free when it takes memory for speed alone (the countdown
+// rule's sets, the mean-field's kept states): its graph and its text buffers
+// (twice 64 MB) come later.
+constexpr size_t kLeaveBytes = size_t(512) << 20;
+bool memory_left(int device) {
+  size_t free_b = 0, total = 0;
+  if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) return false;
+  if (free_b < kLeaveBytes) {
+    cache_trim(device);
+    if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) return false;
+  }
+  return free_b >= kLeaveBytes;
+}
+
+// The countdown rule's state, after everything else that the replay needs: the
+// sets of replicas per infection step, as long as an age may still change, where
+// they take at most set_bytes and either no more than the codes would or leave
+// memory for what comes later, ...
+bool alloc_sets(rp_sim &s) {
+  const PackedLayout &L = s.L;
+  const size_t plane = sizeof(uint32_t) * (size_t)s.N * L.words;
+  s.cd_inf = s.cd.infect_code ? cd_changes(s.cd, s.cd.infect_code, s.T) : std::vector<CdChange>();
+  s.cd_init_ch =
+      s.cd.init_code ? cd_changes(s.cd, s.cd.init_code, s.T + 1) : std::vector<CdChange>();
+  const int32_t slots = s.cd_inf.empty() ? 1 : s.cd_inf.back().age + 1;
+  if ((int64_t)plane * slots > s.set_bytes || (int)s.cd_inf.size() >= kCdSources) return false;
+  const size_t bits = sizeof(uint32_t) * (size_t)L.bit_words * ((size_t)slots + 3);
+  const size_t codes = plane * (8 * (size_t)s.cd.code_bytes);
+  if (s.ring.alloc(plane * slots) == RP_OK && s.ring_bits.alloc(bits) == RP_OK &&
+      (!s.p.record_node_states ||
+       (s.class_a.alloc(plane) == RP_OK && s.class_b.alloc(plane) == RP_OK)) &&
+      (plane * slots <= codes || memory_left(s.g->device))) {
+    s.ring_slots = slots;
+    return true;
+  }
+  for (DevBuf *b : {&s.ring, &s.ring_bits, &s.class_a, &s.class_b}) b->release();
+  return false;
+}
+// ... else codes into the table.
+rp_status alloc_codes(rp_sim &s) {
+  const PackedLayout &L = s.L;
+  RP_TRY(s.mask2.alloc(sizeof(uint32_t) * (size_t)s.N * L.words));
+  RP_TRY(s.codes.alloc((size_t)s.cd.code_bytes * 32 * (size_t)s.N * L.words));  // 8 planes a byte
+  RP_TRY(s.cd_tab.alloc(sizeof(uint32_t) * s.cd.tab.size()));
+  RP_TRY_CUDA(cudaMemcpy(s.cd_tab.ptr, s.cd.tab.data(), sizeof(uint32_t) * s.cd.tab.size(),
                          cudaMemcpyHostToDevice));
   return RP_OK;
 }
@@ -1503,6 +1528,9 @@ RP_API rp_status rp_sim_create_bounded(const rp_graph *h, const rp_params *p,
     RP_TRY(prebuild(*s));
     s->prebuild_ms = ms_since(t0);
   }
+  t0 = std::chrono::steady_clock::now();
+  if (s->path == RP_PATH_BATCHED && s->cd.code_bytes && !alloc_sets(*s)) RP_TRY(alloc_codes(*s));
+  s->alloc_ms += ms_since(t0);
   t0 = std::chrono::steady_clock::now();
   if (!p->record_node_states) RP_TRY(capture(*s));
   s->capture_ms = ms_since(t0);

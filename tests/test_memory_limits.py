@@ -51,3 +51,33 @@ def test_argument_error_before_the_memory_error():
         with pytest.raises(rb.ReplayError, match=f"contact {n - 3} joins") as e:
             rb.Graph.from_arrays(s, s + 5, u, v, 2)
         assert e.value.status == 1
+
+
+def test_sets_of_replicas_leave_room_or_give_way():
+    """Countdown sets of 1.6 GB in ever less memory: every replay whose codes (200 MB) fit is accepted and
+    gives the same counts."""
+    rb = _rb()
+    n, T, M = 20_000, 160, 4096
+    rng = np.random.default_rng(2)
+    u = rng.integers(0, n - 1, 200_000).astype(np.int32)
+    s = synthetic.EPOCH_2000 + rng.integers(0, T * 600, len(u))
+    g = rb.Graph.from_arrays(s, s + 400, u, u + 1, n)
+    kw = dict(M=M, iterations=T, step_size=600.0, window=600, start_time=synthetic.EPOCH_2000, path="batched", seed=2,
+              initial_infected=0.02, infect_prob=0.5, exposed_duration=30_000, infectious_duration=60_000,
+              resistant_duration=0)
+    sim = rb.Simulation(g, **kw)
+    want = sim.run()
+    full = sim.info["device_bytes"]
+    assert full > 1600 * MB
+    sim.close()
+    # from all the sets would take and more, over every size at which a part of them does not fit, to the codes alone
+    tight = full - 1600 * MB + 200 * MB + 192 * MB
+    taken = []
+    for left in [full + 900 * MB, full + 400 * MB, *range(full + 64 * MB, full - 64 * MB, -8 * MB), 1200 * MB, tight]:
+        with memory_left(rb, left):
+            sim = rb.Simulation(g, **kw)
+            taken.append(sim.info["device_bytes"] == full)
+            if left in (full + 64 * MB, tight):
+                np.testing.assert_array_equal(sim.run(), want)
+            sim.close()
+    assert taken[0] and not any(taken[1:])
