@@ -334,8 +334,11 @@ typedef struct rp_meanfield rp_meanfield;
 /* Builds the schedule and every window CSR (int32 contact-second weights) of
  * the replay described by p: n_steps, step_size, start_time, window,
  * ncls_cap, has_exposed and ir_to_s are used; replica and rate fields are
- * ignored.  The adjoint recomputes states between checkpoints taken every
- * `checkpoint_every` steps.  The graph must outlive the handle. */
+ * ignored.  The forward keeps every state for the adjoint (16 (n_steps + 1) +
+ * 8 n_steps bytes a node) where that is at most 4 GiB and leaves 512 MB of the
+ * device free; otherwise it keeps a checkpoint every `checkpoint_every` steps
+ * and the adjoint recomputes the states in between.  The graph must outlive the
+ * handle. */
 RP_API rp_status rp_meanfield_create(const rp_graph *g, const rp_params *p,
                                      int32_t checkpoint_every,
                                      rp_meanfield **out);
@@ -349,7 +352,7 @@ RP_API void rp_meanfield_free(rp_meanfield *m);
  * with ir_to_s).  d_susceptibility: N floats, or NULL for all ones.
  * d_incidence (n_steps floats): expected new infections sum_i S_i P_i of
  * each step; d_xT (4*N floats, optional): the final planes.  Keeps the
- * checkpoints and parameters for rp_meanfield_backward. */
+ * states (or checkpoints) and parameters for rp_meanfield_backward. */
 RP_API rp_status rp_meanfield_forward(rp_meanfield *m, const float *d_x0,
                                       float beta, const float *d_susceptibility,
                                       float p_ei, float p_ir, float p_rs,

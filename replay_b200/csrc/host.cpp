@@ -689,8 +689,8 @@ struct rp_sim {
 
 // Mean-field replay: the schedule and prebuilt window CSRs of a geometric
 // simulation, FP32 probability planes; the forward keeps every state for the
-// adjoint where they fit in kMfKeepBytes (a third of the adjoint's time was
-// recomputing them), else checkpoints every K steps.
+// adjoint where they fit in kMfKeepBytes and leave kLeaveBytes free (a third of
+// the adjoint's time was recomputing them), else checkpoints every K steps.
 constexpr int64_t kMfKeepBytes = 4ll << 30;
 struct rp_meanfield {
   ParkGuard park;  // destroyed last (see rp_sim)
@@ -1902,28 +1902,6 @@ RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
   m->nwarp = mf_warps(N);
   const size_t plane = sizeof(float) * 4 * (size_t)N;
   const size_t per_step = sizeof(float) * (size_t)N;
-  // every state, exp(-beta s e) and exposure of the forward, or checkpoints
-  m->keep = (int64_t)(plane * ((size_t)T + 1) + 2 * per_step * T) <= kMfKeepBytes &&
-            m->ckpt.alloc(plane * ((size_t)T + 1)) == RP_OK &&
-            m->seg_q.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
-            m->seg_e.alloc(per_step * (T > 0 ? T : 1)) == RP_OK;
-  if (!m->keep) {
-    m->n_ckpt = T > 0 ? (T + m->K - 1) / m->K : 1;
-    RP_TRY(m->ckpt.alloc(plane * m->n_ckpt));
-    RP_TRY(m->xa.alloc(plane));
-    RP_TRY(m->xb.alloc(plane));
-    RP_TRY(m->seg_x.alloc(plane * m->K));
-    RP_TRY(m->seg_q.alloc(per_step * m->K));
-    RP_TRY(m->seg_e.alloc(per_step * m->K));
-  }
-  m->cluster = m->keep && T > 0 && N <= kMfClusterNodes;
-  if (m->cluster) {
-    std::vector<MfStep> steps((size_t)T);
-    for (int32_t t = 0; t < T; ++t) steps[t] = MfStep{b.rp_of(t), b.ent_of(t), b.step_scale[t]};
-    RP_TRY(m->steps.alloc(sizeof(MfStep) * (size_t)T));
-    RP_TRY_CUDA(cudaMemcpy(m->steps.ptr, steps.data(), sizeof(MfStep) * (size_t)T,
-                           cudaMemcpyHostToDevice));
-  }
   RP_TRY(m->inc_part.alloc(sizeof(float) * (size_t)m->nwarp * (T > 0 ? T : 1)));
   RP_TRY(m->a0.alloc(plane));
   RP_TRY(m->a1.alloc(plane));
@@ -1943,6 +1921,32 @@ RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
   RP_TRY(m->gx0.alloc(plane));
   RP_TRY(m->gsus.alloc(sizeof(float) * (size_t)N));
   RP_TRY(m->grates.alloc(sizeof(double) * 4));
+  // last: every state, exp(-beta s e) and exposure of the forward, where they fit
+  // and leave memory for the two graphs or take no more than the checkpoints
+  const size_t kept = plane * ((size_t)T + 1) + 2 * per_step * T;
+  m->n_ckpt = T > 0 ? (T + m->K - 1) / m->K : 1;
+  const size_t segment = plane * m->n_ckpt + (plane * 2 + plane * m->K) + 2 * per_step * m->K;
+  m->keep = (int64_t)kept <= kMfKeepBytes && m->ckpt.alloc(plane * ((size_t)T + 1)) == RP_OK &&
+            m->seg_q.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
+            m->seg_e.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
+            (kept <= segment || memory_left(h->g.device));
+  if (!m->keep) {  // or checkpoints
+    for (DevBuf *buf : {&m->ckpt, &m->seg_q, &m->seg_e}) buf->release();
+    RP_TRY(m->ckpt.alloc(plane * m->n_ckpt));
+    RP_TRY(m->xa.alloc(plane));
+    RP_TRY(m->xb.alloc(plane));
+    RP_TRY(m->seg_x.alloc(plane * m->K));
+    RP_TRY(m->seg_q.alloc(per_step * m->K));
+    RP_TRY(m->seg_e.alloc(per_step * m->K));
+  }
+  m->cluster = m->keep && T > 0 && N <= kMfClusterNodes &&
+               m->steps.alloc(sizeof(MfStep) * (size_t)T) == RP_OK;
+  if (m->cluster) {
+    std::vector<MfStep> steps((size_t)T);
+    for (int32_t t = 0; t < T; ++t) steps[t] = MfStep{b.rp_of(t), b.ent_of(t), b.step_scale[t]};
+    RP_TRY_CUDA(cudaMemcpy(m->steps.ptr, steps.data(), sizeof(MfStep) * (size_t)T,
+                           cudaMemcpyHostToDevice));
+  }
   RP_TRY_CUDA(cudaStreamCreateWithFlags(&m->cap, cudaStreamNonBlocking));
   m->rates.has_exposed = p->has_exposed;
   m->rates.ir_to_s = p->ir_to_s;

@@ -103,7 +103,8 @@ class MeanField:
     Keyword arguments follow Simulation: iterations (n_steps), step_size,
     start_time, window, has_exposed, ir_to_s, ncls_cap; checkpoint_every is
     the adjoint's checkpoint interval in steps (states in between are
-    recomputed)."""
+    recomputed); it applies where the states of all steps take more than
+    4 GiB or would leave less than 512 MB of the device free."""
 
     _ALIASES = {"iterations": "n_steps", "static_network_duration": "window"}
 

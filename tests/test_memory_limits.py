@@ -81,3 +81,41 @@ def test_sets_of_replicas_leave_room_or_give_way():
                 np.testing.assert_array_equal(sim.run(), want)
             sim.close()
     assert taken[0] and not any(taken[1:])
+
+
+def test_kept_states_leave_room_or_give_way():
+    """Mean-field states of 2.4 GB in ever less memory: every replay whose checkpoints (0.4 GB) fit is accepted and
+    gives the same values and gradients, bit for bit for the nodes."""
+    rb = _rb()
+    import torch
+    from replay_b200.meanfield import MeanField
+    n, T = 500_000, 200
+    rng = np.random.default_rng(2)
+    u = rng.integers(0, n - 1, 400_000).astype(np.int32)
+    s = synthetic.EPOCH_2000 + rng.integers(0, T * 600, len(u))
+    g = rb.Graph.from_arrays(s, s + 400, u, u + 1, n)
+    x0 = torch.zeros(4, n, device="cuda")
+    x0[0], x0[2] = 0.9, 0.1
+    x0.requires_grad_()
+
+    def passes(left):
+        """Forward and gradient with `left` bytes free before the creation; the bytes that it took."""
+        with memory_left(rb, left):
+            free = torch.cuda.mem_get_info()[0]
+            mf = MeanField(g, iterations=T, step_size=600.0, window=600, start_time=synthetic.EPOCH_2000)
+            took = free - torch.cuda.mem_get_info()[0]
+            inc, xT = mf(x0, 3e-4, p_ei=0.03, p_ir=0.02)
+            (grad,) = torch.autograd.grad(xT[3].sum(), x0)
+            mf.close()
+            return took, xT.detach().cpu().numpy(), grad.cpu().numpy()
+
+    full, want, want_grad = passes(16 << 30)
+    assert full > 2600 * MB  # states and the windows' row pointers
+    kept = []
+    sizes = [full + 900 * MB, full + 400 * MB, *range(full + 128 * MB, full - 64 * MB, -16 * MB), full - 1400 * MB]
+    for left in sizes:
+        took, xT, grad = passes(left)
+        kept.append(took > full - 1000 * MB)
+        np.testing.assert_array_equal(xT, want)
+        np.testing.assert_array_equal(grad, want_grad)
+    assert kept[0] and not any(kept[1:])
