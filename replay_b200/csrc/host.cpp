@@ -307,6 +307,7 @@ struct rp_sim {
   WindowWorkspace wsp2;
   bool overlap = false;
   bool sparse = false;  // windows list their rows with pairs
+  bool frugal = false;  // the least memory: windows one by one, no room to spare
   cudaStream_t side = nullptr;
   cudaEvent_t ev_built[2] = {nullptr, nullptr}, ev_free = nullptr, ev_join = nullptr;
   bool prebuilt = false;
@@ -729,7 +730,8 @@ namespace {
 
 // Builds every window's canonical CSR once into the arena, group by group.
 // The pairs' places are bounded by the candidates, so that one pass is enough;
-// where that bound is more than kArenaBytes, a first pass finds the numbers.
+// where that bound is more than kArenaBytes (or memory is short), a first pass
+// finds the numbers.
 // (One window at a time, each built twice and waited for in between, took
 // 22.4 ms for 168 windows of 20,011 nodes and 36,000 pairs, 1.6 ms now.)
 constexpr int64_t kArenaBytes = 1ll << 30;
@@ -753,7 +755,7 @@ rp_status prebuild(rp_sim &s) {
     RP_TRY_CUDA(cudaStreamSynchronize(st));
     return RP_OK;
   };
-  if ((int64_t)sizeof(int2) * bound > kArenaBytes) {
+  if (s.frugal || (int64_t)sizeof(int2) * bound > kArenaBytes) {
     for (const WindowGroup &g : s.groups) {
       enqueue_window_build(*s.g, s.wsp, g, s.cap, s.weight_kind, true, st);
       enqueue_window_compact(s.wsp, g, s.arena_rp.as<int32_t>() + s.arena_rp_off[g.first], nullptr,
@@ -887,9 +889,9 @@ rp_status sim_setup(rp_sim &s, const Graph &g, const rp_params &p) {
   const bool prebuilt = p.csr_mode == RP_CSR_PREBUILT;
   bool truncate = false;
   for (const WinDesc &d : s.wins) truncate |= d.may_truncate != 0;
-  s.sparse = !prebuilt && !truncate && s.path == RP_PATH_BATCHED &&
+  s.sparse = !s.frugal && !prebuilt && !truncate && s.path == RP_PATH_BATCHED &&
              s.weight_kind == kWeightI32 && sparse_windows(max_cand, s.N);
-  plan_window_groups(s.wins, s.N, false, s.sparse, s.groups);
+  plan_window_groups(s.wins, s.N, s.frugal, s.sparse, s.groups);
   s.win_group.resize(s.wins.size());
   for (size_t k = 0; k < s.groups.size(); ++k)
     for (int32_t w = 0; w < s.groups[k].count; ++w) s.win_group[s.groups[k].first + w] = (int32_t)k;
@@ -1098,9 +1100,11 @@ bool alloc_sets(rp_sim &s) {
   s.cd_init_ch =
       s.cd.init_code ? cd_changes(s.cd, s.cd.init_code, s.T + 1) : std::vector<CdChange>();
   const int32_t slots = s.cd_inf.empty() ? 1 : s.cd_inf.back().age + 1;
-  if ((int64_t)plane * slots > s.set_bytes || (int)s.cd_inf.size() >= kCdSources) return false;
-  const size_t bits = sizeof(uint32_t) * (size_t)L.bit_words * ((size_t)slots + 3);
   const size_t codes = plane * (8 * (size_t)s.cd.code_bytes);
+  if ((int64_t)plane * slots > s.set_bytes || (int)s.cd_inf.size() >= kCdSources ||
+      (s.frugal && plane * slots > codes))
+    return false;
+  const size_t bits = sizeof(uint32_t) * (size_t)L.bit_words * ((size_t)slots + 3);
   if (s.ring.alloc(plane * slots) == RP_OK && s.ring_bits.alloc(bits) == RP_OK &&
       (!s.p.record_node_states ||
        (s.class_a.alloc(plane) == RP_OK && s.class_b.alloc(plane) == RP_OK)) &&
@@ -1134,8 +1138,8 @@ rp_status capture(rp_sim &s) {
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
   e = cudaGraphInstantiate(&s.exec, graph, 0);
   cudaGraphDestroy(graph);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
-  return RP_OK;
+  if (e != cudaSuccess) st = cuda_fail(e, "cudaGraphInstantiate");
+  return e == cudaErrorMemoryAllocation ? RP_ERR_NOMEM : st;
 }
 
 }  // namespace
@@ -1454,19 +1458,8 @@ RP_API void rp_params_default(rp_params *p) {
   p->has_exposed = 1;
 }
 
-RP_API rp_status rp_sim_create(const rp_graph *h, const rp_params *p, rp_sim **out) {
-  return rp_sim_create_batch(h, p, nullptr, 1, out);
-}
-
-RP_API rp_status rp_sim_create_batch(const rp_graph *h, const rp_params *p,
-                                     const int32_t *net_first, int32_t n_networks,
-                                     rp_sim **out) {
-  return rp_sim_create_bounded(h, p, net_first, n_networks, kRingBytes, out);
-}
-
-RP_API rp_status rp_sim_create_bounded(const rp_graph *h, const rp_params *p,
-                                       const int32_t *net_first, int32_t n_networks,
-                                       int64_t set_bytes, rp_sim **out) {
+static rp_status create_sim(const rp_graph *h, const rp_params *p, const int32_t *net_first,
+                            int32_t n_networks, int64_t set_bytes, bool frugal, rp_sim **out) {
   if (!h || !p || !out) {
     set_error("null argument");
     return RP_ERR_ARG;
@@ -1479,6 +1472,7 @@ RP_API rp_status rp_sim_create_bounded(const rp_graph *h, const rp_params *p,
   *out = nullptr;
   std::unique_ptr<rp_sim> s(new rp_sim());
   s->set_bytes = set_bytes;
+  s->frugal = frugal;
   if (net_first) {
     const int32_t N = h->g.n_nodes;
     if (n_networks < 1 || net_first[0] != 0 || net_first[n_networks] != N) {
@@ -1536,6 +1530,24 @@ RP_API rp_status rp_sim_create_bounded(const rp_graph *h, const rp_params *p,
   s->capture_ms = ms_since(t0);
   *out = s.release();
   return RP_OK;
+}
+
+RP_API rp_status rp_sim_create(const rp_graph *h, const rp_params *p, rp_sim **out) {
+  return rp_sim_create_batch(h, p, nullptr, 1, out);
+}
+
+RP_API rp_status rp_sim_create_batch(const rp_graph *h, const rp_params *p,
+                                     const int32_t *net_first, int32_t n_networks,
+                                     rp_sim **out) {
+  return rp_sim_create_bounded(h, p, net_first, n_networks, kRingBytes, out);
+}
+
+RP_API rp_status rp_sim_create_bounded(const rp_graph *h, const rp_params *p,
+                                       const int32_t *net_first, int32_t n_networks,
+                                       int64_t set_bytes, rp_sim **out) {
+  const rp_status st = create_sim(h, p, net_first, n_networks, set_bytes, false, out);
+  // what is taken for speed alone gives way when the rest does not fit
+  return st == RP_ERR_NOMEM ? create_sim(h, p, net_first, n_networks, set_bytes, true, out) : st;
 }
 
 RP_API void rp_sim_free(rp_sim *s) { delete s; }
@@ -1866,8 +1878,8 @@ RP_API rp_status rp_sim_autotune(rp_sim *s, int32_t probe_steps, rp_tune_result 
 
 // ---- mean-field replay --------------------------------------------------
 
-RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
-                                     int32_t checkpoint_every, rp_meanfield **out) {
+static rp_status create_meanfield(const rp_graph *h, const rp_params *p, int32_t checkpoint_every,
+                                  bool frugal, rp_meanfield **out) {
   if (!h || !p || !out) {
     set_error("null argument");
     return RP_ERR_ARG;
@@ -1892,6 +1904,7 @@ RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
   q.beta_per_replica = nullptr;
   q.susceptibility = nullptr;
   rp_sim &b = m->base;
+  b.frugal = frugal;
   RP_TRY(sim_setup(b, h->g, q));
   b.prebuilt = true;
   RP_TRY(prebuild(b));
@@ -1926,7 +1939,8 @@ RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
   const size_t kept = plane * ((size_t)T + 1) + 2 * per_step * T;
   m->n_ckpt = T > 0 ? (T + m->K - 1) / m->K : 1;
   const size_t segment = plane * m->n_ckpt + (plane * 2 + plane * m->K) + 2 * per_step * m->K;
-  m->keep = (int64_t)kept <= kMfKeepBytes && m->ckpt.alloc(plane * ((size_t)T + 1)) == RP_OK &&
+  m->keep = (int64_t)kept <= kMfKeepBytes && (!frugal || kept <= segment) &&
+            m->ckpt.alloc(plane * ((size_t)T + 1)) == RP_OK &&
             m->seg_q.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
             m->seg_e.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
             (kept <= segment || memory_left(h->g.device));
@@ -1952,6 +1966,12 @@ RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
   m->rates.ir_to_s = p->ir_to_s;
   *out = m.release();
   return RP_OK;
+}
+
+RP_API rp_status rp_meanfield_create(const rp_graph *h, const rp_params *p,
+                                     int32_t checkpoint_every, rp_meanfield **out) {
+  const rp_status st = create_meanfield(h, p, checkpoint_every, false, out);
+  return st == RP_ERR_NOMEM ? create_meanfield(h, p, checkpoint_every, true, out) : st;
 }
 
 RP_API void rp_meanfield_free(rp_meanfield *m) { delete m; }

@@ -119,3 +119,30 @@ def test_kept_states_leave_room_or_give_way():
         np.testing.assert_array_equal(xT, want)
         np.testing.assert_array_equal(grad, want_grad)
     assert kept[0] and not any(kept[1:])
+
+
+# windows in groups of 256 MB that list their rows; a window's contacts, mostly the same pairs over and over, in an
+# arena with room for every contact
+@pytest.mark.parametrize("csr,nodes,pairs,contacts,T", [("per-step", 1_500_000, 1_499_999, 400_000, 20),
+                                                        ("prebuilt", 2_000, 50, 6_000_000, 100)])
+def test_windows_give_room_up(csr, nodes, pairs, contacts, T):
+    """In ever less memory, down to what one window at a time takes, a replay is accepted and gives the same counts."""
+    rb = _rb()
+    rng = np.random.default_rng(5)
+    u = rng.integers(0, pairs, contacts).astype(np.int32)
+    s = synthetic.EPOCH_2000 + rng.integers(0, T * 3600, contacts)
+    g = rb.Graph.from_arrays(s, s + 300, u, u + 1, nodes)
+    kw = dict(M=64, iterations=T, step_size=3600.0, window=3600, start_time=synthetic.EPOCH_2000, ncls_cap=False,
+              transition="geometric", beta=1e-4, p_ei=0.1, p_ir=0.1, initial_count=nodes // 20, seed=1, csr=csr)
+    sim = rb.Simulation(g, **kw)
+    want, full = sim.run(), sim.info["device_bytes"]
+    sim.close()
+    least = 200 * MB if csr == "per-step" else full - 48 * MB
+    held = []
+    for left in np.linspace(full + 192 * MB, least, 24):
+        with memory_left(rb, left):
+            sim = rb.Simulation(g, **kw)
+            held.append(sim.info["device_bytes"])
+            np.testing.assert_array_equal(sim.run(), want)
+            sim.close()
+    assert held[0] == full and held[-1] < full - 48 * MB
