@@ -244,12 +244,12 @@ rp_status graph_build_device(Graph &g, const int64_t *start, const int64_t *end,
 rp_status plan_windows(const Graph &g, const std::vector<int64_t> &ws, int64_t length,
                        const std::vector<float> &scale, int64_t cap,
                        std::vector<CandRange> &ranges, std::vector<WinDesc> &wins);
-// One window with caller-owned scratch (kPlanBytes on the device); ranges
-// holds kClasses entries.  Synchronizes st.
-constexpr size_t kPlanBytes = sizeof(int64_t) * 2 * kClasses;
-rp_status plan_window_noalloc(const Graph &g, int64_t ws, int64_t we, float scale, int64_t cap,
-                              int64_t *scratch, CandRange *ranges, WinDesc &out,
-                              cudaStream_t st);
+// One window, planned in the stream: its descriptor, its ranges (kClasses
+// entries) and the number of its candidates stay on the device; with more than
+// `limit` of them the descriptor is of an empty window.
+void enqueue_plan_window(const Graph &g, int64_t ws, int64_t we, float scale, int64_t cap,
+                         int64_t limit, WinDesc *win, CandRange *ranges, int64_t *total,
+                         cudaStream_t st);
 
 // ---- window builder ----------------------------------------------------------
 struct Hit {
