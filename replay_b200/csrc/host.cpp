@@ -342,6 +342,7 @@ struct rp_sim {
   // node-state text mode (rp_sim_run_text)
   rp_text_cb text_cb = nullptr;
   void *text_user = nullptr;
+  bool text_ready = false;  // every buffer below is there (a call may have failed half way)
   int32_t text_rows = 0;  // replica rows per text chunk
   DevBuf text_dev[2], text_seglen, text_segoff;
   char *text_host[2] = {nullptr, nullptr};
@@ -1611,20 +1612,22 @@ RP_API rp_status rp_sim_run_text(rp_sim *s, int32_t *counts, rp_text_cb cb, void
     return RP_ERR_ARG;
   }
   RP_TRY_CUDA(cudaSetDevice(s->g->device));
-  if (!s->text_host[0]) {  // chunk buffers: about 64 MB of text per chunk
+  if (!s->text_ready) {  // chunk buffers: about 64 MB of text per chunk
     const int64_t line = text_line_bound(s->N);
     const int64_t per_row = line * (int64_t)s->N;
     s->text_rows = (int32_t)std::max<int64_t>(1, std::min<int64_t>(s->M, (64ll << 20) / per_row));
     const size_t bytes = (size_t)(per_row * s->text_rows);
     for (int b = 0; b < 2; ++b) {
       RP_TRY(s->text_dev[b].alloc(bytes));
-      RP_TRY_CUDA(cudaMallocHost(&s->text_host[b], bytes));
-      RP_TRY_CUDA(cudaEventCreateWithFlags(&s->text_ev[b], cudaEventDisableTiming));
+      if (!s->text_host[b]) RP_TRY_CUDA(cudaMallocHost(&s->text_host[b], bytes));
+      if (!s->text_ev[b])
+        RP_TRY_CUDA(cudaEventCreateWithFlags(&s->text_ev[b], cudaEventDisableTiming));
     }
-    RP_TRY_CUDA(cudaMallocHost(&s->text_len_host, 2 * sizeof(int64_t)));
+    if (!s->text_len_host) RP_TRY_CUDA(cudaMallocHost(&s->text_len_host, 2 * sizeof(int64_t)));
     const size_t segs = (size_t)(s->text_rows * text_segments(s->N));
     RP_TRY(s->text_seglen.alloc(sizeof(int64_t) * segs));
     RP_TRY(s->text_segoff.alloc(sizeof(int64_t) * (segs + 1)));
+    s->text_ready = true;
   }
   s->text_cb = cb;
   s->text_user = user;

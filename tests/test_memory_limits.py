@@ -146,3 +146,27 @@ def test_windows_give_room_up(csr, nodes, pairs, contacts, T):
             np.testing.assert_array_equal(sim.run(), want)
             sim.close()
     assert held[0] == full and held[-1] < full - 48 * MB
+
+
+def test_text_after_a_call_without_memory():
+    """run_text allocates its buffers at the first call; one that got only a part of them is refused, and so is the
+    next, until there is memory."""
+    rb = _rb()
+    n, M = 20_000, 64
+    s = np.array([synthetic.EPOCH_2000])
+    g = rb.Graph.from_arrays(s, s + 900, [0], [1], n)
+    kw = dict(M=M, iterations=2, step_size=1800.0, window=1800, start_time=synthetic.EPOCH_2000, transition="geometric",
+              beta=1e-3, p_ir=0.1, initial_infected=0.1, record_node_states=True)
+    def text(sim):
+        lines = []
+        sim.run_text(lambda k, ts, data: lines.append((k, data)) and None)
+        return lines
+    want = text(rb.Simulation(g, **kw))
+    assert sum(len(d) for _, d in want) > 3 * n * M * 20
+    sim = rb.Simulation(g, **kw)
+    with memory_left(rb, 100 * MB):  # twice 64 MB of text
+        for _ in range(2):
+            with pytest.raises(rb.ReplayError) as e:
+                text(sim)
+            assert e.value.status == 4
+    assert text(sim) == want
