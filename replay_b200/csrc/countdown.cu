@@ -58,9 +58,9 @@ __device__ __forceinline__ uint32_t tab_next(uint32_t e) { return e & 0xFFFFu; }
 __device__ __forceinline__ uint32_t tab_cls(uint32_t e) { return (e >> 16) & 3u; }
 __device__ __forceinline__ uint32_t tab_inf(uint32_t e) { return (e >> 18) & 1u; }
 
-// Signed per-replica class deltas in a 64-bit word: E, I, R in 16-bit
-// fields (shared-memory counters of one task) or 21-bit fields (the step's
-// event row), added modulo 2^64.
+// Per-replica class deltas in a 64-bit word: E, I, R in 16-bit fields
+// (shared-memory counters of one task, at most 4,096 rows; signed) or 21-bit
+// fields (the step's event row), added modulo 2^64.
 __device__ __forceinline__ unsigned long long cls_enc(uint32_t cls, int bits) {
   return cls == 0 ? 0ull : (1ull << (bits * (int)(cls - 1)));
 }
@@ -546,7 +546,10 @@ __global__ void __launch_bounds__(kCdThreads, 3)
 }
 
 // counts[t][net][r][4] (E, I, R, S) from the initial counts and the per-step
-// signed class deltas.
+// class deltas.  Both are sums modulo 2^64 with E, I and R in fields of 21 bits,
+// and every count fits its field, so that their sum is the next step's counts;
+// one step's delta alone may be too large for a signed field (a network of more
+// than 2^20 nodes whose nodes change class together).
 __global__ void k_cd_finalize(const unsigned long long *__restrict__ init,
                               const unsigned long long *__restrict__ ev, int32_t steps,
                               int32_t per_row, const int32_t *__restrict__ net_size, int32_t m,
@@ -555,24 +558,17 @@ __global__ void k_cd_finalize(const unsigned long long *__restrict__ init,
   if (j >= per_row) return;
   const unsigned long long fm = (1ull << 21) - 1;
   const int64_t N = net_size[j / m];
-  const unsigned long long p = init[j];
-  int64_t E = (int64_t)(p & fm), I = (int64_t)((p >> 21) & fm), R = (int64_t)((p >> 42) & fm);
-  int32_t *o = counts + (int64_t)j * 4;
-  o[0] = (int32_t)E;
-  o[1] = (int32_t)I;
-  o[2] = (int32_t)R;
-  o[3] = (int32_t)(N - E - I - R);
-  for (int32_t t = 0; t < steps; ++t) {
-    int64_t d[3];
-    dec3(ev[(int64_t)t * per_row + j], 21, d);
-    E += d[0];
-    I += d[1];
-    R += d[2];
-    o = counts + ((int64_t)(t + 1) * per_row + j) * 4;
+  unsigned long long p = init[j];
+  for (int32_t t = 0;; ++t) {
+    const int64_t E = (int64_t)(p & fm), I = (int64_t)((p >> 21) & fm),
+                  R = (int64_t)((p >> 42) & fm);
+    int32_t *o = counts + ((int64_t)t * per_row + j) * 4;
     o[0] = (int32_t)E;
     o[1] = (int32_t)I;
     o[2] = (int32_t)R;
     o[3] = (int32_t)(N - E - I - R);
+    if (t == steps) break;
+    p += ev[(int64_t)t * per_row + j];
   }
 }
 
