@@ -331,6 +331,7 @@ struct rp_sim {
   DevBuf codes, cd_tab;
   CdTable cd;
   PackedLayout L{};
+  size_t codes_bytes() const { return (size_t)cd.code_bytes * 32 * (size_t)N * L.words; }
   DevBuf net_size, net_first, net_rows;
   int32_t n_nets = 1;
   std::vector<int32_t> net_bounds;  // n_nets + 1 node offsets (empty: one network)
@@ -530,6 +531,10 @@ struct rp_sim {
   // out and handed to the callback (not capturable).
   rp_status enqueue(cudaStream_t st, rp_state_cb cb, void *user, int *n_kernels,
                     Marks *mk = nullptr) {
+    if (cd.code_bytes && !ring_slots && !cd_tab.ptr) {
+      set_error("no memory for the countdown state");
+      return RP_ERR_NOMEM;
+    }
     int k = 0;
     auto mark = [&](int kind) {
       if (mk) mk->mark(kind);
@@ -1076,11 +1081,13 @@ rp_status alloc_state(rp_sim &s) {
   return RP_OK;
 }
 
-// What a handle leaves free when it takes memory for speed alone (the countdown
+// What a handle leaves free when it takes `bytes` for speed alone (the countdown
 // rule's sets, the mean-field's kept states): its graph and its text buffers
-// (twice 64 MB) come later.
+// (twice 64 MB) come later.  Not asked for up to 256 MB: the question itself takes
+// 0.7 to 3 ms, which would be half of creating a small handle.
 constexpr size_t kLeaveBytes = size_t(512) << 20;
-bool memory_left(int device) {
+bool memory_left(int device, size_t bytes) {
+  if (bytes <= kLeaveBytes / 2) return true;
   size_t free_b = 0, total = 0;
   if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) return false;
   if (free_b < kLeaveBytes) {
@@ -1101,7 +1108,7 @@ bool alloc_sets(rp_sim &s) {
   s.cd_init_ch =
       s.cd.init_code ? cd_changes(s.cd, s.cd.init_code, s.T + 1) : std::vector<CdChange>();
   const int32_t slots = s.cd_inf.empty() ? 1 : s.cd_inf.back().age + 1;
-  const size_t codes = plane * (8 * (size_t)s.cd.code_bytes);
+  const size_t codes = s.codes_bytes();
   if ((int64_t)plane * slots > s.set_bytes || (int)s.cd_inf.size() >= kCdSources ||
       (s.frugal && plane * slots > codes))
     return false;
@@ -1109,7 +1116,7 @@ bool alloc_sets(rp_sim &s) {
   if (s.ring.alloc(plane * slots) == RP_OK && s.ring_bits.alloc(bits) == RP_OK &&
       (!s.p.record_node_states ||
        (s.class_a.alloc(plane) == RP_OK && s.class_b.alloc(plane) == RP_OK)) &&
-      (plane * slots <= codes || memory_left(s.g->device))) {
+      (plane * slots <= codes || memory_left(s.g->device, plane * slots))) {
     s.ring_slots = slots;
     return true;
   }
@@ -1120,10 +1127,40 @@ bool alloc_sets(rp_sim &s) {
 rp_status alloc_codes(rp_sim &s) {
   const PackedLayout &L = s.L;
   RP_TRY(s.mask2.alloc(sizeof(uint32_t) * (size_t)s.N * L.words));
-  RP_TRY(s.codes.alloc((size_t)s.cd.code_bytes * 32 * (size_t)s.N * L.words));  // 8 planes a byte
+  RP_TRY(s.codes.alloc(s.codes_bytes()));
   RP_TRY(s.cd_tab.alloc(sizeof(uint32_t) * s.cd.tab.size()));
   RP_TRY_CUDA(cudaMemcpy(s.cd_tab.ptr, s.cd.tab.data(), sizeof(uint32_t) * s.cd.tab.size(),
                          cudaMemcpyHostToDevice));
+  return RP_OK;
+}
+
+// Codes in place of sets that take more (of a simulation without a captured
+// graph); a run finds neither where even they do not fit.
+rp_status sets_to_codes(rp_sim &s) {
+  if (!s.ring_slots || s.ring.bytes <= s.codes_bytes()) return RP_ERR_NOMEM;
+  s.ring_slots = 0;
+  for (DevBuf *b : {&s.ring, &s.ring_bits, &s.class_a, &s.class_b}) b->release();
+  return alloc_codes(s);
+}
+
+// Text buffers, at the first text run: about 64 MB of text per chunk.
+rp_status alloc_text(rp_sim &s) {
+  if (s.text_ready) return RP_OK;
+  const int64_t line = text_line_bound(s.N);
+  const int64_t per_row = line * (int64_t)s.N;
+  s.text_rows = (int32_t)std::max<int64_t>(1, std::min<int64_t>(s.M, (64ll << 20) / per_row));
+  const size_t bytes = (size_t)(per_row * s.text_rows);
+  for (int b = 0; b < 2; ++b) {
+    RP_TRY(s.text_dev[b].alloc(bytes));
+    if (!s.text_host[b]) RP_TRY_CUDA(cudaMallocHost(&s.text_host[b], bytes));
+    if (!s.text_ev[b])
+      RP_TRY_CUDA(cudaEventCreateWithFlags(&s.text_ev[b], cudaEventDisableTiming));
+  }
+  if (!s.text_len_host) RP_TRY_CUDA(cudaMallocHost(&s.text_len_host, 2 * sizeof(int64_t)));
+  const size_t segs = (size_t)(s.text_rows * text_segments(s.N));
+  RP_TRY(s.text_seglen.alloc(sizeof(int64_t) * segs));
+  RP_TRY(s.text_segoff.alloc(sizeof(int64_t) * (segs + 1)));
+  s.text_ready = true;
   return RP_OK;
 }
 
@@ -1612,26 +1649,12 @@ RP_API rp_status rp_sim_run_text(rp_sim *s, int32_t *counts, rp_text_cb cb, void
     return RP_ERR_ARG;
   }
   RP_TRY_CUDA(cudaSetDevice(s->g->device));
-  if (!s->text_ready) {  // chunk buffers: about 64 MB of text per chunk
-    const int64_t line = text_line_bound(s->N);
-    const int64_t per_row = line * (int64_t)s->N;
-    s->text_rows = (int32_t)std::max<int64_t>(1, std::min<int64_t>(s->M, (64ll << 20) / per_row));
-    const size_t bytes = (size_t)(per_row * s->text_rows);
-    for (int b = 0; b < 2; ++b) {
-      RP_TRY(s->text_dev[b].alloc(bytes));
-      if (!s->text_host[b]) RP_TRY_CUDA(cudaMallocHost(&s->text_host[b], bytes));
-      if (!s->text_ev[b])
-        RP_TRY_CUDA(cudaEventCreateWithFlags(&s->text_ev[b], cudaEventDisableTiming));
-    }
-    if (!s->text_len_host) RP_TRY_CUDA(cudaMallocHost(&s->text_len_host, 2 * sizeof(int64_t)));
-    const size_t segs = (size_t)(s->text_rows * text_segments(s->N));
-    RP_TRY(s->text_seglen.alloc(sizeof(int64_t) * segs));
-    RP_TRY(s->text_segoff.alloc(sizeof(int64_t) * (segs + 1)));
-    s->text_ready = true;
-  }
+  rp_status st = alloc_text(*s);
+  if (st == RP_ERR_NOMEM && sets_to_codes(*s) == RP_OK) st = alloc_text(*s);
+  RP_TRY(st);
   s->text_cb = cb;
   s->text_user = user;
-  rp_status st = s->run_eager(nullptr, nullptr);
+  st = s->run_eager(nullptr, nullptr);
   s->text_cb = nullptr;
   s->text_user = nullptr;
   RP_TRY(st);
@@ -1951,7 +1974,7 @@ static rp_status create_meanfield(const rp_graph *h, const rp_params *p, int32_t
             m->ckpt.alloc(plane * ((size_t)T + 1)) == RP_OK &&
             m->seg_q.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
             m->seg_e.alloc(per_step * (T > 0 ? T : 1)) == RP_OK &&
-            (kept <= segment || memory_left(h->g.device));
+            (kept <= segment || memory_left(h->g.device, kept));
   if (!m->keep) {  // or checkpoints
     for (DevBuf *buf : {&m->ckpt, &m->seg_q, &m->seg_e}) buf->release();
     RP_TRY(m->ckpt.alloc(plane * m->n_ckpt));

@@ -148,6 +148,42 @@ def test_windows_give_room_up(csr, nodes, pairs, contacts, T):
     assert held[0] == full and held[-1] < full - 48 * MB
 
 
+def text(sim):
+    lines = []
+    sim.run_text(lambda k, ts, data: lines.append((k, data)) and None)
+    return lines
+
+
+def test_text_takes_the_place_of_small_sets():
+    """Sets up to 256 MB are taken without a look at what stays free: the first text run turns them into codes."""
+    rb = _rb()
+    n = 20_000
+    s = np.array([synthetic.EPOCH_2000])
+    g = rb.Graph.from_arrays(s, s + 900, [0], [1], n)
+    kw = dict(M=512, iterations=150, step_size=600.0, window=600, start_time=synthetic.EPOCH_2000, path="batched",
+              initial_infected=0.1, infect_prob=0.1, exposed_duration=30_000, infectious_duration=50_000,
+              resistant_duration=0, record_node_states=True)
+
+    def first_lines(sim):
+        lines = []
+
+        def write(k, ts, data):
+            lines.append(data)
+            return k == 2
+        with pytest.raises(rb.ReplayError, match="aborted"):
+            sim.run_text(write)
+        return lines
+    sim = rb.Simulation(g, **kw)
+    want, full = first_lines(sim), sim.info["device_bytes"]
+    sim.close()
+    sets = 132 * n * 64
+    with memory_left(rb, full - sets + 110 * MB):  # the sets, and no room for the text's 128 MB
+        sim = rb.Simulation(g, **kw)
+        assert first_lines(sim) == want
+        assert sim.info["device_bytes"] < full - sets // 2
+        sim.close()
+
+
 def test_text_after_a_call_without_memory():
     """run_text allocates its buffers at the first call; one that got only a part of them is refused, and so is the
     next, until there is memory."""
@@ -157,10 +193,6 @@ def test_text_after_a_call_without_memory():
     g = rb.Graph.from_arrays(s, s + 900, [0], [1], n)
     kw = dict(M=M, iterations=2, step_size=1800.0, window=1800, start_time=synthetic.EPOCH_2000, transition="geometric",
               beta=1e-3, p_ir=0.1, initial_infected=0.1, record_node_states=True)
-    def text(sim):
-        lines = []
-        sim.run_text(lambda k, ts, data: lines.append((k, data)) and None)
-        return lines
     want = text(rb.Simulation(g, **kw))
     assert sum(len(d) for _, d in want) > 3 * n * M * 20
     sim = rb.Simulation(g, **kw)
