@@ -160,6 +160,7 @@ constexpr int kInfectWarpBytes =
     (int)((sizeof(InfectWarp) > sizeof(HeavyWarp) ? sizeof(InfectWarp) : sizeof(HeavyWarp)) + 15) /
     16 * 16;
 constexpr int kInfectDynSmem = kWarps * kInfectWarpBytes;
+static_assert(kHeavyPairs < 1 << 24, "a listed geometric row's pairs beside its row");
 static_assert(3 * (kInfectDynSmem + 1024 + 64) <= 228 * 1024, "three blocks per SM");
 
 // Top 8 uniform bits of replica bit b from a queued word's planes.
@@ -700,8 +701,8 @@ __global__ void __launch_bounds__(kThreads, 3)
               const bool has = len[j] > 0 && (kCountdown || len[j] <= kHeavyPairs);
               const unsigned hm = __ballot_sync(kFull, has);
               if (has) {
-                Q.u.put(nrows + __popc(hm & ((1u << lane) - 1u)), r - r0 + 32 * j + lane, b[j],
-                        len[j]);
+                Q.u.template put<kCountdown>(nrows + __popc(hm & ((1u << lane) - 1u)),
+                                             r - r0 + 32 * j + lane, b[j], len[j]);
               }
               nrows += __popc(hm);
             }
@@ -717,9 +718,8 @@ __global__ void __launch_bounds__(kThreads, 3)
       if (more) {
         n = 0;
         if (ub + lane < nrows) {
-          lrow = r0 + Q.u.row[ub + lane];
-          beg = Q.u.beg[ub + lane];
-          n = Q.u.len[ub + lane];
+          Q.u.template get<kCountdown>(ub + lane, lrow, beg, n);
+          lrow += r0;
           if (d.list.rows) lrow = __ldg(d.list.rows + lrow);
         }
         ub += 32;

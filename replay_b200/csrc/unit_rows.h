@@ -1,7 +1,9 @@
 // The rows of a unit that have pairs, as a warp of k_infect lists them
-// (packed.cu).  A row's pairs have a word of their own: under the countdown rule
-// rows of any length are listed, and a window may hold 2^30 contacts of one
-// pair of nodes (repeated records are not merged in unsorted windows).
+// (packed.cu).  kAnyLength: under the countdown rule rows of any length are
+// listed, and a window may hold 2^30 contacts of one pair of nodes, so that a
+// row's number of pairs has a word of its own.  Geometric rows listed here have
+// at most 48 pairs, which share a word with the row (the separate arrays cost
+// N = 1,000 with 1,000 replicas 2%; the countdown rule gained 5% from them).
 // Header-only so that a host-side test can compile it without the CUDA runtime.
 #pragma once
 #include <cstdint>
@@ -17,15 +19,22 @@ namespace rp {
 constexpr int kUnitRows = 128;  // most rows of a unit
 
 struct UnitRows {
-  int32_t beg[kUnitRows];  // their first pairs
-  int32_t len[kUnitRows];  // their pairs
-  uint8_t row[kUnitRows];  // row (or list entry) in the unit
-  static_assert(kUnitRows <= 256, "a row of the unit in a byte");
+  int32_t beg[kUnitRows];  // first pairs
+  int32_t len[kUnitRows];  // numbers of pairs; or row | pairs << 7
+  uint8_t row[kUnitRows];  // rows (or list entries) in the unit
+  static_assert(kUnitRows <= 128, "a row of the unit in 7 bits");
 
+  template <bool kAnyLength>
   RP_HD void put(int pos, int r, int32_t first, int32_t pairs) {
     beg[pos] = first;
-    len[pos] = pairs;
-    row[pos] = (uint8_t)r;
+    len[pos] = kAnyLength ? pairs : r | pairs << 7;
+    if (kAnyLength) row[pos] = (uint8_t)r;
+  }
+  template <bool kAnyLength>
+  RP_HD void get(int pos, int &r, int32_t &first, int32_t &pairs) const {
+    first = beg[pos];
+    r = kAnyLength ? row[pos] : len[pos] & 127;
+    pairs = kAnyLength ? len[pos] : len[pos] >> 7;
   }
 };
 
