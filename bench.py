@@ -408,7 +408,7 @@ def reference_sample_leg(replay_b200, dev, timed, args):
     out = {"workload": f"reference arm's sample: {sample['n_nodes']} nodes, {len(sample['start'])} contacts, "
                        f"{m} replicas, {p['iterations']} steps, countdown",
            "ms_per_replay": ms, "value": sample["n_nodes"] * m * p["iterations"] / (ms / 1e3), "unit": UNIT,
-           "path": "batched countdown (replica codes)"}
+           "path": "batched countdown (sets of replicas)"}
     sim.close()
     g.close()
     return out

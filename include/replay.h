@@ -306,8 +306,9 @@ RP_API rp_status rp_sim_profile_steps(rp_sim *s, float *step_ms);
  * (192, 384 or the default) are chosen by timing the replay's first
  * `probe_steps` steps with CUDA events, keeping a candidate only when it is
  * 2% faster.  The step kernels split their work by themselves: the height
- * tiles the initial counts and the countdown code table (rings of more than
- * 16 GB), the staging depth has no effect and is kept for its callers.  The
+ * tiles the initial counts and the countdown code table only, and the staging
+ * depth has no effect and is kept for its callers, so that a choice is within
+ * the noise of its timing unless the replay runs by the code table.  The
  * simulation keeps the tuned tiles (and re-captures its CUDA graph); results
  * are unchanged by tiling.  Not for simulations created with
  * record_node_states. */

@@ -34,7 +34,8 @@ def version():
 def release_cached_memory():
     """Returns the device blocks kept from closed graphs and simulations
     (closing a handle keeps its blocks, up to 8 GiB per device, for the
-    next one) to the driver."""
+    next one) and the pinned buffers of large copies (at most 64 MB) to the
+    driver."""
     lib().rp_release_cached_memory()
 
 

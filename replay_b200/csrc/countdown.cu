@@ -1,6 +1,7 @@
 // Batched path, countdown mode: the reference's own transition rules as codes
-// into a table, for replays too large for the sets of replicas further down
-// (those are the usual form: k_cd_flow here, k_infect<true> in packed.cu).
+// into a table, for replays whose sets of replicas, further down, would take more
+// than 16 GB or than the device has left (those are the usual form: k_cd_flow
+// here, k_infect<true> in packed.cu).
 //
 // The reference's own transition rules
 // (initialize_countdown_vector, generate_infectious_vector,

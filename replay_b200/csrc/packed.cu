@@ -35,7 +35,7 @@
 // k_flow (transitions + count reduction), every item set in act or evb:
 //   reads the planes and the item's infection events, draws the bit-sliced
 //   flow uniforms of the E, I (and waning R) replicas, 32 replicas per random
-//   plane (flow_events), applies all moves with bitwise operations, writes the
+//   plane (flow_top, flow_rest), applies all moves with bitwise operations, writes the
 //   planes and mask_{t+1}, and adds every transition event to the step's event
 //   row; k_finalize turns initial counts + events into per-step counts.
 // Every decision uses the state at the start of the step: k_infect reads the
