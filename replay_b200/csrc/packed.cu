@@ -132,9 +132,10 @@ constexpr int kListTurns = 2;
 
 // Per warp: the unit's rows and items, and a queue of exposed words that
 // accumulates over units and is decided 32 words at a time.
+template <bool kCountdown>
 struct InfectWarp {
   uint4 pl[32][2];             // the 8 random planes of each word (round scratch)
-  UnitRows u;                  // the unit's rows with pairs
+  UnitRows<kCountdown> u;      // the unit's rows with pairs
   int32_t list[128];           // items of a batch of 32 rows: row in batch << 5 | column
   uint32_t rmask[32];          // column masks of the batch's rows
   uint4 q[kInfectQueue];       // row, word in the row, exposed replicas, ef(e_max) of the row
@@ -156,12 +157,14 @@ struct HeavyWarp {
   uint32_t C[32];
   int32_t off[32];
 };
+template <bool kCountdown>
 constexpr int kInfectWarpBytes =
-    (int)((sizeof(InfectWarp) > sizeof(HeavyWarp) ? sizeof(InfectWarp) : sizeof(HeavyWarp)) + 15) /
-    16 * 16;
-constexpr int kInfectDynSmem = kWarps * kInfectWarpBytes;
+    (int)((sizeof(InfectWarp<kCountdown>) > sizeof(HeavyWarp) ? sizeof(InfectWarp<kCountdown>)
+                                                              : sizeof(HeavyWarp)) + 15) / 16 * 16;
+template <bool kCountdown>
+constexpr int kInfectDynSmem = kWarps * kInfectWarpBytes<kCountdown>;
 static_assert(kHeavyPairs < 1 << 24, "a listed geometric row's pairs beside its row");
-static_assert(3 * (kInfectDynSmem + 1024 + 64) <= 228 * 1024, "three blocks per SM");
+static_assert(3 * (kInfectDynSmem<true> + 1024 + 64) <= 228 * 1024, "three blocks per SM");
 
 // Top 8 uniform bits of replica bit b from a queued word's planes.
 __device__ __forceinline__ uint32_t queued_top8(const uint4 (&q)[2], uint32_t b) {
@@ -246,7 +249,7 @@ __device__ __forceinline__ void countdown_decide(const InfectArgs &d, const Step
 // Candidates of the round's words into Q.cl; returns their number.  One lane
 // takes one quad of replicas with an exposed member (a draw covers a quad), so
 // that sparse words share the draws; the events of sure words are set here.
-__device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int at0, int n, int lane,
+__device__ __forceinline__ int countdown_candidates(InfectWarp<true> &Q, int at0, int n, int lane,
                                                     const InfectArgs &d, const StepConsts &c,
                                                     const PackedLayout &L) {
   uint16_t *quads = reinterpret_cast<uint16_t *>(Q.pl[0]);  // lane << 3 | quad, at most 256
@@ -309,7 +312,7 @@ __device__ __forceinline__ int countdown_candidates(InfectWarp &Q, int at0, int 
 // rounds; fewer than 32 left over are carried to the next round unless
 // `drain` is set.  Events are OR-ed into their words and flag their items.
 template <bool kCountdown>
-__device__ __forceinline__ void infect_round(InfectWarp &Q, int at0, int n, bool drain, int lane,
+__device__ __forceinline__ void infect_round(InfectWarp<kCountdown> &Q, int at0, int n, bool drain, int lane,
                                              const PackedLayout &L, const InfectArgs &d,
                                              const StepConsts &c) {
   // ---- bound test, one word per lane ----
@@ -600,7 +603,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   }
   if (!kCountdown && (n_heavy | n_huge)) {
     const int nws = (L.words + 31) / 32;
-    HeavyWarp &H = *reinterpret_cast<HeavyWarp *>(s_dyn + warp * kInfectWarpBytes);
+    HeavyWarp &H = *reinterpret_cast<HeavyWarp *>(s_dyn + warp * kInfectWarpBytes<kCountdown>);
     HeavyUnit h;
     // Rows of more than kHugePairs pairs first: the block's warps share the
     // pairs, warp 0 adds their planes, and the decisions are shared again.
@@ -621,7 +624,7 @@ __global__ void __launch_bounds__(kThreads, 3)
         H.C[lane] = X;
         __syncthreads();
         for (int v = 1; v < kWarps && warp == 0; ++v) {
-          const HeavyWarp &Hv = *reinterpret_cast<const HeavyWarp *>(s_dyn + v * kInfectWarpBytes);
+          const HeavyWarp &Hv = *reinterpret_cast<const HeavyWarp *>(s_dyn + v * kInfectWarpBytes<kCountdown>);
           X |= Hv.C[lane];
           uint32_t cy = 0;
           for (int k = 0; k < min(h.nb, 32); ++k) {
@@ -638,7 +641,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
   }
 
-  InfectWarp &Q = *reinterpret_cast<InfectWarp *>(s_dyn + warp * kInfectWarpBytes);
+  InfectWarp<kCountdown> &Q = *reinterpret_cast<InfectWarp<kCountdown> *>(s_dyn + warp * kInfectWarpBytes<kCountdown>);
   if (lane == 0) Q.nk = 0;
   __syncwarp();
   int nq = 0;  // queued words
@@ -701,8 +704,8 @@ __global__ void __launch_bounds__(kThreads, 3)
               const bool has = len[j] > 0 && (kCountdown || len[j] <= kHeavyPairs);
               const unsigned hm = __ballot_sync(kFull, has);
               if (has) {
-                Q.u.template put<kCountdown>(nrows + __popc(hm & ((1u << lane) - 1u)),
-                                             r - r0 + 32 * j + lane, b[j], len[j]);
+                Q.u.put(nrows + __popc(hm & ((1u << lane) - 1u)), r - r0 + 32 * j + lane, b[j],
+                        len[j]);
               }
               nrows += __popc(hm);
             }
@@ -718,7 +721,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       if (more) {
         n = 0;
         if (ub + lane < nrows) {
-          Q.u.template get<kCountdown>(ub + lane, lrow, beg, n);
+          Q.u.get(ub + lane, lrow, beg, n);
           lrow += r0;
           if (d.list.rows) lrow = __ldg(d.list.rows + lrow);
         }
@@ -1377,10 +1380,10 @@ int task_grid(int n_tasks, int per_sm) {
 
 rp_status packed_prepare() {
   cudaError_t e = cudaFuncSetAttribute(
-      k_infect<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfectDynSmem);
+      k_infect<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInfectDynSmem<false>);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_infect<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kInfectDynSmem);
+                             kInfectDynSmem<true>);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_infect)");
   e = cudaFuncSetAttribute(k_flow, cudaFuncAttributeMaxDynamicSharedMemorySize, kFlowDynSmem);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(k_flow)");
@@ -1455,7 +1458,7 @@ void packed_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *en
   d.step = step;
   d.scale = scale;
   set_infect_units(L, list.rows ? list.bound : L.n_nodes, d);
-  k_infect<false><<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
+  k_infect<false><<<unit_grid(d.n_units), kThreads, kInfectDynSmem<false>, st>>>(L, d, c);
 }
 
 void cd_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entries,
@@ -1473,7 +1476,7 @@ void cd_infect(const PackedLayout &L, const int32_t *row_ptr, const int2 *entrie
   d.evb = evb;
   d.step = step;
   set_infect_units(L, L.n_nodes, d);
-  k_infect<true><<<unit_grid(d.n_units), kThreads, kInfectDynSmem, st>>>(L, d, c);
+  k_infect<true><<<unit_grid(d.n_units), kThreads, kInfectDynSmem<true>, st>>>(L, d, c);
 }
 
 void packed_flow(const PackedLayout &L, uint32_t *mask, uint32_t *sa, uint32_t *sb, uint32_t *evs,

@@ -18,23 +18,38 @@ namespace rp {
 
 constexpr int kUnitRows = 128;  // most rows of a unit
 
+template <bool kAnyLength>
 struct UnitRows {
-  int32_t beg[kUnitRows];  // first pairs
-  int32_t len[kUnitRows];  // numbers of pairs; or row | pairs << 7
-  uint8_t row[kUnitRows];  // rows (or list entries) in the unit
+  int32_t word[kUnitRows];  // row (or list entry) in the unit | pairs << 7
+  int32_t beg[kUnitRows];   // first pairs
   static_assert(kUnitRows <= 128, "a row of the unit in 7 bits");
 
-  template <bool kAnyLength>
   RP_HD void put(int pos, int r, int32_t first, int32_t pairs) {
+    word[pos] = r | pairs << 7;
     beg[pos] = first;
-    len[pos] = kAnyLength ? pairs : r | pairs << 7;
-    if (kAnyLength) row[pos] = (uint8_t)r;
   }
-  template <bool kAnyLength>
   RP_HD void get(int pos, int &r, int32_t &first, int32_t &pairs) const {
+    r = word[pos] & 127;
+    pairs = word[pos] >> 7;
     first = beg[pos];
-    r = kAnyLength ? row[pos] : len[pos] & 127;
-    pairs = kAnyLength ? len[pos] : len[pos] >> 7;
+  }
+};
+
+template <>
+struct UnitRows<true> {
+  int32_t len[kUnitRows];  // numbers of pairs
+  int32_t beg[kUnitRows];
+  uint8_t row[kUnitRows];
+
+  RP_HD void put(int pos, int r, int32_t first, int32_t pairs) {
+    len[pos] = pairs;
+    beg[pos] = first;
+    row[pos] = (uint8_t)r;
+  }
+  RP_HD void get(int pos, int &r, int32_t &first, int32_t &pairs) const {
+    r = row[pos];
+    pairs = len[pos];
+    first = beg[pos];
   }
 };
 

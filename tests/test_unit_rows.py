@@ -14,25 +14,26 @@ HARNESS = r'''
 #include <cstdio>
 #include "unit_rows.h"
 int main() {
-  static rp::UnitRows u;
+  static rp::UnitRows<true> u;
+  static rp::UnitRows<false> g;
   const int32_t lens[] = {1, 2, 48, (1 << 24) - 1, 1 << 24, (1 << 24) + 1, (1 << 25) + 100, 1 << 30, INT32_MAX};
   const int k = sizeof(lens) / sizeof(lens[0]);
-  for (int p = 0; p < rp::kUnitRows; ++p) u.put<true>(p, rp::kUnitRows - 1 - p, INT32_MAX - p, lens[p % k]);
+  for (int p = 0; p < rp::kUnitRows; ++p) u.put(p, rp::kUnitRows - 1 - p, INT32_MAX - p, lens[p % k]);
   for (int p = 0; p < rp::kUnitRows; ++p) {
     int r;
     int32_t first, pairs;
-    u.get<true>(p, r, first, pairs);
+    u.get(p, r, first, pairs);
     if (r != rp::kUnitRows - 1 - p || first != INT32_MAX - p || pairs != lens[p % k]) {
       printf("row %d: %d %d %d\n", p, r, first, pairs);
       return 1;
     }
   }
   // geometric rows: the longer ones go another way (kHeavyPairs)
-  for (int p = 0; p < rp::kUnitRows; ++p) u.put<false>(p, rp::kUnitRows - 1 - p, INT32_MAX - p, 1 + p % 48);
+  for (int p = 0; p < rp::kUnitRows; ++p) g.put(p, rp::kUnitRows - 1 - p, INT32_MAX - p, 1 + p % 48);
   for (int p = 0; p < rp::kUnitRows; ++p) {
     int r;
     int32_t first, pairs;
-    u.get<false>(p, r, first, pairs);
+    g.get(p, r, first, pairs);
     if (r != rp::kUnitRows - 1 - p || first != INT32_MAX - p || pairs != 1 + p % 48) return 1;
   }
   return 0;
